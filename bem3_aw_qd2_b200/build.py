@@ -21,7 +21,7 @@ LIB = os.path.join(HERE, "lib")
 INCLUDE = os.path.join(ROOT, "include")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CUDA_SOURCES = ["bem_assemble.cu", "bem_solve.cu", "bem_lu.cu", "bem_capi.cu", "bem_static.cu", "bem_mixed.cu",
-                "bem_server.cu", "bem_transform.cu", "bem_gmres.cu", "bem_tc.cu"]
+                "bem_server.cu", "bem_transform.cu", "bem_gmres.cu", "bem_tc.cu", "bem_smooth.cu"]
 HOST_SOURCES = ["host/aqd2_io.c", "host/aqd2_init.c", "host/aqd2_gpu.c"]
 REFERENCE = os.environ.get("BEM_REFERENCE_DIR", "/root/reference")
 
@@ -55,7 +55,7 @@ def build(force=False, verbose=False):
     gpu_so = os.path.join(LIB, "libbemgpu.so")
     if force or _stale(gpu_so, _deps((".cu", ".cuh", ".h"))):
         cmd = [nvcc, *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
-               "-diag-suppress", "550,177", "-o", gpu_so] + [os.path.join(CSRC, s) for s in CUDA_SOURCES] + \
+               "-diag-suppress", "550,177", "-t", "0", "-o", gpu_so] + [os.path.join(CSRC, s) for s in CUDA_SOURCES] + \
               []
         if verbose:
             print(" ".join(cmd))

@@ -10,9 +10,12 @@
 // Work is split by pair class, each class in its own kernel:
 //   classify  geometric F, dF/dt on 12x12 points for every (p, s); flags the
 //             near-singular pairs (|dF/dt| > 0.5, d3qd2_elem.c:851,537)
-//   regular   12x12 points: periodic domain one thread per point (each point is
-//             a full quasi-periodic Green's function, ~100 lattice terms);
-//             free-space domain one thread per pair (cheap integrand)
+//   regular   periodic domain: lattice images in closed form + an expansion of
+//             the rest (bem_smooth.cu); where that does not apply (no pair lists,
+//             a body much taller than the period) and for pairs with a point on
+//             the lattice plane, one thread per point, each a full
+//             quasi-periodic Green's function of ~100 lattice terms.
+//             free-space domain: one thread per pair (cheap integrand)
 //   near      64x64 points for flagged pairs, one block per pair
 //   self      singular polar quadrature on the collocation element, one block
 //             per collocation node
@@ -22,7 +25,9 @@
 #include <stdint.h>
 #include "bem_qpgf.cuh"
 #include "bem_geom.cuh"
+#include "bem_tiers.cuh"
 #include "bem_kernels.h"
+#include "bem_smooth.h"
 
 
 // ------------------------------------------------------------------ helpers
@@ -115,39 +120,13 @@ __device__ __forceinline__ void geomF(const double vR[3], const double vW[3], co
 // |W| has complex zeros near the element, which the shorter rules feel first;
 // at a quarter the 6-point tier is off by 1e-11); other quads keep tier 2 or
 // the reference rule.
-struct bem_far { int on; double d1x, d1y, d2x, d2y, idet, k; };
-__device__ __forceinline__ bool quad_tier_shape(const bem_el &el) {
-  double c1[3], c2[3], c3[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) { c1[d] = el.cr[d][1]; c2[d] = el.cr[d][2]; c3[d] = el.cr[d][3]; }
-  const double n0 = c1[1] * c2[2] - c1[2] * c2[1], n1 = c1[2] * c2[0] - c1[0] * c2[2], n2 = c1[0] * c2[1] - c1[1] * c2[0];
-  const double nn = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-  const double l1 = sqrt(dot3(c1, c1)), l2 = sqrt(dot3(c2, c2));
-  const double lmin = fmin(l1, l2), lmax = fmax(l1, l2);
-  return nn > 0.0 && fabs(c3[0] * n0 + c3[1] * n1 + c3[2] * n2) <= 0.1 * lmin * nn && lmax <= 3.0 * lmin;
-}
+struct bem_far { int on, split; double d1x, d1y, d2x, d2y, idet, k; };
 // (distance from the element's centre (a triangle's centroid) to the nearest
 // lattice image of rt) / (the element's circumradius R about that centre),
 // squared, and (k R)^2.
 __device__ __forceinline__ double pair_ratio2(const bem_far &fr, const bem_el &el, const double rt[3], bool tri,
                                               double &kR2) {
-  // corners (+-1, +-1) of a quad, (1, 0), (-1/2, +-sqrt3/2) of a triangle
-  double R2 = 0.0;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    double sz = (c == 1 || c == 2) ? 1.0 : -1.0, se = c >= 2 ? 1.0 : -1.0;
-    if (tri) {
-      sz = c == 0 ? 1.0 : -0.5;
-      se = c == 0 ? 0.0 : (c == 1 ? 0.5 * BEM_SQ3 : -0.5 * BEM_SQ3);
-    }
-    double v2 = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double v = el.cr[d][1] * sz + el.cr[d][2] * se + el.cr[d][3] * sz * se;
-      v2 += v * v;
-    }
-    R2 = fmax(R2, v2);
-  }
+  const double R2 = el_circum2(el, tri);
   kR2 = fr.k * fr.k * R2;
   const double vz = rt[2] - el.cr[2][0];
   const double vx = rt[0] - el.cr[0][0], vy = rt[1] - el.cr[1][0];
@@ -166,33 +145,13 @@ __device__ __forceinline__ double pair_ratio2(const bem_far &fr, const bem_el &e
 // stop on rounding-decided zeros, so its values at its own points are not a
 // smooth function that another rule could reproduce.
 #define BEM_FAR_PLANE_TOL 1e-10
-// point (i, j) of tier t's rule: Gauss on a quad; on a triangle the collapsed
-// (Duffy) rule over the whole reference triangle, (z, e) = (1 - 3u/2,
-// sqrt3/2 u (1 - 2v)) for (u, v) in [0, 1]^2, weight u w_u w_v
-__device__ __forceinline__ void tier_point(int t, bool tri, int i, int j, double &z, double &e) {
-  if (tri) {
-    const double u = 0.5 * (c_q.xt[t][i] + 1.0), v = 0.5 * (c_q.xt[t][j] + 1.0);
-    z = 1.0 - 1.5 * u;
-    e = 0.5 * BEM_SQ3 * u * (1.0 - 2.0 * v);
-  } else {
-    z = c_q.xt[t][i];
-    e = c_q.xt[t][j];
-  }
-}
 // tier of a regular pair, or -1 for the reference's rule (whose points the
 // caller has checked against the lattice plane); none of the tier's points
-// may lie within BEM_FAR_PLANE_TOL of rt's lattice plane either
+// may lie within BEM_FAR_PLANE_TOL of rt's lattice plane either (-2: one does)
 __device__ __forceinline__ int far_tier(const bem_far &fr, const bem_el &el, const double rt[3], bool tri) {
   double kR2;
   const double r2 = pair_ratio2(fr, el, rt, tri, kR2);
-  if (kR2 > 1.0) return -1;
-  int t;
-  if (tri)  // flat triangles converge faster: 7 points from 6 R, 6 from 12 R (k R <= 0.5)
-    t = r2 >= 144.0 && kR2 <= 0.25 ? 4 : r2 >= 36.0 && kR2 <= 0.25 ? 3 : r2 >= 25.0 ? 2 : r2 >= 12.25 ? 1 : r2 >= 9.0 ? 0 : -1;
-  else if (!quad_tier_shape(el))
-    t = r2 >= 25.0 ? 2 : -1;
-  else
-    t = r2 >= 625.0 && kR2 <= 0.04 ? 4 : r2 >= 64.0 && kR2 <= 0.25 ? 3 : r2 >= 25.0 ? 2 : r2 >= 12.25 ? 1 : r2 >= 9.0 ? 0 : -1;
+  const int t = tier_of(r2, kR2, tri, tri || quad_tier_shape(el));
   if (t < 0) return -1;
   // |z(zeta, eta) - c0z| <= |c1z| + |c2z| + |c3z| over the element
   const double zr = fabs(el.cr[2][1]) + fabs(el.cr[2][2]) + fabs(el.cr[2][3]);
@@ -202,7 +161,7 @@ __device__ __forceinline__ int far_tier(const bem_far &fr, const bem_el &el, con
     double z, e, r[3], w[3];
     tier_point(t, tri, ij / n, ij % n, z, e);
     bem_rw(el, z, e, r, w);
-    if (fabs(r[2] - rt[2]) < BEM_FAR_PLANE_TOL) return -1;
+    if (fabs(r[2] - rt[2]) < BEM_FAR_PLANE_TOL) return -2;
   }
   return t;
 }
@@ -230,12 +189,13 @@ __device__ __forceinline__ unsigned long long plist_base(const bem_plist &L) {
 __device__ __forceinline__ long long plist_pair(const bem_plist &L, unsigned long long base, long long pair0, long long u) {
   return L.e ? (long long)L.e[base + u] : pair0 + u;
 }
-__device__ __forceinline__ int plist_of_flag(uint8_t fl) { return fl == 0 ? 0 : fl >= 3 ? fl - 2 : -1; }
+__device__ __forceinline__ int plist_of_flag(uint8_t fl) { return fl == 0 || fl == BEM_FL_REF ? 0 : fl >= 3 ? fl - 2 : -1; }
 
 __global__ void __launch_bounds__(128) k_classify(bem_dom_dev D, bem_far fr, double *__restrict__ rowF,
                                                    int *__restrict__ near_s, int *__restrict__ near_n,
                                                    uint8_t *__restrict__ flag, unsigned *status,
-                                                   unsigned *__restrict__ lcnt) {
+                                                   unsigned *__restrict__ lcnt, unsigned *__restrict__ lst,
+                                                   unsigned long long lcap) {
   const int p = blockIdx.x;
   if (bem_pad_row(D, p)) {
     for (int s = threadIdx.x; s < D.ne; s += blockDim.x) flag[(size_t)p * D.ne + s] = 0;
@@ -295,9 +255,16 @@ __global__ void __launch_bounds__(128) k_classify(bem_dom_dev D, bem_far fr, dou
         if (k < D.near_cap) list[k] = s;
       } else {
         sF += F; sFz += Fz; sFe += Fe;
-        if (fr.on && rzmin >= BEM_FAR_PLANE_TOL) {
-          const int tier = far_tier(fr, el, nd.rt, tri);
+        if ((fr.on || fr.split) && rzmin >= BEM_FAR_PLANE_TOL) {
+          const int tier = fr.on ? far_tier(fr, el, nd.rt, tri) : -1;
           if (tier >= 0) fl = (uint8_t)(3 + tier);
+          else if (fr.split && tier == -1) fl = BEM_FL_REF;
+        }
+        if (fr.split && fl == 0) {
+          // a point on the lattice plane: listed for the lattice-sum kernels
+          // (any order: each pair writes its own entries)
+          const unsigned u = atomicAdd(lcnt + BEM_PC_PLANE, 1u);
+          if (u < lcap) lst[u] = (unsigned)((size_t)p * D.ne + s);
         }
       }
     }
@@ -826,7 +793,8 @@ template <class BA>
 __global__ void NP_BOUNDS k_q0_near(bem_dom_dev D, const __grid_constant__ bem_qp q0, const int *__restrict__ near_s,
                                                         const int *__restrict__ near_n, double *G0,
                                                         double *H0, double *__restrict__ nearF, unsigned *status,
-                                                        unsigned long long *terms, const __grid_constant__ BA B) {
+                                                        unsigned long long *terms, const __grid_constant__ BA B, int split) {
+  // split: everything but the home image is in G and H already (bem_smooth.cu), which G0 is added to;
   // blocks (p, y) take the node's near pairs y, y + gridDim.y, ...; a batch:
   // block (p, y, b) those of instance b, and instance 0 alone writes the geometric sums
   const int p = blockIdx.x, nn = near_n[p];
@@ -879,8 +847,9 @@ __global__ void NP_BOUNDS k_q0_near(bem_dom_dev D, const __grid_constant__ bem_q
       reg_point(el, nd, tri, pt, z, e, wt, vR, vW);
       on_plane |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
     }
-    if (!__syncthreads_or(on_plane)) {
-      for (int pt = threadIdx.x; pt < nreg; pt += NP_THREADS) {
+    const bool plane = __syncthreads_or(on_plane), add = split && !plane;
+    if (!plane) {
+      for (int pt = threadIdx.x; pt < nreg && !split; pt += NP_THREADS) {
         double z, e, wt, vR[3], vW[3], N[4];
         reg_point(el, nd, tri, pt, z, e, wt, vR, vW);
         bem_gval gv, g0;
@@ -919,7 +888,8 @@ __global__ void NP_BOUNDS k_q0_near(bem_dom_dev D, const __grid_constant__ bem_q
       const int c = threadIdx.x;
       double *dst = c < 8 ? G : H;
       const int a = (c & 7) >> 1, part = c & 1;
-      dst[2 * ((size_t)p * N + 4 * s + a) + part] = v[c];
+      double &o = dst[2 * ((size_t)p * N + 4 * s + a) + part];
+      o = add ? o + v[c] : v[c];
     } else if (threadIdx.x < 19 && nearF) {
       nearF[((size_t)p * D.near_cap + k) * 3 + (threadIdx.x - 16)] = v[threadIdx.x] * BEM_I_FP;
     }
@@ -1000,7 +970,7 @@ template <class BA>
 __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_qp q0, double *G0,
                                                         double *H0, double *__restrict__ selfF,
                                                         unsigned *status, unsigned long long *terms,
-                                                        const __grid_constant__ BA B) {
+                                                        const __grid_constant__ BA B, int split) {
   const int p = blockIdx.x;
   const int t = p >> 2, tn = p & 3;
   const int te = abs(D.sid[t]) - 1;
@@ -1047,8 +1017,9 @@ __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_q
     reg_point(el, nd, false, pt, z, e, wt, vR, vW);
     on_plane |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
   }
-  if (!__syncthreads_or(on_plane)) {
-    for (int pt = threadIdx.x; pt < BEM_GLN * BEM_GLN; pt += NP_THREADS) {
+  const bool meets = __syncthreads_or(on_plane), add = split && !meets;
+  if (!meets) {
+    for (int pt = threadIdx.x; pt < BEM_GLN * BEM_GLN && !split; pt += NP_THREADS) {
       double z, e, wt, vR[3], vW[3], N[4];
       reg_point(el, nd, false, pt, z, e, wt, vR, vW);
       bem_gval gv, g0;
@@ -1104,7 +1075,8 @@ __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_q
     const int c = threadIdx.x;
     double *dst = c < 8 ? G : H;
     const int a = (c & 7) >> 1, part = c & 1;
-    dst[2 * ((size_t)p * N + 4 * t + a) + part] = all[c];
+    double &o = dst[2 * ((size_t)p * N + 4 * t + a) + part];
+    o = add ? o + all[c] : all[c];
   } else if (threadIdx.x == 16) {
     const double bdC = bem_bdC(el);
     const double F0 = plane ? 0.0 : all[16] * BEM_I_FP * bdC;
@@ -1544,7 +1516,9 @@ __global__ void __launch_bounds__(NP_THREADS, FS_SELF_MINB) k_fs_self(bem_dom_de
 // Jacobian vector J = cw0 2 / (3 sqrt3) the integrands are the quad kernel's.
 __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ bem_qp q, double *__restrict__ G,
                                         double *__restrict__ H, double *__restrict__ selfF, unsigned *status,
-                                        unsigned long long *terms) {
+                                        unsigned long long *terms, int split) {
+  // split: everything but the home image is in G and H already (bem_smooth.cu): G0 on the polar
+  // rule is added to them, unless a point of this rule or of the regular one lies on the lattice plane
   const int p = blockIdx.x;
   const int t = p >> 2, tn = p & 3;
   const int te = abs(D.sid[t]) - 1;
@@ -1565,6 +1539,24 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
   for (int c = 0; c < 16; ++c) v[c] = 0.0;
   unsigned st = 0;
   unsigned long long nterm = 0, npt = 0;
+  bool meets = !split;
+  if (split) {
+    bem_node nd;
+    double w0[3];
+    bem_rw(el, zt, et, nd.rt, w0);
+    for (int pt = threadIdx.x; pt < 3 * BEM_GLN * BEM_GLN; pt += NP_THREADS) {
+      double z, e, wt, vR[3], vW[3];
+      reg_point(el, nd, true, pt, z, e, wt, vR, vW);
+      meets |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
+    }
+  }
+  for (int full = split ? 0 : 1; full < 2; ++full) {
+  if (full && split) {
+    if (!__syncthreads_or(meets)) break;
+    meets = true;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = 0.0;
+  }
   for (int pt = threadIdx.x; pt < 384 * BEM_GLN; pt += NP_THREADS) {
     const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
     const polar_pt tp = polar_theta(th, idx);
@@ -1578,10 +1570,16 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
     double K[3];
     bem_K(el, rr, cth, sth, zt, et, K);
     bem_gval gv;
-    const int rc = bem_qpgf(q, rr * K[0], rr * K[1], rr * K[2], gv, wts);
-    if (rc < 0) st |= (rc == -12 || rc == -23) ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT;
-    nterm += rc > 0 ? (unsigned long long)rc : 0ULL;
-    ++npt;
+    if (full) {
+      const int rc = bem_qpgf(q, rr * K[0], rr * K[1], rr * K[2], gv, wts);
+      if (rc < 0) st |= (rc == -12 || rc == -23) ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT;
+      nterm += rc > 0 ? (unsigned long long)rc : 0ULL;
+      ++npt;
+    } else {
+      const double vR[3] = {rr * K[0], rr * K[1], rr * K[2]};
+      meets |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
+      bem_g0(q.k, vR, gv);
+    }
     const cplx g = cscale(gv.g, aJ * rr * w);
     const cplx h = cscale(cadd(cadd(cscale(gv.gx, J[0]), cscale(gv.gy, J[1])), cscale(gv.gz, J[2])), rr * w);
     double N[4];
@@ -1594,6 +1592,8 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
       v[8 + 2 * a + 1] += h.im * N[a];
     }
   }
+  }
+  const bool add = split && !__syncthreads_or(nterm != 0);
   count_work(terms + 2, nterm, npt);
   set_status(status, st);
   __shared__ double sm[16 * (NP_THREADS / 32) + 16];
@@ -1603,7 +1603,8 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
     const int c = threadIdx.x;
     double *dst = c < 8 ? G : H;
     const int a = (c & 7) >> 1, part = c & 1;
-    dst[2 * ((size_t)p * N + 4 * t + a) + part] = v[c];
+    double &o = dst[2 * ((size_t)p * N + 4 * t + a) + part];
+    o = add ? o + v[c] : v[c];
   } else if (threadIdx.x < 19) {
     selfF[3 * p + (threadIdx.x - 16)] = 0.0;
   }
@@ -1953,7 +1954,7 @@ extern "C" int bem_set_constants(const double *xl, const double *wl, const doubl
   for (int n = 1; n <= BEM_W_TAB; ++n) wc.tab[n - 1] = exp(-wc.a2 * n * n);
   if (cudaMemcpyToSymbol(c_q, &qq, sizeof(qq)) != cudaSuccess) return -1;
   if (cudaMemcpyToSymbol(c_w, &wc, sizeof(wc)) != cudaSuccess) return -1;
-  return 0;
+  return bem_smooth_set_constants(&qq, &wc);
 }
 
 extern "C" int bem_launch_faddeeva(const double *z, int n, double *w, cudaStream_t st) {
@@ -1973,6 +1974,7 @@ extern "C" int bem_launch_qpgf(const bem_qp *q, const double *r, int n, double *
 static bem_far far_params(const bem_dom_dev *D, const bem_qp *q, int periodic) {
   bem_far fr;
   fr.on = periodic && D->far_rule;
+  fr.split = 0;
   fr.d1x = q->d1x; fr.d1y = q->d1y; fr.d2x = q->d2x; fr.d2y = q->d2y;
   fr.idet = q->idet;
   fr.k = q->k;
@@ -2050,27 +2052,41 @@ extern "C" int bem_launch_assemble(const bem_dom_dev *D, const bem_qp *q, int pe
       return -1;
   }
   const long long npairs = (long long)N * D->ne;
-  // compacted pair lists for the periodic domain when the scratch holds them
+  // pair lists for the periodic domain when the scratch holds them
   const bool lists = periodic && S->plist && S->pcount && (unsigned long long)npairs <= S->pcap &&
                      npairs <= 0xffffffffLL;
-  if (lists && cudaMemsetAsync(S->pcount, 0, 2 * BEM_NLIST * sizeof(unsigned), st) != cudaSuccess) return -1;
+  const int split = lists && S->sm && S->sm->on;
+  if (lists && cudaMemsetAsync(S->pcount, 0, 16 * sizeof(unsigned), st) != cudaSuccess) return -1;
   if (ev) cudaEventRecord(ev[0], st);
-  k_classify<<<N, 128, 0, st>>>(*D, far_params(D, q, periodic), S->rowF, S->near_s, S->near_n, S->flag, S->status,
-                                lists ? S->pcount : nullptr);
+  bem_far fr = far_params(D, q, periodic);
+  fr.split = split;
+  k_classify<<<N, 128, 0, st>>>(*D, fr, S->rowF, S->near_s, S->near_n, S->flag, S->status,
+                                lists ? S->pcount : nullptr, S->plist, S->pcap);
   bem_count_launches(1);
-  if (lists) {
+  if (lists && !split) {
     k_plist_fill<<<N, 128, 0, st>>>(*D, S->flag, S->plist, S->pcount, S->pcap);
     bem_count_launches(1);
   }
   if (ev) cudaEventRecord(ev[1], st);
   if (periodic) {
-    if (lists) {
-      // one resident wave (RP_MINB / FP_MINB blocks per SM) striding over each list
-      int dev = 0, nsm = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess ||
-          cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0)
-        return -1;
-      const unsigned grid = RP_MINB * (unsigned)nsm, grid_far = FP_MINB * (unsigned)nsm;
+    // one resident wave (RP_MINB / FP_MINB blocks per SM) striding over each list
+    int dev = 0, nsm = 0;
+    if (lists && (cudaGetDevice(&dev) != cudaSuccess ||
+                  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0))
+      return -1;
+    const unsigned grid = RP_MINB * (unsigned)nsm, grid_far = FP_MINB * (unsigned)nsm;
+    if (split) {
+      if (bem_launch_smooth(S->sm, D, q, 1, &G, &H, S, st)) return -1;
+      // pairs with a point on the lattice plane
+      const bem_plist Lpl = {S->plist, S->pcount + BEM_PC_PLANE, 0};
+      k_q0_regular<bat_none><<<grid, RP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, S->flag, G, H, S->status, S->terms, 0, npairs,
+                                                                    Lpl, k_nobat);
+      bem_count_launches(1);
+      if (D->has_tri) {
+        k_q0_regular_tri<<<grid, RP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, S->flag, G, H, S->status, S->terms, 0, npairs, Lpl);
+        bem_count_launches(1);
+      }
+    } else if (lists) {
       const bem_plist Lreg = {S->plist, S->pcount, 0};
       k_q0_regular<bat_none><<<grid, RP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, S->flag, G, H, S->status, S->terms, 0, npairs, Lreg,
                                                                          k_nobat);
@@ -2098,13 +2114,13 @@ extern "C" int bem_launch_assemble(const bem_dom_dev *D, const bem_qp *q, int pe
     }
     if (ev) cudaEventRecord(ev[2], st);
     k_q0_near<bat_none><<<dim3(N, near_grid_y(D)), NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, S->near_s, S->near_n, G, H, S->nearF,
-                                                                              S->status, S->terms, k_nobat);
+                                                                              S->status, S->terms, k_nobat, split);
     bem_count_launches(1);
     if (ev) cudaEventRecord(ev[3], st);
-    k_q0_self<bat_none><<<N, NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, G, H, S->selfF, S->status, S->terms, k_nobat);
+    k_q0_self<bat_none><<<N, NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, G, H, S->selfF, S->status, S->terms, k_nobat, split);
     bem_count_launches(1);
     if (D->has_tri) {
-      k_q0_self_tri<<<N, NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, G, H, S->selfF, S->status, S->terms);
+      k_q0_self_tri<<<N, NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, G, H, S->selfF, S->status, S->terms, split);
       bem_count_launches(1);
     }
   } else {
@@ -2146,17 +2162,23 @@ extern "C" int bem_launch_assemble_batch(const bem_dom_dev *D, const bem_qp *q, 
   if (D->has_tri) return -2;
   const long long npairs = (long long)N * D->ne;
   if (!(S->plist && S->pcount && (unsigned long long)npairs <= S->pcap && npairs <= 0xffffffffLL)) return -2;
-  if (cudaMemsetAsync(S->pcount, 0, 2 * BEM_NLIST * sizeof(unsigned), st) != cudaSuccess) return -1;
-  k_classify<<<N, 128, 0, st>>>(*D, far_params(D, q, 1), S->rowF, S->near_s, S->near_n, S->flag, S->status,
-                                S->pcount);
+  const int split = S->sm && S->sm->on;
+  if (cudaMemsetAsync(S->pcount, 0, 16 * sizeof(unsigned), st) != cudaSuccess) return -1;
+  bem_far fr = far_params(D, q, 1);
+  fr.split = split;
+  k_classify<<<N, 128, 0, st>>>(*D, fr, S->rowF, S->near_s, S->near_n, S->flag, S->status, S->pcount, S->plist, S->pcap);
   bem_count_launches(1);
-  k_plist_fill<<<N, 128, 0, st>>>(*D, S->flag, S->plist, S->pcount, S->pcap);
-  bem_count_launches(1);
+  if (split) {
+    if (bem_launch_smooth(S->sm, D, qps, nb, Gh, Hh, S, st)) return -1;
+  } else {
+    k_plist_fill<<<N, 128, 0, st>>>(*D, S->flag, S->plist, S->pcount, S->pcap);
+    bem_count_launches(1);
+  }
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0)
     return -1;
-  const bem_plist Lreg = {S->plist, S->pcount, 0};
+  const bem_plist Lreg = {S->plist, split ? S->pcount + BEM_PC_PLANE : S->pcount, 0};
   bem_bat B;  // 20 KB on the host stack, copied into each launch's argument block
   for (int b0 = 0; b0 < nb; b0 += BEM_BAT_MAX) {
     B.nb = nb - b0 < BEM_BAT_MAX ? nb - b0 : BEM_BAT_MAX;
@@ -2168,12 +2190,12 @@ extern "C" int bem_launch_assemble_batch(const bem_dom_dev *D, const bem_qp *q, 
     k_q0_regular<bem_bat><<<RP_MINB * (unsigned)nsm, RP_THREADS, BEM_WT_SMEM, st>>>(
         *D, *q, S->flag, nullptr, nullptr, S->status, S->terms, 0, npairs, Lreg, B);
     bem_count_launches(1);
-    if (D->far_rule) launch_far_tiers(D, q, S, nullptr, nullptr, 0, npairs, Lreg, FP_MINB * (unsigned)nsm, st, B);
+    if (D->far_rule && !split) launch_far_tiers(D, q, S, nullptr, nullptr, 0, npairs, Lreg, FP_MINB * (unsigned)nsm, st, B);
     k_q0_near<bem_bat><<<dim3(N, near_grid_y(D), B.nb), NP_THREADS, BEM_WT_SMEM, st>>>(
-        *D, *q, S->near_s, S->near_n, nullptr, nullptr, S->nearF, S->status, S->terms, B);
+        *D, *q, S->near_s, S->near_n, nullptr, nullptr, S->nearF, S->status, S->terms, B, split);
     bem_count_launches(1);
     k_q0_self<bem_bat><<<dim3(N, 1, B.nb), NP_THREADS, BEM_WT_SMEM, st>>>(*D, *q, nullptr, nullptr, S->selfF,
-                                                                       S->status, S->terms, B);
+                                                                       S->status, S->terms, B, split);
     bem_count_launches(1);
   }
   for (int b = 0; b < nb; ++b) {
@@ -2246,7 +2268,7 @@ extern "C" int bem_launch_fs_deriv(const bem_dom_dev *D, double k, bem_scratch *
 extern "C" int bem_launch_classify(const bem_dom_dev *D, const bem_qp *q, int periodic, bem_scratch *S, cudaStream_t st) {
   if (D->ne <= 0) return 0;
   k_classify<<<D->ne * 4, 128, 0, st>>>(*D, far_params(D, q, periodic), S->rowF, S->near_s, S->near_n, S->flag, S->status,
-                                        nullptr);
+                                        nullptr, nullptr, 0);
   bem_count_launches(1);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

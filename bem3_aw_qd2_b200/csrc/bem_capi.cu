@@ -14,6 +14,7 @@
 #include "bem_lattice.h"
 #include "bem_mixed.h"
 #include "bem_lu.h"
+#include "bem_smooth.h"
 #include "bem_count.h"
 #include <atomic>
 
@@ -49,6 +50,10 @@ struct bemgpu_ctx {
   double *fout = nullptr, *rc_d = nullptr;
   double *wtab = nullptr;  // real-space term table of the Ewald sums (A, B at eta_run)
   double *stab = nullptr;  // evanescent spectral order table (at eta_run)
+  // images + expansion of the periodic domain (bem_smooth.cu): its tables, and
+  // its workspace where the global matrix is too small to lend its own
+  bem_smooth sm;
+  double *sm_tab = nullptr, *sm_buf = nullptr;
   double zspan = 0.0;      // height of the mesh (z extent of all elements)
   double pw[16] = {};      // incident plane wave (bemgpu_problem.pw)
   int far_rule = 1;        // shorter rules for regular pairs of the periodic domain (bemgpu_set_far_rule)
@@ -203,7 +208,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
       dfree(S->rowF); dfree(S->near_s); dfree(S->near_n); dfree(S->nearF); dfree(S->selfF); dfree(S->flag);
     }
     dfree(c->scr.plist); dfree(c->scr.pcount);
-    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->b0); dfree(c->B3s);
+    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_buf); dfree(c->b0); dfree(c->B3s);
     for (int d = 0; d < BEMGPU_MAXDOM; ++d) { dfree(c->Wd[d]); dfree(c->cinv[d]); dfree(c->Gc[d]); }
     dfree(c->B3c);
     dfree(c->dGc); dfree(c->dHc);
@@ -219,6 +224,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
   c->nctr = 0;
   c->ntgt = 0;
   c->loaded = false;
+  c->sm.on = 0;
 }
 
 extern "C" int bemgpu_create(int device, void *stream, bemgpu_ctx **out) {
@@ -385,6 +391,30 @@ static int build_stab(bemgpu_ctx *c) {
   return 0;
 }
 
+// Tables and workspace of the split c->sm for the instances qps[0 .. inst).
+// One instance's workspace lies in the global matrix, which holds nothing
+// between the start of an assembly and the gather after it, where that is
+// large enough (all but small problems).
+static int smooth_setup(bemgpu_ctx *c, int inst, const bem_qp *qps) {
+  c->sm.inst = inst;
+  c->sm.first = 0;
+  c->scr.sm = &c->sm;
+  if (!c->sm.on) return 0;
+  std::vector<double> h(bem_smooth_layout(&c->sm).total);
+  bem_smooth_tables(&c->sm, qps, h.data());
+  CK(falloc(c, &c->sm_tab, h.size()), "expansion tables");
+  CK(cudaMemcpyAsync(c->sm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
+  c->sm.tab = c->sm_tab;
+  const size_t need = bem_smooth_ws_doubles(&c->sm, c->dom_ne[0]);
+  if (inst == 1 && need <= 2 * (size_t)c->n * c->n) {
+    c->sm.ws = c->A;
+  } else {
+    CK(falloc(c, &c->sm_buf, need), "expansion workspace");
+    c->sm.ws = c->sm_buf;
+  }
+  return 0;
+}
+
 extern "C" int bemgpu_load(bemgpu_ctx *c, const bemgpu_problem *pr) {
   CK(cudaSetDevice(c->device), "set device");
   // the previous problem's work ends before its buffers are reused
@@ -541,6 +571,8 @@ extern "C" int bemgpu_load(bemgpu_ctx *c, const bemgpu_problem *pr) {
   CK(falloc(c, &c->A, 2 * n * n), "A");
   CK(falloc(c, &c->b, 2 * n), "b");
   CK(falloc(c, &c->tpv, 6 * (size_t)c->NN), "tpv");
+  bem_smooth_plan(&c->sm, &c->qp, pr->cr, pr->npe, pr->sid, c->dom_ne[0]);
+  if (smooth_setup(c, 1, &c->qp)) return -1;
   for (int d = 0; d < nd; ++d) {
     const size_t N = 4 * (size_t)c->dom_ne[d];
     CK(falloc(c, &c->Wd[d], 2 * N * N), "dpv factors");
@@ -809,6 +841,13 @@ extern "C" int bemgpu_batch_load(bemgpu_ctx *c, int nb, const bemgpu_problem *co
     I.qp.st = I.stab;
   }
   c->bat_cur = 0;
+  std::vector<bem_qp> qps(nb);
+  for (int b = 0; b < nb; ++b) qps[b] = c->bat[b].qp;
+  if (smooth_setup(c, nb, qps.data())) {
+    batch_clear(c);
+    c->sm.on = 0;
+    return -1;
+  }
   return 0;
 }
 
@@ -854,6 +893,7 @@ extern "C" int bemgpu_batch_select(bemgpu_ctx *c, int b) {
   c->H[0] = I.H;
   c->qp = I.qp;
   c->bat_cur = b;
+  c->sm.first = b;
   c->factored = false;
   // the interior domains' matrices are the batch's: their dpv factors, once
   // made by a solve, serve every instance
@@ -1560,6 +1600,13 @@ extern "C" int bemgpu_transform_mesh(bemgpu_ctx *c, const double *rv, double th,
   }
   c->zspan = zhi - zlo;
   if (build_stab(c)) return -1;
+  // and its ball the split into images and expansion
+  std::vector<int> sid(c->dom_ne[0]), npe(c->Ne);
+  CK(cudaMemcpyAsync(sid.data(), c->sid, sid.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "mesh transform");
+  CK(cudaMemcpyAsync(npe.data(), c->npe, npe.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "mesh transform");
+  CK(cudaStreamSynchronize(c->stream), "mesh transform");
+  bem_smooth_plan(&c->sm, &c->qp, cr.data(), npe.data(), sid.data(), c->dom_ne[0]);
+  if (smooth_setup(c, 1, &c->qp)) return -1;
   // every matrix and factor belongs to the old placement
   c->factored = false;
   c->int_valid = false;

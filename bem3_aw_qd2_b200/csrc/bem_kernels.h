@@ -25,13 +25,19 @@ struct bem_scratch {
   int *near_n;      // [N]
   double *nearF;    // [N][near_cap][3]
   double *selfF;    // [N][3]
-  uint8_t *flag;    // [N][ne] 0 regular, 1 near-singular, 2 self, 3 + t regular on shorter-rule tier t
+  uint8_t *flag;    // [N][ne] 0 regular, 1 near-singular, 2 self, 3 + t regular on shorter-rule tier t;
+                    // with the smooth split also BEM_FL_REF, and 0 means a point on the lattice plane
   unsigned *plist;  // [pcap] periodic-domain pair lists p * ne + s: regular, then tier 0, 1, ... (optional)
-  unsigned *pcount; // [16] list lengths, then the fill counters
+  unsigned *pcount; // [16] list lengths, then the fill counters; [BEM_PC_PLANE] pairs on the lattice plane
   unsigned long long pcap;
   unsigned *status; // BEM_ST_* bits
   unsigned long long *terms;  // [6] lattice terms of regular / near / self pairs, then point counts
+  // periodic domain: images + expansion in place of the regular pairs' lattice
+  // sums (bem_smooth.h), when set and on
+  const struct bem_smooth *sm = nullptr;
 };
+#define BEM_FL_REF 8     // regular pair on the 12 x 12 rule, no point on the lattice plane
+#define BEM_PC_PLANE 12
 
 extern "C" {
 // the periodic domain of nb problems that differ only in the Bloch wave

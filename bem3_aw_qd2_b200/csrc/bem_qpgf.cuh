@@ -69,7 +69,7 @@ __device__ __forceinline__ double bem_sinc(double x, double sinx) {
 #ifndef BEM_QPGF_ATTR
 #define BEM_QPGF_ATTR
 #endif
-__device__ BEM_FADDEEVA_ATTR cplx bem_faddeeva(double xr, double yi) {
+static __device__ BEM_FADDEEVA_ATTR cplx bem_faddeeva(double xr, double yi) {
   if (xr == 0.0) return cmk(erfcx(yi), xr);  // w(iy) = erfcx(y), keep the sign of 0
   const double x = fabs(xr), ya = fabs(yi);
   if (ya >= 7.0 || (x >= 6.0 && ya >= 0.1)) {
@@ -277,7 +277,7 @@ __device__ __forceinline__ bem_dd dd_mul(bem_dd x, bem_dd y) {
 __device__ __forceinline__ bem_dd dd_scale(bem_dd x, double s) {  // s a power of two
   return {x.hi * s, x.lo * s};
 }
-__device__ __noinline__ double bem_exp_cr(double a) {
+static __device__ __noinline__ double bem_exp_cr(double a) {
   if (!(a > -700.0 && a < 700.0)) return exp(a);
   const double ln2_hi = 0.69314718055994528623, ln2_lo = 2.3190468138462995584e-17;
   const double n = rint(a * 1.4426950408889634074);
@@ -319,7 +319,7 @@ __device__ __forceinline__ double bem_ewald_eta(const bem_qp &q, double rx, doub
 // The lattice-plane forms below run for a few points of a mesh only; they are
 // kept out of line so that the hot loops' code stays small.
 // Propagating order on the plane: 2 (ef Re w(bn ve) - 1) as the reference rounds it.
-__device__ __noinline__ double ew_plane_residue(const bem_qp &q, int n1, int n2, double bn2, double bn, double ve) {
+static __device__ __noinline__ double ew_plane_residue(const bem_qp &q, int n1, int n2, double bn2, double bn, double ve) {
   // On the lattice plane ef Re w(bn ve) - 1 is zero up to rounding; the
   // reference's rows stop on an identically zero z-derivative sum, so the
   // residue must be the reference's rounded value: the host's table at
@@ -336,7 +336,7 @@ __device__ __noinline__ double ew_plane_residue(const bem_qp &q, int n1, int n2,
 // rounding alone; the rows' stopping tests see that zero, so both are formed
 // exactly as the reference forms them (ebz = exp(bn z), f2 with 1/ebz;
 // d3_qpgf_d2.c:2003-2007).
-__device__ __noinline__ double2 ew_plane_evanescent(double bn, double ve, double rz, double azve) {
+static __device__ __noinline__ double2 ew_plane_evanescent(double bn, double ve, double rz, double azve) {
   const double ebz = bem_exp_cr(__dmul_rn(bn, rz)), bvr = __dmul_rn(bn, ve);
   return make_double2(__dmul_rn(ebz, erfc(__dadd_rn(bvr, azve))),
                       __dmul_rn(__ddiv_rn(1.0, ebz), erfc(__dadd_rn(bvr, -azve))));
@@ -451,7 +451,7 @@ __device__ __forceinline__ cplx cconj(cplx a) { return cmk(a.re, -a.im); }
 // The lattice rows are walked exactly as in the reference (centre, then up,
 // then down, each stopped by the reference's tests); the Bloch phases along a
 // row are advanced by a unit complex factor, so a row costs one sincos.
-__device__ BEM_QPGF_ATTR int bem_qpgf_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval &out,
+static __device__ BEM_QPGF_ATTR int bem_qpgf_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval &out,
                                             const double2 *wts = nullptr) {
   const double ve = bem_ewald_eta(q, rx, ry, rz);
   const double ke = q.k * ve, ke2 = ke * ke, ive = 1.0 / ve;
@@ -554,7 +554,7 @@ __device__ BEM_QPGF_ATTR int bem_qpgf_ewald(const bem_qp &q, double rx, double r
 }
 
 // Pure spectral sum in the home cell (d3hm_qpgf_d2v1_fd_sd, d3_qpgf_d2.c:745-885).
-__device__ BEM_QPGF_ATTR int bem_qpgf_spectral(const bem_qp &q, double rx, double ry, double rz, bem_gval &out) {
+static __device__ BEM_QPGF_ATTR int bem_qpgf_spectral(const bem_qp &q, double rx, double ry, double rz, bem_gval &out) {
   if (rz == 0.0) return -14;
   const double eps = BEM_MEPS, az = fabs(rz);
   int cc = 0;
@@ -619,7 +619,7 @@ __device__ BEM_QPGF_ATTR int bem_qpgf_spectral(const bem_qp &q, double rx, doubl
 
 // G_qp and grad G_qp at r (d3hm_qpgf_d2_v1, d3_qpgf_d2.c:124-176 and the cell
 // reduction of :409-438).  Returns #terms (> 0) or the reference's negative code.
-__device__ BEM_QPGF_ATTR int bem_qpgf(const bem_qp &q, double rx, double ry, double rz, bem_gval &out,
+static __device__ BEM_QPGF_ATTR int bem_qpgf(const bem_qp &q, double rx, double ry, double rz, bem_gval &out,
                                       const double2 *wts = nullptr) {
   bool spectral = false;
   if (!q.ewald_only) {
@@ -656,7 +656,7 @@ struct bem_gval2 { cplx g, d[3], d2[6]; };
 
 __device__ __forceinline__ cplx cmuli(cplx a) { return cmk(-a.im, a.re); }  // i a
 
-__device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
+static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
   const double ve = bem_ewald_eta(q, rx, ry, rz);
   const double ke = q.k * ve, ke2 = ke * ke, ive = 1.0 / ve;
   const bool tab = q.wt != nullptr && ve == q.eta_run;
@@ -818,7 +818,7 @@ __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz,
   return cc;
 }
 
-__device__ int bem_qpgf2_spectral(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
+static __device__ int bem_qpgf2_spectral(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
   if (rz == 0.0) return -14;
   const double eps = BEM_MEPS, az = fabs(rz);
   int cc = 0;
@@ -891,7 +891,7 @@ __device__ int bem_qpgf2_spectral(const bem_qp &q, double rx, double ry, double 
   return cc;
 }
 
-__device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &out) {
+static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &out) {
   bool spectral = false;
   if (!q.ewald_only) {
     const double az = fabs(rz);

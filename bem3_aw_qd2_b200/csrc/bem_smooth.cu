@@ -1,0 +1,1012 @@
+// Regular part of the periodic domain's coefficient matrices without lattice
+// sums per quadrature point.
+//
+// The quasi-periodic Green's function of R = y - x (source minus collocation
+// point) is split into the lattice images that can come near,
+//   G_qp(R) = sum_{l in I} e^{i k_par . R_l} e^{ik|R + R_l|} / (4 pi |R + R_l|) + G_s(R),
+// and a rest G_s that solves the Helmholtz equation in |R| < c, c the distance
+// of the nearest image left in it.  With the body inside a ball of radius R0
+// about its centre, c > 2 R0, the rest is an expansion in regular waves,
+//   G_s(y - x) = sum_{lm, l'm'} phi_lm(y) T_lm,l'm' phi_l'm'(x),
+// which separates source and target: the integrals over the elements become
+// one matrix V = [int N_a |W| phi | int N_a W . grad phi] (K x 8 ne), the
+// targets one matrix A = U T, and the rest of every pair of G and H one real
+// matrix product on the FP64 tensor cores.  The reference sums about 110
+// lattice terms at each of the 36 to 144 points of every pair
+// (q0_bil_dcoef_v2_cc.c:129-204 over d3_qpgf_d2.c:124-176); here a pair costs
+// 16 K multiply-adds of the product and a closed form per image and point.
+//
+// The images keep the quadrature rule of their own distance (bem_tiers.cuh), so
+// every part meets the accuracy of the pairwise rules; pairs with a point on
+// the lattice plane through their node stay with the kernels that sum the
+// lattice point by point (the reference's sums stop on rounding there).
+//
+// 216-quad sphere, square lattice of 0.8 wavelengths (5 images, K = 1296): 1.8 ms
+// in place of 17.3 ms of lattice sums at the points; the whole solve 28.5 ->
+// 11.9 ms, of the 1536-quad sphere 957 -> 374 ms, of 320 triangles 70 -> 29 ms.
+//
+// phi_lm(y) = g_l(k r) R_lm((y - centre) / R0), g_l(z) = (2l + 1)!! j_l(z) / z^l
+// (entire, near 1), R_lm real orthonormal solid harmonics: no zeros of j_l, no
+// large or small factors.  The coefficients of G_s come from its values and
+// radial derivatives on the sphere |R| = 2 R0 (Ewald sums at about 3000 points),
+// projected on spherical harmonics; T from them by the addition theorem, its
+// Gaunt integrals by Gauss-Legendre quadrature (exact for these degrees).
+#include "bem_count.h"
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <math.h>
+#include <algorithm>
+#include <vector>
+#include "bem_qpgf.cuh"
+#include "bem_geom.cuh"
+#include "bem_tiers.cuh"
+#include "bem_kernels.h"
+#include "bem_smooth.h"
+
+extern "C" int bem_smooth_set_constants(const void *quad, const void *wc) {
+  if (cudaMemcpyToSymbol(c_q, quad, sizeof(bem_quad)) != cudaSuccess) return -1;
+  if (cudaMemcpyToSymbol(c_w, wc, sizeof(bem_wconst)) != cudaSuccess) return -1;
+  return 0;
+}
+
+// ------------------------------------------------------------------ host: the split
+// |j_l(z)| = z^l g_l / (2l + 1)!! and |h_l(z)| for l = 0 .. n
+static void bessel_sizes(int n, double z, std::vector<double> &j, std::vector<double> *h) {
+  const int top = n + 20 + (int)z;
+  std::vector<double> g(top + 2);
+  for (int l = top; l <= top + 1; ++l) {
+    double t = 1.0, s = 1.0;
+    for (int m = 1; m < 200 && fabs(t) > 1e-20 * fabs(s); ++m) {
+      t *= -0.5 * z * z / (m * (2.0 * l + 2.0 * m + 1.0));
+      s += t;
+    }
+    g[l] = s;
+  }
+  for (int l = top; l > 0; --l) g[l - 1] = g[l] - z * z / ((2.0 * l + 1.0) * (2.0 * l + 3.0)) * g[l + 1];
+  j.assign(n + 1, 0.0);
+  double f = 1.0;
+  for (int l = 0; l <= n; ++l) {
+    j[l] = f * g[l];
+    f *= z / (2.0 * l + 3.0);
+  }
+  if (!h) return;
+  h->assign(n + 1, 0.0);
+  double y0 = -cos(z) / z, y1 = -cos(z) / (z * z) - sin(z) / z;
+  for (int l = 0; l <= n; ++l) {
+    (*h)[l] = sqrt(j[l] * j[l] + y0 * y0);
+    const double y2 = (2.0 * l + 3.0) / z * y1 - y0;
+    y0 = y1;
+    y1 = y2;
+  }
+}
+// smallest degree whose terms k (2l + 1) |j_l(k a) h_l(k b)| beyond it stay
+// below tol / scale; -1: none up to lim
+static int degree_for(double k, double a, double b, double scale, double tol, int lim) {
+  std::vector<double> j, h;
+  bessel_sizes(lim + 4, k * a, j, nullptr);
+  std::vector<double> jb;
+  bessel_sizes(lim + 4, k * b, jb, &h);
+  for (int l = lim; l >= 0; --l) {
+    const double e = k * (2.0 * (l + 1) + 1.0) * fabs(j[l + 1]) * h[l + 1] * scale;
+    if (!(e <= tol)) return l == lim ? -1 : l + 1;
+  }
+  return 0;
+}
+
+void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int *npe, const int *sid, int ne) {
+  S->on = 0;
+  if (ne <= 0) return;
+  // the ball of the body: corners (+-1, +-1) of a quad, (1, 0), (-1/2,
+  // +-sqrt3/2) of a triangle; every point of an element is a convex
+  // combination of its corners
+  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+  auto corners = [&](int s, double (*v)[3]) {
+    const int e = abs(sid[s]) - 1, n = npe[e] == 3 ? 3 : 4;
+    const double zq[4] = {-1, 1, 1, -1}, eq[4] = {-1, -1, 1, 1};
+    const double zt[3] = {1.0, -0.5, -0.5}, et[3] = {0.0, 0.86602540378443864676, -0.86602540378443864676};
+    for (int c = 0; c < n; ++c) {
+      const double z = n == 3 ? zt[c] : zq[c], w = n == 3 ? et[c] : eq[c];
+      for (int d = 0; d < 3; ++d) {
+        const double *r = cr + (size_t)e * 12 + 4 * d;
+        v[c][d] = r[0] + r[1] * z + r[2] * w + r[3] * z * w;
+      }
+    }
+    return n;
+  };
+  double v[4][3];
+  for (int s = 0; s < ne; ++s) {
+    const int n = corners(s, v);
+    for (int c = 0; c < n; ++c)
+      for (int d = 0; d < 3; ++d) { lo[d] = std::min(lo[d], v[c][d]); hi[d] = std::max(hi[d], v[c][d]); }
+  }
+  for (int d = 0; d < 3; ++d) S->ctr[d] = 0.5 * (lo[d] + hi[d]);
+  double R2 = 0.0;
+  for (int s = 0; s < ne; ++s) {
+    const int n = corners(s, v);
+    for (int c = 0; c < n; ++c) {
+      double r2 = 0.0;
+      for (int d = 0; d < 3; ++d) r2 += (v[c][d] - S->ctr[d]) * (v[c][d] - S->ctr[d]);
+      R2 = std::max(R2, r2);
+    }
+  }
+  S->R0 = sqrt(R2) * (1.0 + 1e-12);
+  S->rho = 2.0 * S->R0;
+  S->k = q->k;
+  if (!(S->R0 > 0.0) || !std::isfinite(S->R0)) return;
+  // lattice points by distance
+  struct pt { double r; int a, b; };
+  std::vector<pt> P;
+  const double reach = 12.0 * S->R0 + 4.0 * (hypot(q->d1x, q->d1y) + hypot(q->d2x, q->d2y));
+  const int n1 = (int)(reach * hypot(q->g1x, q->g1y) / (2.0 * M_PI)) + 1, n2 = (int)(reach * hypot(q->g2x, q->g2y) / (2.0 * M_PI)) + 1;
+  if ((double)n1 * n2 > 1e5) return;
+  for (int a = -n1; a <= n1; ++a)
+    for (int b = -n2; b <= n2; ++b) P.push_back({hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y), a, b});
+  std::stable_sort(P.begin(), P.end(), [](const pt &x, const pt &y) { return x.r < y.r; });
+  // the cheapest split, in FP64 operations: per pair about 45 points of 66 for
+  // each image and 16 multiply-adds for each of the K functions (G and H of 4
+  // entries, complex); once, A = U T, the samples (110 lattice terms each, a
+  // tenth of the GPU busy) and T.  Summed point by point a pair takes about 8e5.
+  const double pairs = 4.0 * ne * ne;
+  double best = 4e5 * pairs;
+  for (size_t c = 1; c < P.size() && c <= BEM_SM_MAXIMG; ++c) {
+    if (P[c].r <= P[c - 1].r * (1.0 + 1e-9)) continue;  // whole shells only
+    const double cut = P[c].r;
+    if (cut <= S->rho * 1.05) continue;
+    // tail relative to 1 / (4 pi 2 R0), six images on the first shell left in
+    const int lmax = degree_for(S->k, S->R0, cut - S->R0, 6.0 * S->rho, 1e-15, BEM_SM_MAXL);
+    if (lmax < 0) continue;
+    int Lmax = degree_for(S->k, S->rho, cut, 6.0 * S->rho, 1e-15, 2 * BEM_SM_MAXL);
+    if (Lmax < 0 || Lmax > 2 * lmax) Lmax = 2 * lmax;
+    const double K = (lmax + 1.0) * (lmax + 1.0), nt = lmax + 0.5 * Lmax + 1.0;
+    const double cost = pairs * ((c - 1) * 45.0 * 66.0 + 16.0 * K) + 4.0 * ne * 2.0 * K * K +
+                        nt * (2.0 * Lmax + 2.0) * 1.2e5 + 0.125 * K * K * lmax * nt;
+    if (cost < best) {
+      best = cost;
+      S->on = 1;
+      S->lmax = lmax;
+      S->Lmax = Lmax;
+      S->nimg = (int)c;
+      for (size_t i = 0; i < c; ++i) { S->l1[i] = P[i].a; S->l2[i] = P[i].b; }
+    }
+  }
+  if (!S->on) return;
+  S->K = (S->lmax + 1) * (S->lmax + 1);
+  S->Kp = (S->K + 15) / 16 * 16;
+  // Gauss-Legendre nodes in cos(theta): exact for products of three harmonics
+  // (degree 2 lmax + Lmax), an even number (no node on the lattice plane)
+  S->nt = (2 * S->lmax + S->Lmax) / 2 + 1;
+  S->nt += S->nt & 1;
+  S->nphi = 2 * S->Lmax + 2;
+}
+
+bem_smooth_tab bem_smooth_layout(const bem_smooth *S) {
+  bem_smooth_tab t;
+  int o = 0;
+  auto put = [&o](int n) { const int p = o; o += n; return p; };
+  t.x = put(S->nt);
+  t.w = put(S->nt);
+  t.ca = put(S->Lmax + 1);
+  t.cb = put(S->Lmax + 1);
+  t.dL = put(S->Lmax + 1);
+  t.el = put(S->lmax + 1);
+  t.rec = put((S->Lmax + 1) * (S->Lmax + 2));
+  t.img = put(3 * S->nimg * S->inst);
+  t.total = o;
+  return t;
+}
+
+void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h) {
+  const bem_smooth_tab t = bem_smooth_layout(S);
+  const int n = S->nt, L = S->Lmax;
+  // Gauss-Legendre by Newton's method on P_n
+  for (int i = 0; i < n / 2; ++i) {
+    double z = cos(M_PI * (i + 0.75) / (n + 0.5)), dp = 1.0;
+    for (int it = 0; it < 60; ++it) {
+      double p0 = 1.0, p1 = z;
+      for (int m = 2; m <= n; ++m) {
+        const double p2 = ((2.0 * m - 1.0) * z * p1 - (m - 1.0) * p0) / m;
+        p0 = p1;
+        p1 = p2;
+      }
+      dp = n * (z * p1 - p0) / (z * z - 1.0);
+      const double dz = p1 / dp;
+      z -= dz;
+      if (fabs(dz) < 1e-16) break;
+    }
+    h[t.x + i] = z;
+    h[t.x + n - 1 - i] = -z;
+    h[t.w + i] = h[t.w + n - 1 - i] = 2.0 / ((1.0 - z * z) * dp * dp);
+  }
+  // u_LM and rho u'_LM / (L + 1) are sigma_LM times g_L(k rho) and
+  // (L g_L - z^2 g_{L+1} / (2L + 3)) / (L + 1): both used, no zero shared
+  std::vector<double> j;
+  const double z = S->k * S->rho;
+  bessel_sizes(L + 1, z, j, nullptr);
+  std::vector<double> g(L + 2);
+  double f = 1.0;
+  for (int l = 0; l <= L + 1; ++l) {
+    g[l] = j[l] / f;
+    f *= z / (2.0 * l + 3.0);
+  }
+  const double kR0 = S->k * S->R0;
+  double dl = 1.0, el = 1.0;
+  for (int l = 0; l <= L; ++l) {
+    const double a = g[l], b = (l * g[l] - z * z / (2.0 * l + 3.0) * g[l + 1]) / (l + 1.0), s = 1.0 / (a * a + b * b);
+    h[t.ca + l] = a * s;
+    h[t.cb + l] = b * s / (l + 1.0);
+    // (2L + 1)!! / (k rho)^L and (k R0)^l / (2l + 1)!!: j_l in terms of g_l and R_lm
+    h[t.dL + l] = dl;
+    dl *= (2.0 * l + 3.0) / z;
+    if (l <= S->lmax) h[t.el + l] = el;
+    el *= kR0 / (2.0 * l + 3.0);
+  }
+  // Theta_lm = a (z Theta_{l-1,m} - b s Theta_{l-2,m}), and Theta_mm at l = m
+  double mm = 0.28209479177387814347;  // 1 / sqrt(4 pi)
+  for (int m = 0; m <= L; ++m) {
+    for (int l = m; l <= L; ++l) {
+      double *r = h + t.rec + l * (l + 1) + 2 * m;
+      if (l == m) {
+        r[0] = mm;
+        r[1] = 0.0;
+      } else {
+        r[0] = sqrt((4.0 * l * l - 1.0) / ((double)l * l - (double)m * m));
+        r[1] = sqrt(((l - 1.0) * (l - 1.0) - (double)m * m) / (4.0 * (l - 1.0) * (l - 1.0) - 1.0));
+      }
+    }
+    mm *= sqrt((2.0 * m + 3.0) / (2.0 * m + 2.0));
+  }
+  for (int b = 0; b < S->inst; ++b)
+    for (int i = 0; i < S->nimg; ++i) {
+      const bem_qp &q = qps[b];
+      const double sx = S->l1[i] * q.d1x + S->l2[i] * q.d2x, sy = S->l1[i] * q.d1y + S->l2[i] * q.d2y;
+      double *m = h + t.img + 3 * (b * S->nimg + i);
+      m[0] = sx;
+      m[1] = sy;
+      m[2] = (q.kx * sx + q.ky * sy) * 0.31830988618379067154;  // phase / pi
+    }
+}
+
+// ------------------------------------------------------------------ device view
+struct sm_dev {
+  int lmax, Lmax, K, Kp, nt, nphi, nimg;
+  double cx, cy, cz, R0, iR0, kR0, rho, k;
+  const double *x, *w, *ca, *cb, *dL, *el, *rec, *img;
+  double *plm;            // [lm >= 0][nt] normalised Legendre functions P_lm(x_t)
+  double *samp;           // [nb][2][nt][nphi] complex: G_s and rho dG_s/drho
+  double *sig;            // [nb][(Lmax + 1)^2] complex
+  double *T;              // [nb][Kp][2 Kp]: T^t, real and imaginary parts
+  double *U, *V, *A;      // [4 ne][Kp], [Kp][8 ne], [nb][4 ne][2 Kp]
+};
+struct sm_ws { size_t plm, samp, sig, T, U, V, A, total; };
+static sm_ws ws_layout(const bem_smooth *S, int ne, int nb) {
+  sm_ws w;
+  size_t o = 0;
+  auto put = [&o](size_t n) { const size_t p = o; o += (n + 31) / 32 * 32; return p; };
+  const size_t L = S->Lmax, Kp = S->Kp;
+  w.plm = put((L + 1) * (L + 2) / 2 * S->nt);
+  w.samp = put((size_t)nb * 4 * S->nt * S->nphi);
+  w.sig = put((size_t)nb * 2 * (L + 1) * (L + 1));
+  w.T = put((size_t)nb * 2 * Kp * Kp);
+  w.U = put(4 * (size_t)ne * Kp);
+  w.V = put(8 * (size_t)ne * Kp);
+  w.A = put((size_t)nb * 8 * ne * Kp);
+  w.total = o;
+  return w;
+}
+size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne) {
+  return ws_layout(S, ne, std::min(S->inst, BEM_SM_BAT)).total;
+}
+
+struct sm_qps { bem_qp q[BEM_SM_BAT]; };
+struct sm_out { double *G[BEM_SM_BAT], *H[BEM_SM_BAT]; };
+
+// the closed form of one image at P = R + R_l, times e^{i pi ph}: value g and
+// the factor f of its gradient f P
+__device__ __forceinline__ void sm_image(double kpi, double k, double px, double py, double pz2, double ph, double &gr,
+                                         double &gi, double &fr, double &fi) {
+  const double r2 = fma(px, px, fma(py, py, pz2));
+  const double ir = rsqrt(r2), r = r2 * ir;
+  double s, c;
+  sincospi(fma(kpi, r, ph), &s, &c);
+  gr = ir * c;
+  gi = ir * s;
+  const double ir2 = ir * ir, kr = k * r;
+  fr = -ir2 * fma(kr, gi, gr);
+  fi = ir2 * fma(kr, gr, -gi);
+}
+
+// ------------------------------------------------------------------ coefficients of the rest
+// Blocks below nsamp: G_s and its radial derivative at the sphere points
+// (one thread per point and instance).  The others: P_lm at the nodes.
+#define SMP_TH 32
+__global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm_dev S, const __grid_constant__ sm_qps Q,
+                                                      int nsamp, int nb, unsigned *status) {
+  if ((int)blockIdx.x < nsamp) {
+    const int b = blockIdx.y, i = blockIdx.x * SMP_TH + threadIdx.x;
+    if (i >= S.nt * S.nphi) return;
+    const bem_qp &q = Q.q[b];
+    const int t = i / S.nphi, jp = i % S.nphi;
+    const double ct = S.x[t], sn = sqrt((1.0 - ct) * (1.0 + ct));
+    double sp, cp;
+    sincospi(2.0 * jp / S.nphi, &sp, &cp);
+    const double ux = sn * cp, uy = sn * sp, X = S.rho * ux, Y = S.rho * uy, Z = S.rho * ct;
+    bem_gval gv;
+    const int rc = bem_qpgf(q, X, Y, Z, gv);
+    if (rc < 0) atomicOr(status, rc == -12 || rc == -23 ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT);
+    double ur = 0, ui = 0, xr = 0, xi = 0;  // the images' value and radial derivative, times 4 pi
+    const double kpi = S.k * 0.31830988618379067154;
+    for (int m = 0; m < S.nimg; ++m) {
+      const double *im = S.img + 3 * (b * S.nimg + m);
+      const double px = X + im[0], py = Y + im[1];
+      double gr, gi, fr, fi;
+      sm_image(kpi, S.k, px, py, Z * Z, im[2], gr, gi, fr, fi);
+      const double d = px * ux + py * uy + Z * ct;
+      ur += gr;
+      ui += gi;
+      xr += fr * d;
+      xi += fi * d;
+    }
+    const double c4 = BEM_I_FP;
+    double *o = S.samp + 2 * ((size_t)b * 2 * S.nt * S.nphi + i), *o2 = o + 2 * (size_t)S.nt * S.nphi;
+    o[0] = gv.g.re - c4 * ur;
+    o[1] = gv.g.im - c4 * ui;
+    o2[0] = S.rho * (gv.gx.re * ux + gv.gy.re * uy + gv.gz.re * ct - c4 * xr);
+    o2[1] = S.rho * (gv.gx.im * ux + gv.gy.im * uy + gv.gz.im * ct - c4 * xi);
+    return;
+  }
+  if (blockIdx.y) return;
+  // P_lm(x_t): one thread per (m, t), upward in l
+  const int i = (blockIdx.x - nsamp) * SMP_TH + threadIdx.x;
+  if (i >= (S.Lmax + 1) * S.nt) return;
+  const int m = i / S.nt, t = i % S.nt;
+  const double ct = S.x[t], sn = sqrt((1.0 - ct) * (1.0 + ct));
+  double p1 = S.rec[m * (m + 1) + 2 * m], p0 = 0.0;
+  for (int a = 0; a < m; ++a) p1 *= sn;
+  for (int l = m; l <= S.Lmax; ++l) {
+    if (l > m) {
+      const double *r = S.rec + l * (l + 1) + 2 * m;
+      const double p2 = r[0] * (ct * p1 - r[1] * p0);
+      p0 = p1;
+      p1 = p2;
+    }
+    S.plm[(size_t)(l * (l + 1) / 2 + m) * S.nt + t] = p1;
+  }
+}
+
+// sigma_LM of one order M and instance: Fourier sums in phi at every node,
+// then Legendre sums
+#define SMC_TH 128
+#define SM_MAXNT (3 * BEM_SM_MAXL + 4)
+__global__ void __launch_bounds__(SMC_TH) k_sm_coef(const __grid_constant__ sm_dev S) {
+  __shared__ double F[4][SM_MAXNT];
+  const int M = (int)blockIdx.x - S.Lmax, b = blockIdx.y;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const double2 *u = reinterpret_cast<const double2 *>(S.samp) + (size_t)b * 2 * S.nt * S.nphi;
+  const double2 *du = u + (size_t)S.nt * S.nphi;
+  for (int t = wid; t < S.nt; t += SMC_TH / 32) {
+    double a[4] = {0, 0, 0, 0};
+    for (int j = lane; j < S.nphi; j += 32) {
+      int e = (int)(((long long)M * j) % S.nphi);
+      double s, c;
+      sincospi(-2.0 * e / S.nphi, &s, &c);
+      const double2 x = u[(size_t)t * S.nphi + j], y = du[(size_t)t * S.nphi + j];
+      a[0] += x.x * c - x.y * s;
+      a[1] += x.x * s + x.y * c;
+      a[2] += y.x * c - y.y * s;
+      a[3] += y.x * s + y.y * c;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) a[c] += __shfl_down_sync(0xffffffffu, a[c], o);
+    if (lane == 0) {
+      const double f = S.w[t] * 2.0 * CUDART_PI / S.nphi;
+      for (int c = 0; c < 4; ++c) F[c][t] = a[c] * f;
+    }
+  }
+  __syncthreads();
+  const int am = abs(M);
+  for (int l = am + threadIdx.x; l <= S.Lmax; l += SMC_TH) {
+    const double *p = S.plm + (size_t)(l * (l + 1) / 2 + am) * S.nt;
+    double a[4] = {0, 0, 0, 0};
+    for (int t = 0; t < S.nt; ++t)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) a[c] += p[t] * F[c][t];
+    double *o = S.sig + 2 * ((size_t)b * (S.Lmax + 1) * (S.Lmax + 1) + l * l + l + M);
+    o[0] = S.ca[l] * a[0] + S.cb[l] * a[2];
+    o[1] = S.ca[l] * a[1] + S.cb[l] * a[3];
+  }
+}
+
+// position of the real function (l, m): cosine (or m = 0) and sine
+__device__ __forceinline__ int sm_idx(int l, int m, int sine) { return l * l + (m ? 2 * m - 1 + sine : 0); }
+
+// T_lm,l'm' = 4 pi sum_L sigma_{L,m-m'} i^{l-l'-L} C (2L+1)!! ... with
+// C = int Y*_lm Y_l'm' Y_{L,m-m'} = 2 pi int P_lm P_l'm' P_L|m-m'| d(cos theta)
+// (harmonics without the Condon-Shortley sign, Y_{l,-m} = conj Y_lm), in the
+// real basis.  Block: (l, m >= 0); thread: (l', m' >= 0).  The integrand is
+// even: half the nodes.  Stored transposed, row l'm', columns lm (real part)
+// and Kp + lm (imaginary part).
+#define SMT_TH 64
+__global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev S) {
+  extern __shared__ double sm_raw[];  // [nt / 2][SMT_TH]
+  const int b = blockIdx.z;
+  int l = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
+  while ((l + 1) * (l + 2) / 2 <= (int)blockIdx.x) ++l;
+  while (l * (l + 1) / 2 > (int)blockIdx.x) --l;
+  const int m = (int)blockIdx.x - l * (l + 1) / 2;
+  const int i2 = blockIdx.y * SMT_TH + threadIdx.x;
+  const int nlm = (S.lmax + 1) * (S.lmax + 2) / 2;
+  const bool live = i2 < nlm;
+  int l2 = 0, m2 = 0;
+  if (live) {
+    l2 = (int)((sqrt(8.0 * i2 + 1.0) - 1.0) * 0.5);
+    while ((l2 + 1) * (l2 + 2) / 2 <= i2) ++l2;
+    while (l2 * (l2 + 1) / 2 > i2) --l2;
+    m2 = i2 - l2 * (l2 + 1) / 2;
+  }
+  const int nh = S.nt / 2;
+  double *pr = sm_raw + threadIdx.x;
+  const double *p1 = S.plm + (size_t)blockIdx.x * S.nt, *p2 = S.plm + (size_t)(live ? i2 : 0) * S.nt;
+  for (int t = 0; t < nh; ++t) pr[t * SMT_TH] = 4.0 * CUDART_PI * S.w[t] * p1[t] * p2[t];
+  if (!live) return;
+  const double *sg = S.sig + 2 * (size_t)b * (S.Lmax + 1) * (S.Lmax + 1);
+  // tp[0]: T_{m,m'}, tp[1]: T_{-m,-m'}, tp[2]: T_{m,-m'}, tp[3]: T_{-m,m'}
+  cplx tp[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tp[c] = cmk(0.0, 0.0);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    if (v && (m == 0 || m2 == 0)) break;
+    const int M = v ? m + m2 : m - m2, aM = abs(M);
+    int L0 = max(abs(l - l2), aM);
+    L0 += (L0 + l + l2) & 1;
+    for (int L = L0; L <= min(l + l2, S.Lmax); L += 2) {
+      const double *pL = S.plm + (size_t)(L * (L + 1) / 2 + aM) * S.nt;
+      double G = 0.0;
+      for (int t = 0; t < nh; ++t) G = fma(pr[t * SMT_TH], pL[t], G);
+      // i^{l - l' - L}, l - l' - L even
+      const double f = ((l - l2 - L) & 2) ? -G * S.dL[L] : G * S.dL[L];
+      const double *sp = sg + 2 * (L * L + L + M), *sn = sg + 2 * (L * L + L - M);
+      tp[2 * v].re += f * sp[0];
+      tp[2 * v].im += f * sp[1];
+      tp[2 * v + 1].re += f * sn[0];
+      tp[2 * v + 1].im += f * sn[1];
+    }
+  }
+  const double sc = 4.0 * CUDART_PI * S.el[l] * S.el[l2];
+  double *T = S.T + (size_t)b * 2 * S.Kp * S.Kp;
+  auto put = [&](int r, int c, cplx z) {  // entry (source function r, target function c)
+    T[(size_t)c * 2 * S.Kp + r] = sc * z.re;
+    T[(size_t)c * 2 * S.Kp + S.Kp + r] = sc * z.im;
+  };
+  const int rc = sm_idx(l, m, 0), rs = rc + 1, cc = sm_idx(l2, m2, 0), cs = cc + 1;
+  const double h2 = 0.70710678118654752440;
+  if (m == 0 && m2 == 0) {
+    put(rc, cc, tp[0]);
+  } else if (m == 0) {
+    // phi*_{+-m'} = (c -+ i s) / sqrt2: T_{0,m'}, T_{0,-m'} (tp[0], tp[1])
+    put(rc, cc, cscale(cadd(tp[0], tp[1]), h2));
+    put(rc, cs, cscale(cmuli(csub(tp[1], tp[0])), h2));
+  } else if (m2 == 0) {
+    put(rc, cc, cscale(cadd(tp[0], tp[1]), h2));
+    put(rs, cc, cscale(cmuli(csub(tp[0], tp[1])), h2));
+  } else {
+    const cplx a = tp[0], d = tp[1], e = tp[2], g = tp[3];  // ++, --, +-, -+
+    put(rc, cc, cscale(cadd(cadd(a, d), cadd(e, g)), 0.5));
+    put(rs, cs, cscale(csub(cadd(a, d), cadd(e, g)), 0.5));
+    // c, s': -i s' over the sign of m'; s, c': +i s over the sign of m
+    put(rc, cs, cscale(cmuli(csub(cadd(d, e), cadd(a, g))), 0.5));
+    put(rs, cc, cscale(cmuli(csub(cadd(a, e), cadd(d, g))), 0.5));
+  }
+}
+
+// ------------------------------------------------------------------ functions at nodes and over elements
+// g_l(z), l = 0 .. n + 1, into g[l * stride] by downward recurrence
+__device__ __forceinline__ void sm_gl(int n, double z2, double *g, int stride) {
+  const int top = n + 1;
+  double a = 0.0, b = 0.0;
+#pragma unroll 1
+  for (int w = 0; w < 2; ++w) {
+    const int l = top + 1 - w;
+    double t = 1.0, s = 1.0;
+    for (int m = 1; m < 100; ++m) {
+      t *= -0.5 * z2 / (m * (2.0 * l + 2.0 * m + 1.0));
+      s += t;
+      if (fabs(t) < 1e-18 * fabs(s)) break;
+    }
+    if (w == 0) a = s;
+    else b = s;
+  }
+  g[top * stride] = b;  // g_top, a = g_{top + 1}
+  for (int l = top; l > 0; --l) {
+    const double c = b - z2 / ((2.0 * l + 1.0) * (2.0 * l + 3.0)) * a;
+    a = b;
+    b = c;
+    g[(l - 1) * stride] = c;
+  }
+}
+
+// U[p][lm] = phi_lm(x_p): a warp per node, a lane per order m
+#define SMU_TH 128
+__global__ void __launch_bounds__(SMU_TH) k_sm_targets(const __grid_constant__ sm_dev S, bem_dom_dev D) {
+  __shared__ double g[SMU_TH / 32][BEM_SM_MAXL + 2];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p = blockIdx.x * (SMU_TH / 32) + wid;
+  if (p >= 4 * D.ne) return;
+  const int te = abs(D.sid[p >> 2]) - 1;
+  double *U = S.U + (size_t)p * S.Kp;
+  const bool pad = (p & 3) == 3 && D.has_tri && D.npe[te] == 3;
+  if (pad) {
+    for (int c = lane; c < S.Kp; c += 32) U[c] = 0.0;
+    return;
+  }
+  for (int c = S.K + lane; c < S.Kp; c += 32) U[c] = 0.0;
+  const double *r = D.ren + (size_t)te * 12 + (p & 3) * 3;
+  const double x = (r[0] - S.cx) * S.iR0, y = (r[1] - S.cy) * S.iR0, z = (r[2] - S.cz) * S.iR0;
+  const double s2 = x * x + y * y + z * z;
+  if (lane == 0) sm_gl(S.lmax, S.kR0 * S.kR0 * s2, g[wid], 1);
+  __syncwarp();
+  for (int m = lane; m <= S.lmax; m += 32) {
+    double C = 1.0, Sn = 0.0;  // Re, Im (x + iy)^m
+    for (int a = 0; a < m; ++a) {
+      const double c2 = C * x - Sn * y;
+      Sn = C * y + Sn * x;
+      C = c2;
+    }
+    if (m) { C *= 1.4142135623730950488; Sn *= 1.4142135623730950488; }
+    double t1 = S.rec[m * (m + 1) + 2 * m], t0 = 0.0;
+    for (int l = m; l <= S.lmax; ++l) {
+      if (l > m) {
+        const double *rr = S.rec + l * (l + 1) + 2 * m;
+        const double t2 = rr[0] * (z * t1 - rr[1] * s2 * t0);
+        t0 = t1;
+        t1 = t2;
+      }
+      const double v = g[wid][l] * t1;
+      U[sm_idx(l, m, 0)] = v * C;
+      if (m) U[sm_idx(l, m, 1)] = v * Sn;
+    }
+  }
+}
+
+// V[lm][4 s + a] = int N_a |W| phi_lm, V[lm][4 ne + 4 s + a] = int N_a W . grad phi_lm
+// over element s, on the reference's 12 x 12 rule (3 parts of it on a
+// triangle).  Block: (element, order m); a thread per point walks l and leaves
+// the four values of each l in shared memory, then a thread per value sums
+// over the points.
+#define SMV_PT (BEM_GLN * BEM_GLN)
+#define SMV_TH 160
+__global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ sm_dev S, bem_dom_dev D) {
+  extern __shared__ double sm_raw[];
+  const int s = blockIdx.x, m = blockIdx.y, tid = threadIdx.x;
+  const int se = abs(D.sid[s]) - 1;
+  const bool tri = D.has_tri && D.npe[se] == 3;
+  const int nl = S.lmax + 1 - m, nf = m ? 2 : 1;  // functions per degree
+  double *Nw = sm_raw;                  // [4][SMV_PT] weight times N_a
+  double *val = Nw + 4 * SMV_PT;        // [nl][2 nf][SMV_PT]
+  const int nout = nl * 2 * nf;
+  const size_t N8 = 8 * (size_t)D.ne;
+  double acc[4] = {0, 0, 0, 0};
+  bem_el el;
+  bem_load_el(D.cr, D.cw, se, el);
+  for (int part = 0; part < (tri ? 3 : 1); ++part) {
+    if (part) __syncthreads();
+    if (tid < SMV_PT) {
+      const int i = tid / BEM_GLN, j = tid % BEM_GLN;
+      double zt = c_q.xl[i], et = c_q.xl[j], wt = c_q.wl[i] * c_q.wl[j];
+      if (tri) {
+        wt *= bem_tri_wfac(zt, et);
+        bem_tri_point(part, c_q.xl[i], c_q.xl[j], zt, et);
+      }
+      double r[3], W[3], Nn[4];
+      bem_rw(el, zt, et, r, W);
+      bem_Nn(tri, zt, et, Nn);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) Nw[a * SMV_PT + tid] = Nn[a] * wt;
+      const double aW = sqrt(W[0] * W[0] + W[1] * W[1] + W[2] * W[2]);
+      const double x = (r[0] - S.cx) * S.iR0, y = (r[1] - S.cy) * S.iR0, z = (r[2] - S.cz) * S.iR0;
+      const double s2 = x * x + y * y + z * z;
+      const double wx = W[0] * S.iR0, wy = W[1] * S.iR0, wz = W[2] * S.iR0;
+      const double wr = wx * x + wy * y + wz * z;
+      // Re, Im (x + iy)^m and their derivatives along W
+      double C = 1.0, Sn = 0.0, C0 = 0.0, S0 = 0.0;
+      for (int a = 0; a < m; ++a) {
+        C0 = C;
+        S0 = Sn;
+        const double c2 = C * x - Sn * y;
+        Sn = C * y + Sn * x;
+        C = c2;
+      }
+      double dC = m * (wx * C0 - wy * S0), dS = m * (wx * S0 + wy * C0);
+      if (m) {
+        const double q2 = 1.4142135623730950488;
+        C *= q2; Sn *= q2; dC *= q2; dS *= q2;
+      }
+      // g_l downward from l = lmax + 1, kept in the value slots until used
+      const double z2 = S.kR0 * S.kR0 * s2, kk2 = S.kR0 * S.kR0;
+      // upward walk needs g_l and g_{l+1}: g is computed into val[l - m][0]
+      // (read before it is overwritten) with g_{lmax + 1} kept in a register
+      double gtop;
+      {
+        double a = 0.0, b = 0.0;
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {
+          const int l = S.lmax + 2 - w;
+          double t = 1.0, sum = 1.0;
+          for (int q = 1; q < 100; ++q) {
+            t *= -0.5 * z2 / (q * (2.0 * l + 2.0 * q + 1.0));
+            sum += t;
+            if (fabs(t) < 1e-18 * fabs(sum)) break;
+          }
+          if (w == 0) a = sum;
+          else b = sum;
+        }
+        gtop = b;
+        for (int l = S.lmax + 1; l > m; --l) {
+          const double c = b - z2 / ((2.0 * l + 1.0) * (2.0 * l + 3.0)) * a;
+          a = b;
+          b = c;
+          val[(size_t)(l - 1 - m) * 2 * nf * SMV_PT + tid] = c;
+        }
+      }
+      double t1 = S.rec[m * (m + 1) + 2 * m], t0 = 0.0;  // Theta
+      double p1 = 0.0, p0 = 0.0, q1 = 0.0, q0 = 0.0;     // dTheta/dz, dTheta/ds
+      for (int l = m; l <= S.lmax; ++l) {
+        if (l > m) {
+          const double *rr = S.rec + l * (l + 1) + 2 * m;
+          const double ra = rr[0], rb = rr[1];
+          const double t2 = ra * (z * t1 - rb * s2 * t0);
+          const double p2 = ra * (t1 + z * p1 - rb * s2 * p0);
+          const double q2 = ra * (z * q1 - rb * (t0 + s2 * q0));
+          t0 = t1; t1 = t2;
+          p0 = p1; p1 = p2;
+          q0 = q1; q1 = q2;
+        }
+        double *v = val + (size_t)(l - m) * 2 * nf * SMV_PT + tid;
+        const double g = v[0], gn = l < S.lmax ? v[2 * nf * SMV_PT] : gtop;
+        // W . grad (g Theta C) = [g (wz P + 2 wr Q) - wr kk^2 g_{l+1} / (2l + 3) Theta] C + g Theta W . grad C
+        const double gt = g * t1;
+        const double f = g * (wz * p1 + 2.0 * wr * q1) - wr * kk2 * gn / (2.0 * l + 3.0) * t1;
+        v[0] = aW * gt * C;
+        v[SMV_PT] = f * C + gt * dC;
+        if (nf == 2) {
+          v[2 * SMV_PT] = aW * gt * Sn;
+          v[3 * SMV_PT] = f * Sn + gt * dS;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < nout) {
+      const double *v = val + (size_t)tid * SMV_PT;
+      const int q0 = tid % SMV_PT;  // another first point per thread: the rows are a multiple of 32 banks apart
+      for (int q = 0; q < SMV_PT; ++q) {
+        const int qq = q + q0 < SMV_PT ? q + q0 : q + q0 - SMV_PT;
+        const double x = v[qq];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) acc[a] = fma(x, Nw[a * SMV_PT + qq], acc[a]);
+      }
+    }
+  }
+  if (tid < nout) {
+    const int l = m + tid / (2 * nf), r = tid % (2 * nf);  // r: value, derivative (, sine value, derivative)
+    double *o = S.V + (size_t)sm_idx(l, m, r >> 1) * N8 + ((r & 1) ? 4 * (size_t)D.ne : 0) + 4 * (size_t)s;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) o[a] = acc[a];
+  }
+  if (m == 0 && tid < 8)  // padding rows of V
+    for (int r = S.K; r < S.Kp; ++r)
+      S.V[(size_t)r * N8 + (tid < 4 ? 0 : 4 * (size_t)D.ne) + 4 * (size_t)s + (tid & 3)] = 0.0;
+}
+
+// ------------------------------------------------------------------ real matrix product on the FP64 tensor cores
+// C = A B, A M x K (row-major, lda), B K x N (row-major, ldb), K a multiple of
+// 16, lda and ldb even.  128 x 64 tiles, 8 warps of 32 x 32, mma m16n8k8,
+// operands through a 3-stage ring of 16-deep slices filled by 16-byte
+// asynchronous copies; row strides of 20 and 68 doubles keep the fragment
+// loads free of bank conflicts.  ILV: rows 2p and 2p + 1 are the real and
+// imaginary parts of row p of a complex result whose columns below N / 2 go to
+// G and the others to H (leading dimension N / 2).
+#define GM_BM 128
+#define GM_BN 64
+#define GM_BK 16
+#define GM_ST 3
+#define GM_LDA 20
+#define GM_LDB 68
+#define GM_TH 256
+#define GM_STAGE (GM_BM * GM_LDA + GM_BK * GM_LDB)
+#define GM_SMEM (GM_ST * GM_STAGE * 8)
+__device__ __forceinline__ void gm_cp16(double *dst, const double *src, bool live) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = live ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void gm_mma(const double (&a)[4], const double (&b)[2], double (&d)[4]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+template <bool ILV>
+__global__ void __launch_bounds__(GM_TH, 2) k_sm_gemm(const double *A0, size_t strideA, int lda, const double *B0,
+                                                      size_t strideB, int ldb, int M, int N, int K, double *C0,
+                                                      size_t strideC, int ldc, const __grid_constant__ sm_out O) {
+  extern __shared__ __align__(16) double gm_smem[];
+  const double *A = A0 + blockIdx.z * strideA, *B = B0 + blockIdx.z * strideB;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = lane >> 2, q = lane & 3;
+  const int rb = blockIdx.y * GM_BM, cb = blockIdx.x * GM_BN;
+  const int wm = (wid & 3) * 32, wn = (wid >> 2) * 32;
+  auto fill = [&](int st, int k0) {
+    double *As = gm_smem + st * GM_STAGE, *Bs = As + GM_BM * GM_LDA;
+#pragma unroll
+    for (int i = 0; i < GM_BM * GM_BK / 2 / GM_TH; ++i) {
+      const int e = t + i * GM_TH, r = e >> 3, c = (e & 7) * 2;
+      const bool live = rb + r < M;
+      gm_cp16(As + r * GM_LDA + c, A + (size_t)(live ? rb + r : 0) * lda + k0 + c, live);
+    }
+#pragma unroll
+    for (int i = 0; i < GM_BK * GM_BN / 2 / GM_TH; ++i) {
+      const int e = t + i * GM_TH, r = e >> 5, c = (e & 31) * 2;
+      const bool live = cb + c < N;
+      gm_cp16(Bs + r * GM_LDB + c, B + (size_t)(k0 + r) * ldb + (live ? cb + c : 0), live);
+    }
+  };
+  double acc[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0;
+  const int nk = K / GM_BK;
+#pragma unroll
+  for (int s = 0; s < GM_ST - 1; ++s) {
+    if (s < nk) fill(s, s * GM_BK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GM_ST - 2) : "memory");
+    __syncthreads();  // slice kt is in, and every warp is done with slice kt - 1
+    if (kt + GM_ST - 1 < nk) fill((kt + GM_ST - 1) % GM_ST, (kt + GM_ST - 1) * GM_BK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const double *As = gm_smem + (kt % GM_ST) * GM_STAGE, *Bs = As + GM_BM * GM_LDA;
+#pragma unroll
+    for (int k8 = 0; k8 < GM_BK; k8 += 8) {
+      double a[2][4], b[4][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[i][c] = As[(wm + i * 16 + g + (c & 1) * 8) * GM_LDA + k8 + q + (c >> 1) * 4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) b[j][c] = Bs[(k8 + q + c * 4) * GM_LDB + wn + j * 8 + g];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gm_mma(a[i], b[j], acc[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = rb + wm + i * 16 + g + 8 * h, col = cb + wn + j * 8 + 2 * q;
+        const double d0 = acc[i][j][2 * h], d1 = acc[i][j][2 * h + 1];
+        if (!ILV) {
+          if (row < M && col < N)
+            *reinterpret_cast<double2 *>(C0 + blockIdx.z * strideC + (size_t)row * ldc + col) = make_double2(d0, d1);
+        } else {
+          // the lane four away holds the other part of the same row of G, H:
+          // the even row's lane takes column col, the odd row's col + 1
+          const bool odd = g & 1;
+          const double other = __shfl_xor_sync(0xffffffffu, odd ? d0 : d1, 4);
+          const int cc = col + (odd ? 1 : 0), N2 = N / 2;
+          const double2 z = odd ? make_double2(other, d1) : make_double2(d0, other);
+          if (row < M && cc < N) {
+            double *dst = (cc < N2 ? O.G[blockIdx.z] : O.H[blockIdx.z]) + 2 * ((size_t)(row >> 1) * N2 + (cc < N2 ? cc : cc - N2));
+            *reinterpret_cast<double2 *>(dst) = z;
+          }
+        }
+      }
+}
+
+// ------------------------------------------------------------------ images
+// The images of every pair off the lattice plane, in closed form, added to G
+// and H: LP lanes per pair, each a share of the rule's points.  The home
+// image of a regular pair takes the pair's own rule (its flag); the others
+// share the points of the rule for the nearest of them, so that an element's
+// geometry is formed once for all.  A warp takes the longest rule its pairs
+// ask for.  FP64 pipe: about 66 operations per image and point.
+#define SMI_TH 128
+__device__ __forceinline__ int sm_rule_points(int n, bool tri) { return n == BEM_GLN ? (tri ? 3 : 1) * BEM_GLN * BEM_GLN : n * n; }
+template <int LP>
+__global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__ sm_dev S, bem_dom_dev D, int far_rule,
+                                                         const uint8_t *__restrict__ flag,
+                                                         const __grid_constant__ sm_out O) {
+  __shared__ double im[3 * BEM_SM_MAXIMG];
+  const int b = blockIdx.y;
+  for (int e = threadIdx.x; e < 3 * S.nimg; e += SMI_TH) im[e] = S.img[3 * b * S.nimg + e];
+  __syncthreads();
+  const long long npairs = 4LL * D.ne * D.ne;
+  const long long pair = ((long long)blockIdx.x * SMI_TH + threadIdx.x) / LP;
+  const int sub = threadIdx.x % LP;
+  const bool in = pair < npairs;
+  const int p = in ? (int)(pair / D.ne) : 0, s = in ? (int)(pair % D.ne) : 0;
+  const int fl = in ? flag[pair] : 0;
+  const int te = abs(D.sid[p >> 2]) - 1, se = abs(D.sid[s]) - 1;
+  const bool tri = D.has_tri && __ldg(D.npe + se) == 3;
+  const bool live = in && fl != 0 && !((p & 3) == 3 && D.has_tri && __ldg(D.npe + te) == 3);
+  bem_el el;
+  bem_load_el(D.cr, D.cw, se, el);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) el.cr[d][0] -= __ldg(D.ren + (size_t)te * 12 + (p & 3) * 3 + d);  // r is R now
+  int n1 = 0, n2 = 0;
+  if (live) {
+    if (fl >= 3) n1 = fl == BEM_FL_REF ? BEM_GLN : BEM_TIER_N0 - (fl - 3);
+    n2 = BEM_GLN;
+    if (far_rule && S.nimg > 1) {
+      double d2 = 1e300;
+      for (int m = 1; m < S.nimg; ++m) {
+        const double x = el.cr[0][0] + im[3 * m], y = el.cr[1][0] + im[3 * m + 1];
+        d2 = fmin(d2, fma(x, x, y * y));
+      }
+      d2 = fma(el.cr[2][0], el.cr[2][0], d2);
+      const double R2 = el_circum2(el, tri);
+      const int t = tier_of(d2 / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
+      if (t >= 0) n2 = BEM_TIER_N0 - t;
+    }
+    if (S.nimg == 1) n2 = 0;
+  }
+  const int w1 = __reduce_max_sync(0xffffffffu, n1);
+  n1 = n1 ? w1 : 0;
+  n2 = __reduce_max_sync(0xffffffffu, n2);
+  double v[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) v[c] = 0.0;
+  const double k = S.k, kpi = S.k * 0.31830988618379067154;
+#pragma unroll 1
+  for (int grp = 0; grp < 2; ++grp) {
+    if (grp == 0 ? n1 == 0 : (!live || n2 == 0)) continue;
+    const int n = grp == 0 ? n1 : n2;
+    const int m0 = grp, m1 = grp == 0 ? 1 : S.nimg, np = sm_rule_points(n, tri);
+    const int t = BEM_TIER_N0 - n;
+#pragma unroll 1
+    for (int pt = sub; pt < np; pt += LP) {
+      double z, e, wt;
+      if (n == BEM_GLN) {
+        const int part = pt / (BEM_GLN * BEM_GLN), ij = pt % (BEM_GLN * BEM_GLN);
+        const double a = c_q.xl[ij / BEM_GLN], c = c_q.xl[ij % BEM_GLN];
+        z = a;
+        e = c;
+        wt = c_q.wl[ij / BEM_GLN] * c_q.wl[ij % BEM_GLN];
+        if (tri) {
+          bem_tri_point(part, a, c, z, e);
+          wt *= bem_tri_wfac(a, c);
+        }
+      } else {
+        const int i = pt / n, j = pt - i * n;
+        tier_point(t, tri, i, j, z, e);
+        wt = c_q.wt[t][i] * c_q.wt[t][j];
+        if (tri) wt *= 0.125 * (c_q.xt[t][i] + 1.0);
+      }
+      double R[3], W[3];
+      bem_rw(el, z, e, R, W);
+      const double rz2 = R[2] * R[2], rzw = R[2] * W[2];
+      double gr = 0.0, gi = 0.0, hr = 0.0, hi = 0.0;
+#pragma unroll 2
+      for (int m = m0; m < m1; ++m) {
+        const double px = R[0] + im[3 * m], py = R[1] + im[3 * m + 1];
+        double a, c, fr, fi;
+        sm_image(kpi, k, px, py, rz2, im[3 * m + 2], a, c, fr, fi);
+        const double dw = fma(px, W[0], fma(py, W[1], rzw));
+        gr += a;
+        gi += c;
+        hr = fma(fr, dw, hr);
+        hi = fma(fi, dw, hi);
+      }
+      const double aw = sqrt(W[0] * W[0] + W[1] * W[1] + W[2] * W[2]) * wt;
+      gr *= aw; gi *= aw; hr *= wt; hi *= wt;
+      double N[4];
+      bem_Nn(tri, z, e, N);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        v[2 * a] = fma(gr, N[a], v[2 * a]);
+        v[2 * a + 1] = fma(gi, N[a], v[2 * a + 1]);
+        v[8 + 2 * a] = fma(hr, N[a], v[8 + 2 * a]);
+        v[8 + 2 * a + 1] = fma(hi, N[a], v[8 + 2 * a + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = LP / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] += __shfl_down_sync(0xffffffffu, v[c], o, LP);
+  if (live && sub == 0) {
+    const size_t at = (size_t)p * (4 * (size_t)D.ne) + 4 * (size_t)s;
+    double2 *G = reinterpret_cast<double2 *>(O.G[b]) + at, *H = reinterpret_cast<double2 *>(O.H[b]) + at;
+    const int na = tri ? 3 : 4;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (a < na) {
+        double2 x = G[a], y = H[a];
+        x.x = fma(BEM_I_FP, v[2 * a], x.x);
+        x.y = fma(BEM_I_FP, v[2 * a + 1], x.y);
+        y.x = fma(BEM_I_FP, v[8 + 2 * a], y.x);
+        y.y = fma(BEM_I_FP, v[8 + 2 * a + 1], y.y);
+        G[a] = x;
+        H[a] = y;
+      }
+  }
+}
+
+// ------------------------------------------------------------------ launches
+static sm_dev dev_view(const bem_smooth *S, int ne, int b0) {
+  sm_dev d;
+  d.lmax = S->lmax; d.Lmax = S->Lmax; d.K = S->K; d.Kp = S->Kp; d.nt = S->nt; d.nphi = S->nphi; d.nimg = S->nimg;
+  d.cx = S->ctr[0]; d.cy = S->ctr[1]; d.cz = S->ctr[2];
+  d.R0 = S->R0; d.iR0 = 1.0 / S->R0; d.kR0 = S->k * S->R0; d.rho = S->rho; d.k = S->k;
+  const bem_smooth_tab t = bem_smooth_layout(S);
+  d.x = S->tab + t.x; d.w = S->tab + t.w; d.ca = S->tab + t.ca; d.cb = S->tab + t.cb;
+  d.dL = S->tab + t.dL; d.el = S->tab + t.el; d.rec = S->tab + t.rec;
+  d.img = S->tab + t.img + 3 * (size_t)b0 * S->nimg;
+  const sm_ws w = ws_layout(S, ne, std::min(S->inst, BEM_SM_BAT));
+  d.plm = S->ws + w.plm; d.samp = S->ws + w.samp; d.sig = S->ws + w.sig; d.T = S->ws + w.T;
+  d.U = S->ws + w.U; d.V = S->ws + w.V; d.A = S->ws + w.A;
+  return d;
+}
+
+template <int LP>
+static void launch_images(const sm_dev &d, const bem_dom_dev *D, int nb, const uint8_t *flag, const sm_out &O, cudaStream_t st) {
+  const long long th = 4LL * D->ne * D->ne * LP;
+  k_sm_images<LP><<<dim3((unsigned)((th + SMI_TH - 1) / SMI_TH), nb), SMI_TH, 0, st>>>(d, *D, D->far_rule, flag, O);
+}
+
+extern "C" int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
+                                 double *const *H, const bem_scratch *scr, cudaStream_t st) {
+  const int ne = D->ne, N = 4 * ne;
+  const int smem_v = (4 * SMV_PT + std::max(2 * (S->lmax + 1), 4 * S->lmax) * SMV_PT) * (int)sizeof(double);
+  const int smem_t = S->nt / 2 * SMT_TH * (int)sizeof(double);
+  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (cudaFuncSetAttribute(k_sm_sources, at, smem_v) != cudaSuccess || cudaFuncSetAttribute(k_sm_T, at, smem_t) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_gemm<true>, at, GM_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_gemm<false>, at, GM_SMEM) != cudaSuccess)
+    return -1;
+  const long long npairs = (long long)N * ne;
+  const int nlm = (S->lmax + 1) * (S->lmax + 2) / 2;
+  for (int b0 = 0; b0 < nb; b0 += BEM_SM_BAT) {
+    const int n = nb - b0 < BEM_SM_BAT ? nb - b0 : BEM_SM_BAT;
+    const sm_dev d = dev_view(S, ne, nb == 1 ? S->first : b0);
+    sm_qps Q;
+    sm_out O;
+    for (int i = 0; i < BEM_SM_BAT; ++i) {
+      Q.q[i] = qps[b0 + (i < n ? i : 0)];
+      O.G[i] = i < n ? G[b0 + i] : nullptr;
+      O.H[i] = i < n ? H[b0 + i] : nullptr;
+    }
+    const int nsamp = (S->nt * S->nphi + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
+    k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, n, scr->status);
+    k_sm_coef<<<dim3(2 * S->Lmax + 1, n), SMC_TH, 0, st>>>(d);
+    if (cudaMemsetAsync(d.T, 0, (size_t)n * 2 * S->Kp * S->Kp * sizeof(double), st) != cudaSuccess) return -1;
+    k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, smem_t, st>>>(d);
+    bem_count_launches(3);
+    if (b0 == 0) {
+      k_sm_targets<<<(N + SMU_TH / 32 - 1) / (SMU_TH / 32), SMU_TH, 0, st>>>(d, *D);
+      k_sm_sources<<<dim3(ne, S->lmax + 1), SMV_TH, smem_v, st>>>(d, *D);
+      bem_count_launches(2);
+    }
+    const size_t sT = 2 * (size_t)S->Kp * S->Kp, sA = (size_t)N * 2 * S->Kp;
+    k_sm_gemm<false><<<dim3((2 * S->Kp + GM_BN - 1) / GM_BN, (N + GM_BM - 1) / GM_BM, n), GM_TH, GM_SMEM, st>>>(
+        d.U, 0, S->Kp, d.T, sT, 2 * S->Kp, N, 2 * S->Kp, S->Kp, d.A, sA, 2 * S->Kp, O);
+    k_sm_gemm<true><<<dim3((8 * ne + GM_BN - 1) / GM_BN, (2 * N + GM_BM - 1) / GM_BM, n), GM_TH, GM_SMEM, st>>>(
+        d.A, sA, S->Kp, d.V, 0, 8 * ne, 2 * N, 8 * ne, S->Kp, nullptr, 0, 0, O);
+    // lanes per pair: enough threads for several waves of the GPU's 75,000 resident ones
+    const long long work = npairs * n;
+    if (work >= 1500000) launch_images<1>(d, D, n, scr->flag, O, st);
+    else if (work >= 60000) launch_images<4>(d, D, n, scr->flag, O, st);
+    else launch_images<32>(d, D, n, scr->flag, O, st);
+    bem_count_launches(3);
+  }
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+}

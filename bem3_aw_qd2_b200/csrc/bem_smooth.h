@@ -1,0 +1,45 @@
+// The quasi-periodic Green's function of the host domain split into a few
+// lattice images and a smooth rest (bem_smooth.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include "bem_kernels.h"
+
+#define BEM_SM_MAXL 40     // largest degree of the expansion about the body's centre
+#define BEM_SM_MAXIMG 40   // most lattice images taken out
+#define BEM_SM_BAT 8       // instances per launch
+
+// The split of one body and lattice: which images are taken out, and the
+// degrees that represent the rest to FP64 round-off.  Host data; tab is what
+// the device needs of it.
+struct bem_smooth {
+  int on = 0;
+  int lmax = 0, Lmax = 0, K = 0, Kp = 0, nt = 0, nphi = 0, nimg = 0;
+  double ctr[3] = {0, 0, 0}, R0 = 0.0, rho = 0.0, k = 0.0;
+  int l1[BEM_SM_MAXIMG], l2[BEM_SM_MAXIMG];  // the images' lattice indices, (0, 0) first
+  int inst = 1, first = 0;      // instances tab holds; the one a launch for a single instance takes
+  const double *tab = nullptr;  // device copy of the tables bem_smooth_tables writes
+  double *ws = nullptr;         // device workspace of bem_smooth_ws_doubles(...) doubles
+};
+// offsets (doubles) in tab
+struct bem_smooth_tab {
+  int x, w, ca, cb, dL, el, rec, img, total;
+};
+
+// Choose the images and degrees for the elements (cr, npe; ids sid[0 .. ne))
+// of the periodic domain; S.on = 0 where the split does not pay (a body much
+// taller or wider than the lattice period).
+void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int *npe, const int *sid, int ne);
+bem_smooth_tab bem_smooth_layout(const bem_smooth *S);
+// the tables of S->inst instances (qps: their Bloch wave vectors) into h[layout.total]
+void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h);
+size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
+
+extern "C" {
+// constant tables of this translation unit (quad: bem_quad, wc: bem_wconst)
+int bem_smooth_set_constants(const void *quad, const void *wc);
+// G, H of nb instances of the periodic domain: the smooth rest of every pair
+// (written), then the images of every pair off the lattice plane (added; the
+// home image of near-singular and self pairs is left to their own kernels)
+int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
+                      double *const *H, const bem_scratch *scr, cudaStream_t st);
+}
