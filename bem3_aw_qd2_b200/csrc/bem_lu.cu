@@ -8,19 +8,18 @@
 // The matrix is row-major (the layout the assembly writes), factored in place
 // as P A = L U, right-looking, 32 columns per panel.  Per panel three kernels:
 //
-//  k_lu_panel   one thread-block cluster of 8 CTAs picks the panel's 32 pivot
-//               rows by tournament pivoting (communication-avoiding LU): each
-//               CTA runs partial pivoting on its slice of rows, one row per
-//               thread in registers, and passes its winners on; CTA 0 runs
-//               partial pivoting on the winners, which gives the pivot order
-//               and the packed L11\U11, inverts U11 and L11, and lists the row
-//               moves (at most 64 touched positions).  The matrix is not
-//               written here.
+//  k_lu_panel   picks the panel's 32 pivot rows by tournament pivoting
+//               (communication-avoiding LU): each CTA runs partial pivoting on a
+//               slice of 256 rows, one row per thread in registers; the last of
+//               up to eight CTAs to finish goes on with their winners, and so on
+//               up to the root, which gives the pivot order and the packed
+//               L11\U11, inverts U11 and L11, and lists the row moves (at most 64
+//               touched positions).  The matrix is not written here.
 //  k_lu_apply   all SMs: L21 = A21 U11^-1 for every row below the panel,
 //               the row moves on the columns outside the panel, and
 //               U12 = L11^-1 A12 on the pivot rows.
 //  k_lu_update  all SMs: A22 -= L21 U12 on the FP64 tensor cores
-//               (mma.sync m8n8k4 f64; Blackwell's tcgen05 has no FP64 kind),
+//               (mma.sync m16n8k8 f64; Blackwell's tcgen05 has no FP64 kind),
 //               64 x 64 complex tiles, the complex product as four real ones.
 //
 // The sequence of a size and matrix is captured once as a CUDA graph and
@@ -44,14 +43,11 @@
 #define LU_ONE_BLOCK_N 2048  // default of bem_lu.one_block_max
 static_assert(LU_OB == LU_OUTER_W, "the tensor-core update depth is the outer block");
 #define LU_TH 256        // threads of a panel CTA: one row each
-#define LU_CL 8          // CTAs of the panel cluster
 #define LU_MAXP (2 * LU_W)
 #define FULL 0xffffffffu
 
 // integer scratch (bem_lu.piv)
-#define PV_CAND 0                    // [LU_CL][LU_W] candidate rows of each leaf
-#define PV_CCNT (LU_CL * LU_W)       // [LU_CL] candidates per leaf
-#define PV_SEL (PV_CCNT + LU_CL)     // [LU_W] pivot rows in order
+#define PV_SEL 0                     // [LU_W] pivot rows in order
 #define PV_PERM (PV_SEL + LU_W)      // count, then (dst, src) pairs of the row moves
 #define PV_INTS (PV_PERM + 1 + 2 * LU_MAXP)
 // complex scratch (bem_lu.u11)
@@ -109,270 +105,390 @@ __device__ __forceinline__ float2 crcp(float2 a) {
 __device__ __forceinline__ float cabs1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 
 // ---------------------------------------------------------------- partial pivoting in one CTA
+#define LU_SB 8                // columns of a sub-block
+#define LU_NW (LU_TH / 32)     // warps
 template <class C2>
 struct gepp_sh {
-  unsigned wk[2][LU_TH / 32];  // each warp's pivot key
-  C2 prow[2][LU_W], krow[2][LU_W];
-  C2 prcp[2];                  // reciprocal of the pivot
-  int pid[2], kid[2];
+  uint4 wk[2][LU_NW / 4];      // each warp's pivot key
+  C2 row[2][LU_NW][LU_SB];     // its row's sub-block columns
+  C2 rcp[2][LU_NW];            // the reciprocal of its pivot
+  C2 l8[LU_SB][LU_SB];         // multipliers of the sub-block's pivot rows
+  C2 tr[LU_SB][LU_W - LU_SB];  // their columns right of the sub-block
 };
 
-// Pivot key of a candidate: the float bits of |re| + |im| (non-negative floats
-// order as their bits) with the low 8 bits replaced by 255 - t, so that one
-// integer maximum gives the largest value and, among values equal to 2^-15,
-// the lowest row; 0 for a row that takes no part.
+// Pivot key of a candidate: the high word (FP64) or the word (FP32) of |re| +
+// |im| (non-negative numbers order as their bits) with the low 8 bits replaced
+// by 255 - t, so that one integer maximum gives the largest value and, among
+// values equal to 2^-12 (2^-15), the lowest row: a pivot within that of the
+// largest, which keeps partial pivoting's growth bound.  0 for a row that takes
+// no part.
+__device__ __forceinline__ unsigned pivot_key(double a, int t) {
+  return ((unsigned)__double2hiint(a) & 0xFFFFFF00u) | (unsigned)(255 - t);
+}
 __device__ __forceinline__ unsigned pivot_key(float a, int t) {
   return (__float_as_uint(a) & 0xFFFFFF00u) | (unsigned)(255 - t);
 }
-
-// rotate the first L registers by one: v[0] (the finished pivot column)
-// goes to v[L - 1]
-template <int L, class C2>
-__device__ __forceinline__ void rotl(C2 (&v)[LU_W]) {
-  const C2 f = v[0];
-#pragma unroll
-  for (int c = 0; c < L - 1; ++c) v[c] = v[c + 1];
-  v[L - 1] = f;
+// 1 / a for the elimination steps, without a branch (a division's slow path
+// would keep the compiler from scheduling it beside the updates): a scaled by a
+// power of two to |re| + |im| in [1, 2), so that re^2 + im^2 neither over- nor
+// underflows, and 1 / (re^2 + im^2) from the hardware's approximation by one
+// third-order Newton step r (1 + e + e^2), e = 1 - d r.
+__device__ __forceinline__ double2 pivot_rcp(double2 a) {
+  const int e = (__double2hiint(cabs1(a)) >> 20) & 2047;
+  const double sc = __hiloint2double(max(2046 - e, 1) << 20, 0);
+  const double x = a.x * sc, y = a.y * sc, d = fma(x, x, y * y);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double q = fma(-d, r, 1.0);
+  r = fma(r, fma(q, q, q), r) * sc;
+  return make_double2(x * r, -y * r);
 }
-
-// One elimination step j of gepp: v[0] holds column j and v[1 .. 31 - j] the
-// columns still to update; L >= 32 - j is the step's compile-time bound, so
-// that the update and the rotation touch only the live window (the finished
-// columns beyond it stay where they are).
-template <int L, class C2>
-__device__ __forceinline__ void gepp_step(C2 (&v)[LU_W], int &id, int j, int steps, int rr, gepp_sh<C2> &sh,
-                                          unsigned *status) {
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  if (j < steps) {
-    const int b = j & 1;
-    // the pivot: one integer maximum per warp, then over the warps (the
-    // 2^-15 resolution of the key only picks among rows within that much of
-    // the largest, which keeps partial pivoting's growth bound)
-    const unsigned key = __reduce_max_sync(FULL, (t >= j && t < rr) ? pivot_key((float)cabs1(v[0]), t) : 0u);
-    if (lane == 0) sh.wk[b][wid] = key;
-    __syncthreads();
-    unsigned best = sh.wk[b][0];
-#pragma unroll
-    for (int q = 1; q < LU_TH / 32; ++q) best = max(best, sh.wk[b][q]);
-    int p = 255 - (int)(best & 255u);
-    if ((best >> 8) == 0u) {  // no non-zero entry left in the column
-      if (status && t == 0) atomicOr(status, BEM_LU_ST_ZERO);
-      p = j;
-    }
-    if (t == p) {
-#pragma unroll
-      for (int c = 0; c < LU_W; ++c) sh.prow[b][c] = v[c];
-      sh.pid[b] = id;
-      sh.prcp[b] = crcp(v[0]);
-    }
-    if (t == j) {
-#pragma unroll
-      for (int c = 0; c < LU_W; ++c) sh.krow[b][c] = v[c];
-      sh.kid[b] = id;
-    }
-    __syncthreads();
-    if (t == j) {
-#pragma unroll
-      for (int c = 0; c < LU_W; ++c) v[c] = sh.prow[b][c];
-      id = sh.pid[b];
-    } else if (t == p) {
-#pragma unroll
-      for (int c = 0; c < LU_W; ++c) v[c] = sh.krow[b][c];
-      id = sh.kid[b];
-    }
-    if (t > j && t < rr) {
-      const C2 l = cmul(v[0], sh.prcp[b]);
-      v[0] = l;
-#pragma unroll
-      for (int c = 1; c < L; ++c)
-        if (c < LU_W - j) v[c] = cfms(l, sh.prow[b][c], v[c]);
-    }
-  }
-  rotl<L>(v);
+__device__ __forceinline__ float2 pivot_rcp(float2 a) {
+  const int e = (__float_as_int(cabs1(a)) >> 23) & 255;
+  const float sc = __int_as_float(max(254 - e, 1) << 23);
+  const float x = a.x * sc, y = a.y * sc, d = fmaf(x, x, y * y);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  r = fmaf(r, fmaf(-d, r, 1.0f), r) * sc;
+  return make_float2(x * r, -y * r);
 }
+// a pivot that counts as zero: below 2^-141, an FP32 number's smallest 255 steps
+template <class R> __device__ __forceinline__ bool zero_pivot(R a) { return (__float_as_uint((float)a) >> 8) == 0u; }
 
 // Partial pivoting (|re| + |im| as LAPACK's izamax, lowest row on ties) over
-// the rr <= LU_TH rows held one per thread (thread t < rr: values v, matrix
-// row id), w columns.  Afterwards thread i < min(w, rr) holds the i-th pivot
-// row and its id, its values packed (multipliers left of column i, U from i
-// on), columns in order.  A row is kept rotated while it is eliminated: at
-// step j its register 0 holds column j, registers 1 .. 31 - j the columns
-// still to update and the rest the finished ones, so that every register
-// index is a compile-time constant inside one short loop body.
+// the rr <= LU_TH rows held one per thread (thread t < rr: values v), w
+// columns.  Rows stay with their threads: ord becomes the row's place in the
+// pivot order (-1: not picked), and a picked row's v its packed row
+// (multipliers left of the pivot, U from it on).  With rd: the pivots'
+// reciprocals, and a zero pivot reported in status.
 //
-// The steps run in four groups of eight with a shrinking live window of 32,
-// 24, 16 and 8 registers: each group's finished columns end up in the eight
-// registers just past the next group's window (group g's at 24 - 8 g ..
-// 31 - 8 g), which a fixed permutation puts back in order at the end.
+// Latency decides here (32 dependent steps, one CTA), so the columns go in
+// sub-blocks of eight: a step publishes each warp's best row, takes one barrier
+// and updates at most seven columns; the columns right of the sub-block are
+// updated by all eight pivots at once.  A step takes about 450 cycles; one that
+// publishes and updates all 32 columns behind two barriers takes 1900 (panel of
+// n = 1728: 67 -> 40 us, of which the FP64 root 24).  The sub-block is kept
+// in v[0 .. 7] by rotating the registers, so that one short body serves all four.
 template <class C2>
-__device__ void gepp(C2 (&v)[LU_W], int &id, int rr, int w, gepp_sh<C2> &sh, unsigned *status) {
+__device__ void gepp(C2 (&v)[LU_W], int &ord, int rr, int w, gepp_sh<C2> &sh, unsigned *status, C2 *rd) {
+  const int t = threadIdx.x, wid = t >> 5;
   const int steps = min(w, rr);
-  for (int j = 0; j < 8; ++j) gepp_step<32>(v, id, j, steps, rr, sh, status);
-  for (int j = 8; j < 16; ++j) gepp_step<24>(v, id, j, steps, rr, sh, status);
-  for (int j = 16; j < 24; ++j) gepp_step<16>(v, id, j, steps, rr, sh, status);
-  for (int j = 24; j < 32; ++j) gepp_step<8>(v, id, j, steps, rr, sh, status);
-  // registers 24 - 8 g .. 31 - 8 g hold columns 8 g .. 8 g + 7
-  C2 o[LU_W];
+  bool act = t < rr;
+  C2 piv = cone<C2>();  // the pivot of a picked row
+  ord = -1;
+#pragma unroll 1
+  for (int sb = 0; sb < LU_W / LU_SB; ++sb) {
+    const int j0 = sb * LU_SB, cnt = min(LU_SB, steps - j0);  // pivots of this sub-block
 #pragma unroll
-  for (int g = 0; g < 4; ++g)
+    for (int jj = 0; jj < LU_SB; ++jj) {
+      if (jj >= cnt) continue;
+      const int b = jj & 1;
+      const unsigned key = act ? pivot_key(cabs1(v[jj]), t) : 0u;
+      const unsigned wmax = __reduce_max_sync(FULL, key);
+      const C2 rc = pivot_rcp(v[jj]);  // by every row, beside the search
+      if (act && key == wmax) {  // this warp's best row (keys of active rows are distinct)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[8 * g + i] = v[24 - 8 * g + i];
+        for (int c = jj; c < LU_SB; ++c) sh.row[b][wid][c] = v[c];
+        sh.rcp[b][wid] = rc;
+        reinterpret_cast<unsigned *>(sh.wk[b])[wid] = wmax;
+      }
+      if (wmax == 0u && (t & 31) == 0) reinterpret_cast<unsigned *>(sh.wk[b])[wid] = 0u;
+      __syncthreads();
+      const uint4 ka = sh.wk[b][0], kb = sh.wk[b][1];
+      const unsigned best = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kb.x, kb.y), max(kb.z, kb.w)));
+      const int p = 255 - (int)(best & 255u), pw = p >> 5;
+      // no branch from here to the next barrier: every warp waits for the
+      // slowest, and the pivot's warp would pay for both sides
+      ord = t == p ? j0 + jj : ord;
+      piv = t == p ? v[jj] : piv;
+      act = act && t != p;
+      C2 l = cmul(v[jj], sh.rcp[b][pw]);
+      v[jj] = act ? l : v[jj];
+      l = act ? l : czero<C2>();
 #pragma unroll
-  for (int c = 0; c < LU_W; ++c) v[c] = o[c];
-}
-
-template <class C2>
-__device__ __forceinline__ void load_row(C2 (&v)[LU_W], const C2 *A, long lda, int row, int k, int w) {
-  const C2 *p = A + (size_t)(row < 0 ? 0 : row) * lda + k;
+      for (int c = jj + 1; c < LU_SB; ++c) v[c] = cfms(l, sh.row[b][pw][c], v[c]);
+    }
+    if (sb < LU_W / LU_SB - 1 && cnt > 0) {
+      // the columns right of the sub-block: U there from the pivot rows
+      // (unit lower solve, a thread per column), then every other row
+      const int nrem = LU_W - LU_SB - j0;
+      const int i = ord - j0;
+      if (i >= 0) {
 #pragma unroll
-  for (int c = 0; c < LU_W; ++c) v[c] = (row >= 0 && c < w) ? p[c] : czero<C2>();
-}
-
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// all threads of all CTAs of the cluster; orders global-memory writes before it
-// with reads after it (release / acquire at cluster scope)
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (int c = 0; c < LU_SB; ++c) sh.l8[i][c] = v[c];
+#pragma unroll
+        for (int c = 0; c < LU_W - LU_SB; ++c)
+          if (c < nrem) sh.tr[i][c] = v[LU_SB + c];
+      }
+      __syncthreads();
+      if (t < nrem) {
+        C2 x[LU_SB];
+#pragma unroll
+        for (int r = 0; r < LU_SB; ++r) x[r] = r < cnt ? sh.tr[r][t] : czero<C2>();
+#pragma unroll
+        for (int r = 1; r < LU_SB; ++r)
+          if (r < cnt)
+#pragma unroll
+            for (int c = 0; c < r; ++c) x[r] = cfms(sh.l8[r][c], x[c], x[r]);
+#pragma unroll
+        for (int r = 0; r < LU_SB; ++r)
+          if (r < cnt) sh.tr[r][t] = x[r];
+      }
+      __syncthreads();
+      if (i >= 0) {
+#pragma unroll
+        for (int c = 0; c < LU_W - LU_SB; ++c)
+          if (c < nrem) v[LU_SB + c] = sh.tr[i][c];
+      } else if (act) {
+#pragma unroll
+        for (int ch = 0; ch < LU_W / LU_SB - 1; ++ch)
+          if (ch * LU_SB < nrem)
+#pragma unroll
+            for (int r = 0; r < LU_SB; ++r)
+              if (r < cnt)
+#pragma unroll
+                for (int c = 0; c < LU_SB; ++c)
+                  v[LU_SB + ch * LU_SB + c] = cfms(v[r], sh.tr[r][ch * LU_SB + c], v[LU_SB + ch * LU_SB + c]);
+      }
+    }
+    // rotate: the finished sub-block goes behind the others
+    C2 f[LU_SB];
+#pragma unroll
+    for (int c = 0; c < LU_SB; ++c) f[c] = v[c];
+#pragma unroll
+    for (int c = 0; c < LU_W - LU_SB; ++c) v[c] = v[c + LU_SB];
+#pragma unroll
+    for (int c = 0; c < LU_SB; ++c) v[LU_W - LU_SB + c] = f[c];
+  }
+  if (rd && ord >= 0) {
+    rd[ord] = crcp(piv);
+    if (zero_pivot(cabs1(piv))) atomicOr(status, BEM_LU_ST_ZERO);  // no non-zero entry was left
+  }
+  __syncthreads();  // the shared buffers may be used again
 }
 
 // ---------------------------------------------------------------- panel
-// the leaves' partial pivoting only selects candidate rows (the root factors
-// the winners from their stored values), so it runs in complex FP32 for
-// either precision of the factorisation
-template <class C2> struct leaf_of { using T = float2; };
-
-__device__ __forceinline__ void load_row_leaf(float2 (&v)[LU_W], const double2 *A, long lda, int row, int k, int w) {
-  const double2 *p = A + (size_t)(row < 0 ? 0 : row) * lda + k;
+// The panel's columns of one row per thread (id: the row, -1 none) into
+// registers, converted to T (the leaves' partial pivoting only selects rows, so
+// it runs in complex FP32 for either precision of the factorisation).  A warp
+// reads four rows' eight columns at a time, whole 128-byte lines, and turns
+// them through stage (32 x 9 of T per warp) so that each lane gets its own row;
+// read row by row the loads take 8000 cycles of the SM's load path, this 1000.
+__device__ __forceinline__ void cvt(double2 x, double2 &y) { y = x; }
+__device__ __forceinline__ void cvt(double2 x, float2 &y) { y = make_float2((float)x.x, (float)x.y); }
+__device__ __forceinline__ void cvt(float2 x, float2 &y) { y = x; }
+template <class T, class C2>
+__device__ __forceinline__ void load_rows(T (&v)[LU_W], const C2 *A, long lda, int id, int k, int w, T *stage) {
+  const int lane = threadIdx.x & 31, sub = lane >> 3, col = lane & 7;
+  T *s = stage + (threadIdx.x >> 5) * (32 * 9);
 #pragma unroll
-  for (int c = 0; c < LU_W; ++c) {
-    const double2 x = (row >= 0 && c < w) ? p[c] : make_double2(0.0, 0.0);
-    v[c] = make_float2((float)x.x, (float)x.y);
+  for (int i = 0; i < 8; ++i) {
+    const int row = __shfl_sync(FULL, id, i * 4 + sub);
+    const C2 *p = A + (size_t)(row < 0 ? 0 : row) * lda + k;
+#pragma unroll
+    for (int c = 0; c < LU_W / 8; ++c) {
+      const C2 x = (row >= 0 && c * 8 + col < w) ? p[c * 8 + col] : czero<C2>();
+      cvt(x, v[c * 8 + i]);
+    }
   }
-}
-__device__ __forceinline__ void load_row_leaf(float2 (&v)[LU_W], const float2 *A, long lda, int row, int k, int w) {
-  load_row(v, A, lda, row, k, w);
+#pragma unroll
+  for (int c = 0; c < LU_W / 8; ++c) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[(i * 4 + sub) * 9 + col] = v[c * 8 + i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[c * 8 + i] = s[lane * 9 + i];
+  }
 }
 
 template <class C2>
 struct panel_sh {
   gepp_sh<C2> g;
   gepp_sh<float2> gl;
-  C2 lu[LU_W][LU_W + 1];
-  C2 rd[LU_W];  // reciprocals of U11's diagonal
+  union {
+    struct {
+      C2 lu[LU_W][LU_W + 1];
+      C2 iv[2][LU_W][LU_W + 1];  // U11^-1, L11^-1
+    };
+    C2 stage[LU_NW * 32 * 9];    // load_rows
+  };
+  C2 rd[LU_W];                   // reciprocals of U11's diagonal
   int sel[LU_W], la[LU_W], lb[LU_W];
+  int last;
 };
 
+// X = T^-1 of the two triangles of lu (b = 0: U, b = 1: unit L), by inverting
+// the 8 x 8 diagonal blocks (a warp each) and doubling the block size twice:
+// the off-diagonal block of the inverse is -T22^-1 T21 T11^-1 (L), -T11^-1 T12
+// T22^-1 (U).  All threads; lu complete before, iv complete after.
 template <class C2>
-__global__ void __cluster_dims__(LU_CL, 1, 1) __launch_bounds__(LU_TH, 1)
-    k_lu_panel(C2 *A, long lda, int n, int k, int *pv, C2 *u, unsigned *status) {
+__device__ void tri_inverses(panel_sh<C2> &S, int w) {
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  for (int e = t; e < 2 * LU_W * (LU_W + 1); e += LU_TH) (&S.iv[0][0][0])[e] = czero<C2>();
+  __syncthreads();
+  {
+    const int up = wid < 4, d = (wid & 3) * 8;  // this warp's diagonal block, a lane per column
+    if (lane < 8) {
+      C2 x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = (i == lane) ? cone<C2>() : czero<C2>();
+      if (up) {
+#pragma unroll
+        for (int l = 7; l >= 0; --l) {
+          // an identity beyond a short panel keeps the block regular
+          const C2 dg = d + l < w ? S.rd[d + l] : cone<C2>();
+          x[l] = cmul(x[l], dg);
+#pragma unroll
+          for (int i = 0; i < l; ++i) x[i] = cfms(S.lu[d + i][d + l], x[l], x[i]);
+        }
+      } else {
+#pragma unroll
+        for (int l = 0; l < 8; ++l)
+#pragma unroll
+          for (int i = l + 1; i < 8; ++i) x[i] = cfms(S.lu[d + i][d + l], x[l], x[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) S.iv[up ? 0 : 1][d + i][d + lane] = x[i];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int bs = 8; bs < LU_W; bs *= 2) {
+    // products of bs x bs blocks: 32 / (2 bs) of them for each triangle
+    const int per = bs * bs, tot = 2 * (LU_W / (2 * bs)) * per;
+    C2 y[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + h * LU_TH;
+      y[h] = czero<C2>();
+      if (e < tot) {
+        const int b = e / (tot / 2), r = e % (tot / 2), blk = r / per, i = r % per / bs, j = r % bs;
+        const int o = blk * 2 * bs, ro = b ? o + bs : o, co = b ? o : o + bs;  // the off-diagonal block
+        // T_off T_(column's diagonal)^-1
+        for (int l = 0; l < bs; ++l) y[h] = cfma(S.lu[ro + i][co + l], S.iv[b][co + l][co + j], y[h]);
+      }
+    }
+    // the strictly other triangle of iv holds the intermediate product
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + h * LU_TH;
+      if (e < tot) {
+        const int b = e / (tot / 2), r = e % (tot / 2), blk = r / per, i = r % per / bs, j = r % bs;
+        const int o = blk * 2 * bs, ro = b ? o + bs : o, co = b ? o : o + bs;
+        S.iv[b][co + i][ro + j] = y[h];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + h * LU_TH;
+      if (e < tot) {
+        const int b = e / (tot / 2), r = e % (tot / 2), blk = r / per, i = r % per / bs, j = r % bs;
+        const int o = blk * 2 * bs, ro = b ? o + bs : o, co = b ? o : o + bs;
+        C2 z = czero<C2>();
+        for (int l = 0; l < bs; ++l) z = cfma(S.iv[b][ro + i][ro + l], S.iv[b][co + l][ro + j], z);
+        y[h] = cneg(z);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = t + h * LU_TH;
+      if (e < tot) {
+        const int b = e / (tot / 2), r = e % (tot / 2), blk = r / per, i = r % per / bs, j = r % bs;
+        const int o = blk * 2 * bs, ro = b ? o + bs : o, co = b ? o : o + bs;
+        S.iv[b][ro + i][co + j] = y[h];
+        S.iv[b][co + i][ro + j] = czero<C2>();
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Tournament over ceil(m / LU_TH) leaves: block b eliminates its slice of the
+// panel's rows and leaves its winners; the block that finishes last of up to
+// eight goes on with their winners, and so on up to the root (no block waits
+// for another).  tree: winners [node][1 + LU_W] (count, rows), then a counter
+// per node, zero between launches.
+template <class C2>
+__global__ void __launch_bounds__(LU_TH, 1)
+    k_lu_panel(C2 *A, long lda, int n, int k, int *pv, int *tree, int max_nodes, C2 *u, unsigned *status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   panel_sh<C2> &S = *reinterpret_cast<panel_sh<C2> *>(smem_raw);
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  const int crank = (int)cluster_rank();
   const int w = min(LU_W, n - k), m = n - k;
-  int id = -1;
-  if (m > LU_TH) {
-    // leaves: each CTA a contiguous slice of the panel's rows, in rounds of
-    // LU_TH rows: the winners of a round stay, fresh rows fill the other slots
-    const int q = (m + LU_CL - 1) / LU_CL;
-    const int lo = k + crank * q, hi = min(n, lo + q);
-    int ncand = 0, next = lo;
-    while (next < hi) {
-      const int fresh = min(LU_TH - ncand, hi - next);
-      int row = -1;
-      if (t < ncand) row = id;
-      else if (t < ncand + fresh) row = next + (t - ncand);
-      next += fresh;
-      id = row;
+  int id = -1, rr = m, ord = -1;
+  if (gridDim.x > 1) {
+    int *counter = tree + (size_t)max_nodes * (1 + LU_W);
+    int nn = gridDim.x, node = blockIdx.x, base = 0;  // nodes of this level, this one, the level's first
+    {
+      const int q = (m + nn - 1) / nn, lo = k + node * q, hi = min(n, lo + q);
+      rr = max(0, hi - lo);
+      id = t < rr ? lo + t : -1;
+    }
+    while (true) {
       float2 vl[LU_W];
-      load_row_leaf(vl, A, lda, row, k, w);
-      const int rr = ncand + fresh;
-      gepp(vl, id, rr, w, S.gl, nullptr);
-      ncand = min(w, rr);
+      load_rows(vl, A, lda, id, k, w, reinterpret_cast<float2 *>(S.stage));
+      gepp(vl, ord, rr, w, S.gl, nullptr, (float2 *)nullptr);
+      int *win = tree + (size_t)(base + node) * (1 + LU_W);
+      if (ord >= 0) win[1 + ord] = id;
+      if (t == 0) win[0] = min(w, rr);
+      __threadfence();
       __syncthreads();
+      const int parents = (nn + 7) / 8, par = node / 8;
+      if (t == 0) {
+        const int kids = min(8, nn - par * 8);
+        S.last = atomicAdd(counter + base + nn + par, 1) == kids - 1;
+        if (S.last) counter[base + nn + par] = 0;
+      }
+      __syncthreads();
+      if (!S.last) return;
+      __threadfence();
+      // this block goes on as the parent: its children's winners, one per thread
+      int total = 0, mine = -1;
+      for (int c = par * 8; c < min(nn, par * 8 + 8); ++c) {
+        const int *wc = tree + (size_t)(base + c) * (1 + LU_W);
+        const int cnt = __ldcg(wc);
+        if (t >= total && t < total + cnt) mine = __ldcg(wc + 1 + (t - total));
+        total += cnt;
+      }
+      base += nn;
+      nn = parents;
+      node = par;
+      id = mine;
+      rr = total;
+      if (nn == 1) break;
     }
-    if (t < ncand) pv[PV_CAND + crank * LU_W + t] = id;
-    if (t == 0) pv[PV_CCNT + crank] = ncand;
-    __threadfence();
-  }
-  cluster_sync_all();
-  if (crank != 0) return;
-  // root: partial pivoting over the leaves' winners (or over all rows of a
-  // short panel), with the values kept: the pivot order and L11\U11
-  int rr;
-  if (m > LU_TH) {
-    int total = 0, mine = -1;
-    for (int cc = 0; cc < LU_CL; ++cc) {
-      const int cnt = __ldcg(pv + PV_CCNT + cc);
-      if (t >= total && t < total + cnt) mine = __ldcg(pv + PV_CAND + cc * LU_W + (t - total));
-      total += cnt;
-    }
-    rr = total;
-    id = mine;
   } else {
-    rr = m;
     id = t < m ? k + t : -1;
   }
+  // root: partial pivoting over the last winners (or over all rows of a short
+  // panel), with the values kept: the pivot order and L11\U11
   C2 v[LU_W];
-  load_row(v, A, lda, id, k, w);
-  gepp(v, id, rr, w, S.g, status);
+  load_rows(v, A, lda, id, k, w, S.stage);
+  gepp(v, ord, rr, w, S.g, status, S.rd);
   if (t < LU_W) {
+    S.sel[t] = -1;
+    if (t >= w)
 #pragma unroll
-    for (int c = 0; c < LU_W; ++c) {
-      const C2 x = (t < w) ? v[c] : czero<C2>();
-      S.lu[t][c] = x;
-      u[U_LU + t * LU_W + c] = x;
-    }
-    S.sel[t] = t < w ? id : -1;
-    if (t < w) pv[PV_SEL + t] = id;
+      for (int c = 0; c < LU_W; ++c) S.lu[t][c] = czero<C2>();
   }
-  if (t < LU_W) S.rd[t] = t < w ? crcp(S.lu[t][t]) : czero<C2>();
   __syncthreads();
-  // U11^-1 (warps 0-3) and L11^-1 (warps 4-7), 8 columns a warp, 4 at a
-  // time, column-oriented substitution with lane = row: at step l lane l
-  // finishes x_l, a shuffle hands it to the other lanes, and each lane
-  // removes its u_il x_l (l_il x_l): one short dependent step per row, all
-  // rows of four columns at once
-  {
-    const int i = lane;
-    const bool upper = wid < 4;
-    const int jb = (wid & 3) * 8;
-    for (int half = 0; half < 2; ++half) {
-      C2 x[4];
+  if (ord >= 0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = (i == jb + half * 4 + q && i < w) ? cone<C2>() : czero<C2>();
-      if (upper) {
-        for (int l = LU_W - 1; l >= 0; --l) {
-          const C2 a = S.lu[i][l], d = S.rd[l];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (i == l) x[q] = cmul(x[q], d);
-            const C2 xl = cx<C2>::mk(__shfl_sync(FULL, x[q].x, l), __shfl_sync(FULL, x[q].y, l));
-            if (i < l) x[q] = cfms(a, xl, x[q]);
-          }
-        }
-      } else {
-        for (int l = 0; l < LU_W; ++l) {
-          const C2 a = S.lu[i][l];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const C2 xl = cx<C2>::mk(__shfl_sync(FULL, x[q].x, l), __shfl_sync(FULL, x[q].y, l));
-            if (i > l) x[q] = cfms(a, xl, x[q]);
-          }
-        }
-      }
-      C2 *dst = upper ? u + U_UINV : u + U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = jb + half * 4 + q;
-        // entries outside a short panel (w < 32) are zero
-        dst[i * LU_W + j] = (i < w && j < w) ? x[q] : czero<C2>();
-      }
-    }
+    for (int c = 0; c < LU_W; ++c) S.lu[ord][c] = v[c];
+    S.sel[ord] = id;
+    pv[PV_SEL + ord] = id;
+  }
+  __syncthreads();
+  tri_inverses(S, w);
+  for (int e = t; e < LU_W * LU_W; e += LU_TH) {
+    const int i = e / LU_W, j = e % LU_W;
+    const bool in = i < w && j < w;  // entries outside a short panel (w < 32) are zero
+    u[U_LU + e] = S.lu[i][j];
+    u[U_UINV + e] = in ? S.iv[0][i][j] : czero<C2>();
+    u[U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W) + e] = in ? S.iv[1][i][j] : czero<C2>();
   }
   if (wid == 2) {
     // row moves: pivot row i goes to position k + i; the rows of the pivot
@@ -410,31 +526,48 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
                                                     int *rowmap, unsigned *status) {
   __shared__ C2 sm[LU_W][LU_W + 1];
   __shared__ C2 srow[LU_MAXP][AP_COLS + 1];
-  __shared__ int sdst[LU_MAXP], ssrc[LU_MAXP];
+  __shared__ int sdst[LU_MAXP], ssrc[LU_MAXP], moved[AP_ROWS];
   const int t = threadIdx.x;
   const int w = min(LU_W, n - k);
   const int r0 = k + w;
+  const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
+  const int nCl = (k + AP_COLS - 1) / AP_COLS, nCr = (n - r0 + AP_COLS - 1) / AP_COLS;
+  const int b = blockIdx.x;
+  // everything read through the row list or needed beside it is loaded at
+  // once: the kernel is a chain of latencies, not of work
   int nperm = __ldcg(pv + PV_PERM);
+  int md = k, ms = k;
+  if (t < LU_MAXP) {
+    md = __ldcg(pv + PV_PERM + 1 + 2 * t);
+    ms = __ldcg(pv + PV_PERM + 2 + 2 * t);
+  }
+  const int ci = b - nL;  // column block
+  const bool right = ci >= nCl;
+  const int c0 = right ? r0 + (ci - nCl) * AP_COLS : ci * AP_COLS;
+  const bool u12 = b >= nL && right && c0 < cend;
+  if (b < nL || b >= nL + nCl + nCr || u12) {
+    const C2 *src = u + (u12 ? U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W) : U_UINV);
+#pragma unroll
+    for (int e = t; e < LU_W * LU_W; e += AP_TH) sm[e / LU_W][e % LU_W] = __ldcg(src + e);
+  }
+  if (t < AP_ROWS) moved[t] = 0;
   if (nperm < 0 || nperm > LU_MAXP) {
     if (t == 0) atomicOr(status, BEM_LU_ST_INTERNAL);
     nperm = 0;
   }
-  for (int e = t; e < nperm; e += AP_TH) {
-    int d = __ldcg(pv + PV_PERM + 1 + 2 * e), sr = __ldcg(pv + PV_PERM + 2 + 2 * e);
-    if (d < k || d >= n || sr < k || sr >= n) {  // a row move out of range: report, keep the row
-      if (blockIdx.x == 0) atomicOr(status, BEM_LU_ST_INTERNAL);
-      d = sr = k + (e < w ? e : 0);
+  if (t < nperm) {
+    if (md < k || md >= n || ms < k || ms >= n) {  // a row move out of range: report, keep the row
+      if (b == 0) atomicOr(status, BEM_LU_ST_INTERNAL);
+      md = ms = k + (t < w ? t : 0);
     }
-    sdst[e] = d;
-    ssrc[e] = sr;
+    sdst[t] = md;
+    ssrc[t] = ms;
   }
-  const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
-  const int nCl = (k + AP_COLS - 1) / AP_COLS, nCr = (n - r0 + AP_COLS - 1) / AP_COLS;
-  const int b = blockIdx.x;
   if (b < nL) {
+    // (a launch at n = 1728: 12 us with strided U11^-1 columns per thread and
+    // the loads one after another, 5 us)
     // L21 = A21 U11^-1 in place, for the rows below the pivot block that no move touches
-    for (int e = t; e < LU_W * LU_W; e += AP_TH) sm[e / LU_W][e % LU_W] = __ldcg(u + U_UINV + e);
-    const int row = r0 + b * AP_ROWS + (t >> 2), part = t & 3;
+    const int rb = r0 + b * AP_ROWS, row = rb + (t >> 2), part = t & 3;
     // the row's panel values, loaded at once (independent loads, not a chain)
     C2 a[LU_W];
     {
@@ -443,64 +576,62 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
       for (int l = 0; l < LU_W; ++l) a[l] = (row < n && l < w) ? ap[l] : czero<C2>();
     }
     __syncthreads();
-    bool live = row < n;
-    for (int e = w; e < nperm && live; ++e) live = sdst[e] != row;
+    if (t >= w && t < nperm && md >= rb && md < rb + AP_ROWS) moved[md - rb] = 1;
     C2 x[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) x[c] = czero<C2>();
 #pragma unroll
     for (int l = 0; l < LU_W; ++l)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) x[c] = cfma(a[l], sm[l][part * 8 + c], x[c]);
+      for (int c = 0; c < 8; ++c) x[c] = cfma(a[l], sm[l][part + 4 * c], x[c]);  // four neighbours: no bank conflict
     __syncthreads();  // every read of the row before any write to it
-    if (live) {
+    if (row < n && !moved[t >> 2]) {
       C2 *ap = A + (size_t)row * lda + k;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (part * 8 + c < w) ap[part * 8 + c] = x[c];
+        if (part + 4 * c < w) ap[part + 4 * c] = x[c];
     }
     return;
   }
+  __syncthreads();  // sdst / ssrc, sm
   if (b < nL + nCl + nCr) {
     // the row moves on AP_COLS columns outside the panel; right of the panel
     // and left of cend (the end of the outer block) also U12 = L11^-1 A12 on
     // the pivot block; right of cend the moves alone (U12 there is formed for
     // the whole outer block at once, k_lu_trsm)
-    const int i = b - nL;
-    const bool right = i >= nCl;
-    const int c0 = right ? r0 + (i - nCl) * AP_COLS : i * AP_COLS;
-    const int c1 = min(right ? n : k, c0 + AP_COLS);
-    const int nc = c1 - c0;
-    const bool u12 = right && c0 < cend;
-    if (u12) {
-      const C2 *linv = u + U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W);
-      for (int e = t; e < LU_W * LU_W; e += AP_TH) sm[e / LU_W][e % LU_W] = __ldcg(linv + e);
-    }
-    __syncthreads();  // sdst / ssrc
-    for (int e = t; e < nperm * AP_COLS; e += AP_TH) {
-      const int pr = e / AP_COLS, cc = e % AP_COLS;
-      srow[pr][cc] = cc < nc ? A[(size_t)ssrc[pr] * lda + c0 + cc] : czero<C2>();
+    const int nc = min(right ? n : k, c0 + AP_COLS) - c0;
+    const int cc = t % AP_COLS, grp = t / AP_COLS;  // 8 groups of 16 columns
+#pragma unroll
+    for (int q = 0; q < LU_MAXP * AP_COLS / AP_TH; ++q) {
+      const int pr = grp + q * (AP_TH / AP_COLS);
+      srow[pr][cc] = (pr < nperm && cc < nc) ? A[(size_t)ssrc[pr] * lda + c0 + cc] : czero<C2>();
     }
     __syncthreads();
-    const int cc = t % AP_COLS, grp = t / AP_COLS;  // 8 groups of 16 columns
-    if (cc < nc) {
-      if (u12) {
-        for (int ii = grp; ii < w; ii += AP_TH / AP_COLS) {
-          C2 s = czero<C2>();
-          for (int l = 0; l <= ii; ++l) s = cfma(sm[ii][l], srow[l][cc], s);
-          A[(size_t)(k + ii) * lda + c0 + cc] = s;
-        }
-        for (int e = w + grp; e < nperm; e += AP_TH / AP_COLS) A[(size_t)sdst[e] * lda + c0 + cc] = srow[e][cc];
-      } else {
-        for (int e = grp; e < nperm; e += AP_TH / AP_COLS) A[(size_t)sdst[e] * lda + c0 + cc] = srow[e][cc];
+    if (cc >= nc) return;
+    if (u12) {
+      // four rows at a time (L11^-1 is zero right of its diagonal)
+      C2 s[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] = czero<C2>();
+#pragma unroll 4
+      for (int l = 0; l < LU_W; ++l) {
+        const C2 x = srow[l][cc];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = cfma(sm[grp + 8 * q][l], x, s[q]);
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (grp + 8 * q < w) A[(size_t)(k + grp + 8 * q) * lda + c0 + cc] = s[q];
+    }
+#pragma unroll
+    for (int q = 0; q < LU_MAXP * AP_COLS / AP_TH; ++q) {
+      const int e = grp + q * (AP_TH / AP_COLS);
+      if (e < nperm && !(u12 && e < w)) A[(size_t)sdst[e] * lda + c0 + cc] = srow[e][cc];
     }
     return;
   }
   // last block: the panel columns of the moved rows (the pivot block gets
   // L11\U11, a row moved below it its L21), and the row map
-  for (int e = t; e < LU_W * LU_W; e += AP_TH) sm[e / LU_W][e % LU_W] = __ldcg(u + U_UINV + e);
-  __syncthreads();
   for (int e = t; e < w * LU_W; e += AP_TH) {
     const int ii = e / LU_W, c = e % LU_W;
     if (c < w) A[(size_t)(k + ii) * lda + k + c] = __ldcg(u + U_LU + ii * LU_W + c);
@@ -517,11 +648,11 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
 #pragma unroll
       for (int l = 0; l < LU_W; ++l)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) x[c] = cfma(a[l], sm[l][part * 8 + c], x[c]);
+        for (int c = 0; c < 8; ++c) x[c] = cfma(a[l], sm[l][part + 4 * c], x[c]);
       C2 *ap = A + (size_t)sdst[e] * lda + k;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (part * 8 + c < w) ap[part * 8 + c] = x[c];
+        if (part + 4 * c < w) ap[part + 4 * c] = x[c];
     }
   }
   int old = 0;
@@ -534,92 +665,210 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
 #define UP_BM 64
 #define UP_BN 64
 #define UP_TH 256
-#define UP_LDA 36   // shared-memory row strides (doubles) of the L21 and U12 tiles:
-#define UP_LDB 68   // conflict-free fragment loads
-#define UP_SMEM ((2 * UP_BM * UP_LDA + 2 * LU_W * UP_LDB) * sizeof(double))
+#define UP_BK 16    // depth of a slice
+#define UP_NST 3    // slices in flight
+#define UP_LDA 20   // row strides (complex) of the slices: a quarter warp's 16-byte
+#define UP_LDB 66   // fragment loads fall into distinct banks
+#define UP_STAGE (UP_BM * UP_LDA + UP_BK * UP_LDB)
+#define UP_SMEM (UP_NST * UP_STAGE * sizeof(double2))
 
-// d = a b + d on an 8 x 8 x 4 FP64 tile: a (8 x 4, row) holds a[g][q], b (4 x 8,
-// col) b[q][g], d (8 x 8) d[g][2 q .. 2 q + 1], with g = lane / 4, q = lane % 4
-__device__ __forceinline__ void dmma(double a, double b, double (&d)[2]) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
+// d = a b + d on a 16 x 8 x 8 FP64 tile, g = lane / 4, q = lane % 4: a holds
+// rows g (a[0], a[2]) and g + 8 (a[1], a[3]) at columns q and q + 4, b column g
+// at rows q and q + 4, d rows g and g + 8 at columns 2 q and 2 q + 1
+__device__ __forceinline__ void dmma(const double (&a)[4], double b0, double b1, double (&d)[4]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+// 16 bytes from global to shared memory, asynchronously; zeros when not live
+__device__ __forceinline__ void cp16(double2 *dst, const double2 *src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(live ? 16 : 0)
+               : "memory");
 }
 
 // C -= L U on the FP64 tensor cores: C = A[r0:n, c0:cend), L = A[r0:n, kk:kk+kw),
-// U = A[kk:kk+kw, c0:cend); kw in steps of LU_W staged through shared memory.
-// A panel's update (kk = k, kw = 32, cend = the end of its outer block) and an
-// outer block's (kk = its first column, kw = LU_OB, cend = n) alike.
+// U = A[kk:kk+kw, c0:cend), kw a multiple of 16.  A panel's update (kk = k, kw =
+// 32, cend = the end of its outer block) and an outer block's (kk = its first
+// column, kw = LU_OB, cend = n) alike.  64 x 64 complex tiles, 8 warps of 32 x
+// 16, the complex product as four real ones; L and U pass through a 3-slice ring
+// of shared memory filled by asynchronous copies, so that the tensor pipe does
+// not wait for loads (2 blocks per SM, 112 KB each).
 __global__ void __launch_bounds__(UP_TH, 2) k_lu_update(double2 *A, long lda, int n, int kk, int kw, int r0,
                                                         int c0, int cend) {
-  extern __shared__ __align__(16) double up_smem[];
-  double *Ar = up_smem, *Ai = Ar + UP_BM * UP_LDA, *Br = Ai + UP_BM * UP_LDA, *Bi = Br + LU_W * UP_LDB;
+  extern __shared__ __align__(16) unsigned char up_raw[];
+  double2 *sm = reinterpret_cast<double2 *>(up_raw);
   const int t = threadIdx.x;
   const int rb = r0 + blockIdx.y * UP_BM, cb = c0 + blockIdx.x * UP_BN;
   const int lane = t & 31, wid = t >> 5, g = lane >> 2, q = lane & 3;
-  const int wm = wid & 1, wn = wid >> 1;  // warp tile: 32 rows x 16 columns
-  double cr[4][2][2], ci[4][2][2];
+  const int wm = (wid & 1) * 32, wn = (wid >> 1) * 16;  // warp tile: 32 rows x 16 columns
+  auto fill = [&](int st, int k0) {
+    double2 *As = sm + st * UP_STAGE, *Bs = As + UP_BM * UP_LDA;
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+    for (int i = 0; i < UP_BM * UP_BK / UP_TH; ++i) {
+      const int e = t + i * UP_TH, r = e / UP_BK, c = e % UP_BK;
+      const bool live = rb + r < n;
+      cp16(As + r * UP_LDA + c, A + (size_t)(live ? rb + r : r0) * lda + kk + k0 + c, live);
+    }
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const int row = rb + wm * 32 + mt * 8 + g, col = cb + wn * 16 + nt * 8 + 2 * q;
+    for (int i = 0; i < UP_BK * UP_BN / UP_TH; ++i) {
+      const int e = t + i * UP_TH, r = e / UP_BN, c = e % UP_BN;
+      const bool live = cb + c < cend;
+      cp16(Bs + r * UP_LDB + c, A + (size_t)(kk + k0 + r) * lda + (live ? cb + c : c0), live);
+    }
+  };
+  const int nk = kw / UP_BK;
+#pragma unroll
+  for (int s = 0; s < UP_NST - 1; ++s) {
+    if (s < nk) fill(s, s * UP_BK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  double cr[2][2][4], ci[2][2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int row = rb + wm + i * 16 + g + (c >> 1) * 8, col = cb + wn + j * 8 + 2 * q + (c & 1);
+        const double2 x = (row < n && col < cend) ? A[(size_t)row * lda + col] : cz();
+        cr[i][j][c] = x.x;
+        ci[i][j][c] = x.y;
+      }
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(UP_NST - 2) : "memory");
+    __syncthreads();  // slice kt is in, and every warp is done with slice kt - 1
+    if (kt + UP_NST - 1 < nk) fill((kt + UP_NST - 1) % UP_NST, (kt + UP_NST - 1) * UP_BK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const double2 *As = sm + (kt % UP_NST) * UP_STAGE, *Bs = As + UP_BM * UP_LDA;
+#pragma unroll
+    for (int k8 = 0; k8 < UP_BK; k8 += 8) {
+      double2 b[2][2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) b[j][c] = Bs[(k8 + q + 4 * c) * UP_LDB + wn + j * 8 + g];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const double2 x = (row < n && col + i < cend) ? A[(size_t)row * lda + col + i] : cz();
-        cr[mt][nt][i] = x.x;
-        ci[mt][nt][i] = x.y;
-      }
-    }
-  for (int q0 = 0; q0 < kw; q0 += LU_W) {
-    const int wq = min(LU_W, kw - q0), kc = kk + q0;
-    if (q0) __syncthreads();  // the previous chunk's fragment loads are done
-    for (int e = t; e < UP_BM * LU_W; e += UP_TH) {
-      const int r = e / LU_W, c = e % LU_W;
-      const double2 x = (rb + r < n && c < wq) ? A[(size_t)(rb + r) * lda + kc + c] : cz();
-      Ar[r * UP_LDA + c] = x.x;
-      Ai[r * UP_LDA + c] = x.y;
-    }
-    for (int e = t; e < LU_W * UP_BN; e += UP_TH) {
-      const int r = e / UP_BN, c = e % UP_BN;
-      const double2 x = (r < wq && cb + c < cend) ? A[(size_t)(kc + r) * lda + cb + c] : cz();
-      Br[r * UP_LDB + c] = x.x;
-      Bi[r * UP_LDB + c] = x.y;
-    }
-    __syncthreads();
+        // (cr, ci) -= (ar + i ai)(br + i bi)
+        double nr[4], ai[4];
 #pragma unroll
-    for (int k4 = 0; k4 < LU_W; k4 += 4) {
-      double ar[4], ai[4], br[2], bi[2];
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
-        ar[mt] = Ar[(wm * 32 + mt * 8 + g) * UP_LDA + k4 + q];
-        ai[mt] = Ai[(wm * 32 + mt * 8 + g) * UP_LDA + k4 + q];
-      }
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        br[nt] = Br[(k4 + q) * UP_LDB + wn * 16 + nt * 8 + g];
-        bi[nt] = Bi[(k4 + q) * UP_LDB + wn * 16 + nt * 8 + g];
-      }
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          // (cr, ci) -= (ar + i ai)(br + i bi)
-          dmma(-ar[mt], br[nt], cr[mt][nt]);
-          dmma(ai[mt], bi[nt], cr[mt][nt]);
-          dmma(-ar[mt], bi[nt], ci[mt][nt]);
-          dmma(-ai[mt], br[nt], ci[mt][nt]);
+        for (int c = 0; c < 4; ++c) {
+          const double2 a = As[(wm + i * 16 + g + (c & 1) * 8) * UP_LDA + k8 + q + (c >> 1) * 4];
+          nr[c] = -a.x;
+          ai[c] = a.y;
         }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          dmma(nr, b[j][0].x, b[j][1].x, cr[i][j]);
+          dmma(nr, b[j][0].y, b[j][1].y, ci[i][j]);
+          dmma(ai, b[j][0].y, b[j][1].y, cr[i][j]);
+          dmma(ai, -b[j][0].x, -b[j][1].x, ci[i][j]);
+        }
+      }
     }
   }
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const int row = rb + wm * 32 + mt * 8 + g, col = cb + wn * 16 + nt * 8 + 2 * q;
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-        if (row < n && col + i < cend) A[(size_t)row * lda + col + i] = make_double2(cr[mt][nt][i], ci[mt][nt][i]);
+      for (int c = 0; c < 4; ++c) {
+        const int row = rb + wm + i * 16 + g + (c >> 1) * 8, col = cb + wn + j * 8 + 2 * q + (c & 1);
+        if (row < n && col < cend) A[(size_t)row * lda + col] = make_double2(cr[i][j][c], ci[i][j][c]);
+      }
+}
+
+// The same on the next panel's 32 columns alone, which the next panel waits
+// for: kw = 32, 32 x 32 tiles (4 warps of 16 x 16), so that the few tiles of a
+// strip spread over the SMs and none of a tile's columns is empty; everything
+// in one load.  7.5 us with the 64 x 64 tiles at n = 1728.
+#define SP_B 32
+#define SP_TH 128
+#define SP_LDA 36
+#define SP_LDB 34
+__global__ void __launch_bounds__(SP_TH) k_lu_strip(double2 *A, long lda, int n, int kk, int r0, int c0, int cend) {
+  __shared__ __align__(16) double2 As[SP_B * SP_LDA], Bs[SP_B * SP_LDB];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = lane >> 2, q = lane & 3;
+  const int rb = r0 + blockIdx.x * SP_B, wm = (wid & 1) * 16, wn = (wid >> 1) * 16;
+#pragma unroll
+  for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
+    const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
+    const bool la = rb + r < n, lb = c0 + c < cend;
+    cp16(As + r * SP_LDA + c, A + (size_t)(la ? rb + r : r0) * lda + kk + c, la);
+    cp16(Bs + r * SP_LDB + c, A + (size_t)(kk + r) * lda + (lb ? c0 + c : c0), lb);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  double cr[2][4], ci[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int row = rb + wm + g + (c >> 1) * 8, col = c0 + wn + j * 8 + 2 * q + (c & 1);
+      const double2 x = (row < n && col < cend) ? A[(size_t)row * lda + col] : cz();
+      cr[j][c] = x.x;
+      ci[j][c] = x.y;
+    }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int k8 = 0; k8 < SP_B; k8 += 8) {
+    double nr[4], ai[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const double2 a = As[(wm + g + (c & 1) * 8) * SP_LDA + k8 + q + (c >> 1) * 4];
+      nr[c] = -a.x;
+      ai[c] = a.y;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const double2 b0 = Bs[(k8 + q) * SP_LDB + wn + j * 8 + g], b1 = Bs[(k8 + q + 4) * SP_LDB + wn + j * 8 + g];
+      dmma(nr, b0.x, b1.x, cr[j]);
+      dmma(nr, b0.y, b1.y, ci[j]);
+      dmma(ai, b0.y, b1.y, cr[j]);
+      dmma(ai, -b0.x, -b1.x, ci[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int row = rb + wm + g + (c >> 1) * 8, col = c0 + wn + j * 8 + 2 * q + (c & 1);
+      if (row < n && col < cend) A[(size_t)row * lda + col] = make_double2(cr[j][c], ci[j][c]);
+    }
+}
+// complex FP32, on the CUDA cores: two rows and four columns per thread
+__global__ void __launch_bounds__(SP_TH) k_lu_strip_c32(float2 *A, long lda, int n, int kk, int r0, int c0, int cend) {
+  __shared__ float2 As[SP_B][SP_B + 1], Bs[SP_B][SP_B + 1];
+  const int t = threadIdx.x, ty = t >> 3, tx = t & 7;
+  const int rb = r0 + blockIdx.x * SP_B;
+  float2 acc[2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int row = rb + ty + 16 * i, col = c0 + tx + 8 * j;
+      acc[i][j] = (row < n && col < cend) ? A[(size_t)row * lda + col] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+  for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
+    const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
+    As[r][c] = rb + r < n ? A[(size_t)(rb + r) * lda + kk + c] : make_float2(0.f, 0.f);
+    Bs[r][c] = c0 + c < cend ? A[(size_t)(kk + r) * lda + c0 + c] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int l = 0; l < SP_B; ++l)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = cfms(As[ty + 16 * i][l], Bs[l][tx + 8 * j], acc[i][j]);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int row = rb + ty + 16 * i, col = c0 + tx + 8 * j;
+      if (row < n && col < cend) A[(size_t)row * lda + col] = acc[i][j];
     }
 }
 
@@ -779,7 +1028,9 @@ __global__ void __launch_bounds__(256) k_resid_z(const double2 *A, int n, const 
     }
 }
 
-__global__ void k_lu_iota(int *rowmap, int n) {
+// the identity row map, and the tournament's counters at zero
+__global__ void k_lu_iota(int *rowmap, int n, int *counter, int nodes) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nodes; i += gridDim.x * blockDim.x) counter[i] = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rowmap[i] = i;
 }
 
@@ -990,6 +1241,7 @@ extern "C" void bem_lu_free(bem_lu *w) {
   if (w->gexec) cudaGraphExecDestroy(w->gexec);
   if (w->graph) cudaGraphDestroy(w->graph);
   cudaFree(w->rowmap);
+  cudaFree(w->tree);
   cudaFree(w->piv);
   cudaFree(w->u11);
   cudaFree(w->status);
@@ -1021,6 +1273,14 @@ static void launch_update(float2 *A, int n, int kk, int kw, int r0, int c0, int 
   k_lu_update_c32<<<grid, UF_TH, 0, st>>>(A, n, n, kk, kw, r0, c0, cend);
 }
 
+// the same on the next panel's columns [c0, cend), at most 32, with kw = 32
+static void launch_strip(double2 *A, int n, int kk, int r0, int c0, int cend, cudaStream_t st) {
+  k_lu_strip<<<(n - r0 + SP_B - 1) / SP_B, SP_TH, 0, st>>>(A, n, n, kk, r0, c0, cend);
+}
+static void launch_strip(float2 *A, int n, int kk, int r0, int c0, int cend, cudaStream_t st) {
+  k_lu_strip_c32<<<(n - r0 + SP_B - 1) / SP_B, SP_TH, 0, st>>>(A, n, n, kk, r0, c0, cend);
+}
+
 // an outer block's update of a complex FP32 factorisation on the tensor cores
 // when the LU has them (returns 1 when launched)
 static int tc_update(bem_lu *w, double2 *, int, int, cudaStream_t) { (void)w; return 0; }
@@ -1028,6 +1288,16 @@ static int tc_update(bem_lu *w, float2 *A, int n, int K, cudaStream_t st) {
   if (!w->tc || !w->tc->ready) return 0;
   bem_tc_launch(w->tc, A, n, n, K, w->status, st);
   return 1;
+}
+
+// nodes of the tournament over n rows
+static int lu_nodes(int n) {
+  int nn = (n + LU_TH - 1) / LU_TH, total = nn;
+  while (nn > 1) {
+    nn = (nn + 7) / 8;
+    total += nn;
+  }
+  return total;
 }
 
 // the launches of one factorisation, in order (captured into the graph, whose
@@ -1040,7 +1310,8 @@ static int tc_update(bem_lu *w, float2 *A, int n, int K, cudaStream_t st) {
 // side stream, beside the next panel); the next row moves wait for the rest.
 template <class C2>
 static int factor_launches(bem_lu *w, C2 *A, int n, cudaStream_t st) {
-  k_lu_iota<<<(n + 255) / 256, 256, 0, st>>>(w->rowmap, n);
+  const int nodes = lu_nodes(n);
+  k_lu_iota<<<(n + 255) / 256, 256, 0, st>>>(w->rowmap, n, w->tree + (size_t)nodes * (1 + LU_W), nodes);
   // up to one_block_max the whole matrix is one outer block (every panel
   // updates the whole trailing matrix: fewer, shorter launches on the
   // critical path of a small factorisation)
@@ -1052,7 +1323,8 @@ static int factor_launches(bem_lu *w, C2 *A, int n, cudaStream_t st) {
     for (int k = K; k < cend; k += LU_W) {
       const int wd = n - k < LU_W ? n - k : LU_W;
       const int r0 = k + wd;
-      k_lu_panel<C2><<<LU_CL, LU_TH, sizeof(panel_sh<C2>), st>>>(A, n, n, k, w->piv, (C2 *)w->u11, w->status);
+      k_lu_panel<C2><<<(n - k + LU_TH - 1) / LU_TH, LU_TH, sizeof(panel_sh<C2>), st>>>(
+          A, n, n, k, w->piv, w->tree, nodes, (C2 *)w->u11, w->status);
       if (pending) {
         CKL(cudaStreamWaitEvent(st, w->ev_join, 0), "LU join");
         pending = false;
@@ -1063,7 +1335,7 @@ static int factor_launches(bem_lu *w, C2 *A, int n, cudaStream_t st) {
                                                     w->status);
       if (r0 < cend) {
         const int nxt = cend - r0 < LU_W ? cend : r0 + LU_W;
-        launch_update(A, n, k, wd, r0, r0, nxt, st);
+        launch_strip(A, n, k, r0, r0, nxt, st);  // wd = 32: only the last panel is narrower
         if (nxt < cend) {
           CKL(cudaEventRecord(w->ev_fork, st), "LU fork");
           CKL(cudaStreamWaitEvent(w->side, w->ev_fork, 0), "LU fork");
@@ -1091,7 +1363,9 @@ template <class C2>
 static int lu_factor(bem_lu *w, void *Av, int n, cudaStream_t st) {
   if (n <= 0) return 0;
   C2 *A = (C2 *)Av;
-  if (grow_bytes(w, (void **)&w->rowmap, &w->rowmap_cap, (size_t)n * sizeof(int), "row map")) return -1;
+  if (grow_bytes(w, (void **)&w->rowmap, &w->rowmap_cap, (size_t)n * sizeof(int), "row map") ||
+      grow_bytes(w, (void **)&w->tree, &w->tree_cap, (size_t)lu_nodes(n) * (2 + LU_W) * sizeof(int), "tournament"))
+    return -1;
   const int tcmode = (sizeof(C2) == sizeof(float2) && w->tc && w->tc->ready) ? w->tc->nprod : 0;
   if (!(w->gexec && w->g_A == Av && w->g_n == n && w->g_tc == tcmode && w->g_obm == w->one_block_max)) {
     if (w->gexec) cudaGraphExecDestroy(w->gexec);

@@ -17,7 +17,9 @@
 struct bem_lu {
   int *rowmap = nullptr;    // [n] original row of each position after pivoting
   size_t rowmap_cap = 0;
-  int *piv = nullptr;       // panel scratch: selected pivot rows, candidates, permutation list
+  int *piv = nullptr;       // panel scratch: selected pivot rows, permutation list
+  int *tree = nullptr;      // tournament scratch: each node's winners, then a counter per node
+  size_t tree_cap = 0;
   void *u11 = nullptr;      // panel scratch: packed L11\U11, inverse of U11, inverse of L11, staged rows
   unsigned *status = nullptr;
   unsigned *flags = nullptr;  // triangular-solve progress counters (lower, upper), 128 bytes apart
