@@ -22,8 +22,8 @@
 //               (mma.sync m16n8k8 f64; Blackwell's tcgen05 has no FP64 kind),
 //               64 x 64 complex tiles, the complex product as four real ones.
 //
-// The sequence of a size and matrix is captured once as a CUDA graph and
-// replayed.  Solves: forward substitution L y = P b and back substitution
+// A small factorisation's sequence is captured once as a CUDA graph and replayed,
+// a large one runs on two streams of its own (factor_blocks).  Solves: forward substitution L y = P b and back substitution
 // U x = y in one launch each, one CTA per 32-row block; blocks are written in
 // dependency order and a block folds in each block it needs as soon as a
 // progress counter in global memory has passed it (bounded waits: a wait that
@@ -39,7 +39,7 @@
 
 #define LU_W BEM_LU_W
 #define LU_OB BEM_LU_OB  // outer block: panels whose updates right of it are delayed and applied at once
-#define LU_NSLOT (LU_OB / LU_W)
+#define LU_NSLOT (2 * LU_OB / LU_W)  // panel slots (row moves, L11^-1): two outer blocks in work
 #define LU_ONE_BLOCK_N 2048  // default of bem_lu.one_block_max
 static_assert(LU_OB == LU_OUTER_W, "the tensor-core update depth is the outer block");
 #define LU_TH 256        // threads of a panel CTA: one row each
@@ -48,14 +48,18 @@ static_assert(LU_OB == LU_OUTER_W, "the tensor-core update depth is the outer bl
 
 // integer scratch (bem_lu.piv)
 #define PV_SEL 0                     // [LU_W] pivot rows in order
-#define PV_PERM (PV_SEL + LU_W)      // count, then (dst, src) pairs of the row moves
-#define PV_INTS (PV_PERM + 1 + 2 * LU_MAXP)
+#define PV_LIST (1 + 2 * LU_MAXP)    // count, then (dst, src) pairs of the row moves
+#define PV_PERM (PV_SEL + LU_W)      // [LU_NSLOT] lists, one per panel of two outer blocks
+#define PV_INTS (PV_PERM + LU_NSLOT * PV_LIST)
 // complex scratch (bem_lu.u11)
 #define U_LU 0                       // [LU_W][LU_W] packed L11\U11, row i = pivot row i
 #define U_UINV (LU_W * LU_W)         // U11^-1 (upper)
 #define U_STAGE (2 * LU_W * LU_W)    // panel values of the rows moved out of the pivot block
-#define U_LINV (3 * LU_W * LU_W)     // [LU_NSLOT] L11^-1 (unit lower) of each panel of the outer block
+#define U_LINV (3 * LU_W * LU_W)     // [LU_NSLOT] L11^-1 (unit lower) of each panel of two outer blocks
 #define U_COUNT ((3 + LU_NSLOT) * LU_W * LU_W)
+
+// the slot of the panel at column k
+__host__ __device__ __forceinline__ int lu_slot(int k) { return k % (2 * LU_OB) / LU_W; }
 
 // ---------------------------------------------------------------- complex helpers
 // complex double (double2) and complex float (float2): the same code in both
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(LU_TH, 1)
     const bool in = i < w && j < w;  // entries outside a short panel (w < 32) are zero
     u[U_LU + e] = S.lu[i][j];
     u[U_UINV + e] = in ? S.iv[0][i][j] : czero<C2>();
-    u[U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W) + e] = in ? S.iv[1][i][j] : czero<C2>();
+    u[U_LINV + lu_slot(k) * (LU_W * LU_W) + e] = in ? S.iv[1][i][j] : czero<C2>();
   }
   if (wid == 2) {
     // row moves: pivot row i goes to position k + i; the rows of the pivot
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(LU_TH, 1)
     if (displaced) S.lb[__popc(bb & lt)] = k + i;
     __syncwarp();
     const int cnt = __popc(ba);
-    int *perm = pv + PV_PERM;
+    int *perm = pv + PV_PERM + lu_slot(k) * PV_LIST;
     if (lane == 0) perm[0] = w + cnt;
     if (i < w) { perm[1 + 2 * i] = k + i; perm[2 + 2 * i] = p; }
     if (lane < cnt) { perm[1 + 2 * (w + lane)] = S.la[lane]; perm[2 + 2 * (w + lane)] = S.lb[lane]; }
@@ -522,7 +526,7 @@ __global__ void __launch_bounds__(LU_TH, 1)
 #define AP_COLS 16   // columns of a row-move block
 
 template <class C2>
-__global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int k, int cend, const int *pv, const C2 *u,
+__global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int k, int cbeg, int cend, const int *pv, const C2 *u,
                                                     int *rowmap, unsigned *status) {
   __shared__ C2 sm[LU_W][LU_W + 1];
   __shared__ C2 srow[LU_MAXP][AP_COLS + 1];
@@ -531,22 +535,23 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
   const int w = min(LU_W, n - k);
   const int r0 = k + w;
   const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
-  const int nCl = (k + AP_COLS - 1) / AP_COLS, nCr = (n - r0 + AP_COLS - 1) / AP_COLS;
+  const int nCl = (k - cbeg + AP_COLS - 1) / AP_COLS, nCr = (cend - r0 + AP_COLS - 1) / AP_COLS;
   const int b = blockIdx.x;
+  pv += PV_PERM + lu_slot(k) * PV_LIST;
   // everything read through the row list or needed beside it is loaded at
   // once: the kernel is a chain of latencies, not of work
-  int nperm = __ldcg(pv + PV_PERM);
+  int nperm = __ldcg(pv);
   int md = k, ms = k;
   if (t < LU_MAXP) {
-    md = __ldcg(pv + PV_PERM + 1 + 2 * t);
-    ms = __ldcg(pv + PV_PERM + 2 + 2 * t);
+    md = __ldcg(pv + 1 + 2 * t);
+    ms = __ldcg(pv + 2 + 2 * t);
   }
   const int ci = b - nL;  // column block
   const bool right = ci >= nCl;
-  const int c0 = right ? r0 + (ci - nCl) * AP_COLS : ci * AP_COLS;
-  const bool u12 = b >= nL && right && c0 < cend;
+  const int c0 = right ? r0 + (ci - nCl) * AP_COLS : cbeg + ci * AP_COLS;
+  const bool u12 = b >= nL && b < nL + nCl + nCr && right;
   if (b < nL || b >= nL + nCl + nCr || u12) {
-    const C2 *src = u + (u12 ? U_LINV + (k % LU_OB) / LU_W * (LU_W * LU_W) : U_UINV);
+    const C2 *src = u + (u12 ? U_LINV + lu_slot(k) * (LU_W * LU_W) : U_UINV);
 #pragma unroll
     for (int e = t; e < LU_W * LU_W; e += AP_TH) sm[e / LU_W][e % LU_W] = __ldcg(src + e);
   }
@@ -595,11 +600,10 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
   }
   __syncthreads();  // sdst / ssrc, sm
   if (b < nL + nCl + nCr) {
-    // the row moves on AP_COLS columns outside the panel; right of the panel
-    // and left of cend (the end of the outer block) also U12 = L11^-1 A12 on
-    // the pivot block; right of cend the moves alone (U12 there is formed for
-    // the whole outer block at once, k_lu_trsm)
-    const int nc = min(right ? n : k, c0 + AP_COLS) - c0;
+    // the row moves on AP_COLS of the outer block's columns [cbeg, cend) outside
+    // the panel; right of the panel also U12 = L11^-1 A12 on the pivot block
+    // (outside the outer block the moves wait for k_lu_swap)
+    const int nc = min(right ? cend : k, c0 + AP_COLS) - c0;
     const int cc = t % AP_COLS, grp = t / AP_COLS;  // 8 groups of 16 columns
 #pragma unroll
     for (int q = 0; q < LU_MAXP * AP_COLS / AP_TH; ++q) {
@@ -661,13 +665,56 @@ __global__ void __launch_bounds__(AP_TH) k_lu_apply(C2 *A, long lda, int n, int 
   if (t < nperm) rowmap[sdst[t]] = old;
 }
 
+// The row moves of the np panels from column K on, on the columns [0, left) and
+// [cbeg, cend), AP_COLS columns per CTA, panel after panel: kept back from the
+// columns outside the outer block until the previous block's trailing update,
+// which runs beside the panels, is done with their rows.
+template <class C2>
+__global__ void __launch_bounds__(AP_TH) k_lu_swap(C2 *A, long lda, int n, int K, int np, int left, int cbeg, int cend,
+                                                   const int *pv) {
+  __shared__ C2 srow[LU_MAXP][AP_COLS + 1];
+  __shared__ int sdst[LU_OB / LU_W][LU_MAXP], ssrc[LU_OB / LU_W][LU_MAXP], scnt[LU_OB / LU_W];
+  const int t = threadIdx.x;
+  const int nCl = (left + AP_COLS - 1) / AP_COLS;
+  const bool right = (int)blockIdx.x >= nCl;
+  const int c0 = right ? cbeg + ((int)blockIdx.x - nCl) * AP_COLS : (int)blockIdx.x * AP_COLS;
+  const int nc = min(right ? cend : left, c0 + AP_COLS) - c0;
+  for (int e = t; e < np * LU_MAXP; e += AP_TH) {
+    const int s = e / LU_MAXP, i = e % LU_MAXP;
+    const int *l = pv + PV_PERM + lu_slot(K + s * LU_W) * PV_LIST;
+    int d = __ldcg(l + 1 + 2 * i), sr = __ldcg(l + 2 + 2 * i);
+    const int cnt = __ldcg(l);
+    if (i == 0) scnt[s] = cnt < 0 || cnt > LU_MAXP ? 0 : cnt;  // (k_lu_apply reports a list out of range)
+    if (d < K || d >= n || sr < K || sr >= n) d = sr = K;
+    sdst[s][i] = d;
+    ssrc[s][i] = sr;
+  }
+  __syncthreads();
+  const int cc = t % AP_COLS, grp = t / AP_COLS;
+  for (int s = 0; s < np; ++s) {
+    const int cnt = scnt[s];
+#pragma unroll
+    for (int q = 0; q < LU_MAXP * AP_COLS / AP_TH; ++q) {
+      const int e = grp + q * (AP_TH / AP_COLS);
+      if (e < cnt && cc < nc) srow[e][cc] = A[(size_t)ssrc[s][e] * lda + c0 + cc];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < LU_MAXP * AP_COLS / AP_TH; ++q) {
+      const int e = grp + q * (AP_TH / AP_COLS);
+      if (e < cnt && cc < nc) A[(size_t)sdst[s][e] * lda + c0 + cc] = srow[e][cc];
+    }
+    __syncthreads();  // the moves of panel s before the reads of panel s + 1
+  }
+}
+
 // ---------------------------------------------------------------- trailing update
 #define UP_BM 64
 #define UP_BN 64
 #define UP_TH 256
-#define UP_BK 16    // depth of a slice
-#define UP_NST 3    // slices in flight
-#define UP_LDA 20   // row strides (complex) of the slices: a quarter warp's 16-byte
+#define UP_BK 8     // depth of a slice
+#define UP_NST 5    // slices in flight
+#define UP_LDA 12   // row strides (complex) of the slices: a quarter warp's 16-byte
 #define UP_LDB 66   // fragment loads fall into distinct banks
 #define UP_STAGE (UP_BM * UP_LDA + UP_BK * UP_LDB)
 #define UP_SMEM (UP_NST * UP_STAGE * sizeof(double2))
@@ -688,12 +735,16 @@ __device__ __forceinline__ void cp16(double2 *dst, const double2 *src, bool live
 }
 
 // C -= L U on the FP64 tensor cores: C = A[r0:n, c0:cend), L = A[r0:n, kk:kk+kw),
-// U = A[kk:kk+kw, c0:cend), kw a multiple of 16.  A panel's update (kk = k, kw =
+// U = A[kk:kk+kw, c0:cend), kw a multiple of 8.  A panel's update (kk = k, kw =
 // 32, cend = the end of its outer block) and an outer block's (kk = its first
 // column, kw = LU_OB, cend = n) alike.  64 x 64 complex tiles, 8 warps of 32 x
-// 16, the complex product as four real ones; L and U pass through a 3-slice ring
-// of shared memory filled by asynchronous copies, so that the tensor pipe does
-// not wait for loads (2 blocks per SM, 112 KB each).
+// 16, the complex product as four real ones; L and U pass through a ring of
+// slices in shared memory filled by asynchronous copies (2 blocks per SM, 103 KB
+// each), C is fetched into L2 meanwhile and met at the end.  30.7 TFLOP/s over a
+// factorisation of n = 12288, 36.5 being what the instruction alone reaches;
+// filling the ring and meeting C take 6 us of a tile's 35.  Blocks that took
+// several tiles, the next one's first slices on their way while one ends, were
+// slower (30.1), as were 16-deep slices (29.8).
 __global__ void __launch_bounds__(UP_TH, 2) k_lu_update(double2 *A, long lda, int n, int kk, int kw, int r0,
                                                         int c0, int cend) {
   extern __shared__ __align__(16) unsigned char up_raw[];
@@ -702,6 +753,7 @@ __global__ void __launch_bounds__(UP_TH, 2) k_lu_update(double2 *A, long lda, in
   const int rb = r0 + blockIdx.y * UP_BM, cb = c0 + blockIdx.x * UP_BN;
   const int lane = t & 31, wid = t >> 5, g = lane >> 2, q = lane & 3;
   const int wm = (wid & 1) * 32, wn = (wid >> 1) * 16;  // warp tile: 32 rows x 16 columns
+  const int nk = kw / UP_BK;
   auto fill = [&](int st, int k0) {
     double2 *As = sm + st * UP_STAGE, *Bs = As + UP_BM * UP_LDA;
 #pragma unroll
@@ -717,7 +769,6 @@ __global__ void __launch_bounds__(UP_TH, 2) k_lu_update(double2 *A, long lda, in
       cp16(Bs + r * UP_LDB + c, A + (size_t)(kk + k0 + r) * lda + (live ? cb + c : c0), live);
     }
   };
-  const int nk = kw / UP_BK;
 #pragma unroll
   for (int s = 0; s < UP_NST - 1; ++s) {
     if (s < nk) fill(s, s * UP_BK);
@@ -729,76 +780,92 @@ __global__ void __launch_bounds__(UP_TH, 2) k_lu_update(double2 *A, long lda, in
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int row = rb + wm + i * 16 + g + (c >> 1) * 8, col = cb + wn + j * 8 + 2 * q + (c & 1);
-        const double2 x = (row < n && col < cend) ? A[(size_t)row * lda + col] : cz();
-        cr[i][j][c] = x.x;
-        ci[i][j][c] = x.y;
-      }
-  for (int kt = 0; kt < nk; ++kt) {
+      for (int c = 0; c < 4; ++c) cr[i][j][c] = ci[i][j][c] = 0.0;
+  {
+    const int row = rb + (t >> 2), col = cb + (t & 3) * 16;
+#pragma unroll
+    for (int c = 0; c < 16; c += 8)
+      if (row < n && col + c < cend) asm volatile("prefetch.global.L2 [%0];" ::"l"(A + (size_t)row * lda + col + c));
+  }
+  int st = 0;
+  for (int it = 0; it < nk; ++it) {
     asm volatile("cp.async.wait_group %0;" ::"n"(UP_NST - 2) : "memory");
-    __syncthreads();  // slice kt is in, and every warp is done with slice kt - 1
-    if (kt + UP_NST - 1 < nk) fill((kt + UP_NST - 1) % UP_NST, (kt + UP_NST - 1) * UP_BK);
+    __syncthreads();  // this slice is in, and every warp is done with the one before
+    if (it + UP_NST - 1 < nk) fill(st == 0 ? UP_NST - 1 : st - 1, (it + UP_NST - 1) * UP_BK);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const double2 *As = sm + (kt % UP_NST) * UP_STAGE, *Bs = As + UP_BM * UP_LDA;
+    const double2 *As = sm + st * UP_STAGE, *Bs = As + UP_BM * UP_LDA;
+    st = st == UP_NST - 1 ? 0 : st + 1;
+    double2 b[2][2];
 #pragma unroll
-    for (int k8 = 0; k8 < UP_BK; k8 += 8) {
-      double2 b[2][2];
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int c = 0; c < 2; ++c) b[j][c] = Bs[(q + 4 * c) * UP_LDB + wn + j * 8 + g];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) b[j][c] = Bs[(k8 + q + 4 * c) * UP_LDB + wn + j * 8 + g];
+    for (int i = 0; i < 2; ++i) {
+      // (cr, ci) -= (ar + i ai)(br + i bi)
+      double nr[4], ai[4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        // (cr, ci) -= (ar + i ai)(br + i bi)
-        double nr[4], ai[4];
+      for (int c = 0; c < 4; ++c) {
+        const double2 a = As[(wm + i * 16 + g + (c & 1) * 8) * UP_LDA + q + (c >> 1) * 4];
+        nr[c] = -a.x;
+        ai[c] = a.y;
+      }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const double2 a = As[(wm + i * 16 + g + (c & 1) * 8) * UP_LDA + k8 + q + (c >> 1) * 4];
-          nr[c] = -a.x;
-          ai[c] = a.y;
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          dmma(nr, b[j][0].x, b[j][1].x, cr[i][j]);
-          dmma(nr, b[j][0].y, b[j][1].y, ci[i][j]);
-          dmma(ai, b[j][0].y, b[j][1].y, cr[i][j]);
-          dmma(ai, -b[j][0].x, -b[j][1].x, ci[i][j]);
-        }
+      for (int j = 0; j < 2; ++j) {
+        dmma(nr, b[j][0].x, b[j][1].x, cr[i][j]);
+        dmma(nr, b[j][0].y, b[j][1].y, ci[i][j]);
+        dmma(ai, b[j][0].y, b[j][1].y, cr[i][j]);
+        dmma(ai, -b[j][0].x, -b[j][1].x, ci[i][j]);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < 2; ++i) {
+    // eight loads in flight, then eight stores (one by one each load would wait
+    // for the store before it)
+    double2 x[2][4];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int row = rb + wm + i * 16 + g + (c >> 1) * 8, col = cb + wn + j * 8 + 2 * q + (c & 1);
-        if (row < n && col < cend) A[(size_t)row * lda + col] = make_double2(cr[i][j][c], ci[i][j][c]);
+        x[j][c] = (row < n && col < cend) ? A[(size_t)row * lda + col] : cz();
       }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int row = rb + wm + i * 16 + g + (c >> 1) * 8, col = cb + wn + j * 8 + 2 * q + (c & 1);
+        if (row < n && col < cend)
+          A[(size_t)row * lda + col] = make_double2(x[j][c].x + cr[i][j][c], x[j][c].y + ci[i][j][c]);
+      }
+  }
 }
 
-// The same on the next panel's 32 columns alone, which the next panel waits
-// for: kw = 32, 32 x 32 tiles (4 warps of 16 x 16), so that the few tiles of a
-// strip spread over the SMs and none of a tile's columns is empty; everything
-// in one load.  7.5 us with the 64 x 64 tiles at n = 1728.
+// The same on a few panels' columns, which the next panel waits for: 32 x 32
+// tiles (4 warps of 16 x 16), so that the few tiles of a strip spread over the
+// SMs and none of a tile's columns is empty; 32 of the kw columns of L in one
+// load.  kw = 32 at n = 1728: 3.2 us, 7.5 with the 64 x 64 tiles.
 #define SP_B 32
 #define SP_TH 128
 #define SP_LDA 36
 #define SP_LDB 34
-__global__ void __launch_bounds__(SP_TH) k_lu_strip(double2 *A, long lda, int n, int kk, int r0, int c0, int cend) {
+__global__ void __launch_bounds__(SP_TH) k_lu_strip(double2 *A, long lda, int n, int kk, int kw, int r0, int c0, int cend) {
   __shared__ __align__(16) double2 As[SP_B * SP_LDA], Bs[SP_B * SP_LDB];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, g = lane >> 2, q = lane & 3;
   const int rb = r0 + blockIdx.x * SP_B, wm = (wid & 1) * 16, wn = (wid >> 1) * 16;
+  c0 += blockIdx.y * SP_B;
+  auto fill = [&](int k0) {
 #pragma unroll
-  for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
-    const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
-    const bool la = rb + r < n, lb = c0 + c < cend;
-    cp16(As + r * SP_LDA + c, A + (size_t)(la ? rb + r : r0) * lda + kk + c, la);
-    cp16(Bs + r * SP_LDB + c, A + (size_t)(kk + r) * lda + (lb ? c0 + c : c0), lb);
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
+      const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
+      const bool la = rb + r < n, lb = c0 + c < cend;
+      cp16(As + r * SP_LDA + c, A + (size_t)(la ? rb + r : r0) * lda + kk + k0 + c, la);
+      cp16(Bs + r * SP_LDB + c, A + (size_t)(kk + k0 + r) * lda + (lb ? c0 + c : c0), lb);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fill(0);
   double cr[2][4], ci[2][4];
 #pragma unroll
   for (int j = 0; j < 2; ++j)
@@ -809,24 +876,30 @@ __global__ void __launch_bounds__(SP_TH) k_lu_strip(double2 *A, long lda, int n,
       cr[j][c] = x.x;
       ci[j][c] = x.y;
     }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-#pragma unroll
-  for (int k8 = 0; k8 < SP_B; k8 += 8) {
-    double nr[4], ai[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double2 a = As[(wm + g + (c & 1) * 8) * SP_LDA + k8 + q + (c >> 1) * 4];
-      nr[c] = -a.x;
-      ai[c] = a.y;
+  for (int k0 = 0; k0 < kw; k0 += SP_B) {
+    if (k0) {
+      __syncthreads();  // the previous columns' fragment loads are done
+      fill(k0);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const double2 b0 = Bs[(k8 + q) * SP_LDB + wn + j * 8 + g], b1 = Bs[(k8 + q + 4) * SP_LDB + wn + j * 8 + g];
-      dmma(nr, b0.x, b1.x, cr[j]);
-      dmma(nr, b0.y, b1.y, ci[j]);
-      dmma(ai, b0.y, b1.y, cr[j]);
-      dmma(ai, -b0.x, -b1.x, ci[j]);
+    for (int k8 = 0; k8 < SP_B; k8 += 8) {
+      double nr[4], ai[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const double2 a = As[(wm + g + (c & 1) * 8) * SP_LDA + k8 + q + (c >> 1) * 4];
+        nr[c] = -a.x;
+        ai[c] = a.y;
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const double2 b0 = Bs[(k8 + q) * SP_LDB + wn + j * 8 + g], b1 = Bs[(k8 + q + 4) * SP_LDB + wn + j * 8 + g];
+        dmma(nr, b0.x, b1.x, cr[j]);
+        dmma(nr, b0.y, b1.y, ci[j]);
+        dmma(ai, b0.y, b1.y, cr[j]);
+        dmma(ai, -b0.x, -b1.x, ci[j]);
+      }
     }
   }
 #pragma unroll
@@ -838,10 +911,11 @@ __global__ void __launch_bounds__(SP_TH) k_lu_strip(double2 *A, long lda, int n,
     }
 }
 // complex FP32, on the CUDA cores: two rows and four columns per thread
-__global__ void __launch_bounds__(SP_TH) k_lu_strip_c32(float2 *A, long lda, int n, int kk, int r0, int c0, int cend) {
+__global__ void __launch_bounds__(SP_TH) k_lu_strip_c32(float2 *A, long lda, int n, int kk, int kw, int r0, int c0, int cend) {
   __shared__ float2 As[SP_B][SP_B + 1], Bs[SP_B][SP_B + 1];
   const int t = threadIdx.x, ty = t >> 3, tx = t & 7;
   const int rb = r0 + blockIdx.x * SP_B;
+  c0 += blockIdx.y * SP_B;
   float2 acc[2][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -850,19 +924,22 @@ __global__ void __launch_bounds__(SP_TH) k_lu_strip_c32(float2 *A, long lda, int
       const int row = rb + ty + 16 * i, col = c0 + tx + 8 * j;
       acc[i][j] = (row < n && col < cend) ? A[(size_t)row * lda + col] : make_float2(0.f, 0.f);
     }
+  for (int k0 = 0; k0 < kw; k0 += SP_B) {
+    if (k0) __syncthreads();
 #pragma unroll
-  for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
-    const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
-    As[r][c] = rb + r < n ? A[(size_t)(rb + r) * lda + kk + c] : make_float2(0.f, 0.f);
-    Bs[r][c] = c0 + c < cend ? A[(size_t)(kk + r) * lda + c0 + c] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
+    for (int i = 0; i < SP_B * SP_B / SP_TH; ++i) {
+      const int e = t + i * SP_TH, r = e / SP_B, c = e % SP_B;
+      As[r][c] = rb + r < n ? A[(size_t)(rb + r) * lda + kk + k0 + c] : make_float2(0.f, 0.f);
+      Bs[r][c] = c0 + c < cend ? A[(size_t)(kk + k0 + r) * lda + c0 + c] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
 #pragma unroll 8
-  for (int l = 0; l < SP_B; ++l)
+    for (int l = 0; l < SP_B; ++l)
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = cfms(As[ty + 16 * i][l], Bs[l][tx + 8 * j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = cfms(As[ty + 16 * i][l], Bs[l][tx + 8 * j], acc[i][j]);
+  }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -927,72 +1004,92 @@ __global__ void __launch_bounds__(UF_TH) k_lu_update_c32(float2 *A, long lda, in
 
 // ---------------------------------------------------------------- U12 of an outer block
 // U12 = L11^-1 A12 in place for the outer block's rows K .. K + ob - 1 and the
-// columns right of it (L11 unit lower, in A's strictly lower part, its
+// columns [cbeg, cend) right of it (L11 unit lower, in A's strictly lower part, its
 // diagonal blocks' inverses in the LINV slots): block row ib gets
-// Linv_ib (A12_ib - sum_{jb < ib} L_ib,jb U12_jb).  One CTA per TR_NC
-// columns; thread (i, c) holds row i of a block row and columns c, c + 4,
-// c + 8, c + 12 (conflict-free shared-memory reads: a warp reads 8 rows of L
-// at one column and 4 consecutive columns of X).
-#define TR_TH 128
+// Linv_ib (A12_ib - sum_{jb < ib} L_ib,jb U12_jb).  One CTA per TR_NC columns;
+// thread (i, cq) holds row i of a block row and columns cq, cq + 8.  The ten
+// 32 x 32 blocks pass through two buffers of shared memory, each loaded into
+// registers while the one before it is used: 41 -> 15 us at n = 4096 against
+// loads between barriers.
+#define TR_TH 256
 #define TR_NC 16
 template <class C2>
 struct trsm_sh {
   C2 X[LU_OB][TR_NC + 1];
-  C2 L[LU_W][LU_W + 1];
+  C2 L[2][LU_W][LU_W + 1];
   C2 Y[LU_W][TR_NC + 1];
 };
 template <class C2>
-__global__ void __launch_bounds__(TR_TH) k_lu_trsm(C2 *A, long lda, int n, int K, int ob, const C2 *u) {
+__global__ void __launch_bounds__(TR_TH) k_lu_trsm(C2 *A, long lda, int K, int ob, int cbeg, int cend, const C2 *u) {
   extern __shared__ __align__(16) unsigned char tr_raw[];
   trsm_sh<C2> &S = *reinterpret_cast<trsm_sh<C2> *>(tr_raw);
   const int t = threadIdx.x;
-  const int c0 = K + ob + blockIdx.x * TR_NC;
+  const int c0 = cbeg + blockIdx.x * TR_NC;
   const int nbk = ob / LU_W;
-  for (int e = t; e < ob * TR_NC; e += TR_TH) {
+  constexpr int PF = LU_W * LU_W / TR_TH;
+  C2 pf[PF];
+  // block (ib, jb) of L11, or the inverse of diagonal block ib (jb = ib)
+  auto fetch = [&](int ib, int jb) {
+#pragma unroll
+    for (int h = 0; h < PF; ++h) {
+      const int e = t + h * TR_TH, r = e / LU_W, c = e % LU_W;
+      pf[h] = jb < ib ? A[(size_t)(K + ib * LU_W + r) * lda + K + jb * LU_W + c]
+                      : __ldcg(u + U_LINV + lu_slot(K + ib * LU_W) * (LU_W * LU_W) + e);
+    }
+  };
+  fetch(0, 0);
+#pragma unroll
+  for (int e = t; e < LU_OB * TR_NC; e += TR_TH) {
     const int r = e / TR_NC, c = e % TR_NC;
-    S.X[r][c] = c0 + c < n ? A[(size_t)(K + r) * lda + c0 + c] : czero<C2>();
+    S.X[r][c] = (r < ob && c0 + c < cend) ? A[(size_t)(K + r) * lda + c0 + c] : czero<C2>();
   }
-  const int i = t >> 2, cq = t & 3;  // row i of a block row, columns cq + 4 j
+  const int i = t >> 3, cq = t & 7;  // row i of a block row, columns cq, cq + 8
+  int buf = 0;
   for (int ib = 0; ib < nbk; ++ib) {
-    C2 acc[4];
-    __syncthreads();
+    C2 acc[2];
+    for (int jb = 0; jb <= ib; ++jb) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = S.X[ib * LU_W + i][cq + 4 * j];
-    for (int jb = 0; jb < ib; ++jb) {
-      for (int e = t; e < LU_W * LU_W; e += TR_TH) {
-        const int r = e / LU_W, c = e % LU_W;
-        S.L[r][c] = A[(size_t)(K + ib * LU_W + r) * lda + K + jb * LU_W + c];
+      for (int h = 0; h < PF; ++h) {
+        const int e = t + h * TR_TH;
+        S.L[buf][e / LU_W][e % LU_W] = pf[h];
       }
-      __syncthreads();
-#pragma unroll 8
-      for (int l = 0; l < LU_W; ++l) {
-        const C2 lv = S.L[i][l];
+      if (jb < ib) fetch(ib, jb + 1);
+      else if (ib + 1 < nbk) fetch(ib + 1, 0);
+      if (jb == 0) {
+        if (ib == 0) __syncthreads();  // X is in
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = cfms(lv, S.X[jb * LU_W + l][cq + 4 * j], acc[j]);
+        for (int j = 0; j < 2; ++j) acc[j] = S.X[ib * LU_W + i][cq + 8 * j];
       }
-      __syncthreads();
-    }
+      if (jb == ib)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) S.Y[i][cq + 4 * j] = acc[j];
-    const C2 *linv = u + U_LINV + ib * (LU_W * LU_W);
-    for (int e = t; e < LU_W * LU_W; e += TR_TH) S.L[e / LU_W][e % LU_W] = __ldcg(linv + e);
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = czero<C2>();
+        for (int j = 0; j < 2; ++j) S.Y[i][cq + 8 * j] = acc[j];
+      __syncthreads();  // L (and X of the blocks above, Y) are in; the other buffer is free
+      if (jb < ib) {
 #pragma unroll 8
-    for (int l = 0; l < LU_W; ++l) {
-      const C2 lv = S.L[i][l];
+        for (int l = 0; l < LU_W; ++l) {
+          const C2 lv = S.L[buf][i][l];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[j] = cfma(lv, S.Y[l][cq + 4 * j], acc[j]);
+          for (int j = 0; j < 2; ++j) acc[j] = cfms(lv, S.X[jb * LU_W + l][cq + 8 * j], acc[j]);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) acc[j] = czero<C2>();
+#pragma unroll 8
+        for (int l = 0; l < LU_W; ++l) {
+          const C2 lv = S.L[buf][i][l];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) acc[j] = cfma(lv, S.Y[l][cq + 8 * j], acc[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) S.X[ib * LU_W + i][cq + 8 * j] = acc[j];
+      }
+      buf ^= 1;
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) S.X[ib * LU_W + i][cq + 4 * j] = acc[j];
-    __syncthreads();  // Y and L are rewritten by the next block row
   }
   __syncthreads();
   for (int e = t; e < ob * TR_NC; e += TR_TH) {
     const int r = e / TR_NC, c = e % TR_NC;
-    if (c0 + c < n) A[(size_t)(K + r) * lda + c0 + c] = S.X[r][c];
+    if (c0 + c < cend) A[(size_t)(K + r) * lda + c0 + c] = S.X[r][c];
   }
 }
 
@@ -1227,9 +1324,14 @@ extern "C" int bem_lu_init(bem_lu *w, int device) {
     snprintf(w->err, sizeof(w->err), "triangular solve: no resident block");
     return -1;
   }
-  CKL(cudaStreamCreateWithFlags(&w->side, cudaStreamNonBlocking), "LU side stream");
+  // the panels' blocks (on hi) go before those of the update that runs beside them
+  int lo = 0, hi = 0;
+  CKL(cudaDeviceGetStreamPriorityRange(&lo, &hi), "LU streams");
+  CKL(cudaStreamCreateWithPriority(&w->side, cudaStreamNonBlocking, lo), "LU side stream");
+  CKL(cudaStreamCreateWithPriority(&w->hi, cudaStreamNonBlocking, hi), "LU streams");
   CKL(cudaEventCreateWithFlags(&w->ev_fork, cudaEventDisableTiming), "LU events");
   CKL(cudaEventCreateWithFlags(&w->ev_join, cudaEventDisableTiming), "LU events");
+  CKL(cudaEventCreateWithFlags(&w->ev_st, cudaEventDisableTiming), "LU events");
   CKL(cudaMalloc(&w->piv, PV_INTS * sizeof(int)), "LU scratch");
   CKL(cudaMalloc(&w->u11, U_COUNT * sizeof(double2)), "LU scratch");
   CKL(cudaMalloc(&w->status, sizeof(unsigned)), "LU status");
@@ -1249,7 +1351,9 @@ extern "C" void bem_lu_free(bem_lu *w) {
   cudaFree(w->y);
   if (w->ev_fork) cudaEventDestroy(w->ev_fork);
   if (w->ev_join) cudaEventDestroy(w->ev_join);
+  if (w->ev_st) cudaEventDestroy(w->ev_st);
   if (w->side) cudaStreamDestroy(w->side);
+  if (w->hi) cudaStreamDestroy(w->hi);
   *w = bem_lu();
 }
 
@@ -1273,20 +1377,21 @@ static void launch_update(float2 *A, int n, int kk, int kw, int r0, int c0, int 
   k_lu_update_c32<<<grid, UF_TH, 0, st>>>(A, n, n, kk, kw, r0, c0, cend);
 }
 
-// the same on the next panel's columns [c0, cend), at most 32, with kw = 32
-static void launch_strip(double2 *A, int n, int kk, int r0, int c0, int cend, cudaStream_t st) {
-  k_lu_strip<<<(n - r0 + SP_B - 1) / SP_B, SP_TH, 0, st>>>(A, n, n, kk, r0, c0, cend);
+// the same on a few panels' columns [c0, cend), kw a multiple of 32
+static void launch_strip(double2 *A, int n, int kk, int kw, int r0, int c0, int cend, cudaStream_t st) {
+  k_lu_strip<<<dim3((n - r0 + SP_B - 1) / SP_B, (cend - c0 + SP_B - 1) / SP_B), SP_TH, 0, st>>>(A, n, n, kk, kw, r0, c0, cend);
 }
-static void launch_strip(float2 *A, int n, int kk, int r0, int c0, int cend, cudaStream_t st) {
-  k_lu_strip_c32<<<(n - r0 + SP_B - 1) / SP_B, SP_TH, 0, st>>>(A, n, n, kk, r0, c0, cend);
+static void launch_strip(float2 *A, int n, int kk, int kw, int r0, int c0, int cend, cudaStream_t st) {
+  k_lu_strip_c32<<<dim3((n - r0 + SP_B - 1) / SP_B, (cend - c0 + SP_B - 1) / SP_B), SP_TH, 0, st>>>(A, n, n, kk, kw, r0, c0, cend);
 }
 
-// an outer block's update of a complex FP32 factorisation on the tensor cores
-// when the LU has them (returns 1 when launched)
-static int tc_update(bem_lu *w, double2 *, int, int, cudaStream_t) { (void)w; return 0; }
-static int tc_update(bem_lu *w, float2 *A, int n, int K, cudaStream_t st) {
+// an outer block's update right of the next block's columns, for a complex FP32
+// factorisation on the tensor cores when the LU has them (returns 1 when
+// launched): its first column tile (as wide as an outer block), or the others
+static int tc_update(bem_lu *w, double2 *, int, int, bool, cudaStream_t) { (void)w; return 0; }
+static int tc_update(bem_lu *w, float2 *A, int n, int K, bool first, cudaStream_t st) {
   if (!w->tc || !w->tc->ready) return 0;
-  bem_tc_launch(w->tc, A, n, n, K, w->status, st);
+  bem_tc_launch(w->tc, A, n, n, K, first, w->status, st);
   return 1;
 }
 
@@ -1300,62 +1405,109 @@ static int lu_nodes(int n) {
   return total;
 }
 
-// the launches of one factorisation, in order (captured into the graph, whose
-// replays count them).  Outer blocks of LU_OB columns: each panel's update
-// covers only the rest of its outer block; the columns right of the block get
-// the row moves as the panels go, then U12 (k_lu_trsm) and one rank-LU_OB
-// update, so the trailing matrix is read and written once per outer block
-// instead of once per panel.  Look-ahead: a panel's update is split into the
-// next panel's 32 columns (on st, before the next panel) and the rest (on the
-// side stream, beside the next panel); the next row moves wait for the rest.
+// One outer block (n <= one_block_max): the launches in order, captured into a
+// graph whose replays count them.  Look-ahead: a panel's update is split into
+// the next panel's 32 columns (on st, before the next panel) and the rest (on
+// the side stream, beside the next panel); the next row moves wait for the rest.
 template <class C2>
-static int factor_launches(bem_lu *w, C2 *A, int n, cudaStream_t st) {
+static int factor_one(bem_lu *w, C2 *A, int n, cudaStream_t st) {
   const int nodes = lu_nodes(n);
   k_lu_iota<<<(n + 255) / 256, 256, 0, st>>>(w->rowmap, n, w->tree + (size_t)nodes * (1 + LU_W), nodes);
-  // up to one_block_max the whole matrix is one outer block (every panel
-  // updates the whole trailing matrix: fewer, shorter launches on the
-  // critical path of a small factorisation)
-  const int one_block = w->one_block_max > 0 ? w->one_block_max : LU_ONE_BLOCK_N;
-  const int obw = n <= one_block ? n : LU_OB;
   bool pending = false;  // update work on the side stream not yet joined
-  for (int K = 0; K < n; K += obw) {
-    const int cend = n - K < obw ? n : K + obw;
-    for (int k = K; k < cend; k += LU_W) {
-      const int wd = n - k < LU_W ? n - k : LU_W;
-      const int r0 = k + wd;
-      k_lu_panel<C2><<<(n - k + LU_TH - 1) / LU_TH, LU_TH, sizeof(panel_sh<C2>), st>>>(
-          A, n, n, k, w->piv, w->tree, nodes, (C2 *)w->u11, w->status);
-      if (pending) {
-        CKL(cudaStreamWaitEvent(st, w->ev_join, 0), "LU join");
-        pending = false;
+  for (int k = 0; k < n; k += LU_W) {
+    const int wd = n - k < LU_W ? n - k : LU_W;
+    const int r0 = k + wd;
+    k_lu_panel<C2><<<(n - k + LU_TH - 1) / LU_TH, LU_TH, sizeof(panel_sh<C2>), st>>>(
+        A, n, n, k, w->piv, w->tree, nodes, (C2 *)w->u11, w->status);
+    if (pending) CKL(cudaStreamWaitEvent(st, w->ev_join, 0), "LU join");
+    pending = false;
+    const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
+    const int nC = (k + AP_COLS - 1) / AP_COLS + (n - r0 + AP_COLS - 1) / AP_COLS;
+    k_lu_apply<C2><<<nL + nC + 1, AP_TH, 0, st>>>(A, n, n, k, 0, n, w->piv, (const C2 *)w->u11, w->rowmap, w->status);
+    if (r0 < n) {  // wd = 32: only the last panel is narrower
+      const int nxt = n - r0 < LU_W ? n : r0 + LU_W;
+      launch_strip(A, n, k, LU_W, r0, r0, nxt, st);
+      if (nxt < n) {
+        CKL(cudaEventRecord(w->ev_fork, st), "LU fork");
+        CKL(cudaStreamWaitEvent(w->side, w->ev_fork, 0), "LU fork");
+        launch_update(A, n, k, wd, r0, nxt, n, w->side);
+        CKL(cudaEventRecord(w->ev_join, w->side), "LU join");
+        pending = true;
       }
-      const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
-      const int nC = (k + AP_COLS - 1) / AP_COLS + (n - r0 + AP_COLS - 1) / AP_COLS;
-      k_lu_apply<C2><<<nL + nC + 1, AP_TH, 0, st>>>(A, n, n, k, cend, w->piv, (const C2 *)w->u11, w->rowmap,
-                                                    w->status);
-      if (r0 < cend) {
-        const int nxt = cend - r0 < LU_W ? cend : r0 + LU_W;
-        launch_strip(A, n, k, r0, r0, nxt, st);  // wd = 32: only the last panel is narrower
-        if (nxt < cend) {
-          CKL(cudaEventRecord(w->ev_fork, st), "LU fork");
-          CKL(cudaStreamWaitEvent(w->side, w->ev_fork, 0), "LU fork");
-          launch_update(A, n, k, wd, r0, nxt, cend, w->side);
-          CKL(cudaEventRecord(w->ev_join, w->side), "LU join");
-          pending = true;
-        }
-      }
-    }
-    if (pending) {
-      CKL(cudaStreamWaitEvent(st, w->ev_join, 0), "LU join");
-      pending = false;
-    }
-    if (cend < n) {
-      k_lu_trsm<C2><<<(n - cend + TR_NC - 1) / TR_NC, TR_TH, sizeof(trsm_sh<C2>), st>>>(A, n, n, K, cend - K,
-                                                                                         (const C2 *)w->u11);
-      if (tc_update(w, A, n, K, st) == 0) launch_update(A, n, K, cend - K, cend, cend, n, st);
     }
   }
   CKL(cudaGetLastError(), "LU launch");
+  return 0;
+}
+
+// Outer blocks of LU_OB columns, two lanes.  hi (high priority): a block's panels,
+// which update only the rest of their block, and then the same block's row
+// moves, U12 and update on the next block's columns alone, so that the next
+// panels can go on.  lo: the block's row moves on all other columns, U12 and the
+// rank-LU_OB update right of the next block, its first LU_OB columns ahead of the
+// rest because hi needs them one block later.  hi runs up to a block ahead: the
+// panels, bound by latency (a half of the time at n = 4096 when they run by
+// themselves), hide behind the updates.  Launched on the streams, not as a
+// graph: a graph's launches do not keep the lanes' priorities.
+template <class C2>
+static int factor_blocks(bem_lu *w, C2 *A, int n, cudaStream_t st) {
+  const int nodes = lu_nodes(n);
+  cudaStream_t hi = w->hi, lo = w->side;
+  unsigned long long count = 1;
+  CKL(cudaEventRecord(w->ev_st, st), "LU start");
+  CKL(cudaStreamWaitEvent(hi, w->ev_st, 0), "LU start");
+  CKL(cudaStreamWaitEvent(lo, w->ev_st, 0), "LU start");
+  k_lu_iota<<<(n + 255) / 256, 256, 0, hi>>>(w->rowmap, n, w->tree + (size_t)nodes * (1 + LU_W), nodes);
+  const C2 *u = (const C2 *)w->u11;
+  for (int K = 0; K < n; K += LU_OB) {
+    const int cend = n - K < LU_OB ? n : K + LU_OB, np = (cend - K + LU_W - 1) / LU_W;
+    const int c1 = n - cend < LU_OB ? n : cend + LU_OB;  // end of the next block
+    const int c2 = n - c1 < LU_OB ? n : c1 + LU_OB;      // and of the one after
+    for (int k = K; k < cend; k += LU_W) {
+      const int r0 = n - k < LU_W ? n : k + LU_W;
+      k_lu_panel<C2><<<(n - k + LU_TH - 1) / LU_TH, LU_TH, sizeof(panel_sh<C2>), hi>>>(
+          A, n, n, k, w->piv, w->tree, nodes, (C2 *)w->u11, w->status);
+      const int nL = (n - r0 + AP_ROWS - 1) / AP_ROWS;
+      const int nC = (k - K + AP_COLS - 1) / AP_COLS + (cend - r0 + AP_COLS - 1) / AP_COLS;
+      k_lu_apply<C2><<<nL + nC + 1, AP_TH, 0, hi>>>(A, n, n, k, K, cend, w->piv, u, w->rowmap, w->status);
+      if (r0 < cend) launch_strip(A, n, k, LU_W, r0, r0, cend, hi);
+      count += r0 < cend ? 3 : 2;
+    }
+    // lo's update of the next block's columns by the previous block (it also
+    // ends lo's use of that block's slots, which the next block's panels take)
+    if (K > 0) CKL(cudaStreamWaitEvent(hi, w->ev_join, 0), "LU join");
+    CKL(cudaEventRecord(w->ev_fork, hi), "LU fork");
+    CKL(cudaStreamWaitEvent(lo, w->ev_fork, 0), "LU fork");
+    if (cend < n) {
+      const int nc = (c1 - cend + AP_COLS - 1) / AP_COLS;
+      k_lu_swap<C2><<<nc, AP_TH, 0, hi>>>(A, n, n, K, np, 0, cend, c1, w->piv);
+      k_lu_trsm<C2><<<(c1 - cend + TR_NC - 1) / TR_NC, TR_TH, sizeof(trsm_sh<C2>), hi>>>(A, n, K, LU_OB, cend, c1, u);
+      launch_strip(A, n, K, LU_OB, cend, cend, c1, hi);
+      count += 3;
+    }
+    const int nsw = (K + AP_COLS - 1) / AP_COLS + (n - c1 + AP_COLS - 1) / AP_COLS;
+    if (nsw > 0) {
+      k_lu_swap<C2><<<nsw, AP_TH, 0, lo>>>(A, n, n, K, np, K, c1, n, w->piv);
+      ++count;
+    }
+    if (c1 < n) {
+      k_lu_trsm<C2><<<(n - c1 + TR_NC - 1) / TR_NC, TR_TH, sizeof(trsm_sh<C2>), lo>>>(A, n, K, LU_OB, c1, n, u);
+      if (!tc_update(w, A, n, K, true, lo)) launch_update(A, n, K, LU_OB, cend, c1, c2, lo);
+      else ++count;
+      count += 2;
+    }
+    CKL(cudaEventRecord(w->ev_join, lo), "LU join");
+    if (c2 < n) {
+      if (!tc_update(w, A, n, K, false, lo)) launch_update(A, n, K, LU_OB, cend, c2, n, lo);
+      ++count;
+    }
+  }
+  CKL(cudaGetLastError(), "LU launch");
+  CKL(cudaEventRecord(w->ev_join, lo), "LU end");
+  CKL(cudaStreamWaitEvent(hi, w->ev_join, 0), "LU end");
+  CKL(cudaEventRecord(w->ev_st, hi), "LU end");
+  CKL(cudaStreamWaitEvent(st, w->ev_st, 0), "LU end");
+  bem_count_launches(count);
   return 0;
 }
 
@@ -1366,16 +1518,16 @@ static int lu_factor(bem_lu *w, void *Av, int n, cudaStream_t st) {
   if (grow_bytes(w, (void **)&w->rowmap, &w->rowmap_cap, (size_t)n * sizeof(int), "row map") ||
       grow_bytes(w, (void **)&w->tree, &w->tree_cap, (size_t)lu_nodes(n) * (2 + LU_W) * sizeof(int), "tournament"))
     return -1;
-  const int tcmode = (sizeof(C2) == sizeof(float2) && w->tc && w->tc->ready) ? w->tc->nprod : 0;
-  if (!(w->gexec && w->g_A == Av && w->g_n == n && w->g_tc == tcmode && w->g_obm == w->one_block_max)) {
+  if (n > (w->one_block_max > 0 ? w->one_block_max : LU_ONE_BLOCK_N)) return factor_blocks(w, A, n, st);
+  if (!(w->gexec && w->g_A == Av && w->g_n == n && w->g_fp == (int)sizeof(C2))) {
     if (w->gexec) cudaGraphExecDestroy(w->gexec);
     if (w->graph) cudaGraphDestroy(w->graph);
     w->gexec = nullptr;
     w->graph = nullptr;
-    CKL(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "LU capture");
-    const int rc = factor_launches(w, A, n, st);
+    CKL(cudaStreamBeginCapture(w->hi, cudaStreamCaptureModeThreadLocal), "LU capture");
+    const int rc = factor_one(w, A, n, w->hi);
     cudaGraph_t g = nullptr;
-    const cudaError_t ce = cudaStreamEndCapture(st, &g);
+    const cudaError_t ce = cudaStreamEndCapture(w->hi, &g);
     if (rc) {
       if (g) cudaGraphDestroy(g);
       return rc;
@@ -1386,10 +1538,9 @@ static int lu_factor(bem_lu *w, void *Av, int n, cudaStream_t st) {
     size_t nodes = 0;
     CKL(cudaGraphGetNodes(g, nullptr, &nodes), "LU graph");
     w->g_nodes = nodes;
-    w->g_obm = w->one_block_max;
     w->g_A = Av;
     w->g_n = n;
-    w->g_tc = tcmode;
+    w->g_fp = (int)sizeof(C2);
   }
   CKL(cudaGraphLaunch(w->gexec, st), "LU graph launch");
   bem_count_launches(w->g_nodes);

@@ -53,11 +53,11 @@ __device__ __forceinline__ float tf32_hi(float x) {
 }
 
 __global__ void k_tc_pack(const float2 *__restrict__ M, long lda, int n, int K, int r0, int nprod,
-                          float *__restrict__ Ap, float *__restrict__ Bp, int rows, int ntiles) {
+                          float *__restrict__ Ap, float *__restrict__ Bp, int rows, int tile0, int ntiles) {
   const int kp = TC_KR * nprod;
   // A'': one thread per (row, k)
   const long na = (long)rows * LU_OUTER_W;
-  const long nb = (long)ntiles * TC_NC * LU_OUTER_W;
+  const long nb = (long)(ntiles - tile0) * TC_NC * LU_OUTER_W;  // sub-tiles tile0 .. ntiles - 1
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < na + nb; e += (long)gridDim.x * blockDim.x) {
     if (e < na) {
       const int r = (int)(e / LU_OUTER_W), kk = (int)(e % LU_OUTER_W);
@@ -75,7 +75,7 @@ __global__ void k_tc_pack(const float2 *__restrict__ M, long lda, int n, int K, 
       }
     } else {
       const long f = e - na;
-      const int cc = (int)(f / LU_OUTER_W), kk = (int)(f % LU_OUTER_W);
+      const int cc = tile0 * TC_NC + (int)(f / LU_OUTER_W), kk = (int)(f % LU_OUTER_W);
       const int col = r0 + cc;
       const float2 b = col < n ? M[(size_t)(K + kk) * lda + col] : make_float2(0.f, 0.f);
       const int tile = cc / TC_NC, j = cc % TC_NC;
@@ -177,7 +177,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // and a B box (TC_M rows x 128 bytes each)
 __global__ void __launch_bounds__(TC_TH, 2)
     k_tc_update(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, float2 *C, long ldc,
-                int n, int r0, int nbox, unsigned *status) {
+                int n, int r0, int nbox, int tile0, unsigned *status) {
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[TC_STAGES], bar_empty[TC_STAGES], bar_done;
   __shared__ uint32_t tmem_base;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(TC_TH, 2)
   unsigned char *sm = (unsigned char *)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int row_tile = r0 + blockIdx.y * TC_M;   // matrix row of the tile's first row
-  const int col_tile = blockIdx.x;               // column tile (TC_NC x TC_NS complex columns)
+  const int col_tile = tile0 + blockIdx.x;       // column tile (TC_NC x TC_NS complex columns)
   if (t == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init(&bar_full[s], 1);
@@ -369,17 +369,23 @@ extern "C" int bem_tc_prepare(bem_tc *t, int n, int nprod) {
   return 0;
 }
 
-extern "C" void bem_tc_launch(bem_tc *t, float2 *M, long lda, int n, int K, unsigned *status, cudaStream_t st) {
+extern "C" void bem_tc_launch(bem_tc *t, float2 *M, long lda, int n, int K, bool first, unsigned *status,
+                              cudaStream_t st) {
+  static_assert(TC_NC * TC_NS == LU_OUTER_W, "a column tile is an outer block");
   const int r0 = K + LU_OUTER_W;
   const int rows = n - r0;
-  if (rows <= 0) return;
   const int ctiles = (rows + TC_NC * TC_NS - 1) / (TC_NC * TC_NS), rtiles = (rows + TC_M - 1) / TC_M;
+  if (ctiles < 2) return;
   const int subtiles = ctiles * TC_NS;  // 64-column sub-tiles packed (the last ones may lie past n)
-  const long work = (long)rows * LU_OUTER_W + (long)subtiles * TC_NC * LU_OUTER_W;
-  const int pb = (int)((work + 255) / 256 < 8192 ? (work + 255) / 256 : 8192);
-  k_tc_pack<<<pb, 256, 0, st>>>(M, lda, n, K, r0, t->nprod, t->Ap, t->Bp, rows, subtiles);
+  if (first) {
+    const long work = (long)rows * LU_OUTER_W + (long)(subtiles - TC_NS) * TC_NC * LU_OUTER_W;
+    const int pb = (int)((work + 255) / 256 < 8192 ? (work + 255) / 256 : 8192);
+    k_tc_pack<<<pb, 256, 0, st>>>(M, lda, n, K, r0, t->nprod, t->Ap, t->Bp, rows, TC_NS, subtiles);
+  }
   const int nbox = TC_KR * t->nprod / TC_BOX_K;
-  k_tc_update<<<dim3(ctiles, rtiles), TC_TH, tc_smem(), st>>>(t->tmA, t->tmB, M, lda, n, r0, nbox, status);
+  const int tile0 = first ? 1 : 2, nt = first ? 1 : ctiles - 2;
+  if (nt > 0)
+    k_tc_update<<<dim3(nt, rtiles), TC_TH, tc_smem(), st>>>(t->tmA, t->tmB, M, lda, n, r0, nbox, tile0, status);
 }
 
 extern "C" void bem_tc_free(bem_tc *t) {

@@ -19,9 +19,10 @@ extern "C" {
 // packed-operand buffers and TMA maps for systems up to n (no allocation
 // inside a stream capture: call before capturing)
 int bem_tc_prepare(bem_tc *t, int n, int nprod);
-// pack and launch the update of the outer block starting at column K of the
-// row-major complex FP32 matrix M: M[r0:n, r0:n] -= M[r0:n, K:r0] M[K:r0, r0:n],
-// r0 = K + LU_OUTER_W
-void bem_tc_launch(bem_tc *t, float2 *M, long lda, int n, int K, unsigned *status, cudaStream_t st);
+// the update of the outer block starting at column K of the row-major complex
+// FP32 matrix M, right of the next block's columns: M[r0:n, c0:n] -= M[r0:n, K:r0]
+// M[K:r0, c0:n], r0 = K + LU_OUTER_W, c0 = r0 + LU_OUTER_W.  first: pack the
+// operands and update the first LU_OUTER_W of those columns; otherwise the others
+void bem_tc_launch(bem_tc *t, float2 *M, long lda, int n, int K, bool first, unsigned *status, cudaStream_t st);
 void bem_tc_free(bem_tc *t);
 }
