@@ -142,12 +142,13 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
   for (int a = -n1; a <= n1; ++a)
     for (int b = -n2; b <= n2; ++b) P.push_back({hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y), a, b});
   std::stable_sort(P.begin(), P.end(), [](const pt &x, const pt &y) { return x.r < y.r; });
-  // the cheapest split, in FP64 operations: per pair about 45 points of 66 for
-  // each image and 16 multiply-adds for each of the K functions (G and H of 4
-  // entries, complex); once, A = U T, the samples (110 lattice terms each, a
-  // tenth of the GPU busy) and T.  Summed point by point a pair takes about 8e5.
+  // the cheapest split, in FP64 operations at the rates that the kernels reach
+  // (images 0.55 of the pipe, the product 0.7): per pair about 45 points of 66
+  // for each image and 16 multiply-adds for each of the K functions (G and H of
+  // 4 entries, complex); once, A = U T, the samples (about 300 terms of 100 each)
+  // and T.  Summed point by point a pair takes about 8e5 at half the pipe.
   const double pairs = 4.0 * ne * ne;
-  double best = 4e5 * pairs;
+  double best = 1e6 * pairs;
   for (size_t c = 1; c < P.size() && c <= BEM_SM_MAXIMG; ++c) {
     if (P[c].r <= P[c - 1].r * (1.0 + 1e-9)) continue;  // whole shells only
     const double cut = P[c].r;
@@ -158,18 +159,41 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
     int Lmax = degree_for(S->k, S->rho, cut, 6.0 * S->rho, 1e-15, 2 * BEM_SM_MAXL);
     if (Lmax < 0 || Lmax > 2 * lmax) Lmax = 2 * lmax;
     const double K = (lmax + 1.0) * (lmax + 1.0), nt = lmax + 0.5 * Lmax + 1.0;
-    const double cost = pairs * ((c - 1) * 45.0 * 66.0 + 16.0 * K) + 4.0 * ne * 2.0 * K * K +
-                        nt * (2.0 * Lmax + 2.0) * 1.2e5 + 0.125 * K * K * lmax * nt;
+    const double cost = pairs * ((c - 1) * 45.0 * 66.0 / 0.55 + 16.0 * K / 0.7) + 4.0 * ne * 2.0 * K * K / 0.7 +
+                        nt * (2.0 * Lmax + 2.0) * 3e4 + 0.25 * K * K * lmax * nt;
     if (cost < best) {
       best = cost;
       S->on = 1;
       S->lmax = lmax;
       S->Lmax = Lmax;
       S->nimg = (int)c;
+      S->cut = cut - S->rho;
       for (size_t i = 0; i < c; ++i) { S->l1[i] = P[i].a; S->l2[i] = P[i].b; }
     }
   }
   if (!S->on) return;
+  // windows of the samples' Ewald sums: the reference's parameter below its cap
+  // (k^2 eta^2 < 3); terms to e^{-40} of the leading one; the images among them
+  S->eta = std::min(q->eta0, 0.98 * sqrt(3.0) / S->k);
+  const double cutr = S->rho + 2.0 * S->eta * sqrt(40.0 + S->k * S->k * S->eta * S->eta);
+  const double cuts = sqrt(40.0 / (S->eta * S->eta) + S->k * S->k);
+  const double tp = 2.0 * M_PI;
+  S->r1 = (int)(cutr * hypot(q->g1x, q->g1y) / tp) + 1;
+  S->r2 = (int)(cutr * hypot(q->g2x, q->g2y) / tp) + 1;
+  for (int i = 0; i < S->nimg; ++i) {
+    S->r1 = std::max(S->r1, abs(S->l1[i]));
+    S->r2 = std::max(S->r2, abs(S->l2[i]));
+  }
+  // a_n = -k_par + n g: |n1 - k_par . d1 / 2 pi| <= |a| |d1| / 2 pi, and for n2
+  S->s1 = (int)(cuts * hypot(q->d1x, q->d1y) / tp) + 2;
+  S->s2 = (int)(cuts * hypot(q->d2x, q->d2y) / tp) + 2;
+  // a batch's instances share the window: centred on n2 = 0, wide enough for |k_par| <= k
+  S->sc2 = 0;
+  S->s2 += (int)(S->k * hypot(q->d2x, q->d2y) / tp) + 1;
+  if ((double)(2 * S->r1 + 1) * (2 * S->r2 + 1) > 20000.0 || (double)(2 * S->s1 + 1) * (2 * S->s2 + 1) > 20000.0) {
+    S->on = 0;
+    return;
+  }
   S->K = (S->lmax + 1) * (S->lmax + 1);
   S->Kp = (S->K + 15) / 16 * 16;
   // Gauss-Legendre nodes in cos(theta): exact for products of three harmonics
@@ -268,10 +292,13 @@ void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h) {
 
 // ------------------------------------------------------------------ device view
 struct sm_dev {
-  int lmax, Lmax, K, Kp, nt, nphi, nimg;
-  double cx, cy, cz, R0, iR0, kR0, rho, k;
+  int lmax, Lmax, K, Kp, nt, nphi, nimg, nlm;  // nlm: pairs (l, m >= 0) up to Lmax
+  double cx, cy, cz, R0, iR0, kR0, rho, k, cut;
+  double eta;                       // Ewald parameter of the samples
+  int nreal, r1, r2, nspec, s1, s2, sc2;  // its windows: l1 in [-r1, r1], l2 in [-r2, r2]; n1 - nc1 in [-s1, s1], ...
+  int iml[2 * BEM_SM_MAXIMG];       // the images' indices
   const double *x, *w, *ca, *cb, *dL, *el, *rec, *img;
-  double *plm;            // [lm >= 0][nt] normalised Legendre functions P_lm(x_t)
+  double *plm;            // [nt][lm >= 0] normalised Legendre functions P_lm(x_t)
   double *samp;           // [nb][2][nt][nphi] complex: G_s and rho dG_s/drho
   double *sig;            // [nb][(Lmax + 1)^2] complex
   double *T;              // [nb][Kp][2 Kp]: T^t, real and imaginary parts
@@ -316,13 +343,19 @@ __device__ __forceinline__ void sm_image(double kpi, double k, double px, double
 }
 
 // ------------------------------------------------------------------ coefficients of the rest
-// Blocks below nsamp: G_s and its radial derivative at the sphere points
-// (one thread per point and instance).  The others: P_lm at the nodes.
-#define SMP_TH 32
+// Warps below nsamp blocks: G_s and its radial derivative at the sphere points.
+// A warp takes a point, its lanes the terms of an Ewald sum over fixed windows:
+// lattice points within |P| < 2 eta sqrt(40 + k^2 eta^2) of a point of the ball
+// |R| <= 2 R0, orders with |beta| eta < sqrt(40 + ...): every term above 1e-17
+// of the leading one, with no stopping tests, which a chain of dependent terms
+// would wait for (220 us with a thread per point and the adaptive sums of
+// bem_qpgf, 65 us like this).  eta keeps k eta below the reference's cap sqrt(3), so that
+// e^{k^2 eta^2} costs no digits.  The other blocks: P_lm at the nodes.
+#define SMP_TH 128
 __global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm_dev S, const __grid_constant__ sm_qps Q,
-                                                      int nsamp, int nb, unsigned *status) {
+                                                      int nsamp, unsigned *status) {
   if ((int)blockIdx.x < nsamp) {
-    const int b = blockIdx.y, i = blockIdx.x * SMP_TH + threadIdx.x;
+    const int b = blockIdx.y, lane = threadIdx.x & 31, i = blockIdx.x * (SMP_TH / 32) + (threadIdx.x >> 5);
     if (i >= S.nt * S.nphi) return;
     const bem_qp &q = Q.q[b];
     const int t = i / S.nphi, jp = i % S.nphi;
@@ -330,35 +363,95 @@ __global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm
     double sp, cp;
     sincospi(2.0 * jp / S.nphi, &sp, &cp);
     const double ux = sn * cp, uy = sn * sp, X = S.rho * ux, Y = S.rho * uy, Z = S.rho * ct;
-    bem_gval gv;
-    const int rc = bem_qpgf(q, X, Y, Z, gv);
-    if (rc < 0) atomicOr(status, rc == -12 || rc == -23 ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT);
-    double ur = 0, ui = 0, xr = 0, xi = 0;  // the images' value and radial derivative, times 4 pi
-    const double kpi = S.k * 0.31830988618379067154;
-    for (int m = 0; m < S.nimg; ++m) {
-      const double *im = S.img + 3 * (b * S.nimg + m);
-      const double px = X + im[0], py = Y + im[1];
-      double gr, gi, fr, fi;
-      sm_image(kpi, S.k, px, py, Z * Z, im[2], gr, gi, fr, fi);
-      const double d = px * ux + py * uy + Z * ct;
-      ur += gr;
-      ui += gi;
-      xr += fr * d;
-      xi += fi * d;
+    const double ve = S.eta, ke = q.k * ve, kpi = S.k * 0.31830988618379067154;
+    double ur = 0, ui = 0, xr = 0, xi = 0;
+    // real-space terms less the images taken out, times 4 pi
+    for (int e = lane; e < S.nreal; e += 32) {
+      const int l1 = e / (2 * S.r2 + 1) - S.r1, l2 = e % (2 * S.r2 + 1) - S.r2;
+      const double sx = l1 * q.d1x + l2 * q.d2x, sy = l1 * q.d1y + l2 * q.d2y;
+      const double px = X + sx, py = Y + sy, r2 = px * px + py * py + Z * Z;
+      bool out = false;  // one of the images: its closed form is not part of G_s
+      for (int m = 0; m < S.nimg; ++m) out |= S.iml[2 * m] == l1 && S.iml[2 * m + 1] == l2;
+      const double arg = ke * ke - r2 / (4.0 * ve * ve);
+      if (arg < -42.0 && !out) continue;
+      const double ph = (q.kx * sx + q.ky * sy) * 0.31830988618379067154, d = px * ux + py * uy + Z * ct;
+      double s, c;
+      sincospi(ph, &s, &c);
+      double a = 0.0, f = 0.0;
+      const double ir = rsqrt(r2), r = r2 * ir;
+      if (arg >= -42.0) {
+        const cplx w = bem_faddeeva(ke, r / (2.0 * ve));
+        const double ef = exp(arg);
+        a = ir * ef * w.re;
+        f = -ir * ir * ef * (ir * w.re - q.k * w.im + 0.56418958354775628695 / ve);
+      }
+      ur += c * a;
+      ui += s * a;
+      xr += c * f * d;
+      xi += s * f * d;
+      if (out) {
+        double gr, gi, fr, fi;
+        sm_image(kpi, S.k, px, py, Z * Z, ph, gr, gi, fr, fi);
+        ur -= gr;
+        ui -= gi;
+        xr -= fr * d;
+        xi -= fi * d;
+      }
     }
-    const double c4 = BEM_I_FP;
-    double *o = S.samp + 2 * ((size_t)b * 2 * S.nt * S.nphi + i), *o2 = o + 2 * (size_t)S.nt * S.nphi;
-    o[0] = gv.g.re - c4 * ur;
-    o[1] = gv.g.im - c4 * ui;
-    o2[0] = S.rho * (gv.gx.re * ux + gv.gy.re * uy + gv.gz.re * ct - c4 * xr);
-    o2[1] = S.rho * (gv.gx.im * ux + gv.gy.im * uy + gv.gz.im * ct - c4 * xi);
+    ur *= BEM_I_FP; ui *= BEM_I_FP; xr *= BEM_I_FP; xi *= BEM_I_FP;
+    // spectral terms (ew_spec_term)
+    const double c2 = 0.25 * q.aidet, dz = Z / (2.0 * ve);
+    bool ray = false;
+    for (int e = lane; e < S.nspec; e += 32) {
+      const int n1 = q.nc1 + e / (2 * S.s2 + 1) - S.s1, n2 = S.sc2 + e % (2 * S.s2 + 1) - S.s2;
+      const double ax = bem_an(-q.kx, n1, q.g1x, n2, q.g2x), ay = bem_an(-q.ky, n1, q.g1y, n2, q.g2y);
+      const double bn2 = __dadd_rn(__dadd_rn(__dmul_rn(q.k, q.k), -__dmul_rn(ax, ax)), -__dmul_rn(ay, ay));
+      if (bn2 * ve * ve < -42.0) continue;
+      double s, c;
+      sincos(ax * X + ay * Y, &s, &c);
+      const double da = ax * ux + ay * uy;
+      cplx F, D;  // sum of F_n and its z-derivative factor, before the phase
+      if (bn2 > 0.0) {
+        const double bn = sqrt(bn2), ef = exp(bn2 * ve * ve - dz * dz);
+        const cplx ff = cexpi(bn * Z), w = bem_faddeeva(bn * ve, dz);
+        F = cmk(2.0 * ff.re / bn, 2.0 * (ef * w.im + ff.im) / bn);
+        D = cmk(2.0 * (ef * w.re - ff.re), -2.0 * ff.im);
+      } else if (bn2 < 0.0) {
+        const double bn = sqrt(-bn2), bv = bn * ve, eq = exp(-(bv * bv + dz * dz));
+        const double f1 = eq * erfcx(bv + dz), f2 = eq * erfcx(bv - dz);
+        F = cmk(0.0, -(f1 + f2) / bn);
+        D = cmk(f1 - f2, 0.0);
+      } else {
+        ray = true;
+        continue;
+      }
+      const cplx ce = cmk(c, s), Fn = cmul(ce, F), Dn = cmul(ce, D);
+      // value i c2 F, gradient (-c2 a F, c2 D)
+      ur -= c2 * Fn.im;
+      ui += c2 * Fn.re;
+      xr += c2 * (Dn.re * ct - da * Fn.re);
+      xi += c2 * (Dn.im * ct - da * Fn.im);
+    }
+    if (ray) atomicOr(status, BEM_ST_RAYLEIGH);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ur += __shfl_down_sync(0xffffffffu, ur, o);
+      ui += __shfl_down_sync(0xffffffffu, ui, o);
+      xr += __shfl_down_sync(0xffffffffu, xr, o);
+      xi += __shfl_down_sync(0xffffffffu, xi, o);
+    }
+    if (lane == 0) {
+      double2 *o = reinterpret_cast<double2 *>(S.samp) + (size_t)b * 2 * S.nt * S.nphi + i;
+      o[0] = make_double2(ur, ui);
+      o[(size_t)S.nt * S.nphi] = make_double2(S.rho * xr, S.rho * xi);
+    }
     return;
   }
   if (blockIdx.y) return;
   // P_lm(x_t): one thread per (m, t), upward in l
   const int i = (blockIdx.x - nsamp) * SMP_TH + threadIdx.x;
   if (i >= (S.Lmax + 1) * S.nt) return;
-  const int m = i / S.nt, t = i % S.nt;
+  const int m = i % (S.Lmax + 1), t = i / (S.Lmax + 1);
   const double ct = S.x[t], sn = sqrt((1.0 - ct) * (1.0 + ct));
   double p1 = S.rec[m * (m + 1) + 2 * m], p0 = 0.0;
   for (int a = 0; a < m; ++a) p1 *= sn;
@@ -369,7 +462,7 @@ __global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm
       p0 = p1;
       p1 = p2;
     }
-    S.plm[(size_t)(l * (l + 1) / 2 + m) * S.nt + t] = p1;
+    S.plm[(size_t)t * S.nlm + l * (l + 1) / 2 + m] = p1;
   }
 }
 
@@ -407,11 +500,12 @@ __global__ void __launch_bounds__(SMC_TH) k_sm_coef(const __grid_constant__ sm_d
   __syncthreads();
   const int am = abs(M);
   for (int l = am + threadIdx.x; l <= S.Lmax; l += SMC_TH) {
-    const double *p = S.plm + (size_t)(l * (l + 1) / 2 + am) * S.nt;
+    const double *p = S.plm + l * (l + 1) / 2 + am;
     double a[4] = {0, 0, 0, 0};
+#pragma unroll 4
     for (int t = 0; t < S.nt; ++t)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) a[c] += p[t] * F[c][t];
+      for (int c = 0; c < 4; ++c) a[c] += p[(size_t)t * S.nlm] * F[c][t];
     double *o = S.sig + 2 * ((size_t)b * (S.Lmax + 1) * (S.Lmax + 1) + l * l + l + M);
     o[0] = S.ca[l] * a[0] + S.cb[l] * a[2];
     o[1] = S.ca[l] * a[1] + S.cb[l] * a[3];
@@ -447,8 +541,10 @@ __global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev 
   }
   const int nh = S.nt / 2;
   double *pr = sm_raw + threadIdx.x;
-  const double *p1 = S.plm + (size_t)blockIdx.x * S.nt, *p2 = S.plm + (size_t)(live ? i2 : 0) * S.nt;
-  for (int t = 0; t < nh; ++t) pr[t * SMT_TH] = 4.0 * CUDART_PI * S.w[t] * p1[t] * p2[t];
+  const double *p1 = S.plm + blockIdx.x, *p2 = S.plm + (live ? i2 : 0);
+#pragma unroll 4
+  for (int t = 0; t < nh; ++t)
+    pr[t * SMT_TH] = 4.0 * CUDART_PI * S.w[t] * p1[(size_t)t * S.nlm] * p2[(size_t)t * S.nlm];
   if (!live) return;
   const double *sg = S.sig + 2 * (size_t)b * (S.Lmax + 1) * (S.Lmax + 1);
   // tp[0]: T_{m,m'}, tp[1]: T_{-m,-m'}, tp[2]: T_{m,-m'}, tp[3]: T_{-m,m'}
@@ -459,12 +555,20 @@ __global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev 
   for (int v = 0; v < 2; ++v) {
     if (v && (m == 0 || m2 == 0)) break;
     const int M = v ? m + m2 : m - m2, aM = abs(M);
-    int L0 = max(abs(l - l2), aM);
-    L0 += (L0 + l + l2) & 1;
-    for (int L = L0; L <= min(l + l2, S.Lmax); L += 2) {
-      const double *pL = S.plm + (size_t)(L * (L + 1) / 2 + aM) * S.nt;
-      double G = 0.0;
-      for (int t = 0; t < nh; ++t) G = fma(pr[t * SMT_TH], pL[t], G);
+    // L from |l - l'| for every thread (P_LM = 0 below |M|), so that threads of
+    // one l' read neighbouring P_LM
+    for (int L = abs(l - l2); L <= min(l + l2, S.Lmax); L += 2) {
+      if (L < aM) continue;
+      const double *pL = S.plm + L * (L + 1) / 2 + aM;
+      double G = 0.0, G1 = 0.0;
+      int t = 0;
+#pragma unroll 2
+      for (; t + 1 < nh; t += 2) {
+        G = fma(pr[t * SMT_TH], pL[(size_t)t * S.nlm], G);
+        G1 = fma(pr[(t + 1) * SMT_TH], pL[(size_t)(t + 1) * S.nlm], G1);
+      }
+      if (t < nh) G = fma(pr[t * SMT_TH], pL[(size_t)t * S.nlm], G);
+      G += G1;
       // i^{l - l' - L}, l - l' - L even
       const double f = ((l - l2 - L) & 2) ? -G * S.dL[L] : G * S.dL[L];
       const double *sp = sg + 2 * (L * L + L + M), *sn = sg + 2 * (L * L + L - M);
@@ -571,13 +675,15 @@ __global__ void __launch_bounds__(SMU_TH) k_sm_targets(const __grid_constant__ s
 }
 
 // V[lm][4 s + a] = int N_a |W| phi_lm, V[lm][4 ne + 4 s + a] = int N_a W . grad phi_lm
-// over element s, on the reference's 12 x 12 rule (3 parts of it on a
-// triangle).  Block: (element, order m); a thread per point walks l and leaves
+// over element s.  The product with A makes these G_s and W . grad G_s integrated
+// with this rule, so the rule is the one a regular pair takes whose nearest image
+// is at the least distance any image left in has from an element (cut - 2 R0);
+// the reference's 12 x 12 (3 parts of it on a triangle) without the shorter rules.  Block: (element, order m); a thread per point walks l and leaves
 // the four values of each l in shared memory, then a thread per value sums
 // over the points.
 #define SMV_PT (BEM_GLN * BEM_GLN)
 #define SMV_TH 160
-__global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ sm_dev S, bem_dom_dev D) {
+__global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ sm_dev S, bem_dom_dev D, int far_rule) {
   extern __shared__ double sm_raw[];
   const int s = blockIdx.x, m = blockIdx.y, tid = threadIdx.x;
   const int se = abs(D.sid[s]) - 1;
@@ -590,14 +696,29 @@ __global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ s
   double acc[4] = {0, 0, 0, 0};
   bem_el el;
   bem_load_el(D.cr, D.cw, se, el);
-  for (int part = 0; part < (tri ? 3 : 1); ++part) {
+  int tier = -1;
+  if (far_rule) {
+    const double R2 = el_circum2(el, tri);
+    tier = tier_of(S.cut * S.cut / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
+  }
+  const int n = tier < 0 ? BEM_GLN : BEM_TIER_N0 - tier, npt = n * n;
+  for (int part = 0; part < (tri && tier < 0 ? 3 : 1); ++part) {
     if (part) __syncthreads();
-    if (tid < SMV_PT) {
-      const int i = tid / BEM_GLN, j = tid % BEM_GLN;
-      double zt = c_q.xl[i], et = c_q.xl[j], wt = c_q.wl[i] * c_q.wl[j];
-      if (tri) {
-        wt *= bem_tri_wfac(zt, et);
-        bem_tri_point(part, c_q.xl[i], c_q.xl[j], zt, et);
+    if (tid < npt) {
+      const int i = tid / n, j = tid % n;
+      double zt, et, wt;
+      if (tier >= 0) {
+        tier_point(tier, tri, i, j, zt, et);
+        wt = c_q.wt[tier][i] * c_q.wt[tier][j];
+        if (tri) wt *= 0.125 * (c_q.xt[tier][i] + 1.0);
+      } else {
+        zt = c_q.xl[i];
+        et = c_q.xl[j];
+        wt = c_q.wl[i] * c_q.wl[j];
+        if (tri) {
+          wt *= bem_tri_wfac(zt, et);
+          bem_tri_point(part, c_q.xl[i], c_q.xl[j], zt, et);
+        }
       }
       double r[3], W[3], Nn[4];
       bem_rw(el, zt, et, r, W);
@@ -679,9 +800,9 @@ __global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ s
     __syncthreads();
     if (tid < nout) {
       const double *v = val + (size_t)tid * SMV_PT;
-      const int q0 = tid % SMV_PT;  // another first point per thread: the rows are a multiple of 32 banks apart
-      for (int q = 0; q < SMV_PT; ++q) {
-        const int qq = q + q0 < SMV_PT ? q + q0 : q + q0 - SMV_PT;
+      const int q0 = tid % npt;  // another first point per thread: the rows are a multiple of 32 banks apart
+      for (int q = 0; q < npt; ++q) {
+        const int qq = q + q0 < npt ? q + q0 : q + q0 - npt;
         const double x = v[qq];
 #pragma unroll
         for (int a = 0; a < 4; ++a) acc[a] = fma(x, Nw[a * SMV_PT + qq], acc[a]);
@@ -945,8 +1066,13 @@ __global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__
 static sm_dev dev_view(const bem_smooth *S, int ne, int b0) {
   sm_dev d;
   d.lmax = S->lmax; d.Lmax = S->Lmax; d.K = S->K; d.Kp = S->Kp; d.nt = S->nt; d.nphi = S->nphi; d.nimg = S->nimg;
+  d.eta = S->eta;
+  d.r1 = S->r1; d.r2 = S->r2; d.nreal = (2 * S->r1 + 1) * (2 * S->r2 + 1);
+  d.s1 = S->s1; d.s2 = S->s2; d.sc2 = S->sc2; d.nspec = (2 * S->s1 + 1) * (2 * S->s2 + 1);
+  for (int i = 0; i < S->nimg; ++i) { d.iml[2 * i] = S->l1[i]; d.iml[2 * i + 1] = S->l2[i]; }
+  d.nlm = (S->Lmax + 1) * (S->Lmax + 2) / 2;
   d.cx = S->ctr[0]; d.cy = S->ctr[1]; d.cz = S->ctr[2];
-  d.R0 = S->R0; d.iR0 = 1.0 / S->R0; d.kR0 = S->k * S->R0; d.rho = S->rho; d.k = S->k;
+  d.R0 = S->R0; d.iR0 = 1.0 / S->R0; d.kR0 = S->k * S->R0; d.rho = S->rho; d.k = S->k; d.cut = S->cut;
   const bem_smooth_tab t = bem_smooth_layout(S);
   d.x = S->tab + t.x; d.w = S->tab + t.w; d.ca = S->tab + t.ca; d.cb = S->tab + t.cb;
   d.dL = S->tab + t.dL; d.el = S->tab + t.el; d.rec = S->tab + t.rec;
@@ -985,15 +1111,15 @@ extern "C" int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, cons
       O.G[i] = i < n ? G[b0 + i] : nullptr;
       O.H[i] = i < n ? H[b0 + i] : nullptr;
     }
-    const int nsamp = (S->nt * S->nphi + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
-    k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, n, scr->status);
+    const int nsamp = (S->nt * S->nphi * 32 + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
+    k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, scr->status);
     k_sm_coef<<<dim3(2 * S->Lmax + 1, n), SMC_TH, 0, st>>>(d);
     if (cudaMemsetAsync(d.T, 0, (size_t)n * 2 * S->Kp * S->Kp * sizeof(double), st) != cudaSuccess) return -1;
     k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, smem_t, st>>>(d);
     bem_count_launches(3);
     if (b0 == 0) {
       k_sm_targets<<<(N + SMU_TH / 32 - 1) / (SMU_TH / 32), SMU_TH, 0, st>>>(d, *D);
-      k_sm_sources<<<dim3(ne, S->lmax + 1), SMV_TH, smem_v, st>>>(d, *D);
+      k_sm_sources<<<dim3(ne, S->lmax + 1), SMV_TH, smem_v, st>>>(d, *D, D->far_rule);
       bem_count_launches(2);
     }
     const size_t sT = 2 * (size_t)S->Kp * S->Kp, sA = (size_t)N * 2 * S->Kp;

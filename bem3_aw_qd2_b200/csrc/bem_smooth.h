@@ -15,6 +15,9 @@ struct bem_smooth {
   int on = 0;
   int lmax = 0, Lmax = 0, K = 0, Kp = 0, nt = 0, nphi = 0, nimg = 0;
   double ctr[3] = {0, 0, 0}, R0 = 0.0, rho = 0.0, k = 0.0;
+  double cut = 0.0;             // least distance of an image left in from an element, seen from a node
+  double eta = 0.0;             // Ewald parameter and windows of the samples
+  int r1 = 0, r2 = 0, s1 = 0, s2 = 0, sc2 = 0;
   int l1[BEM_SM_MAXIMG], l2[BEM_SM_MAXIMG];  // the images' lattice indices, (0, 0) first
   int inst = 1, first = 0;      // instances tab holds; the one a launch for a single instance takes
   const double *tab = nullptr;  // device copy of the tables bem_smooth_tables writes
