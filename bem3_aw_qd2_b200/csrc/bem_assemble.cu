@@ -8,8 +8,9 @@
 //   dF[p][3] = {(1+)F, dF/dt_zeta, dF/dt_eta}
 //
 // Work is split by pair class, each class in its own kernel:
-//   classify  geometric F, dF/dt on 12x12 points for every (p, s); flags the
-//             near-singular pairs (|dF/dt| > 0.5, d3qd2_elem.c:851,537)
+//   classify  geometric F, dF/dt for every (p, s), on 12x12 points or the
+//             shorter rule of the distance; flags the near-singular pairs
+//             (|dF/dt| > 0.5, d3qd2_elem.c:851,537)
 //   regular   periodic domain: lattice images in closed form + an expansion of
 //             the rest (bem_smooth.cu); where that does not apply (no pair lists,
 //             a body much taller than the period) and for pairs with a point on
@@ -83,8 +84,7 @@ __device__ __forceinline__ void count_work(unsigned long long *ctr, unsigned lon
 // geometric F and its tangential derivatives at one quadrature point:
 // tD = (R.W)/R^3, dF_v = (3 (R.v)(R.W)/R^2 - W.v)/R^3   (q0_bil_dcoef_v2_cc.c:165-200)
 __device__ __forceinline__ void geomF(const double vR[3], const double vW[3], const bem_node &n, double &f, double &fz, double &fe) {
-  const double aR = sqrt(vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2]);
-  const double iR = 1.0 / aR;
+  const double iR = rsqrt(vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2]);
   const double rdW = dot3(vR, vW) * iR;
   const double rdz = dot3(vR, n.vz) * iR, rde = dot3(vR, n.vt) * iR;
   const double Wdz = dot3(vW, n.vz), Wde = dot3(vW, n.vt);
@@ -120,7 +120,7 @@ __device__ __forceinline__ void geomF(const double vR[3], const double vW[3], co
 // |W| has complex zeros near the element, which the shorter rules feel first;
 // at a quarter the 6-point tier is off by 1e-11); other quads keep tier 2 or
 // the reference rule.
-struct bem_far { int on, split; double d1x, d1y, d2x, d2y, idet, k; };
+struct bem_far { int on, split, fs; double d1x, d1y, d2x, d2y, idet, k; };
 // (distance from the element's centre (a triangle's centroid) to the nearest
 // lattice image of rt) / (the element's circumradius R about that centre),
 // squared, and (k R)^2.
@@ -214,39 +214,43 @@ __global__ void __launch_bounds__(128) k_classify(bem_dom_dev D, bem_far fr, dou
   if (threadIdx.x == 0) cnt = 0;
   __syncthreads();
   double sF = 0, sFz = 0, sFe = 0;
-  for (int s = threadIdx.x; s < D.ne; s += blockDim.x) {
-    const int se = abs(D.sid[s]) - 1;
+  for (int s0 = 0; s0 < D.ne; s0 += blockDim.x) {
+    const int s = s0 + threadIdx.x;
+    const bool valid = s < D.ne;
+    const int se = abs(D.sid[valid ? s : 0]) - 1;
+    const bool self = se == te, tri = bem_is_tri(D, se);
+    bem_el el;
+    bem_load_el(D.cr, D.cw, se, el);
+    // the geometric sums on the rule of the element's distance (tier_free); a
+    // warp takes the longest its pairs ask for
+    const double R2 = el_circum2(el, tri);
+    const double dx = el.cr[0][0] - nd.rt[0], dy = el.cr[1][0] - nd.rt[1], dz = el.cr[2][0] - nd.rt[2];
+    const double r2 = (dx * dx + dy * dy + dz * dz) / R2;
+    const bool shape = tri || quad_tier_shape(el);
+    int n = 0;
+    if (valid && !self) {
+      const int t = D.far_rule ? tier_free(r2, 0.0, shape) : -1;
+      n = t < 0 ? BEM_GLN : BEM_TIER_N0 - t;
+    }
+    n = __reduce_max_sync(0xffffffffu, n);
+    if (!valid) continue;
     uint8_t fl = 0;
-    if (se == te) {
+    if (self) {
       fl = 2;  // self pair
     } else {
-      bem_el el;
-      bem_load_el(D.cr, D.cw, se, el);
-      const bool tri = bem_is_tri(D, se);
-      double F = 0, Fz = 0, Fe = 0, rzmin = 1e300;
-      for (int part = 0; part < (tri ? 3 : 1); ++part)
-        for (int i = 0; i < BEM_GLN; ++i) {
-          double f = 0, fz = 0, fe = 0;
-          for (int j = 0; j < BEM_GLN; ++j) {
-            double z = c_q.xl[i], e = c_q.xl[j], wf = 1.0;
-            if (tri) {
-              bem_tri_point(part, z, e, z, e);
-              wf = bem_tri_wfac(c_q.xl[i], c_q.xl[j]);
-            }
-            double vR[3], vW[3];
-            bem_rw(el, z, e, vR, vW);
-            for (int d = 0; d < 3; ++d) vR[d] -= nd.rt[d];
-            rzmin = fmin(rzmin, fabs(vR[2]));
-            double a, b, c;
-            geomF(vR, vW, nd, a, b, c);
-            f += c_q.wl[j] * wf * a;
-            fz += c_q.wl[j] * wf * b;
-            fe += c_q.wl[j] * wf * c;
-          }
-          F += c_q.wl[i] * f;
-          Fz += c_q.wl[i] * fz;
-          Fe += c_q.wl[i] * fe;
-        }
+      double F = 0, Fz = 0, Fe = 0;
+      const int np = rule_npts(n, tri);
+      for (int pt = 0; pt < np; ++pt) {
+        double z, e, wt, vR[3], vW[3];
+        rule_pt(n, tri, pt, z, e, wt);
+        bem_rw(el, z, e, vR, vW);
+        for (int d = 0; d < 3; ++d) vR[d] -= nd.rt[d];
+        double a, b, c;
+        geomF(vR, vW, nd, a, b, c);
+        F += wt * a;
+        Fz += wt * b;
+        Fe += wt * c;
+      }
       F *= BEM_I_FP; Fz *= BEM_I_FP; Fe *= BEM_I_FP;
       if (D.sid[s] < 0) { F = -F; Fz = -Fz; Fe = -Fe; }  // bil_convert_CC / _dCC
       if (fabs(Fz) > BEM_CBD_SDF || fabs(Fe) > BEM_CBD_SDF) {
@@ -255,6 +259,22 @@ __global__ void __launch_bounds__(128) k_classify(bem_dom_dev D, bem_far fr, dou
         if (k < D.near_cap) list[k] = s;
       } else {
         sF += F; sFz += Fz; sFe += Fe;
+        // free space: the rule of the distance (k_fs_regular)
+        if (fr.fs) {
+          const int t = tier_free(r2, fr.k * fr.k * R2, shape);
+          if (t >= 0) fl = (uint8_t)(3 + t);
+        }
+        // the reference's points' least height over the node's lattice plane,
+        // where the element reaches that plane at all
+        double rzmin = 1e300;
+        if ((fr.on || fr.split) &&
+            fabs(dz) <= fabs(el.cr[2][1]) + fabs(el.cr[2][2]) + fabs(el.cr[2][3]) + 2.0 * BEM_FAR_PLANE_TOL)
+          for (int pt = 0; pt < rule_npts(BEM_GLN, tri); ++pt) {
+            double z, e, wt, vR[3], vW[3];
+            rule_pt(BEM_GLN, tri, pt, z, e, wt);
+            bem_rw(el, z, e, vR, vW);
+            rzmin = fmin(rzmin, fabs(vR[2] - nd.rt[2]));
+          }
         if ((fr.on || fr.split) && rzmin >= BEM_FAR_PLANE_TOL) {
           const int tier = fr.on ? far_tier(fr, el, nd.rt, tri) : -1;
           if (tier >= 0) fl = (uint8_t)(3 + tier);
@@ -913,6 +933,23 @@ __device__ __forceinline__ polar_pt polar_theta(const double th[5], int idx /* 0
   return r;
 }
 
+// The rule's angles as a table in shared memory (nang <= 512): cosine, sine,
+// radius to the edge, weight.  Each angle serves 12 or 64 radii, whose points
+// otherwise form its four trigonometric functions again.  All threads; the
+// caller synchronises.
+#define POLAR_N 512
+struct polar_tab { double c[POLAR_N], s[POLAR_N], rm[POLAR_N], w[POLAR_N]; };
+__device__ __forceinline__ void polar_fill(polar_tab &T, const double r[5], const double th[5], int nang, unsigned &st) {
+  for (int i = threadIdx.x; i < nang; i += blockDim.x) {
+    const polar_pt tp = polar_theta(th, i);
+    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
+    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
+    sincos(tp.th, &T.s[i], &T.c[i]);
+    T.rm[i] = rm;
+    T.w[i] = tp.wth;
+  }
+}
+
 // geometric F of the element at parameter point (zt,et) by the polar rule (q0_bil_coef_bd_F,
 // q0_bil_dcoef_v2_cc.c:401-454 / bil_sF_theta): returns the un-normalised sum (times bdC/4pi later)
 __device__ double polar_F_partial(const bem_el &el, double zt, double et, unsigned &st) {
@@ -944,17 +981,13 @@ __device__ __forceinline__ double bem_bdC(const bem_el &el) {
 
 // periodic self pair: one block per collocation node p
 // point pt of the polar rule around the node (zt, et) on its own quad: (z, e),
-// the weight with the polar Jacobian, R = rr K from the node, W; false when
-// the rule's radius comes out negative (bad geometry)
-__device__ __forceinline__ bool self_point(const bem_el &el, const double th[5], const double r[5], double zt, double et,
-                                           int pt, double &z, double &e, double &wr, double vR[3], double vW[3]) {
+// the weight with the polar Jacobian, R = rr K from the node, W
+__device__ __forceinline__ void self_point(const bem_el &el, const polar_tab &T, double zt, double et, int pt, double &z,
+                                           double &e, double &wr, double vR[3], double vW[3]) {
   const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
-  const polar_pt tp = polar_theta(th, idx);
-  const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-  double sth, cth;
-  sincos(tp.th, &sth, &cth);
+  const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
   const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-  wr = tp.wth * 0.5 * rm * c_q.wl[ir] * rr;
+  wr = T.w[idx] * 0.5 * rm * c_q.wl[ir] * rr;
   z = rr * cth + zt;
   e = rr * sth + et;
   double K[3];
@@ -963,7 +996,6 @@ __device__ __forceinline__ bool self_point(const bem_el &el, const double th[5],
     vR[d] = rr * K[d];
     vW[d] = el.cw[d][0] + el.cw[d][1] * z + el.cw[d][2] * e;
   }
-  return rm >= 0.0;
 }
 
 template <class BA>
@@ -993,6 +1025,9 @@ __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_q
 #pragma unroll
   for (int c = 0; c < 19; ++c) v[c] = 0.0;
   unsigned st = 0;
+  __shared__ polar_tab T;
+  polar_fill(T, r, th, POLAR_N, st);
+  __syncthreads();
   // the node on its own element
   bem_node nd;
   {
@@ -1004,7 +1039,7 @@ __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_q
   bool on_plane = false;
   for (int pt = threadIdx.x; pt < 512 * BEM_GLN; pt += NP_THREADS) {
     double z, e, wr, vR[3], vW[3], N[4];
-    if (!self_point(el, th, r, zt, et, pt, z, e, wr, vR, vW)) st |= BEM_ST_GEOMETRY;
+    self_point(el, T, zt, et, pt, z, e, wr, vR, vW);
     on_plane |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
     bem_gval g0;
     bem_g0(q.k, vR, g0);
@@ -1040,7 +1075,7 @@ __global__ void NP_BOUNDS k_q0_self(bem_dom_dev D, const __grid_constant__ bem_q
     for (int c = 0; c < 16; ++c) v[c] = 0.0;
     for (int pt = threadIdx.x; pt < 512 * BEM_GLN; pt += NP_THREADS) {
       double z, e, wr, vR[3], vW[3], N[4];
-      self_point(el, th, r, zt, et, pt, z, e, wr, vR, vW);
+      self_point(el, T, zt, et, pt, z, e, wr, vR, vW);
       bem_gval gv;
       const int rc = bem_qpgf(q, vR[0], vR[1], vR[2], gv, wts);
       if (rc < 0) st |= (rc == -12 || rc == -23) ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT;
@@ -1112,8 +1147,8 @@ __device__ __forceinline__ void fs_point(const bem_el &el, const bem_node &nd, d
   double vR[3], vW[3];
   bem_rw(el, z, e, vR, vW);
   for (int d = 0; d < 3; ++d) vR[d] -= nd.rt[d];
-  const double aR = sqrt(vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2]);
-  const double iR = 1.0 / aR;
+  const double R2 = vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2];
+  const double iR = rsqrt(R2), aR = R2 * iR;
   const double aW = sqrt(vW[0] * vW[0] + vW[1] * vW[1] + vW[2] * vW[2]);
   const cplx ce = cexpi(k * aR);
   const cplx cb = cmk(-1.0, k * aR);  // i k R - 1
@@ -1180,15 +1215,19 @@ __device__ __forceinline__ void fs_store(const bem_dom_dev &D, int p, int s, con
   }
 }
 
-// one thread per (p, s) pair, 12x12 points; rows p0 .. p0 + np - 1
+// one thread per (p, s) pair, 12x12 points or a shorter rule (tier_free); rows p0 .. p0 + np - 1
 __global__ void __launch_bounds__(128) k_fs_regular(bem_dom_dev D, double k, const uint8_t *__restrict__ flag,
                                                     double *__restrict__ G, double *__restrict__ H,
                                                     double *__restrict__ dG, double *__restrict__ dH, int p0, int np) {
   const long long pair = (long long)p0 * D.ne + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long total = (long long)(p0 + np) * D.ne;
-  if (pair >= total) return;
-  const int p = (int)(pair / D.ne), s = (int)(pair % D.ne);
-  if (flag[pair] != 0 || bem_pad_row(D, p)) return;
+  const bool in = pair < total;
+  const int p = in ? (int)(pair / D.ne) : p0, s = in ? (int)(pair % D.ne) : 0;
+  const int fl = in ? flag[pair] : 1;
+  const bool live = (fl == 0 || fl >= 3) && !bem_pad_row(D, p);
+  // the rule of the distance; a warp takes the longest its pairs ask for
+  const int n = __reduce_max_sync(0xffffffffu, !live ? 0 : fl == 0 ? BEM_GLN : BEM_TIER_N0 - (fl - 3));
+  if (!live) return;
   bem_node nd;
   int t, te;
   bem_load_node(D, p, nd, t, te);
@@ -1197,18 +1236,13 @@ __global__ void __launch_bounds__(128) k_fs_regular(bem_dom_dev D, double k, con
   bem_load_el(D.cr, D.cw, se, el);
   fs_acc a;
   fs_zero(a);
-  if (bem_is_tri(D, se)) {
-    // lit_dcoef_v2_GL (lit_dcoef_v2.c:185-270): 3 parts x 12 x 12
-    for (int part = 0; part < 3; ++part)
-      for (int i = 0; i < BEM_GLN; ++i)
-        for (int j = 0; j < BEM_GLN; ++j) {
-          double z, e;
-          bem_tri_point(part, c_q.xl[i], c_q.xl[j], z, e);
-          fs_point(el, nd, k, z, e, c_q.wl[i] * c_q.wl[j] * bem_tri_wfac(c_q.xl[i], c_q.xl[j]), a, true);
-        }
-  } else {
-    for (int i = 0; i < BEM_GLN; ++i)
-      for (int j = 0; j < BEM_GLN; ++j) fs_point(el, nd, k, c_q.xl[i], c_q.xl[j], c_q.wl[i] * c_q.wl[j], a);
+  // lit_dcoef_v2_GL (lit_dcoef_v2.c:185-270) on a triangle: 3 parts x 12 x 12
+  const bool tri = bem_is_tri(D, se);
+  const int npt = rule_npts(n, tri);
+  for (int pt = 0; pt < npt; ++pt) {
+    double z, e, wt;
+    rule_pt(n, tri, pt, z, e, wt);
+    fs_point(el, nd, k, z, e, wt, a, tri);
   }
   fs_store(D, p, s, a, G, H, dG, dH, p0);
 }
@@ -1307,16 +1341,15 @@ __global__ void __launch_bounds__(NP_THREADS, FS_SELF_MINB) k_fs_self(bem_dom_de
 #pragma unroll
   for (int c = 0; c < 51; ++c) Av[c] = 0.0;
   unsigned st = 0;
+  __shared__ polar_tab T;
+  polar_fill(T, r, th, POLAR_N, st);
+  __syncthreads();
   // (1) G, H, F over the polar rule with 12 radii from 0 to rm
   for (int pt = threadIdx.x; pt < 512 * BEM_GLN; pt += NP_THREADS) {
     const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-    const double w = tp.wth * 0.5 * rm * c_q.wl[ir];
+    const double w = T.w[idx] * 0.5 * rm * c_q.wl[ir];
     const double z = rr * cth + zt, e = rr * sth + et;
     double K[3], W[3];
     bem_K(el, rr, cth, sth, zt, et, K);
@@ -1338,30 +1371,26 @@ __global__ void __launch_bounds__(NP_THREADS, FS_SELF_MINB) k_fs_self(bem_dom_de
   // (2) D-bar-eps: 512 angles x 64 radii from DEPS to rm
   for (int pt = threadIdx.x; pt < 512 * BEM_GHN; pt += NP_THREADS) {
     const int idx = pt / BEM_GHN, ir = pt % BEM_GHN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * (rm - BEM_DEPS) * c_q.xh[ir] + 0.5 * (rm + BEM_DEPS);
-    const double w = tp.wth * 0.5 * (rm - BEM_DEPS) * c_q.wh[ir];
+    const double w = T.w[idx] * 0.5 * (rm - BEM_DEPS) * c_q.wh[ir];
     const double z = rr * cth + zt, e = rr * sth + et;
     double K[3], W[3];
     bem_K(el, rr, cth, sth, zt, et, K);
     for (int d = 0; d < 3; ++d) W[d] = el.cw[d][0] + el.cw[d][1] * z + el.cw[d][2] * e;
-    const double aK = sqrt(dot3(K, K)), aW = sqrt(dot3(W, W));
-    const double iK = 1.0 / aK;
+    const double K2 = dot3(K, K), iK = rsqrt(K2), aK = K2 * iK, aW = sqrt(dot3(W, W));
+    const double irr = 1.0 / rr;
     const double kR = k * aK * rr;
     const cplx ce = cexpi(kR);
     const cplx cb = cmk(-1.0, kR);
     const cplx cbce = cmul(cb, ce);
     const double KTz = dot3(K, vz), KTe = dot3(K, ve);
     // bil_sdG_Db_r: cb ce / aK^2 / r * (K.vt/aK) * N * aW
-    const double gfac = w * iK * iK / rr * aW * iK;
+    const double gfac = w * iK * iK * irr * aW * iK;
     const cplx dgz = cscale(cbce, gfac * KTz), dge = cscale(cbce, gfac * KTe);
     // bil_sdHz_Db_r: ce/(r aK^5) ((kR^2 + 3cb) K.vt cth - cb aK^2), then * sth (outer)
     // bil_sdHe_Db_r: same with sth inside and cth outer
-    const double i5 = 1.0 / (rr * aK * aK * aK * aK * aK);
+    const double i5 = irr * iK * (iK * iK) * (iK * iK);
     const cplx kk3 = cmk(kR * kR + 3.0 * cb.re, 3.0 * cb.im);
     const cplx hz = cscale(cmul(ce, csub(cscale(kk3, KTz * cth), cscale(cb, aK * aK))), w * i5 * sth);
     const cplx he = cscale(cmul(ce, csub(cscale(kk3, KTe * sth), cscale(cb, aK * aK))), w * i5 * cth);
@@ -1538,6 +1567,9 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
 #pragma unroll
   for (int c = 0; c < 16; ++c) v[c] = 0.0;
   unsigned st = 0;
+  __shared__ polar_tab T;
+  polar_fill(T, r, th, 384, st);
+  __syncthreads();
   unsigned long long nterm = 0, npt = 0;
   bool meets = !split;
   if (split) {
@@ -1559,13 +1591,9 @@ __global__ void NP_BOUNDS k_q0_self_tri(bem_dom_dev D, const __grid_constant__ b
   }
   for (int pt = threadIdx.x; pt < 384 * BEM_GLN; pt += NP_THREADS) {
     const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-    const double w = tp.wth * 0.5 * rm * c_q.wl[ir];
+    const double w = T.w[idx] * 0.5 * rm * c_q.wl[ir];
     const double z = rr * cth + zt, e = rr * sth + et;
     double K[3];
     bem_K(el, rr, cth, sth, zt, et, K);
@@ -1640,16 +1668,15 @@ __global__ void __launch_bounds__(NP_THREADS) k_fs_self_tri(bem_dom_dev D, doubl
 #pragma unroll
   for (int c = 0; c < 24; ++c) v[c] = 0.0;
   unsigned st = 0;
+  __shared__ polar_tab T;
+  polar_fill(T, r, th, 384, st);
+  __syncthreads();
   // (1) G: 3 x 128 angles x 12 radii from 0 to the edge (lit_sG_r: e^{ik aK r} / aK N)
   for (int pt = threadIdx.x; pt < 384 * BEM_GLN; pt += NP_THREADS) {
     const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-    const double w = tp.wth * 0.5 * rm * c_q.wl[ir];
+    const double w = T.w[idx] * 0.5 * rm * c_q.wl[ir];
     double K[3];
     bem_K(el, rr, cth, sth, zt, et, K);
     const double aK = sqrt(dot3(K, K));
@@ -1662,13 +1689,9 @@ __global__ void __launch_bounds__(NP_THREADS) k_fs_self_tri(bem_dom_dev D, doubl
   // (2) D-bar-eps: 3 x 128 angles x 64 radii from DEPS to the edge (lit_sdG_Db_r)
   for (int pt = threadIdx.x; pt < 384 * BEM_GHN; pt += NP_THREADS) {
     const int idx = pt / BEM_GHN, ir = pt % BEM_GHN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * (rm - BEM_DEPS) * c_q.xh[ir] + 0.5 * (rm + BEM_DEPS);
-    const double w = tp.wth * 0.5 * (rm - BEM_DEPS) * c_q.wh[ir];
+    const double w = T.w[idx] * 0.5 * (rm - BEM_DEPS) * c_q.wh[ir];
     double K[3];
     bem_K(el, rr, cth, sth, zt, et, K);
     const double aK = sqrt(dot3(K, K)), iK = 1.0 / aK;
@@ -1971,13 +1994,15 @@ extern "C" int bem_launch_qpgf(const bem_qp *q, const double *r, int n, double *
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-static bem_far far_params(const bem_dom_dev *D, const bem_qp *q, int periodic) {
+// (k: the domain's wave number)
+static bem_far far_params(const bem_dom_dev *D, const bem_qp *q, int periodic, double k) {
   bem_far fr;
   fr.on = periodic && D->far_rule;
   fr.split = 0;
+  fr.fs = !periodic && D->far_rule;
   fr.d1x = q->d1x; fr.d1y = q->d1y; fr.d2x = q->d2x; fr.d2y = q->d2y;
   fr.idet = q->idet;
-  fr.k = q->k;
+  fr.k = periodic ? q->k : k;
   return fr;
 }
 
@@ -2058,7 +2083,7 @@ extern "C" int bem_launch_assemble(const bem_dom_dev *D, const bem_qp *q, int pe
   const int split = lists && S->sm && S->sm->on;
   if (lists && cudaMemsetAsync(S->pcount, 0, 16 * sizeof(unsigned), st) != cudaSuccess) return -1;
   if (ev) cudaEventRecord(ev[0], st);
-  bem_far fr = far_params(D, q, periodic);
+  bem_far fr = far_params(D, q, periodic, k);
   fr.split = split;
   k_classify<<<N, 128, 0, st>>>(*D, fr, S->rowF, S->near_s, S->near_n, S->flag, S->status,
                                 lists ? S->pcount : nullptr, S->plist, S->pcap);
@@ -2164,7 +2189,7 @@ extern "C" int bem_launch_assemble_batch(const bem_dom_dev *D, const bem_qp *q, 
   if (!(S->plist && S->pcount && (unsigned long long)npairs <= S->pcap && npairs <= 0xffffffffLL)) return -2;
   const int split = S->sm && S->sm->on;
   if (cudaMemsetAsync(S->pcount, 0, 16 * sizeof(unsigned), st) != cudaSuccess) return -1;
-  bem_far fr = far_params(D, q, 1);
+  bem_far fr = far_params(D, q, 1, q->k);
   fr.split = split;
   k_classify<<<N, 128, 0, st>>>(*D, fr, S->rowF, S->near_s, S->near_n, S->flag, S->status, S->pcount, S->plist, S->pcap);
   bem_count_launches(1);
@@ -2265,9 +2290,10 @@ extern "C" int bem_launch_fs_deriv(const bem_dom_dev *D, double k, bem_scratch *
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-extern "C" int bem_launch_classify(const bem_dom_dev *D, const bem_qp *q, int periodic, bem_scratch *S, cudaStream_t st) {
+extern "C" int bem_launch_classify(const bem_dom_dev *D, const bem_qp *q, int periodic, double k, bem_scratch *S,
+                                   cudaStream_t st) {
   if (D->ne <= 0) return 0;
-  k_classify<<<D->ne * 4, 128, 0, st>>>(*D, far_params(D, q, periodic), S->rowF, S->near_s, S->near_n, S->flag, S->status,
+  k_classify<<<D->ne * 4, 128, 0, st>>>(*D, far_params(D, q, periodic, k), S->rowF, S->near_s, S->near_n, S->flag, S->status,
                                         nullptr, nullptr, 0);
   bem_count_launches(1);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;

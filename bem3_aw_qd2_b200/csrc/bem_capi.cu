@@ -623,6 +623,11 @@ extern "C" int bemgpu_load(bemgpu_ctx *c, const bemgpu_problem *pr) {
 }
 
 extern "C" int bemgpu_set_far_rule(bemgpu_ctx *c, int on) {
+  if (c->far_rule != (on ? 1 : 0)) {
+    // the free-space domains' matrices of the other rules are not kept
+    c->int_valid = false;
+    for (int d = 0; d < BEMGPU_MAXDOM; ++d) c->int_factored[d] = false;
+  }
   c->far_rule = on ? 1 : 0;
   c->factored = false;
   return 0;
@@ -663,7 +668,7 @@ extern "C" int bemgpu_autotune(bemgpu_ctx *c, double *best_scale) {
   if (!c->bat.empty()) { snprintf(c->err, sizeof(c->err), "a batch is loaded (load a single problem first)"); return -2; }
   if (!c->loaded) { snprintf(c->err, sizeof(c->err), "no problem loaded"); return -2; }
   bem_dom_dev D = dom_view(c, 0);
-  if (bem_launch_classify(&D, &c->qp, 1, &c->scr, c->stream)) return fail(c, "autotune", cudaGetLastError());
+  if (bem_launch_classify(&D, &c->qp, 1, c->k0[0], &c->scr, c->stream)) return fail(c, "autotune", cudaGetLastError());
   double *tab = nullptr, *stab = nullptr;
   CK(dalloc(&tab, BEM_WT_SIZE), "autotune");
   // the rule's scale and its neighbours
@@ -1064,7 +1069,7 @@ static int solve_tail(bemgpu_ctx *c) {
     // of this domain first: the free-space scratch may hold another domain's)
     bem_dom_dev D = dom_view(c, d);
     const int N = 4 * c->dom_ne[d];
-    if (bem_launch_classify(&D, &c->qp, 0, &c->scr1, c->stream)) return fail(c, "classify", cudaGetLastError());
+    if (bem_launch_classify(&D, &c->qp, 0, c->k0[d], &c->scr1, c->stream)) return fail(c, "classify", cudaGetLastError());
     for (int p0 = 0; p0 < N; p0 += c->dgh_rows) {
       const int np = N - p0 < c->dgh_rows ? N - p0 : c->dgh_rows;
       if (bem_launch_fs_deriv(&D, c->k0[d], &c->scr1, p0, np, c->dGc, c->dHc, c->stream) ||

@@ -13,7 +13,7 @@ struct bem_dom_dev {
   const uint8_t *plane;         // 1 if the element is plane (bil_check_plane)
   const int *npe;               // nodes per element: 4 bilinear quad, 3 linear triangle
   int has_tri;                  // any triangle among the domain's elements
-  int far_rule;                 // periodic domain: shorter rules for regular pairs far from every lattice image (k_q0_far)
+  int far_rule;                 // shorter rules for regular pairs far from their singularities (bem_tiers.cuh)
   int near_cap;                 // near-singular sources one collocation node can hold (<= 256):
                                 // the stride of bem_scratch.near_s / nearF
 };
@@ -63,7 +63,7 @@ int bem_launch_bdval(const bem_dom_dev *D, const bem_qp *q, int periodic, double
 int bem_launch_force_bd(const bem_dom_dev *D, int ntgt, const int *tgt_t, const double *tgt_ze, const double *wts,
                         const double *bdv, const double *pw, double k2r, double k2i, const double *rc, double c0,
                         double rho0, double *out, cudaStream_t st);
-int bem_launch_classify(const bem_dom_dev *D, const bem_qp *q, int periodic, bem_scratch *S, cudaStream_t st);
+int bem_launch_classify(const bem_dom_dev *D, const bem_qp *q, int periodic, double k, bem_scratch *S, cudaStream_t st);
 // free-space derivative rows dG, dH of rows p0 .. p0 + np - 1 only (row 2 (p - p0))
 int bem_launch_fs_deriv(const bem_dom_dev *D, double k, bem_scratch *S, int p0, int np, double *dG, double *dH,
                         cudaStream_t st);

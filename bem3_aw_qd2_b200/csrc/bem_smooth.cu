@@ -699,27 +699,14 @@ __global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ s
   int tier = -1;
   if (far_rule) {
     const double R2 = el_circum2(el, tri);
-    tier = tier_of(S.cut * S.cut / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
+    tier = tier_image(S.cut * S.cut / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
   }
   const int n = tier < 0 ? BEM_GLN : BEM_TIER_N0 - tier, npt = n * n;
   for (int part = 0; part < (tri && tier < 0 ? 3 : 1); ++part) {
     if (part) __syncthreads();
     if (tid < npt) {
-      const int i = tid / n, j = tid % n;
       double zt, et, wt;
-      if (tier >= 0) {
-        tier_point(tier, tri, i, j, zt, et);
-        wt = c_q.wt[tier][i] * c_q.wt[tier][j];
-        if (tri) wt *= 0.125 * (c_q.xt[tier][i] + 1.0);
-      } else {
-        zt = c_q.xl[i];
-        et = c_q.xl[j];
-        wt = c_q.wl[i] * c_q.wl[j];
-        if (tri) {
-          wt *= bem_tri_wfac(zt, et);
-          bem_tri_point(part, c_q.xl[i], c_q.xl[j], zt, et);
-        }
-      }
+      rule_pt(n, tri, part * npt + tid, zt, et, wt);
       double r[3], W[3], Nn[4];
       bem_rw(el, zt, et, r, W);
       bem_Nn(tri, zt, et, Nn);
@@ -941,7 +928,6 @@ __global__ void __launch_bounds__(GM_TH, 2) k_sm_gemm(const double *A0, size_t s
 // geometry is formed once for all.  A warp takes the longest rule its pairs
 // ask for.  FP64 pipe: about 66 operations per image and point.
 #define SMI_TH 128
-__device__ __forceinline__ int sm_rule_points(int n, bool tri) { return n == BEM_GLN ? (tri ? 3 : 1) * BEM_GLN * BEM_GLN : n * n; }
 template <int LP>
 __global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__ sm_dev S, bem_dom_dev D, int far_rule,
                                                          const uint8_t *__restrict__ flag,
@@ -975,7 +961,7 @@ __global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__
       }
       d2 = fma(el.cr[2][0], el.cr[2][0], d2);
       const double R2 = el_circum2(el, tri);
-      const int t = tier_of(d2 / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
+      const int t = tier_image(d2 / R2, S.k * S.k * R2, tri, tri || quad_tier_shape(el));
       if (t >= 0) n2 = BEM_TIER_N0 - t;
     }
     if (S.nimg == 1) n2 = 0;
@@ -991,27 +977,11 @@ __global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__
   for (int grp = 0; grp < 2; ++grp) {
     if (grp == 0 ? n1 == 0 : (!live || n2 == 0)) continue;
     const int n = grp == 0 ? n1 : n2;
-    const int m0 = grp, m1 = grp == 0 ? 1 : S.nimg, np = sm_rule_points(n, tri);
-    const int t = BEM_TIER_N0 - n;
+    const int m0 = grp, m1 = grp == 0 ? 1 : S.nimg, np = rule_npts(n, tri);
 #pragma unroll 1
     for (int pt = sub; pt < np; pt += LP) {
       double z, e, wt;
-      if (n == BEM_GLN) {
-        const int part = pt / (BEM_GLN * BEM_GLN), ij = pt % (BEM_GLN * BEM_GLN);
-        const double a = c_q.xl[ij / BEM_GLN], c = c_q.xl[ij % BEM_GLN];
-        z = a;
-        e = c;
-        wt = c_q.wl[ij / BEM_GLN] * c_q.wl[ij % BEM_GLN];
-        if (tri) {
-          bem_tri_point(part, a, c, z, e);
-          wt *= bem_tri_wfac(a, c);
-        }
-      } else {
-        const int i = pt / n, j = pt - i * n;
-        tier_point(t, tri, i, j, z, e);
-        wt = c_q.wt[t][i] * c_q.wt[t][j];
-        if (tri) wt *= 0.125 * (c_q.xt[t][i] + 1.0);
-      }
+      rule_pt(n, tri, pt, z, e, wt);
       double R[3], W[3];
       bem_rw(el, z, e, R, W);
       const double rz2 = R[2] * R[2], rzw = R[2] * W[2];

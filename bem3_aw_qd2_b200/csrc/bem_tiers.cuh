@@ -50,6 +50,47 @@ __device__ __forceinline__ int tier_of(double r2, double kR2, bool tri, bool sha
   if (!shape) return r2 >= 25.0 ? 2 : -1;
   return r2 >= 625.0 && kR2 <= 0.04 ? 4 : r2 >= 64.0 && kR2 <= 0.25 ? 3 : r2 >= 25.0 ? 2 : r2 >= 12.25 ? 1 : r2 >= 9.0 ? 0 : -1;
 }
+// The same for a part of a pair that is not its nearest image: flat quads
+// inside the shape guard reach 2e-13 of the image's largest entry with 7 points
+// from 6 R and with 6 from 10 R (k R <= 0.5; numpy, random directions, twists and
+// aspects inside the guard), so 7 from 7 R and 6 from 12 R here.
+__device__ __forceinline__ int tier_image(double r2, double kR2, bool tri, bool shape) {
+  if (tri || !shape) return tier_of(r2, kR2, tri, shape);
+  if (kR2 > 1.0) return -1;
+  return r2 >= 144.0 && kR2 <= 0.25 ? 4 : r2 >= 49.0 && kR2 <= 0.25 ? 3 : r2 >= 25.0 ? 2 : r2 >= 12.25 ? 1 : r2 >= 9.0 ? 0 : -1;
+}
+// Free space, with the tangential derivatives of G and H (a third-order
+// singularity), and the geometric sums: 1e-14 of the largest entry of each
+// matrix, the rounding of the 144-point sums themselves (numpy, as above; quads
+// and triangles alike): 10 points from 4 R, 9 from 5, 8 from 7, 7 from 9
+// (k R <= 0.5), 6 from 16 (k R <= 0.25).
+__device__ __forceinline__ int tier_free(double r2, double kR2, bool shape) {
+  if (kR2 > 1.0 || !shape) return -1;
+  return r2 >= 256.0 && kR2 <= 0.0625 ? 4 : r2 >= 81.0 && kR2 <= 0.25 ? 3 : r2 >= 49.0 ? 2 : r2 >= 25.0 ? 1 : r2 >= 16.0 ? 0 : -1;
+}
+// points of rule n on an element: 12 is the reference's 12 x 12 (3 parts of it on
+// a triangle), 6 .. 10 a tier's n x n; point pt of it, its weight as those of the
+// 12 x 12 rules (relative to W)
+__device__ __forceinline__ int rule_npts(int n, bool tri) { return n == BEM_GLN && tri ? 3 * BEM_GLN * BEM_GLN : n * n; }
+__device__ __forceinline__ void tier_point(int t, bool tri, int i, int j, double &z, double &e);
+__device__ __forceinline__ void rule_pt(int n, bool tri, int pt, double &z, double &e, double &wt) {
+  if (n == BEM_GLN) {
+    const int part = pt / (BEM_GLN * BEM_GLN), ij = pt % (BEM_GLN * BEM_GLN);
+    const double a = c_q.xl[ij / BEM_GLN], c = c_q.xl[ij % BEM_GLN];
+    z = a;
+    e = c;
+    wt = c_q.wl[ij / BEM_GLN] * c_q.wl[ij % BEM_GLN];
+    if (tri) {
+      bem_tri_point(part, a, c, z, e);
+      wt *= bem_tri_wfac(a, c);
+    }
+  } else {
+    const int t = BEM_TIER_N0 - n, i = pt / n, j = pt - i * n;
+    tier_point(t, tri, i, j, z, e);
+    wt = c_q.wt[t][i] * c_q.wt[t][j];
+    if (tri) wt *= 0.125 * (c_q.xt[t][i] + 1.0);
+  }
+}
 // point (i, j) of tier t's rule: Gauss on a quad; on a triangle the collapsed
 // (Duffy) rule over the whole reference triangle, (z, e) = (1 - 3u/2,
 // sqrt3/2 u (1 - 2v)) for (u, v) in [0, 1]^2, weight u w_u w_v

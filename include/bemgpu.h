@@ -89,9 +89,9 @@ int bemgpu_load(bemgpu_ctx *ctx, const bemgpu_problem *prob);
 #define BEMGPU_EWALD_RULE 0.0
 int bemgpu_set_ewald_scale(bemgpu_ctx *ctx, double scale);
 
-/* Quadrature of the regular pairs of the periodic domain (no counterpart in
+/* Quadrature of the regular pairs (no counterpart in
  * the reference, which uses its 12 x 12 Gauss rule for every regular pair,
- * on each of 3 parts of a triangle): on = 1 (the default) uses a shorter
+ * on each of 3 parts of a triangle): on = 1 (the default) uses, in the periodic domain, a shorter
  * n x n rule (Gauss on a quad, collapsed over a whole triangle) where the
  * source element's centre is at least d circumradii R from the nearest
  * lattice image of the collocation node:
@@ -102,8 +102,11 @@ int bemgpu_set_ewald_scale(bemgpu_ctx *ctx, double scale);
  * is at most a tenth of the shorter half-side and whose half-sides are within
  * 3x (every triangle).  Each reproduces the reference's integrals to about
  * 1e-13 of the pair's largest entry with up to 4 (quads) or 12 (triangles)
- * times fewer Green's-function values; on = 0 keeps the reference's rules
- * everywhere.  Applies from the next assembly. */
+ * times fewer Green's-function values.  The free-space domains and the
+ * geometric sums take such rules by the distance from the node itself, from
+ * farther out (10 from 4, 9 from 5, 8 from 7, 7 from 9, 6 from 16), where they
+ * reach 1e-14 with the tangential derivatives.  on = 0 keeps the reference's
+ * rules everywhere.  Applies from the next assembly. */
 int bemgpu_set_far_rule(bemgpu_ctx *ctx, int on);
 /* Regular pairs of the periodic domain by rule in the last assembly:
  * counts[0] on the reference's 12 x 12 rule, counts[1 .. 5] on the 10, 9, 8,
