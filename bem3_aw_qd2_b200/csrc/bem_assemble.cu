@@ -27,6 +27,7 @@
 #include "bem_qpgf.cuh"
 #include "bem_geom.cuh"
 #include "bem_tiers.cuh"
+#include "bem_rules.cuh"
 #include "bem_kernels.h"
 #include "bem_smooth.h"
 
@@ -55,7 +56,6 @@ __device__ __forceinline__ void bem_load_node(const bem_dom_dev &D, int p, bem_n
   for (int d = 0; d < 3; ++d) { n.vz[d] /= az; n.vt[d] /= ae; }
 }
 
-__device__ __forceinline__ double dot3(const double a[3], const double b[3]) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 
 // element e (0-based) is a linear triangle
 __device__ __forceinline__ bool bem_is_tri(const bem_dom_dev &D, int e) { return D.has_tri && __ldg(D.npe + e) == 3; }
@@ -65,7 +65,6 @@ __device__ __forceinline__ bool bem_pad_row(const bem_dom_dev &D, int p) {
   return (p & 3) == 3 && bem_is_tri(D, abs(D.sid[p >> 2]) - 1);
 }
 
-__device__ __forceinline__ void set_status(unsigned *st, unsigned bits) { if (bits) atomicOr(st, bits); }
 
 // warp-aggregated work counters (lattice terms and Green's-function points);
 // every lane of the warp must call it
@@ -140,11 +139,6 @@ __device__ __forceinline__ double pair_ratio2(const bem_far &fr, const bem_el &e
     }
   return dmin2 / R2;
 }
-// Quadrature points closer than this to the lattice plane through the node
-// keep a pair on the reference's rule: there the reference's lattice sums
-// stop on rounding-decided zeros, so its values at its own points are not a
-// smooth function that another rule could reproduce.
-#define BEM_FAR_PLANE_TOL 1e-10
 // tier of a regular pair, or -1 for the reference's rule (whose points the
 // caller has checked against the lattice plane); none of the tier's points
 // may lie within BEM_FAR_PLANE_TOL of rt's lattice plane either (-2: one does)
@@ -702,26 +696,6 @@ __global__ void __launch_bounds__(FP_THREADS, FP_MINB) k_q0_far(bem_dom_dev D, c
 // ------------------------------------------------------------------ periodic near-singular pairs
 // 64x64 points (q0_bil_dcoef_v2_cc_GH, q0_bil_dcoef_v2_cc.c:206-281).
 #define NP_THREADS 256
-// The home-cell image of the quasi-periodic Green's function: the free-space
-// e^{ikR} / (4 pi R) and its gradient at r, in bem_qpgf's conventions.  The
-// near-singular and self integrals split G_qp = G0 + (G_qp - G0): G0 carries
-// the whole singularity and costs a sincos, so it is integrated on the
-// reference's own points (64 x 64 Gauss, the polar rule); the rest is smooth
-// over the element (its nearest singularities are the other lattice images)
-// and is integrated on the 12 x 12 Gauss rule of regular pairs, a lattice sum
-// at 144 points instead of 4096 or 6144.
-__device__ __forceinline__ void bem_g0(double k, const double vR[3], bem_gval &o) {
-  const double R2 = vR[0] * vR[0] + vR[1] * vR[1] + vR[2] * vR[2];
-  const double R = sqrt(R2), iR = 1.0 / R;
-  const cplx ce = cexpi(k * R);
-  const double c4 = 0.07957747154594766788 * iR;  // 1 / (4 pi R)
-  o.g = cscale(ce, c4);
-  // (i k R - 1) e^{ikR} / (4 pi R^3) times r
-  const cplx f = cscale(cmul(cmk(-1.0, k * R), ce), c4 * iR * iR);
-  o.gx = cscale(f, vR[0]);
-  o.gy = cscale(f, vR[1]);
-  o.gz = cscale(f, vR[2]);
-}
 // accumulate a point's G and H contributions: g = gv.g |W| wg, h = (grad gv . W) wh
 __device__ __forceinline__ void acc_gh(double (&v)[19], const bem_gval &gv, const double vW[3], double wg, double wh,
                                        const double N[4]) {
@@ -922,63 +896,6 @@ __global__ void NP_BOUNDS k_q0_near(bem_dom_dev D, const __grid_constant__ bem_q
 // 4 sub-triangles x (2 x 64) angles x 12 radii (q0_bil_coef_bd, q0_bil_coef.c:246-338,
 // and bil_coef_bd, bil_coef.c:244-342).  The angular rule of the reference
 // splits each sub-triangle's angle range in two halves with 64 points each.
-struct polar_pt { double th, wth; int j; };
-__device__ __forceinline__ polar_pt polar_theta(const double th[5], int idx /* 0..511 */) {
-  const int j = idx >> 7, h = (idx >> 6) & 1, m = idx & 63;
-  const double t0 = th[j], t1 = th[j + 1];
-  polar_pt r;
-  r.th = h == 0 ? 0.25 * (t1 - t0) * c_q.xh[m] + 0.25 * (t1 + 3.0 * t0) : 0.25 * (t1 - t0) * c_q.xh[m] + 0.25 * (3.0 * t1 + t0);
-  r.wth = c_q.wh[m] * 0.25 * (t1 - t0);
-  r.j = j;
-  return r;
-}
-
-// The rule's angles as a table in shared memory (nang <= 512): cosine, sine,
-// radius to the edge, weight.  Each angle serves 12 or 64 radii, whose points
-// otherwise form its four trigonometric functions again.  All threads; the
-// caller synchronises.
-#define POLAR_N 512
-struct polar_tab { double c[POLAR_N], s[POLAR_N], rm[POLAR_N], w[POLAR_N]; };
-__device__ __forceinline__ void polar_fill(polar_tab &T, const double r[5], const double th[5], int nang, unsigned &st) {
-  for (int i = threadIdx.x; i < nang; i += blockDim.x) {
-    const polar_pt tp = polar_theta(th, i);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    sincos(tp.th, &T.s[i], &T.c[i]);
-    T.rm[i] = rm;
-    T.w[i] = tp.wth;
-  }
-}
-
-// geometric F of the element at parameter point (zt,et) by the polar rule (q0_bil_coef_bd_F,
-// q0_bil_dcoef_v2_cc.c:401-454 / bil_sF_theta): returns the un-normalised sum (times bdC/4pi later)
-__device__ double polar_F_partial(const bem_el &el, double zt, double et, unsigned &st) {
-  double r[5], th[5];
-  bem_node_r_th(zt, et, r, th);
-  double acc = 0.0;
-  for (int idx = threadIdx.x; idx < 512; idx += blockDim.x) {
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
-    double inner = 0.0;
-    for (int ir = 0; ir < BEM_GLN; ++ir) {
-      const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-      double K[3];
-      bem_K(el, rr, cth, sth, zt, et, K);
-      const double aK = sqrt(K[0] * K[0] + K[1] * K[1] + K[2] * K[2]);
-      inner += c_q.wl[ir] / (aK * aK * aK) * cth * sth;
-    }
-    acc += tp.wth * 0.5 * rm * inner;
-  }
-  return acc;
-}
-
-__device__ __forceinline__ double bem_bdC(const bem_el &el) {
-  return el.cr[0][1] * el.cw[0][2] + el.cr[1][1] * el.cw[1][2] + el.cr[2][1] * el.cw[2][2];
-}
-
 // periodic self pair: one block per collocation node p
 // point pt of the polar rule around the node (zt, et) on its own quad: (z, e),
 // the weight with the polar Jacobian, R = rr K from the node, W

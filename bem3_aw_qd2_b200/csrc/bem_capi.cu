@@ -53,7 +53,7 @@ struct bemgpu_ctx {
   // images + expansion of the periodic domain (bem_smooth.cu): its tables, and
   // its workspace where the global matrix is too small to lend its own
   bem_smooth sm;
-  double *sm_tab = nullptr, *sm_buf = nullptr;
+  double *sm_tab = nullptr, *sm_keep = nullptr, *sm_buf = nullptr;
   double zspan = 0.0;      // height of the mesh (z extent of all elements)
   double pw[16] = {};      // incident plane wave (bemgpu_problem.pw)
   int far_rule = 1;        // shorter rules for regular pairs of the periodic domain (bemgpu_set_far_rule)
@@ -208,7 +208,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
       dfree(S->rowF); dfree(S->near_s); dfree(S->near_n); dfree(S->nearF); dfree(S->selfF); dfree(S->flag);
     }
     dfree(c->scr.plist); dfree(c->scr.pcount);
-    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_buf); dfree(c->b0); dfree(c->B3s);
+    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->b0); dfree(c->B3s);
     for (int d = 0; d < BEMGPU_MAXDOM; ++d) { dfree(c->Wd[d]); dfree(c->cinv[d]); dfree(c->Gc[d]); }
     dfree(c->B3c);
     dfree(c->dGc); dfree(c->dHc);
@@ -405,6 +405,9 @@ static int smooth_setup(bemgpu_ctx *c, int inst, const bem_qp *qps) {
   CK(falloc(c, &c->sm_tab, h.size()), "expansion tables");
   CK(cudaMemcpyAsync(c->sm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
   c->sm.tab = c->sm_tab;
+  CK(falloc(c, &c->sm_keep, bem_smooth_keep_doubles(&c->sm)), "expansion");
+  c->sm.keep = c->sm_keep;
+  c->sm.have0 = c->sm.have1 = 0;
   const size_t need = bem_smooth_ws_doubles(&c->sm, c->dom_ne[0]);
   if (inst == 1 && need <= 2 * (size_t)c->n * c->n) {
     c->sm.ws = c->A;
@@ -1310,6 +1313,16 @@ static int ensure_force_targets(bemgpu_ctx *c);
 static int ensure_centres(bemgpu_ctx *c);
 static bem_dom_dev dom_view(bemgpu_ctx *c, int d);
 
+// boundary sums of the periodic domain: with images and expansion where the
+// problem takes the split, point by point otherwise
+static int bdval0(bemgpu_ctx *c, const bem_dom_dev *D, int type, int n, const int *t, const double *ze, double *out) {
+  if (c->sm.on)
+    return bem_launch_bdsum(&c->sm, D, &c->qp, type, n, t, ze, c->P[0], c->dP[0], c->pv[0], c->dpv[0], out, c->status,
+                            c->stream);
+  return bem_launch_bdval(D, &c->qp, 1, c->k0[0], type, n, t, ze, c->P[0], c->dP[0], c->pv[0], c->dpv[0], out, c->status,
+                          c->stream);
+}
+
 extern "C" int bemgpu_force(bemgpu_ctx *c, int type, const double *rc, double *F, double *N) {
   if (!c->loaded) { snprintf(c->err, sizeof(c->err), "no problem loaded"); return -2; }
   CK(cudaMemcpyAsync(c->rc_d, rc, 3 * sizeof(double), cudaMemcpyHostToDevice, c->stream), "rc");
@@ -1319,8 +1332,7 @@ extern "C" int bemgpu_force(bemgpu_ctx *c, int type, const double *rc, double *F
       // boundary values at the centres of the domain-0 triangles (lit_force_4p's 4th point)
       if (ensure_centres(c)) return -1;
       bem_dom_dev D = dom_view(c, 0);
-      if (bem_launch_bdval(&D, &c->qp, 1, c->k0[0], 0, c->nctr, c->ctr_t, c->ctr_ze, c->P[0], c->dP[0], c->pv[0],
-                           c->dpv[0], c->ctr_bdv, c->status, c->stream))
+      if (bdval0(c, &D, 0, c->nctr, c->ctr_t, c->ctr_ze, c->ctr_bdv))
         return fail(c, "force", cudaGetLastError());
       ctr = c->ctr_idx;
     }
@@ -1331,8 +1343,7 @@ extern "C" int bemgpu_force(bemgpu_ctx *c, int type, const double *rc, double *F
     // boundary values at the rule points of every domain-0 element, then the stress integral
     if (ensure_force_targets(c)) return -1;
     bem_dom_dev D = dom_view(c, 0);
-    if (bem_launch_bdval(&D, &c->qp, 1, c->k0[0], 1, c->ntgt, c->tgt_t, c->tgt_ze, c->P[0], c->dP[0], c->pv[0], c->dpv[0], c->bdv,
-                         c->status, c->stream) ||
+    if (bdval0(c, &D, 1, c->ntgt, c->tgt_t, c->tgt_ze, c->bdv) ||
         bem_launch_force_bd(&D, c->ntgt, c->tgt_t, c->tgt_ze, c->tgt_w, c->bdv, c->pw_d, c->k2[0], c->k2[1], c->rc_d,
                             c->c0[0], c->rho0[0], c->fout, c->stream))
       return fail(c, "force", cudaGetLastError());
@@ -1413,8 +1424,9 @@ extern "C" int bemgpu_boundary_field(bemgpu_ctx *c, int d, int type, int n, cons
   bem_dom_dev D = dom_view(c, d);
   CK(cudaMemcpyAsync(c->pt_t, t, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream), "targets");
   CK(cudaMemcpyAsync(c->pt_in, ze, 2 * sizeof(double) * n, cudaMemcpyHostToDevice, c->stream), "targets");
-  if (bem_launch_bdval(&D, &c->qp, d == 0, c->k0[d], type, n, c->pt_t, c->pt_in, c->P[d], c->dP[d], c->pv[d],
-                       c->dpv[d], c->pt_out, c->status, c->stream))
+  if (d == 0 ? bdval0(c, &D, type, n, c->pt_t, c->pt_in, c->pt_out)
+             : bem_launch_bdval(&D, &c->qp, 0, c->k0[d], type, n, c->pt_t, c->pt_in, c->P[d], c->dP[d], c->pv[d],
+                                c->dpv[d], c->pt_out, c->status, c->stream))
     return fail(c, "boundary field", cudaGetLastError());
   CK(cudaMemcpyAsync(out, c->pt_out, 9 * sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream), "boundary field");
   CK(cudaStreamSynchronize(c->stream), "boundary field");

@@ -34,7 +34,7 @@ struct bem_scratch {
   unsigned long long *terms;  // [6] lattice terms of regular / near / self pairs, then point counts
   // periodic domain: images + expansion in place of the regular pairs' lattice
   // sums (bem_smooth.h), when set and on
-  const struct bem_smooth *sm = nullptr;
+  struct bem_smooth *sm = nullptr;
 };
 #define BEM_FL_REF 8     // regular pair on the 12 x 12 rule, no point on the lattice plane
 #define BEM_PC_PLANE 12

@@ -17,75 +17,11 @@
 // Bloch phase.  Rules: type 0 4 nodes, 1 9-point, 2 12x12 GL, 3 64x64 GL.
 #pragma once
 
+#include "bem_rules.cuh"
+
 #define FIELD_THREADS 128
 
 struct fld_acc { double s0r, s0i, s1[6], f, df[3], s2[6]; };  // 18 doubles
-
-// rule point idx of a source element: parameter point, weight, node flag
-__device__ __forceinline__ int rule_points(int type) {
-  return type == 0 ? 4 : (type == 1 ? 9 : (type == 2 ? BEM_GLN * BEM_GLN : BEM_GHN * BEM_GHN));
-}
-
-__device__ __forceinline__ void rule_point(int type, int i, double &z, double &e, double &w) {
-  if (type == 0) { z = c_q.zt[i]; e = c_q.et[i]; w = 1.0; }
-  else if (type == 1) { z = c_q.z9[i]; e = c_q.e9[i]; w = c_q.w9[i]; }
-  else if (type == 2) { z = c_q.xl[i / BEM_GLN]; e = c_q.xl[i % BEM_GLN]; w = c_q.wl[i / BEM_GLN] * c_q.wl[i % BEM_GLN]; }
-  else { z = c_q.xh[i / BEM_GHN]; e = c_q.xh[i % BEM_GHN]; w = c_q.wh[i / BEM_GHN] * c_q.wh[i % BEM_GHN]; }
-}
-
-// Rules on a triangle source (q0_lit_coef_4p / _7p / _GL / _GH, q0_lit_coef.c:10-250):
-// type 0: the 3 nodes and the centre (weights 25/48 x 3, -27/48), 1: 7-point rule,
-// 2, 3: the 3-part 12 x 12 / 64 x 64 rules.  w multiplies W = cw0 (twice the area).
-__device__ __forceinline__ int tri_rule_points(int type) {
-  return type == 0 ? 4 : (type == 1 ? 7 : 3 * (type == 2 ? BEM_GLN * BEM_GLN : BEM_GHN * BEM_GHN));
-}
-__device__ __forceinline__ void tri_rule_point(int type, int i, double &z, double &e, double &w) {
-  if (type == 0) {
-    if (i < 3) bem_tri_node(i, z, e);
-    else z = e = 0.0;
-    w = 0.5 * (i < 3 ? 25.0 / 48.0 : -27.0 / 48.0);
-  } else if (type == 1) {
-    // the 7-point rule (zt_37, et_37, wt_37, bem3_aw_qd2.c:1012-1021)
-    const double n0 = 0.3480702390148154917985, n1 = 0.2052130961576726346557;
-    const double n2 = 0.6028753385763033130539, n3 = 0.3554395089236065568357;
-    const double v0 = 0.1259391805448271525957, v1 = 0.1323941527885061807376, v2 = 0.225;
-    const double zz[7] = {-n0, 2.0 * n0, -n0, n1, -2.0 * n1, n1, 0.0}, ee[7] = {-n2, 0.0, n2, n3, 0.0, -n3, 0.0};
-    z = zz[i];
-    e = ee[i];
-    w = 0.5 * (i < 3 ? v0 : (i < 6 ? v1 : v2));
-  } else {
-    const int n = type == 2 ? BEM_GLN : BEM_GHN;
-    const double *x = type == 2 ? c_q.xl : c_q.xh, *wq = type == 2 ? c_q.wl : c_q.wh;
-    const int part = i / (n * n), ij = i % (n * n), a = ij / n, b = ij % n;
-    bem_tri_point(part, x[a], x[b], z, e);
-    w = wq[a] * wq[b] * bem_tri_wfac(x[a], x[b]);
-  }
-}
-
-// boundary values of source element s interpolated at (z,e); type 0 uses the
-// node value itself (the 4-point rule sits on the nodes; the triangle's centre
-// point takes the mean of its 3 nodes)
-__device__ __forceinline__ void interp_bv(int type, int i, double z, double e, int s, const double *P, const double *dP,
-                                          const double *pv, const double *dpv, cplx &Pn, cplx &dPn, cplx pvn[3],
-                                          cplx dpvn[3], bool tri = false) {
-  double N[4];
-  if (type == 0 && !(tri && i == 3)) {
-    for (int a = 0; a < 4; ++a) N[a] = a == i ? 1.0 : 0.0;
-  } else {
-    bem_Nn(tri, z, e, N);
-  }
-  Pn = dPn = cmk(0, 0);
-  for (int c = 0; c < 3; ++c) pvn[c] = dpvn[c] = cmk(0, 0);
-  for (int a = 0; a < 4; ++a) {
-    const size_t o = (size_t)s * 4 + a;
-    Pn = cadd(Pn, cscale(cmk(P[2 * o], P[2 * o + 1]), N[a]));
-    dPn = cadd(dPn, cscale(cmk(dP[2 * o], dP[2 * o + 1]), N[a]));
-    for (int c = 0; c < 3; ++c) {
-      pvn[c] = cadd(pvn[c], cscale(cmk(pv[2 * (3 * o + c)], pv[2 * (3 * o + c) + 1]), N[a]));
-      dpvn[c] = cadd(dpvn[c], cscale(cmk(dpv[2 * (3 * o + c)], dpv[2 * (3 * o + c) + 1]), N[a]));
-    }
-  }
-}
 
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm /* NV*(FIELD_THREADS/32) + NV */) {
@@ -297,15 +233,14 @@ __global__ void __launch_bounds__(FIELD_THREADS) k_bdval(bem_dom_dev D, const __
   else bem_node_r_th(zt, et, r, th);
   const bool plane = D.plane[te] != 0;
   const double sgt = D.sid[t] < 0 ? -1.0 : 1.0, bdC = bem_bdC(elt);
+  __shared__ polar_tab T;
+  polar_fill(T, r, th, ttri ? 384 : 512, st);
+  __syncthreads();
   for (int pt = threadIdx.x; pt < (ttri ? 384 : 512) * BEM_GLN; pt += FIELD_THREADS) {
     const int idx = pt / BEM_GLN, ir = pt % BEM_GLN;
-    const polar_pt tp = polar_theta(th, idx);
-    const double rm = bem_rmax(r[tp.j], r[tp.j + 1], th[tp.j], th[tp.j + 1], tp.th);
-    if (rm < 0.0) st |= BEM_ST_GEOMETRY;
-    double sth, cth;
-    sincos(tp.th, &sth, &cth);
+    const double rm = T.rm[idx], sth = T.s[idx], cth = T.c[idx];
     const double rr = 0.5 * rm * (c_q.xl[ir] + 1.0);
-    const double w = tp.wth * 0.5 * rm * c_q.wl[ir] * rr;
+    const double w = T.w[idx] * 0.5 * rm * c_q.wl[ir] * rr;
     const double z = rr * cth + zt, e = rr * sth + et;
     double K[3], vR[3], vW[3];
     bem_K(elt, rr, cth, sth, zt, et, K);

@@ -41,6 +41,7 @@
 #include "bem_geom.cuh"
 #include "bem_tiers.cuh"
 #include "bem_kernels.h"
+#include "bem_rules.cuh"
 #include "bem_smooth.h"
 
 extern "C" int bem_smooth_set_constants(const void *quad, const void *wc) {
@@ -95,6 +96,7 @@ static int degree_for(double k, double a, double b, double scale, double tol, in
 
 void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int *npe, const int *sid, int ne) {
   S->on = 0;
+  S->have0 = S->have1 = 0;
   if (ne <= 0) return;
   // the ball of the body: corners (+-1, +-1) of a quad, (1, 0), (-1/2,
   // +-sqrt3/2) of a triangle; every point of an element is a convex
@@ -172,6 +174,13 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
     }
   }
   if (!S->on) return;
+  // degrees for one point's rest at |R| <= (i + 1) 2 R0 / 8 (the gradient's terms are
+  // those of the value times l / |R|)
+  for (int i = 0; i < 8; ++i) {
+    const double f = (i + 1) / 8.0;
+    const int l = degree_for(S->k, f * S->rho, S->cut + S->rho, 6.0 * S->rho, f * 1e-15, S->Lmax);
+    S->lcut[i] = l < 0 ? S->Lmax : l;
+  }
   // windows of the samples' Ewald sums: the reference's parameter below its cap
   // (k^2 eta^2 < 3); terms to e^{-40} of the leading one; the images among them
   S->eta = std::min(q->eta0, 0.98 * sqrt(3.0) / S->k);
@@ -297,32 +306,47 @@ struct sm_dev {
   double eta;                       // Ewald parameter of the samples
   int nreal, r1, r2, nspec, s1, s2, sc2;  // its windows: l1 in [-r1, r1], l2 in [-r2, r2]; n1 - nc1 in [-s1, s1], ...
   int iml[2 * BEM_SM_MAXIMG];       // the images' indices
+  int lcut[8];                      // degrees of the expansion about a point at |R| <= (i + 1) 2 R0 / 8
   const double *x, *w, *ca, *cb, *dL, *el, *rec, *img;
   double *plm;            // [nt][lm >= 0] normalised Legendre functions P_lm(x_t)
   double *samp;           // [nb][2][nt][nphi] complex: G_s and rho dG_s/drho
   double *sig;            // [nb][(Lmax + 1)^2] complex
   double *T;              // [nb][Kp][2 Kp]: T^t, real and imaginary parts
+  double *Z, *Zt;         // densities of boundary sums: [32][Kp][8], [Kp][8]
   double *U, *V, *A;      // [4 ne][Kp], [Kp][8 ne], [nb][4 ne][2 Kp]
 };
-struct sm_ws { size_t plm, samp, sig, T, U, V, A, total; };
-static sm_ws ws_layout(const bem_smooth *S, int ne, int nb) {
-  sm_ws w;
+// What stays valid after an assembly (for boundary sums): Legendre functions,
+// samples, sigma, T of up to BEM_SM_BAT instances, the densities
+struct sm_keep { size_t plm, samp, sig, T, Z, Zt, total; };
+static sm_keep keep_layout(const bem_smooth *S) {
+  sm_keep w;
   size_t o = 0;
   auto put = [&o](size_t n) { const size_t p = o; o += (n + 31) / 32 * 32; return p; };
-  const size_t L = S->Lmax, Kp = S->Kp;
+  const size_t L = S->Lmax, Kp = S->Kp, nb = std::min(S->inst, BEM_SM_BAT);
   w.plm = put((L + 1) * (L + 2) / 2 * S->nt);
-  w.samp = put((size_t)nb * 4 * S->nt * S->nphi);
-  w.sig = put((size_t)nb * 2 * (L + 1) * (L + 1));
-  w.T = put((size_t)nb * 2 * Kp * Kp);
-  w.U = put(4 * (size_t)ne * Kp);
-  w.V = put(8 * (size_t)ne * Kp);
-  w.A = put((size_t)nb * 8 * ne * Kp);
+  w.samp = put(nb * 4 * S->nt * S->nphi);
+  w.sig = put(nb * 2 * (L + 1) * (L + 1));
+  w.T = put(nb * 2 * Kp * Kp);
+  w.Z = put(32 * Kp * 8);
+  w.Zt = put((Kp + 1) * 8);
   w.total = o;
   return w;
 }
-size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne) {
-  return ws_layout(S, ne, std::min(S->inst, BEM_SM_BAT)).total;
+size_t bem_smooth_keep_doubles(const bem_smooth *S) { return keep_layout(S).total; }
+// and an assembly's scratch
+struct sm_ws { size_t U, V, A, total; };
+static sm_ws ws_layout(const bem_smooth *S, int ne) {
+  sm_ws w;
+  size_t o = 0;
+  auto put = [&o](size_t n) { const size_t p = o; o += (n + 31) / 32 * 32; return p; };
+  const size_t Kp = S->Kp, nb = std::min(S->inst, BEM_SM_BAT);
+  w.U = put(4 * (size_t)ne * Kp);
+  w.V = put(8 * (size_t)ne * Kp);
+  w.A = put(nb * 8 * ne * Kp);
+  w.total = o;
+  return w;
 }
+size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne) { return ws_layout(S, ne).total; }
 
 struct sm_qps { bem_qp q[BEM_SM_BAT]; };
 struct sm_out { double *G[BEM_SM_BAT], *H[BEM_SM_BAT]; };
@@ -674,6 +698,84 @@ __global__ void __launch_bounds__(SMU_TH) k_sm_targets(const __grid_constant__ s
   }
 }
 
+// The values of order m at a point (r, W): for each degree l the rows |W| phi and
+// W . grad phi of the cosine (and of the sine) function, SMV_PT apart, at val.
+#define SMV_PT (BEM_GLN * BEM_GLN)
+__device__ __forceinline__ void sm_point_values(const sm_dev &S, int m, int nf, const double r[3], const double W[3],
+                                                double *val) {
+        const double aW = sqrt(W[0] * W[0] + W[1] * W[1] + W[2] * W[2]);
+        const double x = (r[0] - S.cx) * S.iR0, y = (r[1] - S.cy) * S.iR0, z = (r[2] - S.cz) * S.iR0;
+        const double s2 = x * x + y * y + z * z;
+        const double wx = W[0] * S.iR0, wy = W[1] * S.iR0, wz = W[2] * S.iR0;
+        const double wr = wx * x + wy * y + wz * z;
+        // Re, Im (x + iy)^m and their derivatives along W
+        double C = 1.0, Sn = 0.0, C0 = 0.0, S0 = 0.0;
+        for (int a = 0; a < m; ++a) {
+          C0 = C;
+          S0 = Sn;
+          const double c2 = C * x - Sn * y;
+          Sn = C * y + Sn * x;
+          C = c2;
+        }
+        double dC = m * (wx * C0 - wy * S0), dS = m * (wx * S0 + wy * C0);
+        if (m) {
+          const double q2 = 1.4142135623730950488;
+          C *= q2; Sn *= q2; dC *= q2; dS *= q2;
+        }
+        // g_l downward from l = lmax + 1, kept in the value slots until used
+        const double z2 = S.kR0 * S.kR0 * s2, kk2 = S.kR0 * S.kR0;
+        // upward walk needs g_l and g_{l+1}: g is computed into val[l - m][0]
+        // (read before it is overwritten) with g_{lmax + 1} kept in a register
+        double gtop;
+        {
+          double a = 0.0, b = 0.0;
+  #pragma unroll 1
+          for (int w = 0; w < 2; ++w) {
+            const int l = S.lmax + 2 - w;
+            double t = 1.0, sum = 1.0;
+            for (int q = 1; q < 100; ++q) {
+              t *= -0.5 * z2 / (q * (2.0 * l + 2.0 * q + 1.0));
+              sum += t;
+              if (fabs(t) < 1e-18 * fabs(sum)) break;
+            }
+            if (w == 0) a = sum;
+            else b = sum;
+          }
+          gtop = b;
+          for (int l = S.lmax + 1; l > m; --l) {
+            const double c = b - z2 / ((2.0 * l + 1.0) * (2.0 * l + 3.0)) * a;
+            a = b;
+            b = c;
+            val[(size_t)(l - 1 - m) * 2 * nf * SMV_PT] = c;
+          }
+        }
+        double t1 = S.rec[m * (m + 1) + 2 * m], t0 = 0.0;  // Theta
+        double p1 = 0.0, p0 = 0.0, q1 = 0.0, q0 = 0.0;     // dTheta/dz, dTheta/ds
+        for (int l = m; l <= S.lmax; ++l) {
+          if (l > m) {
+            const double *rr = S.rec + l * (l + 1) + 2 * m;
+            const double ra = rr[0], rb = rr[1];
+            const double t2 = ra * (z * t1 - rb * s2 * t0);
+            const double p2 = ra * (t1 + z * p1 - rb * s2 * p0);
+            const double q2 = ra * (z * q1 - rb * (t0 + s2 * q0));
+            t0 = t1; t1 = t2;
+            p0 = p1; p1 = p2;
+            q0 = q1; q1 = q2;
+          }
+          double *v = val + (size_t)(l - m) * 2 * nf * SMV_PT;
+          const double g = v[0], gn = l < S.lmax ? v[2 * nf * SMV_PT] : gtop;
+          // W . grad (g Theta C) = [g (wz P + 2 wr Q) - wr kk^2 g_{l+1} / (2l + 3) Theta] C + g Theta W . grad C
+          const double gt = g * t1;
+          const double f = g * (wz * p1 + 2.0 * wr * q1) - wr * kk2 * gn / (2.0 * l + 3.0) * t1;
+          v[0] = aW * gt * C;
+          v[SMV_PT] = f * C + gt * dC;
+          if (nf == 2) {
+            v[2 * SMV_PT] = aW * gt * Sn;
+            v[3 * SMV_PT] = f * Sn + gt * dS;
+          }
+        }
+}
+
 // V[lm][4 s + a] = int N_a |W| phi_lm, V[lm][4 ne + 4 s + a] = int N_a W . grad phi_lm
 // over element s.  The product with A makes these G_s and W . grad G_s integrated
 // with this rule, so the rule is the one a regular pair takes whose nearest image
@@ -681,7 +783,6 @@ __global__ void __launch_bounds__(SMU_TH) k_sm_targets(const __grid_constant__ s
 // the reference's 12 x 12 (3 parts of it on a triangle) without the shorter rules.  Block: (element, order m); a thread per point walks l and leaves
 // the four values of each l in shared memory, then a thread per value sums
 // over the points.
-#define SMV_PT (BEM_GLN * BEM_GLN)
 #define SMV_TH 160
 __global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ sm_dev S, bem_dom_dev D, int far_rule) {
   extern __shared__ double sm_raw[];
@@ -712,77 +813,7 @@ __global__ void __launch_bounds__(SMV_TH) k_sm_sources(const __grid_constant__ s
       bem_Nn(tri, zt, et, Nn);
 #pragma unroll
       for (int a = 0; a < 4; ++a) Nw[a * SMV_PT + tid] = Nn[a] * wt;
-      const double aW = sqrt(W[0] * W[0] + W[1] * W[1] + W[2] * W[2]);
-      const double x = (r[0] - S.cx) * S.iR0, y = (r[1] - S.cy) * S.iR0, z = (r[2] - S.cz) * S.iR0;
-      const double s2 = x * x + y * y + z * z;
-      const double wx = W[0] * S.iR0, wy = W[1] * S.iR0, wz = W[2] * S.iR0;
-      const double wr = wx * x + wy * y + wz * z;
-      // Re, Im (x + iy)^m and their derivatives along W
-      double C = 1.0, Sn = 0.0, C0 = 0.0, S0 = 0.0;
-      for (int a = 0; a < m; ++a) {
-        C0 = C;
-        S0 = Sn;
-        const double c2 = C * x - Sn * y;
-        Sn = C * y + Sn * x;
-        C = c2;
-      }
-      double dC = m * (wx * C0 - wy * S0), dS = m * (wx * S0 + wy * C0);
-      if (m) {
-        const double q2 = 1.4142135623730950488;
-        C *= q2; Sn *= q2; dC *= q2; dS *= q2;
-      }
-      // g_l downward from l = lmax + 1, kept in the value slots until used
-      const double z2 = S.kR0 * S.kR0 * s2, kk2 = S.kR0 * S.kR0;
-      // upward walk needs g_l and g_{l+1}: g is computed into val[l - m][0]
-      // (read before it is overwritten) with g_{lmax + 1} kept in a register
-      double gtop;
-      {
-        double a = 0.0, b = 0.0;
-#pragma unroll 1
-        for (int w = 0; w < 2; ++w) {
-          const int l = S.lmax + 2 - w;
-          double t = 1.0, sum = 1.0;
-          for (int q = 1; q < 100; ++q) {
-            t *= -0.5 * z2 / (q * (2.0 * l + 2.0 * q + 1.0));
-            sum += t;
-            if (fabs(t) < 1e-18 * fabs(sum)) break;
-          }
-          if (w == 0) a = sum;
-          else b = sum;
-        }
-        gtop = b;
-        for (int l = S.lmax + 1; l > m; --l) {
-          const double c = b - z2 / ((2.0 * l + 1.0) * (2.0 * l + 3.0)) * a;
-          a = b;
-          b = c;
-          val[(size_t)(l - 1 - m) * 2 * nf * SMV_PT + tid] = c;
-        }
-      }
-      double t1 = S.rec[m * (m + 1) + 2 * m], t0 = 0.0;  // Theta
-      double p1 = 0.0, p0 = 0.0, q1 = 0.0, q0 = 0.0;     // dTheta/dz, dTheta/ds
-      for (int l = m; l <= S.lmax; ++l) {
-        if (l > m) {
-          const double *rr = S.rec + l * (l + 1) + 2 * m;
-          const double ra = rr[0], rb = rr[1];
-          const double t2 = ra * (z * t1 - rb * s2 * t0);
-          const double p2 = ra * (t1 + z * p1 - rb * s2 * p0);
-          const double q2 = ra * (z * q1 - rb * (t0 + s2 * q0));
-          t0 = t1; t1 = t2;
-          p0 = p1; p1 = p2;
-          q0 = q1; q1 = q2;
-        }
-        double *v = val + (size_t)(l - m) * 2 * nf * SMV_PT + tid;
-        const double g = v[0], gn = l < S.lmax ? v[2 * nf * SMV_PT] : gtop;
-        // W . grad (g Theta C) = [g (wz P + 2 wr Q) - wr kk^2 g_{l+1} / (2l + 3) Theta] C + g Theta W . grad C
-        const double gt = g * t1;
-        const double f = g * (wz * p1 + 2.0 * wr * q1) - wr * kk2 * gn / (2.0 * l + 3.0) * t1;
-        v[0] = aW * gt * C;
-        v[SMV_PT] = f * C + gt * dC;
-        if (nf == 2) {
-          v[2 * SMV_PT] = aW * gt * Sn;
-          v[3 * SMV_PT] = f * Sn + gt * dS;
-        }
-      }
+      sm_point_values(S, m, nf, r, W, val + tid);
     }
     __syncthreads();
     if (tid < nout) {
@@ -1033,7 +1064,9 @@ __global__ void __launch_bounds__(SMI_TH, 4) k_sm_images(const __grid_constant__
 }
 
 // ------------------------------------------------------------------ launches
-static sm_dev dev_view(const bem_smooth *S, int ne, int b0) {
+// instances b0, b0 + 1, ... of the tables; held: sigma and T of instance b0 where
+// the last launch_rest left them (otherwise at the front, where it will put them)
+static sm_dev dev_view(const bem_smooth *S, int ne, int b0, bool held = false) {
   sm_dev d;
   d.lmax = S->lmax; d.Lmax = S->Lmax; d.K = S->K; d.Kp = S->Kp; d.nt = S->nt; d.nphi = S->nphi; d.nimg = S->nimg;
   d.eta = S->eta;
@@ -1047,10 +1080,40 @@ static sm_dev dev_view(const bem_smooth *S, int ne, int b0) {
   d.x = S->tab + t.x; d.w = S->tab + t.w; d.ca = S->tab + t.ca; d.cb = S->tab + t.cb;
   d.dL = S->tab + t.dL; d.el = S->tab + t.el; d.rec = S->tab + t.rec;
   d.img = S->tab + t.img + 3 * (size_t)b0 * S->nimg;
-  const sm_ws w = ws_layout(S, ne, std::min(S->inst, BEM_SM_BAT));
-  d.plm = S->ws + w.plm; d.samp = S->ws + w.samp; d.sig = S->ws + w.sig; d.T = S->ws + w.T;
-  d.U = S->ws + w.U; d.V = S->ws + w.V; d.A = S->ws + w.A;
+  const sm_keep k = keep_layout(S);
+  const size_t at = held ? b0 - S->have0 : 0;
+  for (int i = 0; i < 8; ++i) d.lcut[i] = S->lcut[i];
+  d.plm = S->keep + k.plm;
+  d.samp = S->keep + k.samp;
+  d.sig = S->keep + k.sig + at * 2 * (S->Lmax + 1) * (S->Lmax + 1);
+  d.T = S->keep + k.T + at * 2 * S->Kp * S->Kp;
+  d.Z = S->keep + k.Z;
+  d.Zt = S->keep + k.Zt;
+  const sm_ws w = ws_layout(S, ne);
+  d.U = S->ws + w.U;
+  d.V = S->ws + w.V;
+  d.A = S->ws + w.A;
   return d;
+}
+
+// sigma and T of n <= BEM_SM_BAT instances from instance b0 on
+static int launch_rest(bem_smooth *S, const bem_qp *qps, int b0, int n, unsigned *status, cudaStream_t st) {
+  const sm_dev d = dev_view(S, 0, b0);
+  sm_qps Q;
+  for (int i = 0; i < BEM_SM_BAT; ++i) Q.q[i] = qps[i < n ? i : 0];
+  const int smem_t = S->nt / 2 * SMT_TH * (int)sizeof(double), nlm = (S->lmax + 1) * (S->lmax + 2) / 2;
+  if (cudaFuncSetAttribute(k_sm_T, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t) != cudaSuccess) return -1;
+  const int nsamp = (S->nt * S->nphi * 32 + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
+  S->have0 = S->have1 = 0;
+  k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, status);
+  k_sm_coef<<<dim3(2 * S->Lmax + 1, n), SMC_TH, 0, st>>>(d);
+  if (cudaMemsetAsync(d.T, 0, (size_t)n * 2 * S->Kp * S->Kp * sizeof(double), st) != cudaSuccess) return -1;
+  k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, smem_t, st>>>(d);
+  bem_count_launches(3);
+  if (cudaPeekAtLastError() != cudaSuccess) return -1;
+  S->have0 = b0;
+  S->have1 = b0 + n;
+  return 0;
 }
 
 template <int LP>
@@ -1059,34 +1122,26 @@ static void launch_images(const sm_dev &d, const bem_dom_dev *D, int nb, const u
   k_sm_images<LP><<<dim3((unsigned)((th + SMI_TH - 1) / SMI_TH), nb), SMI_TH, 0, st>>>(d, *D, D->far_rule, flag, O);
 }
 
-extern "C" int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
+extern "C" int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
                                  double *const *H, const bem_scratch *scr, cudaStream_t st) {
   const int ne = D->ne, N = 4 * ne;
   const int smem_v = (4 * SMV_PT + std::max(2 * (S->lmax + 1), 4 * S->lmax) * SMV_PT) * (int)sizeof(double);
-  const int smem_t = S->nt / 2 * SMT_TH * (int)sizeof(double);
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (cudaFuncSetAttribute(k_sm_sources, at, smem_v) != cudaSuccess || cudaFuncSetAttribute(k_sm_T, at, smem_t) != cudaSuccess ||
+  if (cudaFuncSetAttribute(k_sm_sources, at, smem_v) != cudaSuccess ||
       cudaFuncSetAttribute(k_sm_gemm<true>, at, GM_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(k_sm_gemm<false>, at, GM_SMEM) != cudaSuccess)
     return -1;
   const long long npairs = (long long)N * ne;
-  const int nlm = (S->lmax + 1) * (S->lmax + 2) / 2;
   for (int b0 = 0; b0 < nb; b0 += BEM_SM_BAT) {
     const int n = nb - b0 < BEM_SM_BAT ? nb - b0 : BEM_SM_BAT;
-    const sm_dev d = dev_view(S, ne, nb == 1 ? S->first : b0);
-    sm_qps Q;
+    const int first = nb == 1 ? S->first : b0;
+    if (launch_rest(S, qps + b0, first, n, scr->status, st)) return -1;
+    const sm_dev d = dev_view(S, ne, first);
     sm_out O;
     for (int i = 0; i < BEM_SM_BAT; ++i) {
-      Q.q[i] = qps[b0 + (i < n ? i : 0)];
       O.G[i] = i < n ? G[b0 + i] : nullptr;
       O.H[i] = i < n ? H[b0 + i] : nullptr;
     }
-    const int nsamp = (S->nt * S->nphi * 32 + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
-    k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, scr->status);
-    k_sm_coef<<<dim3(2 * S->Lmax + 1, n), SMC_TH, 0, st>>>(d);
-    if (cudaMemsetAsync(d.T, 0, (size_t)n * 2 * S->Kp * S->Kp * sizeof(double), st) != cudaSuccess) return -1;
-    k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, smem_t, st>>>(d);
-    bem_count_launches(3);
     if (b0 == 0) {
       k_sm_targets<<<(N + SMU_TH / 32 - 1) / (SMU_TH / 32), SMU_TH, 0, st>>>(d, *D);
       k_sm_sources<<<dim3(ne, S->lmax + 1), SMV_TH, smem_v, st>>>(d, *D, D->far_rule);
@@ -1106,3 +1161,5 @@ extern "C" int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, cons
   }
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
+
+#include "bem_bdsum.cuh"

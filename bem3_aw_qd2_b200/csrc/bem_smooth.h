@@ -21,7 +21,10 @@ struct bem_smooth {
   int l1[BEM_SM_MAXIMG], l2[BEM_SM_MAXIMG];  // the images' lattice indices, (0, 0) first
   int inst = 1, first = 0;      // instances tab holds; the one a launch for a single instance takes
   const double *tab = nullptr;  // device copy of the tables bem_smooth_tables writes
-  double *ws = nullptr;         // device workspace of bem_smooth_ws_doubles(...) doubles
+  int lcut[8];                  // degrees of the expansion about a point, by distance
+  double *keep = nullptr;       // device memory of bem_smooth_keep_doubles doubles, kept with the problem
+  int have0 = 0, have1 = 0;     // instances whose expansion keep holds
+  double *ws = nullptr;         // an assembly's scratch, bem_smooth_ws_doubles doubles
 };
 // offsets (doubles) in tab
 struct bem_smooth_tab {
@@ -35,6 +38,7 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
 bem_smooth_tab bem_smooth_layout(const bem_smooth *S);
 // the tables of S->inst instances (qps: their Bloch wave vectors) into h[layout.total]
 void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h);
+size_t bem_smooth_keep_doubles(const bem_smooth *S);
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
 
 extern "C" {
@@ -43,6 +47,11 @@ int bem_smooth_set_constants(const void *quad, const void *wc);
 // G, H of nb instances of the periodic domain: the smooth rest of every pair
 // (written), then the images of every pair off the lattice plane (added; the
 // home image of near-singular and self pairs is left to their own kernels)
-int bem_launch_smooth(const bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
+int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
                       double *const *H, const bem_scratch *scr, cudaStream_t st);
+// k_bdval's sums for targets of the periodic domain (bem_bdsum.cuh); q: the
+// parameters of instance S->first
+int bem_launch_bdsum(bem_smooth *S, const bem_dom_dev *D, const bem_qp *q, int type, int ntgt, const int *tgt_t,
+                     const double *tgt_ze, const double *P, const double *dP, const double *pv, const double *dpv,
+                     double *out, unsigned *status, cudaStream_t st);
 }
