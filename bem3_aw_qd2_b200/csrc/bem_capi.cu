@@ -55,6 +55,9 @@ struct bemgpu_ctx {
   bem_smooth sm;
   double *sm_tab = nullptr, *sm_keep = nullptr, *sm_buf = nullptr;
   double zspan = 0.0;      // height of the mesh (z extent of all elements)
+  double zlo = 0.0;        // and its lower end
+  double *fst = nullptr;   // evanescent order table for field points above or below the mesh
+  size_t fst_cap = 0;
   double pw[16] = {};      // incident plane wave (bemgpu_problem.pw)
   int far_rule = 1;        // shorter rules for regular pairs of the periodic domain (bemgpu_set_far_rule)
   double eta_scale = 0.0;  // Ewald parameter off the lattice plane = eta0 x eta_scale; 0: by rule per problem
@@ -208,7 +211,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
       dfree(S->rowF); dfree(S->near_s); dfree(S->near_n); dfree(S->nearF); dfree(S->selfF); dfree(S->flag);
     }
     dfree(c->scr.plist); dfree(c->scr.pcount);
-    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->b0); dfree(c->B3s);
+    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->fst); dfree(c->b0); dfree(c->B3s);
     for (int d = 0; d < BEMGPU_MAXDOM; ++d) { dfree(c->Wd[d]); dfree(c->cinv[d]); dfree(c->Gc[d]); }
     dfree(c->B3c);
     dfree(c->dGc); dfree(c->dHc);
@@ -472,6 +475,7 @@ extern "C" int bemgpu_load(bemgpu_ctx *c, const bemgpu_problem *pr) {
       if (e == 0 || z[0] + hw > zhi) zhi = z[0] + hw;
     }
     c->zspan = zhi - zlo;
+    c->zlo = zlo;
   }
   if (build_stab(c)) return -1;
   memcpy(c->pw, pr->pw, sizeof(c->pw));
@@ -1393,6 +1397,45 @@ static int ensure_points(bemgpu_ctx *c, int n) {
   return 0;
 }
 
+// The lattice sums of field points: q = c->qp with a spectral order table that
+// reaches from the mesh to the points where that is worth its build.  The
+// context's own table covers distances within the mesh; beyond it a term is two
+// erfcx and an exponential in place of one recurrence, some 4 times the work of
+// the whole term.  A table costs its orders x intervals x degree direct terms, a
+// point about 50 spectral terms for each source.  Distances at which the plane
+// wave sum converges by itself (bem_qpgf2) need no table.
+static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources, bem_qp *q) {
+  *q = c->qp;
+  double reach = 0.0;
+  for (int i = 0; i < n; ++i)
+    reach = std::max(reach, std::max(c->zlo + c->zspan - r[3 * i + 2], r[3 * i + 2] - c->zlo));
+  if (!q->ewald_only) {
+    const double eps = 1e-15;  // the sums' relative error
+    const double zs = std::max(log(q->sel_cp / eps) / q->sel_bp, log(q->sel_cm / eps) / q->sel_bm);
+    if (zs > 0.0) reach = std::min(reach, zs);
+  }
+  if (!(reach > c->zspan) || !(reach < 1e4 * q->eta_run)) return 0;
+  const bem_qp own = *q;
+  const size_t cnt = stab_window(q, reach);
+  if (!cnt || (double)n * sources * 50.0 < 2.0 * cnt) {
+    *q = own;
+    return 0;
+  }
+  if (cnt > c->fst_cap) {
+    dfree(c->fst);
+    c->fst_cap = 0;
+    if (dalloc(&c->fst, cnt) != cudaSuccess) {  // without one, then
+      cudaGetLastError();
+      *q = own;
+      return 0;
+    }
+    c->fst_cap = cnt;
+  }
+  if (bem_launch_stab(q, c->fst, c->stream)) return fail(c, "spectral table", cudaGetLastError());
+  q->st = c->fst;
+  return 0;
+}
+
 extern "C" int bemgpu_field(bemgpu_ctx *c, int d, int type, int n, const double *r, double *out) {
   if (!c->loaded || d < 0 || d > c->MN) { snprintf(c->err, sizeof(c->err), "bad domain %d", d); return -2; }
   const int grad = !(type & BEMGPU_FIELD_POTENTIAL);
@@ -1402,7 +1445,10 @@ extern "C" int bemgpu_field(bemgpu_ctx *c, int d, int type, int n, const double 
   if (ensure_points(c, n)) return -1;
   bem_dom_dev D = dom_view(c, d);
   CK(cudaMemcpyAsync(c->pt_in, r, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, c->stream), "field points");
-  if (bem_launch_field(&D, &c->qp, d == 0, grad, c->k0[d], type, n, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
+  bem_qp q = c->qp;
+  if (d == 0 && field_tables(c, n, r, (long long)c->dom_ne[0] * (type == 0 ? 4 : type == 1 ? 9 : type == 2 ? 144 : 4096), &q))
+    return -1;
+  if (bem_launch_field(&D, &q, d == 0, grad, c->k0[d], type, n, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
                        c->pt_out, c->status, c->stream))
     return fail(c, "field", cudaGetLastError());
   CK(cudaMemcpyAsync(out, c->pt_out, 18 * sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream), "field");
@@ -1616,6 +1662,7 @@ extern "C" int bemgpu_transform_mesh(bemgpu_ctx *c, const double *rv, double th,
     if (e == 0 || z[0] + hw > zhi) zhi = z[0] + hw;
   }
   c->zspan = zhi - zlo;
+  c->zlo = zlo;
   if (build_stab(c)) return -1;
   // and its ball the split into images and expansion
   std::vector<int> sid(c->dom_ne[0]), npe(c->Ne);

@@ -656,7 +656,8 @@ struct bem_gval2 { cplx g, d[3], d2[6]; };
 
 __device__ __forceinline__ cplx cmuli(cplx a) { return cmk(-a.im, a.re); }  // i a
 
-static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
+static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o,
+                                      const double2 *wts) {
   const double ve = bem_ewald_eta(q, rx, ry, rz);
   const double ke = q.k * ve, ke2 = ke * ke, ive = 1.0 / ve;
   const bool tab = q.wt != nullptr && ve == q.eta_run;
@@ -689,7 +690,7 @@ static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, dou
           // A = ef Re w and the first-derivative factor from the table when it applies
           double A, B1;
           if (tab) {
-            const double2 ab = bem_wtab(q, ve, ke, rl2e);
+            const double2 ab = bem_wtab(q, ve, ke, rl2e, wts);
             A = ab.x;
             B1 = 2.0 * ve * irl * irl * irl * ab.y;
           } else {
@@ -735,6 +736,7 @@ static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, dou
   cplx t = cmk(0, 0), td[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)}, t2[6];
   for (int c = 0; c < 6; ++c) t2[c] = cmk(0, 0);
   const double azve = rz / (2.0 * ve), c2pi = 2.0 * isp * ive;
+  const bool stab = ew_spec_tab_ok(q, ve, rz);
   for (int dir = 0; dir < 3; ++dir) {
     int n1 = q.nc1 + (dir == 2 ? -1 : (dir == 1 ? 1 : 0));
     const int step = dir == 2 ? -1 : 1;
@@ -758,23 +760,35 @@ static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, dou
           const double ef = exp(bn2 * ve * ve - azve * azve);
           cplx Fn, dz, dzz;
           int e;
+          double v0, v1;
+          const bool in = stab && ew_spec_tab(q, n1, n2, azve, v0, v1);
           if (bn2 > 0.0) {
             const double bn = sqrt(bn2);
             const cplx ff = cexpi(bn * rz);
-            const cplx w = bem_faddeeva(bn * ve, azve);
-            const cplx F = cmk(2.0 * ff.re, 2.0 * (ef * w.im + ff.im));
-            const cplx Gq = cmk(2.0 * (ef * w.re - ff.re), -2.0 * ff.im);
+            if (!in) {
+              const cplx w = bem_faddeeva(bn * ve, azve);
+              v0 = ef * w.re;
+              v1 = ef * w.im;
+            }
+            const cplx F = cmk(2.0 * ff.re, 2.0 * (v1 + ff.im));
+            const cplx Gq = cmk(2.0 * (v0 - ff.re), -2.0 * ff.im);
             Fn = cscale(cmul(ce, F), 1.0 / bn);
             dz = cmul(ce, Gq);
             dzz = cmul(ce, cadd(cscale(cmuli(F), bn), cmk(c2pi * ef, 0.0)));
             e = 0;
           } else if (bn2 < 0.0) {
-            const double bn = sqrt(-bn2), bv = bn * ve;  // see ew_spec_term
-            const double eq = exp(-(bv * bv + azve * azve));
-            const double f1 = eq * erfcx(bv + azve), f2 = eq * erfcx(bv - azve);
-            Fn = cmul(ce, cmk(0.0, -(f1 + f2) / bn));
-            dz = cscale(ce, f1 - f2);
-            dzz = cscale(ce, -bn * (f1 + f2) + c2pi * ef);
+            if (in) {  // (f1 + f2) / bn, (f1 - f2) / d
+              v1 *= azve;
+            } else {
+              const double bn = sqrt(-bn2), bv = bn * ve;  // see ew_spec_term
+              const double eq = exp(-(bv * bv + azve * azve));
+              const double f1 = eq * erfcx(bv + azve), f2 = eq * erfcx(bv - azve);
+              v0 = (f1 + f2) / bn;
+              v1 = f1 - f2;
+            }
+            Fn = cmul(ce, cmk(0.0, -v0));
+            dz = cscale(ce, v1);
+            dzz = cscale(ce, bn2 * v0 + c2pi * ef);
             e = 1;
           } else {
             return -23;
@@ -891,7 +905,9 @@ static __device__ int bem_qpgf2_spectral(const bem_qp &q, double rx, double ry, 
   return cc;
 }
 
-static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &out) {
+// wts: the kernel's shared-memory copy of the real-space table, or null
+static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &out,
+                                const double2 *wts = nullptr) {
   bool spectral = false;
   if (!q.ewald_only) {
     const double az = fabs(rz);
@@ -902,7 +918,7 @@ static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz
   const int l2 = (int)floor(-(rx * q.d1y - ry * q.d1x) * q.idet + 0.5);
   const double hx = bem_sub2(rx, l1, q.d1x, l2, q.d2x);
   const double hy = bem_sub2(ry, l1, q.d1y, l2, q.d2y);
-  const int e = spectral ? bem_qpgf2_spectral(q, hx, hy, rz, out) : bem_qpgf2_ewald(q, hx, hy, rz, out);
+  const int e = spectral ? bem_qpgf2_spectral(q, hx, hy, rz, out) : bem_qpgf2_ewald(q, hx, hy, rz, out, wts);
   if (e > 0 && (l1 != 0 || l2 != 0)) {
     const cplx cf = cexpi(-(q.kx * (l1 * q.d1x + l2 * q.d2x) + q.ky * (l1 * q.d1y + l2 * q.d2y)));
     out.g = cmul(out.g, cf);
