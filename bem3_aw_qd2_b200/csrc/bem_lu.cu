@@ -1132,17 +1132,19 @@ __global__ void k_lu_iota(int *rowmap, int n, int *counter, int nodes) {
 }
 
 // ---------------------------------------------------------------- triangular solves
+// Bound by a serial chain: block it of 32 unknowns needs block it - 1, so a solve
+// is n / 32 hops from one SM to the next through L2 (the factor's entries stream
+// in beside them).  Everything that does not need the last block's values is done
+// before they arrive: with V the inverse of the diagonal block and M = V times
+// the block beside it, x_it = V (rhs - sum of the others) - M x_{it-1}, and only
+// the last product, one sum over four warps and one store stay on the chain.  The
+// values are their own flag: out starts as all ones (no arithmetic yields that
+// pattern), a reader polls the values that it needs, and a hop has no counter, no
+// fence and no second round trip.  A pair of solves with three right-hand sides
+// at n = 1999: 816 us with substitution in the block behind a counter, 176.
 #define TS_TH 128
 #define TS_WAIT_NS 1000000000ull  // one second
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1153,52 +1155,125 @@ __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-// the two counters (lower, upper solve) sit 128 bytes apart
-#define TS_FSTRIDE 32
-// wait until *cnt > k and return the count seen: a spin of relaxed loads with
-// an acquire fence once it has moved past k; after one second it gives up with
-// BEM_LU_ST_WAIT set (and returns k + 1), and once any wait has given up later
-// waits return at once
-__device__ __forceinline__ unsigned wait_count(const unsigned *cnt, unsigned k, unsigned *status) {
-  unsigned c = ld_acquire(cnt);
-  if (c > k) return c;
-  const unsigned long long t0 = gtimer();
+__device__ __forceinline__ double2 ts_load(const double2 *p) {
+  double2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ts_load(const float2 *p) {
+  float2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool ts_unset(double2 v) {
+  return __double_as_longlong(v.x) == -1ll || __double_as_longlong(v.y) == -1ll;
+}
+__device__ __forceinline__ bool ts_unset(float2 v) { return __float_as_int(v.x) == -1 || __float_as_int(v.y) == -1; }
+// a value with the reserved pattern (a NaN handed in) is stored as another NaN
+__device__ __forceinline__ void ts_store(double2 *p, double2 v) {
+  if (__double_as_longlong(v.x) == -1ll) v.x = __longlong_as_double(0x7ff8000000000000ll);
+  if (__double_as_longlong(v.y) == -1ll) v.y = __longlong_as_double(0x7ff8000000000000ll);
+  asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void ts_store(float2 *p, float2 v) {
+  if (__float_as_int(v.x) == -1) v.x = __int_as_float(0x7fc00000);
+  if (__float_as_int(v.y) == -1) v.y = __int_as_float(0x7fc00000);
+  asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+// The warp's eight unknowns from c0 on, into sx[c][q], once they are written (zero
+// beyond n).  After one second a wait gives up with BEM_LU_ST_WAIT set, and once
+// any wait has given up the others return at their next look.
+template <class C2, int NR>
+__device__ __forceinline__ void ts_get(const C2 *out, int n, int c0, bool next, C2 *sx, unsigned *status) {
+  const int lane = threadIdx.x & 31, c = lane & 7, q = lane >> 3;
+  const bool need = q < NR && c0 + c < n;
+  const C2 *p = out + (need ? (size_t)q * n + c0 + c : 0);
+  C2 v = czero<C2>();
+  bool ok = !need;
+  unsigned long long t0 = 0;
   for (unsigned it = 1;; ++it) {
-    c = ld_relaxed(cnt);
-    if (c > k) {
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      return c;
+    if (!ok) {
+      const C2 x = ts_load(p);
+      if (!ts_unset(x)) {
+        v = x;
+        ok = true;
+      }
     }
-    if ((it & 255) == 0 && (gtimer() - t0 > TS_WAIT_NS || (ld_relaxed(status) & BEM_LU_ST_WAIT))) {
-      atomicOr(status, BEM_LU_ST_WAIT);
-      return k + 1;
+    if (__all_sync(FULL, ok)) break;
+    if (it == 1) t0 = gtimer();
+    if ((it & 255) == 0 &&
+        __any_sync(FULL, gtimer() - t0 > TS_WAIT_NS || (ld_relaxed(status) & BEM_LU_ST_WAIT) != 0)) {
+      if (lane == 0) atomicOr(status, BEM_LU_ST_WAIT);
+      break;
     }
+    if (!next) __nanosleep(100);  // leave the line to the block that is next
   }
+  __syncwarp();
+  if (q < NR) sx[c * NR + q] = v;
+  __syncwarp();
 }
 
 // lower = 1: out = L^-1 (P in), in read through rowmap (unit lower L);
-// lower = 0: out = U^-1 in.  in / out are n x NR column-major.  The 32-row
-// blocks are solved in dependency order (top down for L, bottom up for U): the
-// block of position it needs the blocks of positions 0 .. it-1, each of which
-// it folds in as soon as *cnt (the number of blocks written so far, which
-// grows in position order) has passed it.
+// lower = 0: out = U^-1 in.  in / out are n x NR column-major, out all ones (bits)
+// before.  The 32-row blocks go in dependency order (top down for L, bottom up for
+// U): the block of position it needs those of positions 0 .. it - 1.  All blocks
+// are resident, or take their positions in order.
 template <class C2, int NR>
 __global__ void __launch_bounds__(TS_TH) k_lu_trsv(const C2 *LU, long lda, int n, const int *rowmap, const C2 *in,
-                                                   C2 *out, unsigned *cnt, int lower, unsigned *status) {
-  __shared__ C2 sd[32][33];
-  __shared__ C2 sacc[4][32][NR];
-  __shared__ unsigned sready[2];
+                                                   C2 *out, int lower, unsigned *status) {
+  __shared__ C2 sd[32][33], sv[32][33];
+  __shared__ C2 sx[4][8 * NR];
+  // once M is formed, V's place holds the four warps' sums
+  C2 (*sacc)[32][NR] = reinterpret_cast<C2 (*)[32][NR]>(&sv[0][0]);
+  C2 (*sout)[32][NR] = sacc + 4;
   const int nb = (n + 31) / 32;
   const int t = threadIdx.x, r = t & 31, s = t >> 5;
-  unsigned nwait = 0;
   for (int it = blockIdx.x; it < nb; it += gridDim.x) {
     const int b = lower ? it : nb - 1 - it;
     const int r0 = b * 32, rows = min(32, n - r0);
+    const int row = r0 + r;
+    // V: a warp inverts onto eight columns, a lane per row
     for (int e = t; e < 32 * 32; e += TS_TH) {
       const int i = e >> 5, j = e & 31;
-      sd[i][j] = (i < rows && j < rows) ? LU[(size_t)(r0 + i) * lda + r0 + j] : czero<C2>();
+      sd[i][j] = (i < rows && j < rows) ? LU[(size_t)(r0 + i) * lda + r0 + j] : (i == j ? cone<C2>() : czero<C2>());
     }
-    const int row = r0 + r;
+    __syncthreads();
+    C2 inv[8], m[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      inv[c] = r == 8 * s + c ? cone<C2>() : czero<C2>();
+      m[c] = czero<C2>();
+    }
+    const C2 d = lower ? cone<C2>() : crcp(sd[r][r]);
+#pragma unroll 2
+    for (int kk = 0; kk < 32; ++kk) {
+      const int k = lower ? kk : 31 - kk;
+      const C2 f = sd[r][k];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if (!lower && r == k) inv[c] = cmul(inv[c], d);
+        const C2 w = cx<C2>::mk(__shfl_sync(FULL, inv[c].x, k), __shfl_sync(FULL, inv[c].y, k));
+        if (lower ? r > k : r < k) inv[c] = cfms(f, w, inv[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sv[r][8 * s + c] = inv[c];
+    __syncthreads();
+    const int jl = (lower ? it - 1 : nb - it) * 32;  // the last dependency's columns
+    if (it > 0) {  // M = V times the block beside
+      for (int e = t; e < 32 * 32; e += TS_TH) {
+        const int i = e >> 5, j = e & 31;
+        sd[i][j] = (i < rows && jl + j < n) ? LU[(size_t)(r0 + i) * lda + jl + j] : czero<C2>();
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int j = 0; j < 32; ++j) {
+        const C2 f = sv[r][j];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) m[c] = cfma(f, sd[j][8 * s + c], m[c]);
+      }
+    }
+    __syncthreads();
     C2 acc[NR];
 #pragma unroll
     for (int q = 0; q < NR; ++q) acc[q] = czero<C2>();
@@ -1218,77 +1293,54 @@ __global__ void __launch_bounds__(TS_TH) k_lu_trsv(const C2 *LU, long lda, int n
 #pragma unroll
       for (int cc = 0; cc < 8; ++cc) {
         const int col = jb * 32 + s * 8 + cc;
-        ac[cc] = (it > 0 && r < rows && col < n) ? arow[col] : czero<C2>();
+        ac[cc] = (it > 1 && r < rows && col < n) ? arow[col] : czero<C2>();
       }
     }
-    unsigned ready = 0;
-    for (int k = 0; k < it; ++k) {
+    for (int k = 0; k + 1 < it; ++k) {
       const int jb = lower ? k : nb - 1 - k, jn = lower ? k + 1 : nb - 2 - k;
 #pragma unroll
       for (int cc = 0; cc < 8; ++cc) {
         const int col = jn * 32 + s * 8 + cc;
-        an[cc] = (k + 1 < it && r < rows && col < n) ? arow[col] : czero<C2>();
+        an[cc] = (k + 2 < it && r < rows && col < n) ? arow[col] : czero<C2>();
       }
-      if ((unsigned)k >= ready) {
-        // one thread polls (all threads polling one line starve the block
-        // that publishes it); the barrier passes its acquire on.  The two
-        // slots alternate so a slot is rewritten only after every thread has
-        // passed the barrier that follows its read.
-        if (t == 0) sready[nwait & 1] = wait_count(cnt, (unsigned)k, status);
-        __syncthreads();
-        ready = sready[nwait & 1];
-        ++nwait;
-      }
-      const int c0 = jb * 32 + s * 8;
+      ts_get<C2, NR>(out, n, jb * 32 + s * 8, k + 3 >= it, sx[s], status);
 #pragma unroll
       for (int cc = 0; cc < 8; ++cc) {
-        const int col = c0 + cc;
-        if (col < n)
 #pragma unroll
-          for (int q = 0; q < NR; ++q) acc[q] = cfms(ac[cc], __ldcg(out + (size_t)q * n + col), acc[q]);
+        for (int q = 0; q < NR; ++q) acc[q] = cfms(ac[cc], sx[s][cc * NR + q], acc[q]);
         ac[cc] = an[cc];
       }
     }
 #pragma unroll
     for (int q = 0; q < NR; ++q) sacc[s][r][q] = acc[q];
     __syncthreads();
-    if (s == 0) {
+#pragma unroll
+    for (int q = 0; q < NR; ++q) acc[q] = czero<C2>();
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
-        C2 x = sacc[0][r][q];
-        for (int ss = 1; ss < 4; ++ss) x = cx<C2>::mk(x.x + sacc[ss][r][q].x, x.y + sacc[ss][r][q].y);
-        acc[q] = x;
+        C2 x = sacc[0][8 * s + c][q];
+#pragma unroll
+        for (int u = 1; u < 4; ++u) x = cx<C2>::mk(x.x + sacc[u][8 * s + c][q].x, x.y + sacc[u][8 * s + c][q].y);
+        acc[q] = cfma(inv[c], x, acc[q]);
       }
-      if (lower) {
-        for (int i = 0; i < rows; ++i) {
+    if (it > 0) {
+      ts_get<C2, NR>(out, n, jl + s * 8, true, sx[s], status);
 #pragma unroll
-          for (int q = 0; q < NR; ++q) {
-            const C2 yi = cx<C2>::mk(__shfl_sync(FULL, acc[q].x, i), __shfl_sync(FULL, acc[q].y, i));
-            if (r > i && r < rows) acc[q] = cfms(sd[r][i], yi, acc[q]);
-          }
-        }
-      } else {
-        for (int i = rows - 1; i >= 0; --i) {
-          if (r == i) {
-            const C2 d = crcp(sd[i][i]);
+      for (int c = 0; c < 8; ++c)
 #pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] = cmul(acc[q], d);
-          }
-#pragma unroll
-          for (int q = 0; q < NR; ++q) {
-            const C2 xi = cx<C2>::mk(__shfl_sync(FULL, acc[q].x, i), __shfl_sync(FULL, acc[q].y, i));
-            if (r < i) acc[q] = cfms(sd[r][i], xi, acc[q]);
-          }
-        }
-      }
-      if (r < rows)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) out[(size_t)q * n + row] = acc[q];
-      __threadfence();
-      __syncwarp();
-      if (r == 0) st_release(cnt, (unsigned)it + 1u);
+        for (int q = 0; q < NR; ++q) acc[q] = cfms(m[c], sx[s][c * NR + q], acc[q]);
     }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) sout[s][r][q] = acc[q];
     __syncthreads();
+    if (s < NR && r < rows) {
+      C2 x = sout[0][r][s];
+#pragma unroll
+      for (int u = 1; u < 4; ++u) x = cx<C2>::mk(x.x + sout[u][r][s].x, x.y + sout[u][r][s].y);
+      ts_store(out + (size_t)s * n + row, x);
+    }
   }
 }
 
@@ -1347,7 +1399,6 @@ extern "C" void bem_lu_free(bem_lu *w) {
   cudaFree(w->piv);
   cudaFree(w->u11);
   cudaFree(w->status);
-  cudaFree(w->flags);
   cudaFree(w->y);
   if (w->ev_fork) cudaEventDestroy(w->ev_fork);
   if (w->ev_join) cudaEventDestroy(w->ev_join);
@@ -1552,8 +1603,7 @@ extern "C" int bem_lu_factor_z(bem_lu *w, double *A, int n, cudaStream_t st) { r
 extern "C" int bem_lu_factor_c(bem_lu *w, float *A, int n, cudaStream_t st) { return lu_factor<float2>(w, A, n, st); }
 
 template <class C2, int NR>
-static int launch_trsv(bem_lu *w, const C2 *LU, int n, const C2 *in, C2 *out, unsigned *flags, int lower,
-                       cudaStream_t st) {
+static int launch_trsv(bem_lu *w, const C2 *LU, int n, const C2 *in, C2 *out, int lower, cudaStream_t st) {
   const int nb = (n + 31) / 32;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nb < w->coop_blocks ? nb : w->coop_blocks);
@@ -1564,8 +1614,8 @@ static int launch_trsv(bem_lu *w, const C2 *LU, int n, const C2 *in, C2 *out, un
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  CKL(cudaLaunchKernelEx(&cfg, k_lu_trsv<C2, NR>, LU, (long)n, n, (const int *)w->rowmap, in, out, flags, lower,
-                         w->status),
+  CKL(cudaMemsetAsync(out, 0xff, (size_t)n * NR * sizeof(C2), st), "triangular solve");
+  CKL(cudaLaunchKernelEx(&cfg, k_lu_trsv<C2, NR>, LU, (long)n, n, (const int *)w->rowmap, in, out, lower, w->status),
       "triangular solve");
   bem_count_launches(1);
   return 0;
@@ -1578,18 +1628,16 @@ static int lu_solve(bem_lu *w, const void *LUv, int n, int nrhs, void *Bv, cudaS
     snprintf(w->err, sizeof(w->err), "LU solve: %d right-hand sides (1..4)", nrhs);
     return -1;
   }
-  if (grow_bytes(w, (void **)&w->flags, &w->flags_cap, 2 * TS_FSTRIDE * sizeof(unsigned), "solve flags") ||
-      grow_bytes(w, &w->y, &w->y_cap, (size_t)n * nrhs * sizeof(C2), "solve scratch"))
+  if (grow_bytes(w, &w->y, &w->y_cap, (size_t)n * nrhs * sizeof(C2), "solve scratch"))
     return -1;
   const C2 *LU = (const C2 *)LUv;
   C2 *B = (C2 *)Bv, *Y = (C2 *)w->y;
-  CKL(cudaMemsetAsync(w->flags, 0, 2 * TS_FSTRIDE * sizeof(unsigned), st), "solve flags");
   int rc = 0;
   switch (nrhs) {
-    case 1: rc = launch_trsv<C2, 1>(w, LU, n, B, Y, w->flags, 1, st) || launch_trsv<C2, 1>(w, LU, n, Y, B, w->flags + TS_FSTRIDE, 0, st); break;
-    case 2: rc = launch_trsv<C2, 2>(w, LU, n, B, Y, w->flags, 1, st) || launch_trsv<C2, 2>(w, LU, n, Y, B, w->flags + TS_FSTRIDE, 0, st); break;
-    case 3: rc = launch_trsv<C2, 3>(w, LU, n, B, Y, w->flags, 1, st) || launch_trsv<C2, 3>(w, LU, n, Y, B, w->flags + TS_FSTRIDE, 0, st); break;
-    default: rc = launch_trsv<C2, 4>(w, LU, n, B, Y, w->flags, 1, st) || launch_trsv<C2, 4>(w, LU, n, Y, B, w->flags + TS_FSTRIDE, 0, st); break;
+    case 1: rc = launch_trsv<C2, 1>(w, LU, n, B, Y, 1, st) || launch_trsv<C2, 1>(w, LU, n, Y, B, 0, st); break;
+    case 2: rc = launch_trsv<C2, 2>(w, LU, n, B, Y, 1, st) || launch_trsv<C2, 2>(w, LU, n, Y, B, 0, st); break;
+    case 3: rc = launch_trsv<C2, 3>(w, LU, n, B, Y, 1, st) || launch_trsv<C2, 3>(w, LU, n, Y, B, 0, st); break;
+    default: rc = launch_trsv<C2, 4>(w, LU, n, B, Y, 1, st) || launch_trsv<C2, 4>(w, LU, n, Y, B, 0, st); break;
   }
   return rc ? -1 : 0;
 }

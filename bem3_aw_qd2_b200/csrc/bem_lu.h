@@ -22,8 +22,6 @@ struct bem_lu {
   size_t tree_cap = 0;
   void *u11 = nullptr;      // panel scratch: packed L11\U11, inverse of U11, inverse of L11, staged rows
   unsigned *status = nullptr;
-  unsigned *flags = nullptr;  // triangular-solve progress counters (lower, upper), 128 bytes apart
-  size_t flags_cap = 0;
   void *y = nullptr;          // triangular-solve intermediate (n x nrhs complex)
   size_t y_cap = 0;
   // the factorisation of one (matrix, size) as a CUDA graph, replayed while both stay the same
