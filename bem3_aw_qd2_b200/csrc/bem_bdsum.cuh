@@ -541,18 +541,26 @@ __global__ void __launch_bounds__(SMB_TH, 2) k_sm_bdsum(const __grid_constant__ 
   }
 }
 
+// the densities of a rule's sources with the boundary values given
+static int launch_density(const bem_smooth *S, const sm_dev &d, const bem_dom_dev *D, int type, const double *P,
+                          const double *dP, const double *pv, const double *dpv, cudaStream_t st) {
+  const int smem = (16 + std::max(2 * (S->lmax + 1), 4 * S->lmax)) * SMV_PT * (int)sizeof(double);
+  if (cudaFuncSetAttribute(k_sm_density, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
+  k_sm_density<<<dim3(SMD_NCH, S->lmax + 1), SMD_TH, smem, st>>>(d, *D, type, P, dP, pv, dpv);
+  k_sm_density_sum<<<(8 * S->K + SMB_TH - 1) / SMB_TH, SMB_TH, 0, st>>>(d);
+  k_sm_density_T<<<S->K, SMB_TH, 0, st>>>(d);
+  bem_count_launches(3);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+}
+
 extern "C" int bem_launch_bdsum(bem_smooth *S, const bem_dom_dev *D, const bem_qp *q, int type, int ntgt, const int *tgt_t,
                                 const double *tgt_ze, const double *P, const double *dP, const double *pv,
                                 const double *dpv, double *out, unsigned *status, cudaStream_t st) {
   if (ntgt <= 0) return 0;
   if (!(S->have0 <= S->first && S->first < S->have1) && launch_rest(S, q, S->first, 1, status, st)) return -1;
   const sm_dev d = dev_view(S, D->ne, S->first, true);
-  const int smem = (16 + std::max(2 * (S->lmax + 1), 4 * S->lmax)) * SMV_PT * (int)sizeof(double);
-  if (cudaFuncSetAttribute(k_sm_density, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
-  k_sm_density<<<dim3(SMD_NCH, S->lmax + 1), SMD_TH, smem, st>>>(d, *D, type, P, dP, pv, dpv);
-  k_sm_density_sum<<<(8 * S->K + SMB_TH - 1) / SMB_TH, SMB_TH, 0, st>>>(d);
-  k_sm_density_T<<<S->K, SMB_TH, 0, st>>>(d);
+  if (launch_density(S, d, D, type, P, dP, pv, dpv, st)) return -1;
   k_sm_bdsum<<<ntgt, SMB_TH, 0, st>>>(d, *D, *q, type, tgt_t, tgt_ze, P, dP, pv, dpv, out, status);
-  bem_count_launches(4);
+  bem_count_launches(1);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

@@ -7,6 +7,7 @@
 #include <math.h>
 #include <thread>
 #include <unordered_map>
+#include <algorithm>
 #include <vector>
 #include "../../include/bemgpu.h"
 #include "bem_kernels.h"
@@ -58,6 +59,9 @@ struct bemgpu_ctx {
   double zlo = 0.0;        // and its lower end
   double *fst = nullptr;   // evanescent order table for field points above or below the mesh
   size_t fst_cap = 0;
+  bem_smooth fsm;          // the split for field points, its tables and expansion (of the last call's points)
+  double *fsm_tab = nullptr, *fsm_keep = nullptr;
+  size_t fsm_cap[2] = {0, 0};
   double pw[16] = {};      // incident plane wave (bemgpu_problem.pw)
   int far_rule = 1;        // shorter rules for regular pairs of the periodic domain (bemgpu_set_far_rule)
   double eta_scale = 0.0;  // Ewald parameter off the lattice plane = eta0 x eta_scale; 0: by rule per problem
@@ -211,7 +215,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
       dfree(S->rowF); dfree(S->near_s); dfree(S->near_n); dfree(S->nearF); dfree(S->selfF); dfree(S->flag);
     }
     dfree(c->scr.plist); dfree(c->scr.pcount);
-    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->fst); dfree(c->b0); dfree(c->B3s);
+    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->fst); dfree(c->fsm_tab); dfree(c->fsm_keep); dfree(c->b0); dfree(c->B3s);
     for (int d = 0; d < BEMGPU_MAXDOM; ++d) { dfree(c->Wd[d]); dfree(c->cinv[d]); dfree(c->Gc[d]); }
     dfree(c->B3c);
     dfree(c->dGc); dfree(c->dHc);
@@ -1436,6 +1440,61 @@ static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources
   return 0;
 }
 
+// The points that the split c->fsm takes (their number; order: they first, then the
+// others, empty where that is how they come), planned for the largest ball of those
+// that hold all, 9, 7 or 5 in 10 of the points for which images, expansion and the
+// other points' lattice sums cost least.  Costs in FP64 operations at the kernels'
+// rates: a pair's lattice sum 7e4 with second derivatives, 1.5e4 without, set-up
+// and its launches 1e10 (0.5 ms).  0: none.
+static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int grad, std::vector<int> &order) {
+  const double pair = grad ? 7e4 : 1.5e4, all = (double)n * src * pair;
+  if (!c->sm.on || all < 2e10) return 0;
+  std::vector<double> d(n);
+  for (int i = 0; i < n; ++i)
+    d[i] = sqrt((r[3 * i] - c->sm.ctr[0]) * (r[3 * i] - c->sm.ctr[0]) + (r[3 * i + 1] - c->sm.ctr[1]) * (r[3 * i + 1] - c->sm.ctr[1]) +
+                (r[3 * i + 2] - c->sm.ctr[2]) * (r[3 * i + 2] - c->sm.ctr[2]));
+  for (int i = 0; i < n; ++i)
+    if (!(d[i] < 1e300)) return 0;
+  std::vector<double> by(d);
+  std::sort(by.begin(), by.end());
+  double best = all, Rx = 0.0;
+  for (const double part : {1.0, 0.9, 0.7, 0.5}) {
+    const double R = by[(size_t)ceil(part * n) - 1];
+    const double cost = bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, R, part * n, (double)src) + 1e10 + (1.0 - part) * all;
+    if (cost < best) {
+      best = cost;
+      Rx = R;
+    }
+  }
+  if (!(Rx > 0.0)) return 0;
+  bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, Rx, n, (double)src);
+  std::vector<double> h(bem_smooth_layout(&c->fsm).total);
+  bem_smooth_tables(&c->fsm, &c->qp, h.data());
+  double **p[2] = {&c->fsm_tab, &c->fsm_keep};
+  const size_t need[2] = {h.size(), bem_smooth_keep_doubles(&c->fsm)};
+  for (int i = 0; i < 2; ++i)
+    if (need[i] > c->fsm_cap[i]) {
+      dfree(*p[i]);
+      c->fsm_cap[i] = 0;
+      if (dalloc(p[i], need[i]) != cudaSuccess) {  // lattice sums, then
+        cudaGetLastError();
+        return 0;
+      }
+      c->fsm_cap[i] = need[i];
+    }
+  c->fsm.tab = c->fsm_tab;
+  c->fsm.keep = c->fsm_keep;
+  CK(cudaMemcpyAsync(c->fsm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
+  int near = 0;
+  for (int i = 0; i < n; ++i) near += d[i] <= Rx;
+  if (near < n) {
+    order.resize(n);
+    int a = 0, b = near;
+    for (int i = 0; i < n; ++i) order[d[i] <= Rx ? a++ : b++] = i;
+  }
+  return near;
+}
+
 extern "C" int bemgpu_field(bemgpu_ctx *c, int d, int type, int n, const double *r, double *out) {
   if (!c->loaded || d < 0 || d > c->MN) { snprintf(c->err, sizeof(c->err), "bad domain %d", d); return -2; }
   const int grad = !(type & BEMGPU_FIELD_POTENTIAL);
@@ -1444,15 +1503,38 @@ extern "C" int bemgpu_field(bemgpu_ctx *c, int d, int type, int n, const double 
   if (n <= 0) return 0;
   if (ensure_points(c, n)) return -1;
   bem_dom_dev D = dom_view(c, d);
-  CK(cudaMemcpyAsync(c->pt_in, r, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, c->stream), "field points");
+  const long long src = (long long)c->dom_ne[d] * (type == 0 ? 4 : type == 1 ? 9 : type == 2 ? 144 : 4096);
+  // points of the split first (order: the call's), the others after them
+  std::vector<int> order;
+  const int near = d == 0 ? field_split(c, n, r, src, grad, order) : 0;
+  if (near < 0) return -1;
+  std::vector<double> rs, os;
+  const double *rp = r;
+  if (!order.empty()) {
+    rs.resize(3 * (size_t)n);
+    os.resize(18 * (size_t)n);
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < 3; ++j) rs[3 * (size_t)i + j] = r[3 * (size_t)order[i] + j];
+    rp = rs.data();
+  }
+  CK(cudaMemcpyAsync(c->pt_in, rp, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, c->stream), "field points");
   bem_qp q = c->qp;
-  if (d == 0 && field_tables(c, n, r, (long long)c->dom_ne[0] * (type == 0 ? 4 : type == 1 ? 9 : type == 2 ? 144 : 4096), &q))
-    return -1;
-  if (bem_launch_field(&D, &q, d == 0, grad, c->k0[d], type, n, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
-                       c->pt_out, c->status, c->stream))
+  if (near && (bem_launch_smfield(&c->fsm, &D, &q, grad, type, near, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
+                                  c->pt_out, c->pt_t, c->status, c->stream) ||
+               bem_launch_field(&D, &q, 1, grad, c->k0[d], type, near, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
+                                c->pt_out, c->status, c->pt_t, c->stream)))
     return fail(c, "field", cudaGetLastError());
-  CK(cudaMemcpyAsync(out, c->pt_out, 18 * sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream), "field");
+  if (near < n) {
+    if (d == 0 && field_tables(c, n - near, rp + 3 * (size_t)near, src, &q)) return -1;
+    if (bem_launch_field(&D, &q, d == 0, grad, c->k0[d], type, n - near, c->pt_in + 3 * (size_t)near, c->P[d], c->dP[d],
+                         c->pv[d], c->dpv[d], c->pt_out + 18 * (size_t)near, c->status, nullptr, c->stream))
+      return fail(c, "field", cudaGetLastError());
+  }
+  double *op = order.empty() ? out : os.data();
+  CK(cudaMemcpyAsync(op, c->pt_out, 18 * sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream), "field");
   CK(cudaStreamSynchronize(c->stream), "field");
+  if (!order.empty())
+    for (int i = 0; i < n; ++i) memcpy(out + 18 * (size_t)order[i], op + 18 * (size_t)i, 18 * sizeof(double));
   return 0;
 }
 

@@ -54,7 +54,9 @@ __global__ void __launch_bounds__(FIELD_THREADS) k_field(bem_dom_dev D, const __
                                                          const double *__restrict__ pts, const double *__restrict__ P,
                                                          const double *__restrict__ dP, const double *__restrict__ pv,
                                                          const double *__restrict__ dpv, double *__restrict__ out,
-                                                         unsigned *status) {
+                                                         unsigned *status,
+                                                         const int *__restrict__ only) {
+  if (only && !only[blockIdx.x]) return;
   // the real-space table in shared memory and spectral orders from a table that
   // reaches the points (bemgpu_field): 1500 points of 216 quads on the 9-point rule
   // 15.0 -> 10.9 ms, at 47 % of the FP64 pipe with three blocks an SM (registers)
@@ -345,10 +347,10 @@ __global__ void k_force_bd(bem_dom_dev D, int ntgt, const int *__restrict__ tgt_
 
 extern "C" int bem_launch_field(const bem_dom_dev *D, const bem_qp *q, int periodic, int grad, double k, int type,
                                 int npts, const double *pts, const double *P, const double *dP, const double *pv,
-                                const double *dpv, double *out, unsigned *status, cudaStream_t st) {
+                                const double *dpv, double *out, unsigned *status, const int *only, cudaStream_t st) {
   if (npts <= 0) return 0;
   const int smem = periodic && grad && q->wt ? BEM_WT_SMEM : 0;
-  k_field<<<npts, FIELD_THREADS, smem, st>>>(*D, *q, periodic, grad, k, type, pts, P, dP, pv, dpv, out, status);
+  k_field<<<npts, FIELD_THREADS, smem, st>>>(*D, *q, periodic, grad, k, type, pts, P, dP, pv, dpv, out, status, only);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

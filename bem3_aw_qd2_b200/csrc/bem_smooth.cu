@@ -94,6 +94,20 @@ static int degree_for(double k, double a, double b, double scale, double tol, in
   return 0;
 }
 
+// lattice points by distance, to the reach and four periods (empty: far too many)
+struct sm_pt { double r; int a, b; };
+static std::vector<sm_pt> lattice_by_distance(const bem_qp *q, double reach) {
+  std::vector<sm_pt> P;
+  reach += 4.0 * (hypot(q->d1x, q->d1y) + hypot(q->d2x, q->d2y));
+  const double n1 = floor(reach * hypot(q->g1x, q->g1y) / (2.0 * M_PI)) + 1, n2 = floor(reach * hypot(q->g2x, q->g2y) / (2.0 * M_PI)) + 1;
+  if (!(n1 * n2 <= 1e5)) return P;
+  for (int a = -(int)n1; a <= (int)n1; ++a)
+    for (int b = -(int)n2; b <= (int)n2; ++b) P.push_back({hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y), a, b});
+  std::stable_sort(P.begin(), P.end(), [](const sm_pt &x, const sm_pt &y) { return x.r < y.r; });
+  return P;
+}
+static void finish_plan(bem_smooth *S, const bem_qp *q);
+
 void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int *npe, const int *sid, int ne) {
   S->on = 0;
   S->have0 = S->have1 = 0;
@@ -135,15 +149,7 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
   S->rho = 2.0 * S->R0;
   S->k = q->k;
   if (!(S->R0 > 0.0) || !std::isfinite(S->R0)) return;
-  // lattice points by distance
-  struct pt { double r; int a, b; };
-  std::vector<pt> P;
-  const double reach = 12.0 * S->R0 + 4.0 * (hypot(q->d1x, q->d1y) + hypot(q->d2x, q->d2y));
-  const int n1 = (int)(reach * hypot(q->g1x, q->g1y) / (2.0 * M_PI)) + 1, n2 = (int)(reach * hypot(q->g2x, q->g2y) / (2.0 * M_PI)) + 1;
-  if ((double)n1 * n2 > 1e5) return;
-  for (int a = -n1; a <= n1; ++a)
-    for (int b = -n2; b <= n2; ++b) P.push_back({hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y), a, b});
-  std::stable_sort(P.begin(), P.end(), [](const pt &x, const pt &y) { return x.r < y.r; });
+  const std::vector<sm_pt> P = lattice_by_distance(q, 12.0 * S->R0);
   // the cheapest split, in FP64 operations at the rates that the kernels reach
   // (images 0.55 of the pipe, the product 0.7): per pair about 45 points of 66
   // for each image and 16 multiply-adds for each of the K functions (G and H of
@@ -173,7 +179,54 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
       for (size_t i = 0; i < c; ++i) { S->l1[i] = P[i].a; S->l2[i] = P[i].b; }
     }
   }
-  if (!S->on) return;
+  if (S->on) finish_plan(S, q);
+}
+
+// The split for sums at points up to Rx from the body's centre: the larger ball
+// takes R0's place, the degrees follow from both (a source at R0 against images
+// seen from Rx, a point at Rx against images seen from R0).  Returns the FP64
+// operations of n points and their sources, a large number where there is none.
+double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources) {
+  F->on = 0;
+  F->have0 = F->have1 = 0;
+  F->inst = 1;
+  F->first = 0;
+  F->k = q->k;
+  for (int d = 0; d < 3; ++d) F->ctr[d] = S->ctr[d];
+  F->R0 = std::max(Rx, S->R0) * (1.0 + 1e-12);
+  F->rho = F->R0 + S->R0;
+  double best = 1e300;
+  if (!(F->R0 < 1e3 * S->R0)) return best;
+  const std::vector<sm_pt> P = lattice_by_distance(q, 3.0 * F->rho);
+  for (size_t c = 1; c < P.size() && c <= BEM_SM_MAXIMG; ++c) {
+    if (P[c].r <= P[c - 1].r * (1.0 + 1e-9)) continue;  // whole shells only
+    const double cut = P[c].r;
+    if (cut <= F->rho * 1.05) continue;
+    const int lx = degree_for(F->k, F->R0, cut - S->R0, 6.0 * F->rho, 1e-15, BEM_SM_MAXL);
+    const int ly = degree_for(F->k, S->R0, cut - F->R0, 6.0 * F->rho, 1e-15, BEM_SM_MAXL);
+    if (lx < 0 || ly < 0) continue;
+    const int lmax = std::max(lx, ly);
+    int Lmax = degree_for(F->k, F->rho, cut, 6.0 * F->rho, 1e-15, 2 * BEM_SM_MAXL);
+    if (Lmax < 0 || Lmax > 2 * lmax) Lmax = 2 * lmax;
+    // an image with second derivatives about 160 operations, a pair's own part 400
+    const double K = (lmax + 1.0) * (lmax + 1.0), nt = lmax + 0.5 * Lmax + 1.0;
+    const double cost = n * sources * (400.0 + c * 160.0) / 0.55 + nt * (2.0 * Lmax + 2.0) * 3e4 + 0.25 * K * K * lmax * nt +
+                        sources * K * 60.0;
+    if (cost < best) {
+      best = cost;
+      F->on = 1;
+      F->lmax = lmax;
+      F->Lmax = Lmax;
+      F->nimg = (int)c;
+      F->cut = cut - F->rho;
+      for (size_t i = 0; i < c; ++i) { F->l1[i] = P[i].a; F->l2[i] = P[i].b; }
+    }
+  }
+  if (F->on) finish_plan(F, q);
+  return F->on ? best : 1e300;
+}
+
+static void finish_plan(bem_smooth *S, const bem_qp *q) {
   // degrees for one point's rest at |R| <= (i + 1) 2 R0 / 8 (the gradient's terms are
   // those of the value times l / |R|)
   for (int i = 0; i < 8; ++i) {
@@ -1163,3 +1216,4 @@ extern "C" int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_
 }
 
 #include "bem_bdsum.cuh"
+#include "bem_smfield.cuh"

@@ -38,6 +38,7 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
 bem_smooth_tab bem_smooth_layout(const bem_smooth *S);
 // the tables of S->inst instances (qps: their Bloch wave vectors) into h[layout.total]
 void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h);
+double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources);
 size_t bem_smooth_keep_doubles(const bem_smooth *S);
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
 
@@ -54,4 +55,10 @@ int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, in
 int bem_launch_bdsum(bem_smooth *S, const bem_dom_dev *D, const bem_qp *q, int type, int ntgt, const int *tgt_t,
                      const double *tgt_ze, const double *P, const double *dP, const double *pv, const double *dpv,
                      double *out, unsigned *status, cudaStream_t st);
+// Field sums of k_field at points within the ball of a plan made by
+// bem_smooth_plan_field (bem_smfield.cuh); pts, out as bem_launch_field's, again[i]: 1
+// where a source lies on the lattice plane through point i (out not written)
+int bem_launch_smfield(bem_smooth *F, const bem_dom_dev *D, const bem_qp *q, int grad, int type, int npts,
+                       const double *pts, const double *P, const double *dP, const double *pv, const double *dpv,
+                       double *out, int *again, unsigned *status, cudaStream_t st);
 }
