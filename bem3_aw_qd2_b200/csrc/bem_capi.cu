@@ -1637,37 +1637,29 @@ extern "C" int bemgpu_qpgf(const double *qpar, const double *r, int n, double *G
   if (ensure_constants(nullptr, nullptr, nullptr, nullptr, nullptr) != 0) return -1;
   bem_qp q;
   bem_qp_prepare(qpar, &q);
-  double *wt = nullptr;
-  if (cudaMalloc(&wt, BEM_WT_SIZE * sizeof(double)) != cudaSuccess) return -1;
-  if (bem_launch_wtab(q.k, q.eta_run, wt, 0) != 0) { cudaFree(wt); return -1; }
-  q.wt = wt;
-  q.wt_h = BEM_WT_H;
-  q.wt_n = BEM_WT_N;
   // evanescent order table reaching the points' |z|
   double zmax = 0.0;
   for (int i = 0; i < n; ++i) zmax = fabs(r[3 * i + 2]) > zmax ? fabs(r[3 * i + 2]) : zmax;
-  double *stb = nullptr;
-  const size_t scnt = stab_window(&q, 2.0 * zmax);
-  if (scnt) {
-    if (cudaMalloc(&stb, scnt * sizeof(double)) != cudaSuccess) { cudaFree(wt); return -1; }
-    if (bem_launch_stab(&q, stb, 0) != 0) { cudaFree(wt); cudaFree(stb); return -1; }
-    q.st = stb;
-  }
-  double *dr = nullptr, *dg = nullptr, *ddg = nullptr;
-  int *dret = nullptr;
+  const size_t scnt = stab_window(&q, zmax), N = (size_t)n;
+  // one allocation for the tables, the points and the results (six cost 1 ms)
+  double *buf = nullptr;
+  if (cudaMalloc(&buf, (BEM_WT_SIZE + scnt + 11 * N + (N + 1) / 2) * sizeof(double)) != cudaSuccess) return -1;
+  double *wt = buf, *stb = wt + BEM_WT_SIZE, *dr = stb + scnt, *dg = dr + 3 * N, *ddg = dg + 2 * N;
+  int *dret = (int *)(ddg + 6 * N);
   int rc = -1;
-  if (cudaMalloc(&dr, 3 * sizeof(double) * n) == cudaSuccess && cudaMalloc(&dg, 2 * sizeof(double) * n) == cudaSuccess &&
-      cudaMalloc(&ddg, 6 * sizeof(double) * n) == cudaSuccess && cudaMalloc(&dret, sizeof(int) * n) == cudaSuccess) {
-    cudaMemcpy(dr, r, 3 * sizeof(double) * n, cudaMemcpyHostToDevice);
-    rc = bem_launch_qpgf(&q, dr, n, dg, ddg, dret, 0);
-    if (rc == 0) {
-      if (cudaMemcpy(G, dg, 2 * sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess ||
-          cudaMemcpy(dG, ddg, 6 * sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess ||
-          cudaMemcpy(ret, dret, sizeof(int) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
-        rc = -1;
-    }
+  if (cudaMemcpy(dr, r, 3 * sizeof(double) * N, cudaMemcpyHostToDevice) == cudaSuccess &&
+      bem_launch_wtab(q.k, q.eta_run, wt, 0) == 0 && (scnt == 0 || bem_launch_stab(&q, stb, 0) == 0)) {
+    q.wt = wt;
+    q.wt_h = BEM_WT_H;
+    q.wt_n = BEM_WT_N;
+    if (scnt) q.st = stb;
+    if (bem_launch_qpgf(&q, dr, n, dg, ddg, dret, 0) == 0 &&
+        cudaMemcpy(G, dg, 2 * sizeof(double) * N, cudaMemcpyDeviceToHost) == cudaSuccess &&
+        cudaMemcpy(dG, ddg, 6 * sizeof(double) * N, cudaMemcpyDeviceToHost) == cudaSuccess &&
+        cudaMemcpy(ret, dret, sizeof(int) * N, cudaMemcpyDeviceToHost) == cudaSuccess)
+      rc = 0;
   }
-  cudaFree(dr); cudaFree(dg); cudaFree(ddg); cudaFree(dret); cudaFree(wt); cudaFree(stb);
+  cudaFree(buf);
   return rc;
 }
 
