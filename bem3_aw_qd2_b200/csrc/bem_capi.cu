@@ -54,7 +54,7 @@ struct bemgpu_ctx {
   // images + expansion of the periodic domain (bem_smooth.cu): its tables, and
   // its workspace where the global matrix is too small to lend its own
   bem_smooth sm;
-  double *sm_tab = nullptr, *sm_keep = nullptr, *sm_buf = nullptr;
+  double *sm_buf = nullptr;
   double zspan = 0.0;      // height of the mesh (z extent of all elements)
   double zlo = 0.0;        // and its lower end
   double *fst = nullptr;   // evanescent order table for field points above or below the mesh
@@ -215,7 +215,7 @@ static void free_problem(bemgpu_ctx *c, bool release) {
       dfree(S->rowF); dfree(S->near_s); dfree(S->near_n); dfree(S->nearF); dfree(S->selfF); dfree(S->flag);
     }
     dfree(c->scr.plist); dfree(c->scr.pcount);
-    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_tab); dfree(c->sm_keep); dfree(c->sm_buf); dfree(c->fst); dfree(c->fsm_tab); dfree(c->fsm_keep); dfree(c->b0); dfree(c->B3s);
+    dfree(c->A); dfree(c->b); dfree(c->tpv); dfree(c->B3); dfree(c->wtab); dfree(c->stab); dfree(c->sm_buf); dfree(c->fst); dfree(c->fsm_tab); dfree(c->fsm_keep); dfree(c->b0); dfree(c->B3s);
     for (int d = 0; d < BEMGPU_MAXDOM; ++d) { dfree(c->Wd[d]); dfree(c->cinv[d]); dfree(c->Gc[d]); }
     dfree(c->B3c);
     dfree(c->dGc); dfree(c->dHc);
@@ -409,19 +409,16 @@ static int smooth_setup(bemgpu_ctx *c, int inst, const bem_qp *qps) {
   if (!c->sm.on) return 0;
   std::vector<double> h(bem_smooth_layout(&c->sm).total);
   bem_smooth_tables(&c->sm, qps, h.data());
-  CK(falloc(c, &c->sm_tab, h.size()), "expansion tables");
-  CK(cudaMemcpyAsync(c->sm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
-  c->sm.tab = c->sm_tab;
-  CK(falloc(c, &c->sm_keep, bem_smooth_keep_doubles(&c->sm)), "expansion");
-  c->sm.keep = c->sm_keep;
-  c->sm.have0 = c->sm.have1 = 0;
+  // one allocation: tables, what is kept, and the workspace where it is not in A
+  const size_t tab = (h.size() + 31) / 32 * 32, keep = (bem_smooth_keep_doubles(&c->sm) + 31) / 32 * 32;
   const size_t need = bem_smooth_ws_doubles(&c->sm, c->dom_ne[0]);
-  if (inst == 1 && need <= 2 * (size_t)c->n * c->n) {
-    c->sm.ws = c->A;
-  } else {
-    CK(falloc(c, &c->sm_buf, need), "expansion workspace");
-    c->sm.ws = c->sm_buf;
-  }
+  const bool in_A = inst == 1 && need <= 2 * (size_t)c->n * c->n;
+  CK(falloc(c, &c->sm_buf, tab + keep + (in_A ? 0 : need)), "expansion");
+  CK(cudaMemcpyAsync(c->sm_buf, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
+  c->sm.tab = c->sm_buf;
+  c->sm.keep = c->sm_buf + tab;
+  c->sm.have0 = c->sm.have1 = 0;
+  c->sm.ws = in_A ? c->A : c->sm_buf + tab + keep;
   return 0;
 }
 

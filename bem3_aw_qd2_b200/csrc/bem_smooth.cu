@@ -354,7 +354,7 @@ void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h) {
 
 // ------------------------------------------------------------------ device view
 struct sm_dev {
-  int lmax, Lmax, K, Kp, nt, nphi, nimg, nlm;  // nlm: pairs (l, m >= 0) up to Lmax
+  int lmax, Lmax, Mx, K, Kp, nt, nphi, nimg, nlm;  // nlm: pairs (l, m >= 0) up to Lmax
   double cx, cy, cz, R0, iR0, kR0, rho, k, cut;
   double eta;                       // Ewald parameter of the samples
   int nreal, r1, r2, nspec, s1, s2, sc2;  // its windows: l1 in [-r1, r1], l2 in [-r2, r2]; n1 - nc1 in [-s1, s1], ...
@@ -364,13 +364,14 @@ struct sm_dev {
   double *plm;            // [nt][lm >= 0] normalised Legendre functions P_lm(x_t)
   double *samp;           // [nb][2][nt][nphi] complex: G_s and rho dG_s/drho
   double *sig;            // [nb][(Lmax + 1)^2] complex
+  double *F;              // [nb][Lmax + 1][nt / 2][2 Mx + 1] complex: partial sums over L (k_sm_F)
   double *T;              // [nb][Kp][2 Kp]: T^t, real and imaginary parts
   double *Z, *Zt;         // densities of boundary sums: [32][Kp][8], [Kp][8]
   double *U, *V, *A;      // [4 ne][Kp], [Kp][8 ne], [nb][4 ne][2 Kp]
 };
 // What stays valid after an assembly (for boundary sums): Legendre functions,
 // samples, sigma, T of up to BEM_SM_BAT instances, the densities
-struct sm_keep { size_t plm, samp, sig, T, Z, Zt, total; };
+struct sm_keep { size_t plm, samp, sig, F, T, Z, Zt, total; };
 static sm_keep keep_layout(const bem_smooth *S) {
   sm_keep w;
   size_t o = 0;
@@ -379,6 +380,7 @@ static sm_keep keep_layout(const bem_smooth *S) {
   w.plm = put((L + 1) * (L + 2) / 2 * S->nt);
   w.samp = put(nb * 4 * S->nt * S->nphi);
   w.sig = put(nb * 2 * (L + 1) * (L + 1));
+  w.F = put(nb * 2 * (L + 1) * (S->nt / 2) * (2 * std::min(2 * S->lmax, S->Lmax) + 1));
   w.T = put(nb * 2 * Kp * Kp);
   w.Z = put(32 * Kp * 8);
   w.Zt = put((Kp + 1) * 8);
@@ -592,70 +594,8 @@ __global__ void __launch_bounds__(SMC_TH) k_sm_coef(const __grid_constant__ sm_d
 // position of the real function (l, m): cosine (or m = 0) and sine
 __device__ __forceinline__ int sm_idx(int l, int m, int sine) { return l * l + (m ? 2 * m - 1 + sine : 0); }
 
-// T_lm,l'm' = 4 pi sum_L sigma_{L,m-m'} i^{l-l'-L} C (2L+1)!! ... with
-// C = int Y*_lm Y_l'm' Y_{L,m-m'} = 2 pi int P_lm P_l'm' P_L|m-m'| d(cos theta)
-// (harmonics without the Condon-Shortley sign, Y_{l,-m} = conj Y_lm), in the
-// real basis.  Block: (l, m >= 0); thread: (l', m' >= 0).  The integrand is
-// even: half the nodes.  Stored transposed, row l'm', columns lm (real part)
-// and Kp + lm (imaginary part).
-#define SMT_TH 64
-__global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev S) {
-  extern __shared__ double sm_raw[];  // [nt / 2][SMT_TH]
-  const int b = blockIdx.z;
-  int l = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
-  while ((l + 1) * (l + 2) / 2 <= (int)blockIdx.x) ++l;
-  while (l * (l + 1) / 2 > (int)blockIdx.x) --l;
-  const int m = (int)blockIdx.x - l * (l + 1) / 2;
-  const int i2 = blockIdx.y * SMT_TH + threadIdx.x;
-  const int nlm = (S.lmax + 1) * (S.lmax + 2) / 2;
-  const bool live = i2 < nlm;
-  int l2 = 0, m2 = 0;
-  if (live) {
-    l2 = (int)((sqrt(8.0 * i2 + 1.0) - 1.0) * 0.5);
-    while ((l2 + 1) * (l2 + 2) / 2 <= i2) ++l2;
-    while (l2 * (l2 + 1) / 2 > i2) --l2;
-    m2 = i2 - l2 * (l2 + 1) / 2;
-  }
-  const int nh = S.nt / 2;
-  double *pr = sm_raw + threadIdx.x;
-  const double *p1 = S.plm + blockIdx.x, *p2 = S.plm + (live ? i2 : 0);
-#pragma unroll 4
-  for (int t = 0; t < nh; ++t)
-    pr[t * SMT_TH] = 4.0 * CUDART_PI * S.w[t] * p1[(size_t)t * S.nlm] * p2[(size_t)t * S.nlm];
-  if (!live) return;
-  const double *sg = S.sig + 2 * (size_t)b * (S.Lmax + 1) * (S.Lmax + 1);
-  // tp[0]: T_{m,m'}, tp[1]: T_{-m,-m'}, tp[2]: T_{m,-m'}, tp[3]: T_{-m,m'}
-  cplx tp[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) tp[c] = cmk(0.0, 0.0);
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    if (v && (m == 0 || m2 == 0)) break;
-    const int M = v ? m + m2 : m - m2, aM = abs(M);
-    // L from |l - l'| for every thread (P_LM = 0 below |M|), so that threads of
-    // one l' read neighbouring P_LM
-    for (int L = abs(l - l2); L <= min(l + l2, S.Lmax); L += 2) {
-      if (L < aM) continue;
-      const double *pL = S.plm + L * (L + 1) / 2 + aM;
-      double G = 0.0, G1 = 0.0;
-      int t = 0;
-#pragma unroll 2
-      for (; t + 1 < nh; t += 2) {
-        G = fma(pr[t * SMT_TH], pL[(size_t)t * S.nlm], G);
-        G1 = fma(pr[(t + 1) * SMT_TH], pL[(size_t)(t + 1) * S.nlm], G1);
-      }
-      if (t < nh) G = fma(pr[t * SMT_TH], pL[(size_t)t * S.nlm], G);
-      G += G1;
-      // i^{l - l' - L}, l - l' - L even
-      const double f = ((l - l2 - L) & 2) ? -G * S.dL[L] : G * S.dL[L];
-      const double *sp = sg + 2 * (L * L + L + M), *sn = sg + 2 * (L * L + L - M);
-      tp[2 * v].re += f * sp[0];
-      tp[2 * v].im += f * sp[1];
-      tp[2 * v + 1].re += f * sn[0];
-      tp[2 * v + 1].im += f * sn[1];
-    }
-  }
-  const double sc = 4.0 * CUDART_PI * S.el[l] * S.el[l2];
+// the real functions' entries of T from those of e^{+-i m phi}, e^{+-i m' phi}
+__device__ __forceinline__ void sm_put_T(const sm_dev &S, int b, int l, int m, int l2, int m2, const cplx tp[4], double sc) {
   double *T = S.T + (size_t)b * 2 * S.Kp * S.Kp;
   auto put = [&](int r, int c, cplx z) {  // entry (source function r, target function c)
     T[(size_t)c * 2 * S.Kp + r] = sc * z.re;
@@ -680,6 +620,98 @@ __global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev 
     put(rc, cs, cscale(cmuli(csub(cadd(d, e), cadd(a, g))), 0.5));
     put(rs, cc, cscale(cmuli(csub(cadd(a, e), cadd(d, g))), 0.5));
   }
+}
+
+// T_lm,l'm' = 4 pi sum_L sigma_{L,m-m'} i^{l-l'-L} C (2L+1)!! ... with
+// C = int Y*_lm Y_l'm' Y_{L,m-m'} = 2 pi int P_lm P_l'm' P_L|m-m'| d(cos theta)
+// (harmonics without the Condon-Shortley sign, Y_{l,-m} = conj Y_lm), in the
+// real basis.  The sum over L goes under the integral: with
+// F_M^j(t) = sum of i^-L sigma_LM ... P_L|M|(t) over L <= j, L of j's parity, an entry is
+// one integral of P_lm P_l'm' F_{m-m'}^{l+l'} (L beyond l + l' integrate to zero, but
+// their size would drown the rest; those below |l - l'| only round).  An integral
+// for each L in its place was 16 (lmax 16) to 40 times the multiply-adds: 91 us
+// for 24 quads in a period of 0.8 and 600 us for the field points' ball; with F
+// 20 + 25 us and 110.
+//
+// F: [j <= Lmax][t][M = -Mx .. Mx], a thread per (t, M), its terms in order of L.
+#define SMF_FTH 128
+__global__ void __launch_bounds__(SMF_FTH) k_sm_F(const __grid_constant__ sm_dev S) {
+  const int b = blockIdx.y, nM = 2 * S.Mx + 1, nh = S.nt / 2;
+  const int i = blockIdx.x * SMF_FTH + threadIdx.x;
+  if (i >= nM * nh) return;
+  const int t = i / nM, M = i % nM - S.Mx, aM = abs(M);
+  const double2 *sg = reinterpret_cast<const double2 *>(S.sig) + (size_t)b * (S.Lmax + 1) * (S.Lmax + 1);
+  const double *p = S.plm + (size_t)t * S.nlm + aM;
+  double2 *F = reinterpret_cast<double2 *>(S.F) + (size_t)b * (S.Lmax + 1) * nh * nM + i;
+  double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+  for (int L = 0; L <= S.Lmax; ++L) {
+    if (L >= aM) {
+      const double f = (L & 2) ? -S.dL[L] * p[L * (L + 1) / 2] : S.dL[L] * p[L * (L + 1) / 2];
+      const double2 s = sg[L * L + L + M];
+      acc[0].x = fma(f, s.x, acc[0].x);
+      acc[0].y = fma(f, s.y, acc[0].y);
+    }
+    F[(size_t)L * nh * nM] = acc[0];
+    const double2 x = acc[0];  // the two parities in turn
+    acc[0] = acc[1];
+    acc[1] = x;
+  }
+}
+
+// Block: (l, m >= 0); thread: (l', m' >= 0) from (l, m) on, and the entries with
+// both exchanged (the same integrals, F_M for F_-M).  The integrand is even: half
+// the nodes.  Stored transposed, row l'm', columns lm (real part) and Kp + lm
+// (imaginary part).  Bound by the reads of F through L2.
+#define SMT_TH 64
+__global__ void __launch_bounds__(SMT_TH) k_sm_T(const __grid_constant__ sm_dev S) {
+  const int b = blockIdx.z;
+  auto lm = [](int i, int &l, int &m) {
+    l = (int)((sqrt(8.0 * i + 1.0) - 1.0) * 0.5);
+    while ((l + 1) * (l + 2) / 2 <= i) ++l;
+    while (l * (l + 1) / 2 > i) --l;
+    m = i - l * (l + 1) / 2;
+  };
+  const int i1 = blockIdx.x, i2 = blockIdx.y * SMT_TH + threadIdx.x;
+  const int nlm = (S.lmax + 1) * (S.lmax + 2) / 2;
+  if (i2 < i1 || i2 >= nlm) return;
+  int l, m, l2, m2;
+  lm(i1, l, m);
+  lm(i2, l2, m2);
+  const int nM = 2 * S.Mx + 1, nh = S.nt / 2, sum = l + l2;
+  const int j = sum <= S.Lmax ? sum : S.Lmax - ((S.Lmax ^ sum) & 1);
+  const int M1 = m - m2, M2 = m + m2;
+  const bool on2 = m && m2 && M2 <= S.Mx, on1 = abs(M1) <= S.Mx;
+  const double2 *F = reinterpret_cast<const double2 *>(S.F) + ((size_t)b * (S.Lmax + 1) + j) * nh * nM + S.Mx;
+  const double2 *Fa = F + (on1 ? M1 : 0), *Fb = F - (on1 ? M1 : 0), *Fc = F + (on2 ? M2 : 0), *Fd = F - (on2 ? M2 : 0);
+  const double *p1 = S.plm + i1, *p2 = S.plm + i2;
+  // tp[0]: T_{m,m'}, tp[1]: T_{-m,-m'}, tp[2]: T_{m,-m'}, tp[3]: T_{-m,m'}
+  cplx tp[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tp[c] = cmk(0.0, 0.0);
+#pragma unroll 4
+  for (int t = 0; t < nh; ++t) {
+    const double pr = 4.0 * CUDART_PI * S.w[t] * p1[(size_t)t * S.nlm] * p2[(size_t)t * S.nlm];
+    const size_t o = (size_t)t * nM;
+    const double2 fa = Fa[o], fb = Fb[o], fc = Fc[o], fd = Fd[o];
+    tp[0].re = fma(pr, fa.x, tp[0].re);
+    tp[0].im = fma(pr, fa.y, tp[0].im);
+    tp[1].re = fma(pr, fb.x, tp[1].re);
+    tp[1].im = fma(pr, fb.y, tp[1].im);
+    tp[2].re = fma(pr, fc.x, tp[2].re);
+    tp[2].im = fma(pr, fc.y, tp[2].im);
+    tp[3].re = fma(pr, fd.x, tp[3].re);
+    tp[3].im = fma(pr, fd.y, tp[3].im);
+  }
+  if (!on1) tp[0] = tp[1] = cmk(0.0, 0.0);
+  if (!on2) tp[2] = tp[3] = cmk(0.0, 0.0);
+  // i^{l - l'} beside F's i^{-L}: even exponents together
+  const double sc = 4.0 * CUDART_PI * S.el[l] * S.el[l2];
+  sm_put_T(S, b, l, m, l2, m2, tp, ((l - l2) & 2) ? -sc : sc);
+  if (i2 == i1) return;
+  const cplx x = tp[0];
+  tp[0] = tp[1];
+  tp[1] = x;
+  sm_put_T(S, b, l2, m2, l, m, tp, ((l2 - l) & 2) ? -sc : sc);
 }
 
 // ------------------------------------------------------------------ functions at nodes and over elements
@@ -1139,6 +1171,8 @@ static sm_dev dev_view(const bem_smooth *S, int ne, int b0, bool held = false) {
   d.plm = S->keep + k.plm;
   d.samp = S->keep + k.samp;
   d.sig = S->keep + k.sig + at * 2 * (S->Lmax + 1) * (S->Lmax + 1);
+  d.Mx = std::min(2 * S->lmax, S->Lmax);
+  d.F = S->keep + k.F;
   d.T = S->keep + k.T + at * 2 * S->Kp * S->Kp;
   d.Z = S->keep + k.Z;
   d.Zt = S->keep + k.Zt;
@@ -1154,15 +1188,15 @@ static int launch_rest(bem_smooth *S, const bem_qp *qps, int b0, int n, unsigned
   const sm_dev d = dev_view(S, 0, b0);
   sm_qps Q;
   for (int i = 0; i < BEM_SM_BAT; ++i) Q.q[i] = qps[i < n ? i : 0];
-  const int smem_t = S->nt / 2 * SMT_TH * (int)sizeof(double), nlm = (S->lmax + 1) * (S->lmax + 2) / 2;
-  if (cudaFuncSetAttribute(k_sm_T, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t) != cudaSuccess) return -1;
+  const int nlm = (S->lmax + 1) * (S->lmax + 2) / 2;
   const int nsamp = (S->nt * S->nphi * 32 + SMP_TH - 1) / SMP_TH, nleg = ((S->Lmax + 1) * S->nt + SMP_TH - 1) / SMP_TH;
   S->have0 = S->have1 = 0;
   k_sm_sample<<<dim3(nsamp + nleg, n), SMP_TH, 0, st>>>(d, Q, nsamp, status);
   k_sm_coef<<<dim3(2 * S->Lmax + 1, n), SMC_TH, 0, st>>>(d);
+  k_sm_F<<<dim3(((2 * d.Mx + 1) * (S->nt / 2) + SMF_FTH - 1) / SMF_FTH, n), SMF_FTH, 0, st>>>(d);
   if (cudaMemsetAsync(d.T, 0, (size_t)n * 2 * S->Kp * S->Kp * sizeof(double), st) != cudaSuccess) return -1;
-  k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, smem_t, st>>>(d);
-  bem_count_launches(3);
+  k_sm_T<<<dim3(nlm, (nlm + SMT_TH - 1) / SMT_TH, n), SMT_TH, 0, st>>>(d);
+  bem_count_launches(4);
   if (cudaPeekAtLastError() != cudaSuccess) return -1;
   S->have0 = b0;
   S->have1 = b0 + n;
