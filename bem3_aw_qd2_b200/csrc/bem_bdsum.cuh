@@ -10,7 +10,7 @@
 // rule points the polar rule replaces, and points on the lattice plane through
 // the target, where the reference's sums stop on rounding and are kept), it
 // comes from the expansion about the target (sm_rest).  A 9-point force of 150
-// turned quads takes 0.98 ms for 19.9 of k_bdval; of the sums 0.75 ms.  A target
+// turned quads takes 0.98 ms for 19.9 of k_bdval, 0.89 of it k_sm_bdsum.  A target
 // with a quarter of its points on its plane (flat bodies across z) keeps the
 // lattice sums: there they are the cheaper form.
 #pragma once

@@ -21,9 +21,10 @@
 // the lattice plane through their node stay with the kernels that sum the
 // lattice point by point (the reference's sums stop on rounding there).
 //
-// 216-quad sphere, square lattice of 0.8 wavelengths (5 images, K = 1296): 1.8 ms
-// in place of 17.3 ms of lattice sums at the points; the whole solve 28.5 ->
-// 11.9 ms, of the 1536-quad sphere 957 -> 374 ms, of 320 triangles 70 -> 29 ms.
+// 216-quad sphere, square lattice of 0.8 wavelengths (K = 625): 1.25 ms of kernels in
+// place of 17.3 ms of lattice sums at the points.  The split alone took the whole
+// solve from 28.5 to 11.9 ms, of the 1536-quad sphere from 957 to 374 ms, of 320
+// triangles from 70 to 29 ms.
 //
 // phi_lm(y) = g_l(k r) R_lm((y - centre) / R0), g_l(z) = (2l + 1)!! j_l(z) / z^l
 // (entire, near 1), R_lm real orthonormal solid harmonics: no zeros of j_l, no

@@ -14,8 +14,8 @@ radiation force.  Rank 0 prints one JSON line.
   e2e    the same solves through the drop-in C API with host buffers
          (solve_bieq_aqd2 uploads the element tables, solves, downloads P, dP,
          pv, dpv; force_FN_aqd2 returns F, N)
-  roofline  the dominant kernel (periodic regular-pair assembly), FP64 work
-         = lattice terms x a fixed FP64 operation count per term
+  roofline  the phase that takes most of a solve, the global LU and its solves:
+         (8/3) n^3 real FP64 operations over the phase's CUDA-event time
   cpu_baseline  the reference's own assembly loop (oracle/_ref) timed on a
          bounded sample of collocation elements on the host cores,
          extrapolated linearly in elements, plus the dense solves
@@ -39,29 +39,10 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# FP64 operations per lattice term of the Green's-function sums (real-space or
-# spectral term with its Faddeeva / erfc evaluation, per-point set-up
-# amortised): counted once with ncu's FP64 instruction counters on the first
-# implementation of the periodic regular-pair kernel on the 216-quad sphere
-# (1.88e12 flop / 6.727e9 terms); frozen, never re-tuned.
-C_TERM_FLOPS = 280.0
 # nominal FP64 peak of B200 (148 SMs x 64 FP64 FMA/clk x 2 x 1.965 GHz), for
 # context; the roofline divides by the FP64 rate measured in the run
 # (measured_fp64_peak), as the bf16 and HBM peaks of this pool are measured
 FP64_NOMINAL_TFLOPS = 37.2
-# The regular-pair kernels' hardware readings from one ncu capture of a
-# warm-up assembly of the timed configuration on the 216-quad workload
-# (profiles/k_q0_regular_far_sphere216.md, command given there): FP64 pipe busy
-# fraction (sm__pipe_fp64_cycles_active over active cycles) and DRAM bytes read +
-# written per launch, for k_q0_regular and each shorter-rule tier's k_q0_far<n>.
-# Reported for that workload only.
-NCU_WORKLOAD = "sphere216"
-NCU_REGULAR = {"k_q0_regular": {"fp64_pipe": 0.4343, "dram_bytes": 434432 + 7126272},
-               "k_q0_far<10>": {"fp64_pipe": 0.4598, "dram_bytes": 414720 + 20992},
-               "k_q0_far<9>": {"fp64_pipe": 0.5040, "dram_bytes": 960512 + 305408},
-               "k_q0_far<8>": {"fp64_pipe": 0.5010, "dram_bytes": 817152 + 1160192},
-               "k_q0_far<7>": {"fp64_pipe": 0.4631, "dram_bytes": 1312000 + 1236480},
-               "k_q0_far<6>": {"fp64_pipe": 0.0, "dram_bytes": 85760 + 0}}
 
 
 def measured_fp64_peak():
@@ -508,27 +489,21 @@ def run_stream(args, rank, world):
         dist.destroy_process_group()
 
 
-def roofline_record(achieved, fp64_peak, terms_reg, cnt, workload, out_bytes):
-    """The dominant kernels' roofline: periodic regular-pair assembly
-    (k_q0_regular on the reference's rule, k_q0_far<n> on the shorter rules'
-    tiers, one phase), FP64
-    work = lattice terms counted by the kernels x the frozen per-term count,
-    over the phase's CUDA-event time; beside it the FP64 pipe fraction and DRAM
-    traffic ncu read on the same kernels."""
-    traffic, pipe = None, {k: None for k in NCU_REGULAR}
-    if workload == NCU_WORKLOAD:
-        traffic = sum(v["dram_bytes"] for v in NCU_REGULAR.values())
-        pipe = {k: v["fp64_pipe"] for k, v in NCU_REGULAR.items()}
-    return {"bound": "fp64", "kernel": "k_q0_regular + k_q0_far<10..6> (regular pairs)", "achieved": achieved,
-            "peak": fp64_peak, "unit": "TFLOP/s", "frac": (achieved / fp64_peak) if achieved else None,
-            "traffic": traffic, "traffic_unit": "bytes per assembly over the phase's 6 launches (ncu dram__bytes_read.sum + write.sum)",
-            "algorithmic_bytes": out_bytes,
-            "algorithmic_bytes_what": "G and H of the periodic domain written (the kernels' only DRAM output; "
-                                      "inputs are L2-resident)",
+def roofline_record(n, t_lu, fp64_peak, cnt):
+    """The roofline of the phase that takes most of a solve: the factorisation of
+    the n x n global system with its two triangular solves (k_lu_panel, k_lu_apply,
+    k_lu_strip, k_lu_update, k_lu_trsv), (8/3) n^3 real FP64 operations over the
+    phase's CUDA-event time.  The assembly beside it sums the lattice only for the
+    pairs on a collocation node's lattice plane; their terms are reported."""
+    work = 8.0 / 3.0 * float(n) ** 3
+    achieved = work / t_lu / 1e12 if t_lu > 0 else None
+    return {"bound": "fp64", "kernel": "k_lu_panel + k_lu_apply + k_lu_strip + k_lu_update + k_lu_trsv (global system)",
+            "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
+            "frac": (achieved / fp64_peak) if achieved else None,
+            "algorithmic_bytes": 16 * n * n, "algorithmic_bytes_what": "the matrix, factored in place",
             "peak_source": "of measured: cuBLAS DGEMM 8192^3 in this run (nominal %.1f TFLOP/s)" % FP64_NOMINAL_TFLOPS,
-            "fp64_pipe_frac_ncu": pipe,
-            "work": "%.3e lattice terms x %.0f FP64 ops per launch" % (terms_reg, C_TERM_FLOPS),
-            "mean_terms_per_point": cnt[0] / max(cnt[3], 1)}
+            "work": "%.3e FP64 operations (8/3 n^3, n = %d)" % (work, n),
+            "lattice_terms_per_assembly": cnt[0], "mean_terms_per_point": cnt[0] / max(cnt[3], 1)}
 
 
 def sweep_instances(freqs, dirs, n=16, a=0.8):
@@ -906,9 +881,7 @@ def main():
     names = ["d0_classify", "d0_regular", "d0_near", "d0_self", "d0_diag", "d1_classify", "d1_regular", "d1_near",
              "d1_self", "d1_diag", "gather", "lu_solve", "boundary_values", "dpv_solves"]
     phase_ms = {names[i]: float(ph[i]) for i in range(min(len(names), len(ph)))}
-    terms_reg = cnt[0] / args.steps
-    t_reg = phase_ms.get("d0_regular", float("nan")) / 1000.0
-    achieved = terms_reg * C_TERM_FLOPS / t_reg / 1e12 if t_reg > 0 else None
+    t_lu = phase_ms.get("lu_solve", float("nan")) / 1000.0
     h2d = ne * (12 + 9 + 12 + 12 + 8 + 8 + 8 + 24 + 2) * 8 + ne * (1 + 4 + 1 + 2 + 8) * 4 + ne
     d2h = 2 * (4 * ne) * (2 + 2 + 6 + 6) * 8 + 48 + 4
     lat = sorted(times)
@@ -925,7 +898,7 @@ def main():
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "path": "solve_bieq_aqd2 + force_FN_aqd2 (C ABI, host buffers)"},
         "phase_ms": phase_ms,
-        "roofline": roofline_record(achieved, fp64_peak, terms_reg, cnt, args.workload, 2 * 16 * n_dom ** 2),
+        "roofline": roofline_record(n_glob, t_lu, fp64_peak, [x / args.steps for x in cnt]),
         "clocks": clk,
         "mixed": mixed,
         "gpu_launches": int(launches),
