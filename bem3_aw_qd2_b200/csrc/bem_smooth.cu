@@ -550,18 +550,28 @@ __global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm
 // then Legendre sums
 #define SMC_TH 128
 #define SM_MAXNT (3 * BEM_SM_MAXL + 4)
+#define SMC_NJ ((4 * BEM_SM_MAXL + 2 + 31) / 32)
 __global__ void __launch_bounds__(SMC_TH) k_sm_coef(const __grid_constant__ sm_dev S) {
   __shared__ double F[4][SM_MAXNT];
   const int M = (int)blockIdx.x - S.Lmax, b = blockIdx.y;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double2 *u = reinterpret_cast<const double2 *>(S.samp) + (size_t)b * 2 * S.nt * S.nphi;
   const double2 *du = u + (size_t)S.nt * S.nphi;
+  // a lane's phases, the same at every node (nphi <= 4 BEM_SM_MAXL + 2 angles, 32 apart)
+  double cs[SMC_NJ], sn[SMC_NJ];
+#pragma unroll
+  for (int i = 0; i < SMC_NJ; ++i) {
+    const int j = lane + 32 * i;
+    cs[i] = sn[i] = 0.0;
+    if (j < S.nphi) sincospi(-2.0 * ((M * j) % S.nphi) / S.nphi, &sn[i], &cs[i]);
+  }
   for (int t = wid; t < S.nt; t += SMC_TH / 32) {
     double a[4] = {0, 0, 0, 0};
-    for (int j = lane; j < S.nphi; j += 32) {
-      int e = (int)(((long long)M * j) % S.nphi);
-      double s, c;
-      sincospi(-2.0 * e / S.nphi, &s, &c);
+#pragma unroll
+    for (int i = 0; i < SMC_NJ; ++i) {
+      const int j = lane + 32 * i;
+      if (j >= S.nphi) break;
+      const double s = sn[i], c = cs[i];
       const double2 x = u[(size_t)t * S.nphi + j], y = du[(size_t)t * S.nphi + j];
       a[0] += x.x * c - x.y * s;
       a[1] += x.x * s + x.y * c;
@@ -632,7 +642,7 @@ __device__ __forceinline__ void sm_put_T(const sm_dev &S, int b, int l, int m, i
 // their size would drown the rest; those below |l - l'| only round).  An integral
 // for each L in its place was 16 (lmax 16) to 40 times the multiply-adds: 91 us
 // for 24 quads in a period of 0.8 and 600 us for the field points' ball; with F
-// 20 + 25 us and 110.
+// 20 + 15 us and 100.
 //
 // F: [j <= Lmax][t][M = -Mx .. Mx], a thread per (t, M), its terms in order of L.
 #define SMF_FTH 128
@@ -645,13 +655,14 @@ __global__ void __launch_bounds__(SMF_FTH) k_sm_F(const __grid_constant__ sm_dev
   const double *p = S.plm + (size_t)t * S.nlm + aM;
   double2 *F = reinterpret_cast<double2 *>(S.F) + (size_t)b * (S.Lmax + 1) * nh * nM + i;
   double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-  for (int L = 0; L <= S.Lmax; ++L) {
-    if (L >= aM) {
-      const double f = (L & 2) ? -S.dL[L] * p[L * (L + 1) / 2] : S.dL[L] * p[L * (L + 1) / 2];
-      const double2 s = sg[L * L + L + M];
-      acc[0].x = fma(f, s.x, acc[0].x);
-      acc[0].y = fma(f, s.y, acc[0].y);
-    }
+  for (int L = 0; L < aM && L <= S.Lmax; ++L) F[(size_t)L * nh * nM] = acc[0];
+  // (loads by themselves, so that several degrees' are in flight)
+#pragma unroll 4
+  for (int L = aM; L <= S.Lmax; ++L) {
+    const double d = __ldg(S.dL + L) * __ldg(p + L * (L + 1) / 2), f = (L & 2) ? -d : d;
+    const double2 s = __ldg(sg + L * L + L + M);
+    acc[0].x = fma(f, s.x, acc[0].x);
+    acc[0].y = fma(f, s.y, acc[0].y);
     F[(size_t)L * nh * nM] = acc[0];
     const double2 x = acc[0];  // the two parities in turn
     acc[0] = acc[1];
