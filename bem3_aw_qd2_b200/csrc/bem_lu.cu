@@ -1391,9 +1391,16 @@ extern "C" int bem_lu_init(bem_lu *w, int device) {
   return 0;
 }
 
-extern "C" void bem_lu_free(bem_lu *w) {
+static void drop_graph(bem_lu *w) {
   if (w->gexec) cudaGraphExecDestroy(w->gexec);
   if (w->graph) cudaGraphDestroy(w->graph);
+  w->gexec = nullptr;
+  w->graph = nullptr;
+  w->g_A = nullptr;
+}
+
+extern "C" void bem_lu_free(bem_lu *w) {
+  drop_graph(w);
   cudaFree(w->rowmap);
   cudaFree(w->tree);
   cudaFree(w->piv);
@@ -1566,15 +1573,16 @@ template <class C2>
 static int lu_factor(bem_lu *w, void *Av, int n, cudaStream_t st) {
   if (n <= 0) return 0;
   C2 *A = (C2 *)Av;
-  if (grow_bytes(w, (void **)&w->rowmap, &w->rowmap_cap, (size_t)n * sizeof(int), "row map") ||
-      grow_bytes(w, (void **)&w->tree, &w->tree_cap, (size_t)lu_nodes(n) * (2 + LU_W) * sizeof(int), "tournament"))
+  // the kept graph's kernels write the row map and the tree: it goes where either
+  // moves, also for a system that is factored without a graph
+  const size_t need_map = (size_t)n * sizeof(int), need_tree = (size_t)lu_nodes(n) * (2 + LU_W) * sizeof(int);
+  if (need_map > w->rowmap_cap || need_tree > w->tree_cap) drop_graph(w);
+  if (grow_bytes(w, (void **)&w->rowmap, &w->rowmap_cap, need_map, "row map") ||
+      grow_bytes(w, (void **)&w->tree, &w->tree_cap, need_tree, "tournament"))
     return -1;
   if (n > (w->one_block_max > 0 ? w->one_block_max : LU_ONE_BLOCK_N)) return factor_blocks(w, A, n, st);
   if (!(w->gexec && w->g_A == Av && w->g_n == n && w->g_fp == (int)sizeof(C2))) {
-    if (w->gexec) cudaGraphExecDestroy(w->gexec);
-    if (w->graph) cudaGraphDestroy(w->graph);
-    w->gexec = nullptr;
-    w->graph = nullptr;
+    drop_graph(w);
     CKL(cudaStreamBeginCapture(w->hi, cudaStreamCaptureModeThreadLocal), "LU capture");
     const int rc = factor_one(w, A, n, w->hi);
     cudaGraph_t g = nullptr;

@@ -24,7 +24,8 @@ struct bem_lu {
   unsigned *status = nullptr;
   void *y = nullptr;          // triangular-solve intermediate (n x nrhs complex)
   size_t y_cap = 0;
-  // the factorisation of one (matrix, size) as a CUDA graph, replayed while both stay the same
+  // the factorisation of one (matrix, size) as a CUDA graph, replayed while both stay the
+  // same; dropped when rowmap or tree moves, whose addresses it holds
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   const void *g_A = nullptr;
