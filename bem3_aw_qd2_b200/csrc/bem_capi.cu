@@ -58,10 +58,8 @@ struct bemgpu_ctx {
   double zspan = 0.0;      // height of the mesh (z extent of all elements)
   double zlo = 0.0;        // and its lower end
   double *fst = nullptr;   // evanescent order table for field points above or below the mesh
-  size_t fst_cap = 0;
   bem_smooth fsm;          // the split for field points, its tables and expansion (of the last call's points)
   double *fsm_tab = nullptr, *fsm_keep = nullptr;
-  size_t fsm_cap[2] = {0, 0};
   double pw[16] = {};      // incident plane wave (bemgpu_problem.pw)
   int far_rule = 1;        // shorter rules for regular pairs of the periodic domain (bemgpu_set_far_rule)
   double eta_scale = 0.0;  // Ewald parameter off the lattice plane = eta0 x eta_scale; 0: by rule per problem
@@ -1422,15 +1420,10 @@ static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources
     *q = own;
     return 0;
   }
-  if (cnt > c->fst_cap) {
-    dfree(c->fst);
-    c->fst_cap = 0;
-    if (dalloc(&c->fst, cnt) != cudaSuccess) {  // without one, then
-      cudaGetLastError();
-      *q = own;
-      return 0;
-    }
-    c->fst_cap = cnt;
+  if (falloc(c, &c->fst, cnt) != cudaSuccess) {  // without one, then
+    cudaGetLastError();
+    *q = own;
+    return 0;
   }
   if (bem_launch_stab(q, c->fst, c->stream)) return fail(c, "spectral table", cudaGetLastError());
   q->st = c->fst;
@@ -1467,18 +1460,11 @@ static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int
   bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, Rx, n, (double)src);
   std::vector<double> h(bem_smooth_layout(&c->fsm).total);
   bem_smooth_tables(&c->fsm, &c->qp, h.data());
-  double **p[2] = {&c->fsm_tab, &c->fsm_keep};
-  const size_t need[2] = {h.size(), bem_smooth_keep_doubles(&c->fsm)};
-  for (int i = 0; i < 2; ++i)
-    if (need[i] > c->fsm_cap[i]) {
-      dfree(*p[i]);
-      c->fsm_cap[i] = 0;
-      if (dalloc(p[i], need[i]) != cudaSuccess) {  // lattice sums, then
-        cudaGetLastError();
-        return 0;
-      }
-      c->fsm_cap[i] = need[i];
-    }
+  if (falloc(c, &c->fsm_tab, h.size()) != cudaSuccess ||
+      falloc(c, &c->fsm_keep, bem_smooth_keep_doubles(&c->fsm)) != cudaSuccess) {  // lattice sums, then
+    cudaGetLastError();
+    return 0;
+  }
   c->fsm.tab = c->fsm_tab;
   c->fsm.keep = c->fsm_keep;
   CK(cudaMemcpyAsync(c->fsm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
