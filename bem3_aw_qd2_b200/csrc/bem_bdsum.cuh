@@ -546,9 +546,7 @@ __global__ void __launch_bounds__(SMB_TH, 3) k_sm_bdsum(const __grid_constant__ 
 // the densities of a rule's sources with the boundary values given
 static int launch_density(const bem_smooth *S, const sm_dev &d, const bem_dom_dev *D, int type, const double *P,
                           const double *dP, const double *pv, const double *dpv, cudaStream_t st) {
-  const int smem = (16 + std::max(2 * (S->lmax + 1), 4 * S->lmax)) * SMV_PT * (int)sizeof(double);
-  if (cudaFuncSetAttribute(k_sm_density, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
-  k_sm_density<<<dim3(SMD_NCH, S->lmax + 1), SMD_TH, smem, st>>>(d, *D, type, P, dP, pv, dpv);
+  k_sm_density<<<dim3(SMD_NCH, S->lmax + 1), SMD_TH, sm_point_smem(16, S->lmax), st>>>(d, *D, type, P, dP, pv, dpv);
   k_sm_density_sum<<<(8 * S->K + SMB_TH - 1) / SMB_TH, SMB_TH, 0, st>>>(d);
   k_sm_density_T<<<S->K, SMB_TH, 0, st>>>(d);
   bem_count_launches(3);

@@ -45,11 +45,6 @@
 #include "bem_rules.cuh"
 #include "bem_smooth.h"
 
-extern "C" int bem_smooth_set_constants(const void *quad, const void *wc) {
-  if (cudaMemcpyToSymbol(c_q, quad, sizeof(bem_quad)) != cudaSuccess) return -1;
-  if (cudaMemcpyToSymbol(c_w, wc, sizeof(bem_wconst)) != cudaSuccess) return -1;
-  return 0;
-}
 
 // ------------------------------------------------------------------ host: the split
 // |j_l(z)| = z^l g_l / (2l + 1)!! and |h_l(z)| for l = 0 .. n
@@ -798,6 +793,10 @@ __global__ void __launch_bounds__(SMU_TH) k_sm_targets(const __grid_constant__ s
 // The values of order m at a point (r, W): for each degree l the rows |W| phi and
 // W . grad phi of the cosine (and of the sine) function, SMV_PT apart, at val.
 #define SMV_PT (BEM_GLN * BEM_GLN)
+// shared memory of a kernel that keeps these values, rows more per point beside them
+static int sm_point_smem(int rows, int lmax) {
+  return (rows + std::max(2 * (lmax + 1), 4 * lmax)) * SMV_PT * (int)sizeof(double);
+}
 __device__ __forceinline__ void sm_point_values(const sm_dev &S, int m, int nf, const double r[3], const double W[3],
                                                 double *val) {
         const double aW = sqrt(W[0] * W[0] + W[1] * W[1] + W[2] * W[2]);
@@ -1224,12 +1223,7 @@ static void launch_images(const sm_dev &d, const bem_dom_dev *D, int nb, const u
 extern "C" int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_qp *qps, int nb, double *const *G,
                                  double *const *H, const bem_scratch *scr, cudaStream_t st) {
   const int ne = D->ne, N = 4 * ne;
-  const int smem_v = (4 * SMV_PT + std::max(2 * (S->lmax + 1), 4 * S->lmax) * SMV_PT) * (int)sizeof(double);
-  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (cudaFuncSetAttribute(k_sm_sources, at, smem_v) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sm_gemm<true>, at, GM_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sm_gemm<false>, at, GM_SMEM) != cudaSuccess)
-    return -1;
+  const int smem_v = sm_point_smem(4, S->lmax);
   const long long npairs = (long long)N * ne;
   for (int b0 = 0; b0 < nb; b0 += BEM_SM_BAT) {
     const int n = nb - b0 < BEM_SM_BAT ? nb - b0 : BEM_SM_BAT;
@@ -1263,3 +1257,18 @@ extern "C" int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_
 
 #include "bem_bdsum.cuh"
 #include "bem_smfield.cuh"
+
+// The attributes belong to the device's functions, not to a context: every context sets
+// the same, the most that any degree takes, so that threads with bodies of different
+// degrees leave each other's launches valid.
+extern "C" int bem_smooth_set_constants(const void *quad, const void *wc) {
+  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (cudaMemcpyToSymbol(c_q, quad, sizeof(bem_quad)) != cudaSuccess ||
+      cudaMemcpyToSymbol(c_w, wc, sizeof(bem_wconst)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_sources, at, sm_point_smem(4, BEM_SM_MAXL)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_density, at, sm_point_smem(16, BEM_SM_MAXL)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_gemm<true>, at, GM_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sm_gemm<false>, at, GM_SMEM) != cudaSuccess)
+    return -1;
+  return 0;
+}

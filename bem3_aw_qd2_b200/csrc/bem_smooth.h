@@ -43,7 +43,8 @@ size_t bem_smooth_keep_doubles(const bem_smooth *S);
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
 
 extern "C" {
-// constant tables of this translation unit (quad: bem_quad, wc: bem_wconst)
+// constant tables of this translation unit (quad: bem_quad, wc: bem_wconst) and its
+// kernels' attributes, on the current device
 int bem_smooth_set_constants(const void *quad, const void *wc);
 // G, H of nb instances of the periodic domain: the smooth rest of every pair
 // (written), then the images of every pair off the lattice plane (added; the
