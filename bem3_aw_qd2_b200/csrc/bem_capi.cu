@@ -1430,34 +1430,85 @@ static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources
   return 0;
 }
 
+// Terms of the plane-wave sum at height z over a source, and the height from which
+// bem_qpgf2 takes it alone.
+static double plane_waves(const bem_qp *q, double z) { return 1296.0 / (z * z) * fabs(q->det) * 0.0795774715459476679; }
+static double plane_wave_height(const bem_qp *q) {
+  if (q->ewald_only) return 1e300;
+  const double eps = 1e-15;  // the sums' relative error
+  return std::max(std::max(log(q->sel_cp / eps) / q->sel_bp, log(q->sel_cm / eps) / q->sel_bm), sqrt(plane_waves(q, 1.0) / 250.0));
+}
+
+// FP64 operations of a point's lattice sums for each source, at the rate that k_field
+// reaches (17e12 a second): an Ewald sum 7e4 with second derivatives, 6e4 without, four
+// times that where its parameter is capped next to the source and no table holds its
+// terms; where plane waves alone do, 4e3 and 420 a term, the sources in thirds of the
+// mesh's height.  Measured, ns a pair, 9-point rule: around 216 quads 3.1 (period 0.8),
+// 3.5 (1.5), around 54 quads 18 (3.3); over the centre of the first at 1 wavelength 1.7,
+// at 2 0.61, at 10 0.28.
+static double lattice_cost(const bemgpu_ctx *c, double zs, int grad, double z) {
+  const double ke = c->qp.k * c->qp.eta_run, ewald = (grad ? 7e4 : 6e4) * (ke * ke > 3.0 ? 4.0 : 1.0);
+  double sum = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    const double h = fabs(z - c->zlo - (2 * i + 1) / 6.0 * c->zspan);
+    sum += h > zs ? 4e3 + 420.0 * plane_waves(&c->qp, h) : ewald;
+  }
+  return sum / 3.0;
+}
+
 // The points that the split c->fsm takes (their number; order: they first, then the
 // others, empty where that is how they come), planned for the largest ball of those
 // that hold all, 9, 7 or 5 in 10 of the points for which images, expansion and the
 // other points' lattice sums cost least.  Costs in FP64 operations at the kernels'
-// rates: a pair's lattice sum 7e4 with second derivatives, 1.5e4 without, set-up
-// and its launches 1e10 (0.5 ms).  0: none.
+// rates: a pair's lattice sum lattice_cost, in waves of k_field's blocks (a point each,
+// three an SM; one an SM takes 0.8 of a full wave's time) and whole strides of their
+// threads; the split's set-up and its launches 1e10 (0.5 ms), so that calls below 2e10
+// are not looked at.  0: none.
 static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int grad, std::vector<int> &order) {
-  const double pair = grad ? 7e4 : 1.5e4, all = (double)n * src * pair;
-  if (!c->sm.on || all < 2e10) return 0;
-  std::vector<double> d(n);
-  for (int i = 0; i < n; ++i)
-    d[i] = sqrt((r[3 * i] - c->sm.ctr[0]) * (r[3 * i] - c->sm.ctr[0]) + (r[3 * i + 1] - c->sm.ctr[1]) * (r[3 * i + 1] - c->sm.ctr[1]) +
-                (r[3 * i + 2] - c->sm.ctr[2]) * (r[3 * i + 2] - c->sm.ctr[2]));
-  for (int i = 0; i < n; ++i)
+  if (!c->sm.on || (double)n * src * (grad ? 7e4 : 1.5e4) < 2e10) return 0;
+  const double zs = plane_wave_height(&c->qp), wave = 3.0 * c->lus[0].sms, stride = ceil(src / 128.0) * 128.0;
+  std::vector<double> d(n), cost(n);
+  double sum = 0.0, far = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double x = r[3 * i] - c->sm.ctr[0], y = r[3 * i + 1] - c->sm.ctr[1], z = r[3 * i + 2] - c->sm.ctr[2];
+    d[i] = sqrt(x * x + y * y + z * z);
     if (!(d[i] < 1e300)) return 0;
+    far = std::max(far, d[i]);
+    cost[i] = lattice_cost(c, zs, grad, r[3 * i + 2]);
+    sum += cost[i];
+  }
+  // m points of these costs together
+  auto lattice = [&](int m, double costs) {
+    const double full = floor(m / wave), part = m / wave - full;
+    return m ? costs / m * stride * wave * (full + (part > 0.0 ? 0.7 + 0.3 * part : 0.0)) : 0.0;
+  };
+  const double all = lattice(n, sum);
+  if (all < 2e10) return 0;
   std::vector<double> by(d);
-  std::sort(by.begin(), by.end());
   double best = all, Rx = 0.0;
   for (const double part : {1.0, 0.9, 0.7, 0.5}) {
-    const double R = by[(size_t)ceil(part * n) - 1];
-    const double cost = bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, R, part * n, (double)src) + 1e10 + (1.0 - part) * all;
-    if (cost < best) {
-      best = cost;
+    double R = far, rest = 0.0;
+    int near = n;
+    if (part < 1.0) {
+      auto k = by.begin() + ((size_t)ceil(part * n) - 1);
+      std::nth_element(by.begin(), k, by.end());
+      R = *k;
+      for (int i = near = 0; i < n; ++i) {
+        if (d[i] <= R) ++near;
+        else rest += cost[i];
+      }
+    }
+    const double other = lattice(n - near, rest) + 1e10;
+    const double t = bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, R, near, (double)src, best - other) + other;
+    if (t < best) {
+      best = t;
       Rx = R;
     }
   }
   if (!(Rx > 0.0)) return 0;
-  bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, Rx, n, (double)src);
+  int near = 0;
+  for (int i = 0; i < n; ++i) near += d[i] <= Rx;
+  if (bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, Rx, near, (double)src, 1e300) >= 1e300) return 0;
   std::vector<double> h(bem_smooth_layout(&c->fsm).total);
   bem_smooth_tables(&c->fsm, &c->qp, h.data());
   if (falloc(c, &c->fsm_tab, h.size()) != cudaSuccess ||
@@ -1468,8 +1519,6 @@ static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int
   c->fsm.tab = c->fsm_tab;
   c->fsm.keep = c->fsm_keep;
   CK(cudaMemcpyAsync(c->fsm_tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
-  int near = 0;
-  for (int i = 0; i < n; ++i) near += d[i] <= Rx;
   if (near < n) {
     order.resize(n);
     int a = 0, b = near;

@@ -90,19 +90,44 @@ static int degree_for(double k, double a, double b, double scale, double tol, in
   return 0;
 }
 
-// lattice points by distance, to the reach and four periods (empty: far too many)
-struct sm_pt { double r; int a, b; };
-static std::vector<sm_pt> lattice_by_distance(const bem_qp *q, double reach) {
-  std::vector<sm_pt> P;
-  reach += 4.0 * (hypot(q->d1x, q->d1y) + hypot(q->d2x, q->d2y));
-  const double n1 = floor(reach * hypot(q->g1x, q->g1y) / (2.0 * M_PI)) + 1, n2 = floor(reach * hypot(q->g2x, q->g2y) / (2.0 * M_PI)) + 1;
-  if (!(n1 * n2 <= 1e5)) return P;
-  for (int a = -(int)n1; a <= (int)n1; ++a)
-    for (int b = -(int)n2; b <= (int)n2; ++b) P.push_back({hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y), a, b});
-  std::stable_sort(P.begin(), P.end(), [](const sm_pt &x, const sm_pt &y) { return x.r < y.r; });
-  return P;
+// The BEM_SM_MAXIMG + 1 lattice points nearest to the origin, by distance (those of one
+// distance in order of their indices).  S->np = 0 where the lattice's basis is too
+// skewed, or the body too many periods wide, for a split to be looked for.
+static void nearest_points(bem_smooth *S, const bem_qp *q) {
+  struct pt { double r; int a, b; };
+  S->np = 0;
+  const double g1 = hypot(q->g1x, q->g1y) / (2.0 * M_PI), g2 = hypot(q->g2x, q->g2y) / (2.0 * M_PI);
+  const double wide = 12.0 * S->R0 + 4.0 * (hypot(q->d1x, q->d1y) + hypot(q->d2x, q->d2y));
+  if (!((floor(wide * g1) + 1) * (floor(wide * g2) + 1) <= 1e5)) return;
+  std::vector<pt> P;
+  const size_t want = BEM_SM_MAXIMG + 1;
+  // every point within the reach is listed; a disc of the wanted points' area holds
+  // about as many, a wider one more
+  for (double reach = 1.2 * sqrt(want / (M_PI * q->aidet)); P.size() < want; reach *= 1.4) {
+    P.clear();
+    const int n1 = (int)floor(reach * g1) + 1, n2 = (int)floor(reach * g2) + 1;
+    for (int a = -n1; a <= n1; ++a)
+      for (int b = -n2; b <= n2; ++b) {
+        const double r = hypot(a * q->d1x + b * q->d2x, a * q->d1y + b * q->d2y);
+        if (r <= reach) P.push_back({r, a, b});
+      }
+  }
+  std::stable_sort(P.begin(), P.end(), [](const pt &x, const pt &y) { return x.r < y.r; });
+  S->np = (int)want;
+  for (size_t i = 0; i < want; ++i) {
+    S->pr[i] = P[i].r;
+    S->p1[i] = P[i].a;
+    S->p2[i] = P[i].b;
+  }
 }
 static void finish_plan(bem_smooth *S, const bem_qp *q);
+static void take_images(bem_smooth *S) {
+  S->cut = S->pr[S->nimg] - S->rho;
+  for (int i = 0; i < S->nimg; ++i) {
+    S->l1[i] = S->p1[i];
+    S->l2[i] = S->p2[i];
+  }
+}
 
 void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int *npe, const int *sid, int ne) {
   S->on = 0;
@@ -145,7 +170,7 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
   S->rho = 2.0 * S->R0;
   S->k = q->k;
   if (!(S->R0 > 0.0) || !std::isfinite(S->R0)) return;
-  const std::vector<sm_pt> P = lattice_by_distance(q, 12.0 * S->R0);
+  nearest_points(S, q);
   // the cheapest split, in FP64 operations at the rates that the kernels reach
   // (images 0.55 of the pipe, the product 0.7): per pair about 45 points of 66
   // for each image and 16 multiply-adds for each of the K functions (G and H of
@@ -153,36 +178,44 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
   // and T.  Summed point by point a pair takes about 8e5 at half the pipe.
   const double pairs = 4.0 * ne * ne;
   double best = 1e6 * pairs;
-  for (size_t c = 1; c < P.size() && c <= BEM_SM_MAXIMG; ++c) {
-    if (P[c].r <= P[c - 1].r * (1.0 + 1e-9)) continue;  // whole shells only
-    const double cut = P[c].r;
-    if (cut <= S->rho * 1.05) continue;
+  for (int c = S->np - 1; c >= 1; --c) {
+    if (S->pr[c] <= S->pr[c - 1] * (1.0 + 1e-9)) continue;  // whole shells only
+    const double cut = S->pr[c], images = pairs * (c - 1) * 45.0 * 66.0 / 0.55;
+    if (cut <= S->rho * 1.05) break;
+    if (images >= best) continue;
     // tail relative to 1 / (4 pi 2 R0), six images on the first shell left in
     const int lmax = degree_for(S->k, S->R0, cut - S->R0, 6.0 * S->rho, 1e-15, BEM_SM_MAXL);
     if (lmax < 0) continue;
     int Lmax = degree_for(S->k, S->rho, cut, 6.0 * S->rho, 1e-15, 2 * BEM_SM_MAXL);
     if (Lmax < 0 || Lmax > 2 * lmax) Lmax = 2 * lmax;
     const double K = (lmax + 1.0) * (lmax + 1.0), nt = lmax + 0.5 * Lmax + 1.0;
-    const double cost = pairs * ((c - 1) * 45.0 * 66.0 / 0.55 + 16.0 * K / 0.7) + 4.0 * ne * 2.0 * K * K / 0.7 +
+    const double cost = images + pairs * 16.0 * K / 0.7 + 4.0 * ne * 2.0 * K * K / 0.7 +
                         nt * (2.0 * Lmax + 2.0) * 3e4 + 0.25 * K * K * lmax * nt;
     if (cost < best) {
       best = cost;
       S->on = 1;
       S->lmax = lmax;
       S->Lmax = Lmax;
-      S->nimg = (int)c;
-      S->cut = cut - S->rho;
-      for (size_t i = 0; i < c; ++i) { S->l1[i] = P[i].a; S->l2[i] = P[i].b; }
+      S->nimg = c;
     }
   }
-  if (S->on) finish_plan(S, q);
+  if (!S->on) return;
+  take_images(S);
+  // degrees for one point's rest at |R| <= (i + 1) 2 R0 / 8 (the gradient's terms are
+  // those of the value times l / |R|)
+  for (int i = 0; i < 8; ++i) {
+    const double f = (i + 1) / 8.0;
+    const int l = degree_for(S->k, f * S->rho, S->cut + S->rho, 6.0 * S->rho, f * 1e-15, S->Lmax);
+    S->lcut[i] = l < 0 ? S->Lmax : l;
+  }
+  finish_plan(S, q);
 }
 
 // The split for sums at points up to Rx from the body's centre: the larger ball
 // takes R0's place, the degrees follow from both (a source at R0 against images
-// seen from Rx, a point at Rx against images seen from R0).  Returns the FP64
-// operations of n points and their sources, a large number where there is none.
-double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources) {
+// seen from Rx, a point at Rx against images seen from R0).
+double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources,
+                             double limit) {
   F->on = 0;
   F->have0 = F->have1 = 0;
   F->inst = 1;
@@ -191,45 +224,42 @@ double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q
   for (int d = 0; d < 3; ++d) F->ctr[d] = S->ctr[d];
   F->R0 = std::max(Rx, S->R0) * (1.0 + 1e-12);
   F->rho = F->R0 + S->R0;
-  double best = 1e300;
-  if (!(F->R0 < 1e3 * S->R0)) return best;
-  const std::vector<sm_pt> P = lattice_by_distance(q, 3.0 * F->rho);
-  for (size_t c = 1; c < P.size() && c <= BEM_SM_MAXIMG; ++c) {
-    if (P[c].r <= P[c - 1].r * (1.0 + 1e-9)) continue;  // whole shells only
-    const double cut = P[c].r;
-    if (cut <= F->rho * 1.05) continue;
+  double best = limit;
+  if (!(F->R0 < 1e3 * S->R0)) return 1e300;
+  F->np = S->np;
+  std::copy(S->pr, S->pr + S->np, F->pr);
+  std::copy(S->p1, S->p1 + S->np, F->p1);
+  std::copy(S->p2, S->p2 + S->np, F->p2);
+  for (int c = F->np - 1; c >= 1; --c) {  // as bem_smooth_plan
+    if (F->pr[c] <= F->pr[c - 1] * (1.0 + 1e-9)) continue;
+    // an image with second derivatives about 160 operations, a pair's own part 400
+    const double cut = F->pr[c], images = n * sources * (400.0 + c * 160.0) / 0.55;
+    if (cut <= F->rho * 1.05) break;
+    if (images >= best) continue;
     const int lx = degree_for(F->k, F->R0, cut - S->R0, 6.0 * F->rho, 1e-15, BEM_SM_MAXL);
+    if (lx < 0) continue;
     const int ly = degree_for(F->k, S->R0, cut - F->R0, 6.0 * F->rho, 1e-15, BEM_SM_MAXL);
-    if (lx < 0 || ly < 0) continue;
+    if (ly < 0) continue;
     const int lmax = std::max(lx, ly);
     int Lmax = degree_for(F->k, F->rho, cut, 6.0 * F->rho, 1e-15, 2 * BEM_SM_MAXL);
     if (Lmax < 0 || Lmax > 2 * lmax) Lmax = 2 * lmax;
-    // an image with second derivatives about 160 operations, a pair's own part 400
     const double K = (lmax + 1.0) * (lmax + 1.0), nt = lmax + 0.5 * Lmax + 1.0;
-    const double cost = n * sources * (400.0 + c * 160.0) / 0.55 + nt * (2.0 * Lmax + 2.0) * 3e4 + 0.25 * K * K * lmax * nt +
-                        sources * K * 60.0;
+    const double cost = images + nt * (2.0 * Lmax + 2.0) * 3e4 + 0.25 * K * K * lmax * nt + sources * K * 60.0;
     if (cost < best) {
       best = cost;
       F->on = 1;
       F->lmax = lmax;
       F->Lmax = Lmax;
-      F->nimg = (int)c;
-      F->cut = cut - F->rho;
-      for (size_t i = 0; i < c; ++i) { F->l1[i] = P[i].a; F->l2[i] = P[i].b; }
+      F->nimg = c;
     }
   }
-  if (F->on) finish_plan(F, q);
+  if (!F->on) return 1e300;
+  take_images(F);
+  finish_plan(F, q);
   return F->on ? best : 1e300;
 }
 
 static void finish_plan(bem_smooth *S, const bem_qp *q) {
-  // degrees for one point's rest at |R| <= (i + 1) 2 R0 / 8 (the gradient's terms are
-  // those of the value times l / |R|)
-  for (int i = 0; i < 8; ++i) {
-    const double f = (i + 1) / 8.0;
-    const int l = degree_for(S->k, f * S->rho, S->cut + S->rho, 6.0 * S->rho, f * 1e-15, S->Lmax);
-    S->lcut[i] = l < 0 ? S->Lmax : l;
-  }
   // windows of the samples' Ewald sums: the reference's parameter below its cap
   // (k^2 eta^2 < 3); terms to e^{-40} of the leading one; the images among them
   S->eta = std::min(q->eta0, 0.98 * sqrt(3.0) / S->k);

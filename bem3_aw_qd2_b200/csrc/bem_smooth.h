@@ -19,9 +19,12 @@ struct bem_smooth {
   double eta = 0.0;             // Ewald parameter and windows of the samples
   int r1 = 0, r2 = 0, s1 = 0, s2 = 0, sc2 = 0;
   int l1[BEM_SM_MAXIMG], l2[BEM_SM_MAXIMG];  // the images' lattice indices, (0, 0) first
+  int np = 0;                   // the nearest lattice points, by distance (as many as a split
+  double pr[BEM_SM_MAXIMG + 1]; // can look at: its images and the first shell left in)
+  int p1[BEM_SM_MAXIMG + 1], p2[BEM_SM_MAXIMG + 1];
   int inst = 1, first = 0;      // instances tab holds; the one a launch for a single instance takes
   const double *tab = nullptr;  // device copy of the tables bem_smooth_tables writes
-  int lcut[8];                  // degrees of the expansion about a point, by distance
+  int lcut[8] = {};             // degrees of the expansion about a point, by distance (boundary sums; not a field's plan)
   double *keep = nullptr;       // device memory of bem_smooth_keep_doubles doubles, kept with the problem
   int have0 = 0, have1 = 0;     // instances whose expansion keep holds
   double *ws = nullptr;         // an assembly's scratch, bem_smooth_ws_doubles doubles
@@ -38,7 +41,10 @@ void bem_smooth_plan(bem_smooth *S, const bem_qp *q, const double *cr, const int
 bem_smooth_tab bem_smooth_layout(const bem_smooth *S);
 // the tables of S->inst instances (qps: their Bloch wave vectors) into h[layout.total]
 void bem_smooth_tables(const bem_smooth *S, const bem_qp *qps, double *h);
-double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources);
+// the split for sums at n points up to Rx from the body's centre; returns its operations,
+// 1e300 where there is none of fewer than limit (then F->on = 0)
+double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q, double Rx, double n, double sources,
+                             double limit);
 size_t bem_smooth_keep_doubles(const bem_smooth *S);
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
 
