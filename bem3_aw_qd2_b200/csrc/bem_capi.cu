@@ -1396,40 +1396,6 @@ static int ensure_points(bemgpu_ctx *c, int n) {
   return 0;
 }
 
-// The lattice sums of field points: q = c->qp with a spectral order table that
-// reaches from the mesh to the points where that is worth its build.  The
-// context's own table covers distances within the mesh; beyond it a term is two
-// erfcx and an exponential in place of one recurrence, some 4 times the work of
-// the whole term.  A table costs its orders x intervals x degree direct terms, a
-// point about 50 spectral terms for each source.  Distances at which the plane
-// wave sum converges by itself (bem_qpgf2) need no table.
-static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources, bem_qp *q) {
-  *q = c->qp;
-  double reach = 0.0;
-  for (int i = 0; i < n; ++i)
-    reach = std::max(reach, std::max(c->zlo + c->zspan - r[3 * i + 2], r[3 * i + 2] - c->zlo));
-  if (!q->ewald_only) {
-    const double eps = 1e-15;  // the sums' relative error
-    const double zs = std::max(log(q->sel_cp / eps) / q->sel_bp, log(q->sel_cm / eps) / q->sel_bm);
-    if (zs > 0.0) reach = std::min(reach, zs);
-  }
-  if (!(reach > c->zspan) || !(reach < 1e4 * q->eta_run)) return 0;
-  const bem_qp own = *q;
-  const size_t cnt = stab_window(q, reach);
-  if (!cnt || (double)n * sources * 50.0 < 2.0 * cnt) {
-    *q = own;
-    return 0;
-  }
-  if (falloc(c, &c->fst, cnt) != cudaSuccess) {  // without one, then
-    cudaGetLastError();
-    *q = own;
-    return 0;
-  }
-  if (bem_launch_stab(q, c->fst, c->stream)) return fail(c, "spectral table", cudaGetLastError());
-  q->st = c->fst;
-  return 0;
-}
-
 // Terms of the plane-wave sum at height z over a source, and the height from which
 // bem_qpgf2 takes it alone.
 static double plane_waves(const bem_qp *q, double z) { return 1296.0 / (z * z) * fabs(q->det) * 0.0795774715459476679; }
@@ -1437,6 +1403,64 @@ static double plane_wave_height(const bem_qp *q) {
   if (q->ewald_only) return 1e300;
   const double eps = 1e-15;  // the sums' relative error
   return std::max(std::max(log(q->sel_cp / eps) / q->sel_bp, log(q->sel_cm / eps) / q->sel_bm), sqrt(plane_waves(q, 1.0) / 250.0));
+}
+
+// Points of a call that its estimates look at: all up to 128, else 128 in steps of the
+// golden ratio (a call's order is often that of a grid).
+static std::vector<int> sample_points(int n) {
+  std::vector<int> s(std::min(n, 128));
+  double x = 0.5;
+  for (size_t i = 0; i < s.size(); ++i) {
+    s[i] = n <= 128 ? (int)i : (int)(x * n);
+    x += 0.61803398874989485;
+    x -= floor(x);
+  }
+  return s;
+}
+
+// The lattice sums of field points: q = c->qp, with a spectral order table that reaches
+// from the mesh to the points where that is worth its build; *spec: the second-derivative
+// sums take q's table.  With a term from a table two erfcx and an exponential become one
+// recurrence; the context's own table holds the heights within the mesh.  A table
+// serves a point when it holds three fifths of the heights over the sources at which
+// plane waves alone do not do, and the point keeps the distance from the body's ball
+// below which the Ewald parameter is capped (bem_ewald_eta: a warp would run both forms).
+// A build takes 50 to 90 us and saves a quarter or more of the sums of the points that
+// it serves and the own table does not: 30 points of 96 flat quads, period 1, 9-point
+// rule, 1.03 -> 0.82 ms (7 strides of 128 sources; 3 are worth it), 3000 of them 11.1 ->
+// 6.6.  Within one wave of blocks the slowest point decides, so that second derivatives
+// (whose direct forms are code of their own) ask for every point to be served, beyond
+// it for half.
+static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources, int grad, bem_qp *q, int *spec) {
+  *q = c->qp;
+  const double ke = q->k * q->eta_run, wave = 3.0 * c->lus[0].sms, zs = plane_wave_height(q), *ctr = c->sm.ctr;
+  const double cap = ke * ke > 3.0 ? c->sm.R0 + 2.0 * q->eta_run * sqrt(ke * ke - 3.0) : 0.0;
+  double reach = 0.0;
+  const std::vector<int> sample = sample_points(n);
+  size_t own = 0, served = 0;  // by the context's table, by one of this reach
+  for (const int i : sample) {
+    const double *p = r + 3 * (size_t)i, z = p[2], dx = p[0] - ctr[0], dy = p[1] - ctr[1], dz = z - ctr[2];
+    const double far = std::max(z - c->zlo, c->zlo + c->zspan - z), lo = std::max(0.0, far - c->zspan), hi = std::min(zs, far);
+    if (!(lo < hi) || !(dx * dx + dy * dy + dz * dz >= cap * cap)) continue;
+    ++served;
+    own += std::min(c->zspan, hi) - lo >= 0.6 * (hi - lo);
+    reach = std::max(reach, hi);
+  }
+  const size_t need = grad && n <= wave ? sample.size() : (sample.size() + 1) / 2;
+  *spec = q->st && own >= need;
+  if (own >= need || served < need || ceil(sources / 128.0) * std::max(1.0, n / wave) < 3.0 || !(reach < 1e4 * q->eta_run))
+    return 0;
+  const bem_qp qown = *q;
+  const size_t cnt = stab_window(q, reach);
+  if (!cnt || falloc(c, &c->fst, cnt) != cudaSuccess) {  // too large, or no memory: without one
+    cudaGetLastError();
+    *q = qown;
+    return 0;
+  }
+  if (bem_launch_stab(q, c->fst, c->stream)) return fail(c, "spectral table", cudaGetLastError());
+  q->st = c->fst;
+  *spec = 1;
+  return 0;
 }
 
 // FP64 operations of a point's lattice sums for each source, at the rate that k_field
@@ -1466,49 +1490,67 @@ static double lattice_cost(const bemgpu_ctx *c, double zs, int grad, double z) {
 // are not looked at.  0: none.
 static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int grad, std::vector<int> &order) {
   if (!c->sm.on || (double)n * src * (grad ? 7e4 : 1.5e4) < 2e10) return 0;
-  const double zs = plane_wave_height(&c->qp), wave = 3.0 * c->lus[0].sms, stride = ceil(src / 128.0) * 128.0;
-  std::vector<double> d(n), cost(n);
-  double sum = 0.0, far = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const double x = r[3 * i] - c->sm.ctr[0], y = r[3 * i + 1] - c->sm.ctr[1], z = r[3 * i + 2] - c->sm.ctr[2];
-    d[i] = sqrt(x * x + y * y + z * z);
-    if (!(d[i] < 1e300)) return 0;
-    far = std::max(far, d[i]);
-    cost[i] = lattice_cost(c, zs, grad, r[3 * i + 2]);
-    sum += cost[i];
-  }
-  // m points of these costs together
-  auto lattice = [&](int m, double costs) {
-    const double full = floor(m / wave), part = m / wave - full;
-    return m ? costs / m * stride * wave * (full + (part > 0.0 ? 0.7 + 0.3 * part : 0.0)) : 0.0;
+  const double *ctr = c->sm.ctr, wave = 3.0 * c->lus[0].sms, stride = ceil(src / 128.0) * 128.0;
+  auto dist2 = [&](int i) {
+    const double *p = r + 3 * (size_t)i, x = p[0] - ctr[0], y = p[1] - ctr[1], z = p[2] - ctr[2];
+    return x * x + y * y + z * z;
   };
-  const double all = lattice(n, sum);
-  if (all < 2e10) return 0;
-  std::vector<double> by(d);
-  double best = all, Rx = 0.0;
+  // distance and lattice cost of the points that the estimates look at, by distance
+  const double zs = plane_wave_height(&c->qp);
+  const std::vector<int> sample = sample_points(n);
+  std::vector<std::pair<double, double>> near_cost;
+  double sum = 0.0;
+  for (const int i : sample) {
+    near_cost.emplace_back(dist2(i), lattice_cost(c, zs, grad, r[3 * (size_t)i + 2]));
+    sum += near_cost.back().second;
+  }
+  // m points of this mean cost
+  auto lattice = [&](double m, double cost) {
+    const double full = floor(m / wave), part = m / wave - full;
+    return cost * stride * wave * (full + (part > 0.0 ? 0.7 + 0.3 * part : 0.0));
+  };
+  const double all = lattice(n, sum / sample.size());
+  if (!(all >= 2e10)) return 0;
+  double far = 0.0;
+  bool finite = true;
+  for (int i = 0; i < n; ++i) {
+    const double d2 = dist2(i);
+    finite &= d2 < 1e300;
+    far = std::max(far, d2);
+  }
+  if (!finite) return 0;
+  std::sort(near_cost.begin(), near_cost.end());
+  // (of large calls every point's distance: whether a ball has a split can hang on the last percent)
+  std::vector<double> by;
+  if (all >= 1e11)
+    for (int i = 0; i < n; ++i) by.push_back(dist2(i));
+  double best = all, R2 = 0.0;
   for (const double part : {1.0, 0.9, 0.7, 0.5}) {
-    double R = far, rest = 0.0;
-    int near = n;
+    double d2 = far;
     if (part < 1.0) {
-      auto k = by.begin() + ((size_t)ceil(part * n) - 1);
-      std::nth_element(by.begin(), k, by.end());
-      R = *k;
-      for (int i = near = 0; i < n; ++i) {
-        if (d[i] <= R) ++near;
-        else rest += cost[i];
-      }
+      const size_t k = (size_t)ceil(part * (by.empty() ? sample.size() : n)) - 1;
+      if (!by.empty()) std::nth_element(by.begin(), by.begin() + k, by.end());
+      d2 = by.empty() ? near_cost[k].first : by[k];
     }
-    const double other = lattice(n - near, rest) + 1e10;
-    const double t = bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, R, near, (double)src, best - other) + other;
+    double rest = 0.0;
+    int m = 0;  // sampled points beyond
+    for (const auto &p : near_cost)
+      if (p.first > d2) {
+        rest += p.second;
+        ++m;
+      }
+    const double others = floor((1.0 - part) * n);
+    const double other = (others > 0.0 ? lattice(others, m ? rest / m : sum / sample.size()) : 0.0) + 1e10;
+    const double t = bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, sqrt(d2), n - others, (double)src, best - other) + other;
     if (t < best) {
       best = t;
-      Rx = R;
+      R2 = d2;
     }
   }
-  if (!(Rx > 0.0)) return 0;
+  if (!(R2 > 0.0)) return 0;
   int near = 0;
-  for (int i = 0; i < n; ++i) near += d[i] <= Rx;
-  if (bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, Rx, near, (double)src, 1e300) >= 1e300) return 0;
+  for (int i = 0; i < n; ++i) near += dist2(i) <= R2;
+  if (bem_smooth_plan_field(&c->fsm, &c->sm, &c->qp, sqrt(R2), near, (double)src, 1e300) >= 1e300) return 0;
   std::vector<double> h(bem_smooth_layout(&c->fsm).total);
   bem_smooth_tables(&c->fsm, &c->qp, h.data());
   if (falloc(c, &c->fsm_tab, h.size()) != cudaSuccess ||
@@ -1522,7 +1564,7 @@ static int field_split(bemgpu_ctx *c, int n, const double *r, long long src, int
   if (near < n) {
     order.resize(n);
     int a = 0, b = near;
-    for (int i = 0; i < n; ++i) order[d[i] <= Rx ? a++ : b++] = i;
+    for (int i = 0; i < n; ++i) order[dist2(i) <= R2 ? a++ : b++] = i;
   }
   return near;
 }
@@ -1551,15 +1593,16 @@ extern "C" int bemgpu_field(bemgpu_ctx *c, int d, int type, int n, const double 
   }
   CK(cudaMemcpyAsync(c->pt_in, rp, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, c->stream), "field points");
   bem_qp q = c->qp;
+  int spec = 0;
   if (near && (bem_launch_smfield(&c->fsm, &D, &q, grad, type, near, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
                                   c->pt_out, c->pt_t, c->status, c->stream) ||
                bem_launch_field(&D, &q, 1, grad, c->k0[d], type, near, c->pt_in, c->P[d], c->dP[d], c->pv[d], c->dpv[d],
-                                c->pt_out, c->status, c->pt_t, c->stream)))
+                                c->pt_out, c->status, c->pt_t, 1, c->stream)))
     return fail(c, "field", cudaGetLastError());
   if (near < n) {
-    if (d == 0 && field_tables(c, n - near, rp + 3 * (size_t)near, src, &q)) return -1;
+    if (d == 0 && field_tables(c, n - near, rp + 3 * (size_t)near, src, grad, &q, &spec)) return -1;
     if (bem_launch_field(&D, &q, d == 0, grad, c->k0[d], type, n - near, c->pt_in + 3 * (size_t)near, c->P[d], c->dP[d],
-                         c->pv[d], c->dpv[d], c->pt_out + 18 * (size_t)near, c->status, nullptr, c->stream))
+                         c->pv[d], c->dpv[d], c->pt_out + 18 * (size_t)near, c->status, nullptr, spec, c->stream))
       return fail(c, "field", cudaGetLastError());
   }
   double *op = order.empty() ? out : os.data();

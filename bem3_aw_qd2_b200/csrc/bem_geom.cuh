@@ -72,7 +72,7 @@ __device__ __forceinline__ void bem_rw_ref(const bem_el &el, double z, double e,
   for (int d = 0; d < 3; ++d) {
     r[d] = __dadd_rn(__dadd_rn(__dadd_rn(el.cr[d][0], __dmul_rn(el.cr[d][1], z)), __dmul_rn(el.cr[d][2], e)),
                      __dmul_rn(__dmul_rn(el.cr[d][3], z), e));
-    w[d] = el.cw[d][0] + el.cw[d][1] * z + el.cw[d][2] * e;
+    w[d] = __fma_rn(el.cw[d][2], e, __fma_rn(el.cw[d][1], z, el.cw[d][0]));
   }
 }
 

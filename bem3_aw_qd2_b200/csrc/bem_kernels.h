@@ -53,10 +53,11 @@ int bem_launch_wtab(double k, double ve, double *out, cudaStream_t st);
 // out: st_n1cnt x st_n2cnt x st_nint x BEM_ST_DEG (P, M) pairs)
 int bem_launch_stab(const bem_qp *q, double *out, cudaStream_t st);
 int bem_launch_qpgf(const bem_qp *q, const double *r, int n, double *G, double *dG, int *ret, cudaStream_t st);
+// spec: the second-derivative sums of the periodic domain take q's spectral order table;
 // only: null, or a flag per point (0: left out)
 int bem_launch_field(const bem_dom_dev *D, const bem_qp *q, int periodic, int grad, double k, int type, int npts,
                      const double *pts, const double *P, const double *dP, const double *pv, const double *dpv,
-                     double *out, unsigned *status, const int *only, cudaStream_t st);
+                     double *out, unsigned *status, const int *only, int spec, cudaStream_t st);
 int bem_launch_bdval(const bem_dom_dev *D, const bem_qp *q, int periodic, double k, int type, int ntgt, const int *tgt_t,
                      const double *tgt_ze,
                      const double *P, const double *dP, const double *pv, const double *dpv, double *out,

@@ -50,19 +50,18 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm /* NV*(FIE
 // first-derivative one (q0_coef_rt, d3hm_qpgf_d2_v1), as phi_s_aqd2 and
 // pv_s_bieq_aqd2 form them: the two lattice sums stop differently next to
 // the lattice plane, so each caller gets the one the reference uses.
+// spec: second-derivative sums with q's spectral order table, 1500 points around 216 quads
+// (9-point rule) 15.0 -> 10.9 ms, at 47 % of the FP64 pipe with three blocks an SM
+// (registers); where it does not serve, the direct forms' own code takes 5 to 8 % less
+// than asking the table first.  One choice for a launch: blocks of both kinds side by
+// side were 10 % slower than either.
 __global__ void __launch_bounds__(FIELD_THREADS) k_field(bem_dom_dev D, const __grid_constant__ bem_qp q, int periodic, int grad, double k, int type,
                                                          const double *__restrict__ pts, const double *__restrict__ P,
                                                          const double *__restrict__ dP, const double *__restrict__ pv,
                                                          const double *__restrict__ dpv, double *__restrict__ out,
                                                          unsigned *status,
-                                                         const int *__restrict__ only) {
+                                                         const int *__restrict__ only, int spec) {
   if (only && !only[blockIdx.x]) return;
-  // the real-space table in shared memory and spectral orders from a table that
-  // reaches the points (bemgpu_field): 1500 points of 216 quads on the 9-point rule
-  // 15.0 -> 10.9 ms, at 47 % of the FP64 pipe with three blocks an SM (registers)
-  extern __shared__ double2 wts_s[];
-  const double2 *wts = periodic && grad ? bem_wtab_stage(q, wts_s) : nullptr;
-  __syncthreads();
   const int ip = blockIdx.x;
   const double rt[3] = {pts[3 * ip], pts[3 * ip + 1], pts[3 * ip + 2]};
   const int nr = D.has_tri ? max(rule_points(type), tri_rule_points(type)) : rule_points(type);
@@ -106,7 +105,7 @@ __global__ void __launch_bounds__(FIELD_THREADS) k_field(bem_dom_dev D, const __
       for (int j = 0; j < 3; ++j) dG[j] = dH[j] = cmk(0.0, 0.0);
     } else if (periodic) {
       bem_gval2 gv;
-      const int rc = bem_qpgf2(q, vR[0], vR[1], vR[2], gv, wts);
+      const int rc = bem_qpgf2(q, vR[0], vR[1], vR[2], spec, gv);
       if (rc < 0) st |= (rc == -12 || rc == -23) ? BEM_ST_RAYLEIGH : BEM_ST_QPGF_LIMIT;
       G = cscale(gv.g, aW);
       H = cadd(cadd(cscale(gv.d[0], vW[0]), cscale(gv.d[1], vW[1])), cscale(gv.d[2], vW[2]));
@@ -143,9 +142,7 @@ __global__ void __launch_bounds__(FIELD_THREADS) k_field(bem_dom_dev D, const __
       a[12 + 2 * j] += w * t2.re;
       a[13 + 2 * j] += w * t2.im;
     }
-    const double i3 = iR * iR * iR;
-    a[8] += sg * w * rdW * iR * iR;
-    for (int j = 0; j < 3; ++j) a[9 + j] += sg * w * i3 * (3.0 * vR[j] * iR * rdW - vW[j]);
+    fld_geom(vR, vW, sg * w, a + 8);
   }
   set_status(status, st);
   __shared__ double sm[18 * (FIELD_THREADS / 32) + 18];
@@ -347,10 +344,10 @@ __global__ void k_force_bd(bem_dom_dev D, int ntgt, const int *__restrict__ tgt_
 
 extern "C" int bem_launch_field(const bem_dom_dev *D, const bem_qp *q, int periodic, int grad, double k, int type,
                                 int npts, const double *pts, const double *P, const double *dP, const double *pv,
-                                const double *dpv, double *out, unsigned *status, const int *only, cudaStream_t st) {
+                                const double *dpv, double *out, unsigned *status, const int *only,
+                                int spec, cudaStream_t st) {
   if (npts <= 0) return 0;
-  const int smem = periodic && grad && q->wt ? BEM_WT_SMEM : 0;
-  k_field<<<npts, FIELD_THREADS, smem, st>>>(*D, *q, periodic, grad, k, type, pts, P, dP, pv, dpv, out, status, only);
+  k_field<<<npts, FIELD_THREADS, 0, st>>>(*D, *q, periodic, grad, k, type, pts, P, dP, pv, dpv, out, status, only, spec);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -656,8 +656,9 @@ struct bem_gval2 { cplx g, d[3], d2[6]; };
 
 __device__ __forceinline__ cplx cmuli(cplx a) { return cmk(-a.im, a.re); }  // i a
 
-static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o,
-                                      const double2 *wts) {
+// SPEC: spectral terms from q's order table where it reaches (without: the direct forms alone)
+template <bool SPEC>
+static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &o) {
   const double ve = bem_ewald_eta(q, rx, ry, rz);
   const double ke = q.k * ve, ke2 = ke * ke, ive = 1.0 / ve;
   const bool tab = q.wt != nullptr && ve == q.eta_run;
@@ -690,7 +691,7 @@ static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, dou
           // A = ef Re w and the first-derivative factor from the table when it applies
           double A, B1;
           if (tab) {
-            const double2 ab = bem_wtab(q, ve, ke, rl2e, wts);
+            const double2 ab = bem_wtab(q, ve, ke, rl2e);
             A = ab.x;
             B1 = 2.0 * ve * irl * irl * irl * ab.y;
           } else {
@@ -736,7 +737,7 @@ static __device__ int bem_qpgf2_ewald(const bem_qp &q, double rx, double ry, dou
   cplx t = cmk(0, 0), td[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)}, t2[6];
   for (int c = 0; c < 6; ++c) t2[c] = cmk(0, 0);
   const double azve = rz / (2.0 * ve), c2pi = 2.0 * isp * ive;
-  const bool stab = ew_spec_tab_ok(q, ve, rz);
+  const bool stab = SPEC && ew_spec_tab_ok(q, ve, rz);
   for (int dir = 0; dir < 3; ++dir) {
     int n1 = q.nc1 + (dir == 2 ? -1 : (dir == 1 ? 1 : 0));
     const int step = dir == 2 ? -1 : 1;
@@ -905,9 +906,8 @@ static __device__ int bem_qpgf2_spectral(const bem_qp &q, double rx, double ry, 
   return cc;
 }
 
-// wts: the kernel's shared-memory copy of the real-space table, or null
-static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, bem_gval2 &out,
-                                const double2 *wts = nullptr) {
+// spec: spectral terms from q's order table where it reaches (for a whole launch)
+static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz, int spec, bem_gval2 &out) {
   bool spectral = false;
   if (!q.ewald_only) {
     const double az = fabs(rz);
@@ -918,7 +918,9 @@ static __device__ int bem_qpgf2(const bem_qp &q, double rx, double ry, double rz
   const int l2 = (int)floor(-(rx * q.d1y - ry * q.d1x) * q.idet + 0.5);
   const double hx = bem_sub2(rx, l1, q.d1x, l2, q.d2x);
   const double hy = bem_sub2(ry, l1, q.d1y, l2, q.d2y);
-  const int e = spectral ? bem_qpgf2_spectral(q, hx, hy, rz, out) : bem_qpgf2_ewald(q, hx, hy, rz, out, wts);
+  const int e = spectral ? bem_qpgf2_spectral(q, hx, hy, rz, out)
+                : spec   ? bem_qpgf2_ewald<true>(q, hx, hy, rz, out)
+                         : bem_qpgf2_ewald<false>(q, hx, hy, rz, out);
   if (e > 0 && (l1 != 0 || l2 != 0)) {
     const cplx cf = cexpi(-(q.kx * (l1 * q.d1x + l2 * q.d2x) + q.ky * (l1 * q.d1y + l2 * q.d2y)));
     out.g = cmul(out.g, cf);

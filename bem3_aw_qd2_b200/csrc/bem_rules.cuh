@@ -97,6 +97,21 @@ __device__ __forceinline__ void bd_source_point(const bem_dom_dev &D, int se, bo
   }
 }
 
+// The geometric sum F of a field point and its gradient, times 4 pi: sw (sign and weight)
+// times (R . W) / R^3 to a[0], its gradient to a[1 .. 3].  Over a closed body the sum
+// cancels to 1e-8 of its terms, so every kernel that forms it rounds alike: each
+// operation is spelled out.
+__device__ __forceinline__ void fld_geom(const double R[3], const double W[3], double sw, double *a) {
+  const double r2 = __fma_rn(R[2], R[2], __fma_rn(R[1], R[1], __dmul_rn(R[0], R[0])));
+  const double iR = __ddiv_rn(1.0, __dsqrt_rn(r2));
+  const double rdW = __dmul_rn(__fma_rn(R[2], W[2], __fma_rn(R[1], W[1], __dmul_rn(R[0], W[0]))), iR);
+  a[0] = __fma_rn(__dmul_rn(__dmul_rn(sw, rdW), iR), iR, a[0]);
+  const double s3 = __dmul_rn(sw, __dmul_rn(__dmul_rn(iR, iR), iR));
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    a[1 + j] = __fma_rn(s3, __fma_rn(__dmul_rn(__dmul_rn(3.0, R[j]), iR), rdW, -W[j]), a[1 + j]);
+}
+
 // ------------------------------------------------------------------ polar rule
 struct polar_pt { double th, wth; int j; };
 __device__ __forceinline__ polar_pt polar_theta(const double th[5], int idx /* 0..511 */) {

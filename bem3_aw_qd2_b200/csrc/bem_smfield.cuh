@@ -40,8 +40,7 @@ __global__ void __launch_bounds__(SMF_TH) k_sm_field(const __grid_constant__ sm_
     for (int d = 0; d < 3; ++d) vR[d] = __dsub_rn(vR[d], rt[d]);
     met |= fabs(vR[2]) < BEM_FAR_PLANE_TOL;
     // images: value, gradient, second derivatives along W
-    // (products of their own: those of the geometric sums below stay fused, as k_field's)
-    const double rz2 = __dmul_rn(vR[2], vR[2]), zw = __dmul_rn(vR[2], vW[2]);
+    const double rz2 = vR[2] * vR[2], zw = vR[2] * vW[2];
     double g[2] = {0, 0}, f[6] = {0, 0, 0, 0, 0, 0}, fs[2] = {0, 0}, h[6] = {0, 0, 0, 0, 0, 0};
     for (int m = 0; m < S.nimg; ++m) {
       const double px = vR[0] + im[3 * m], py = vR[1] + im[3 * m + 1];
@@ -95,9 +94,7 @@ __global__ void __launch_bounds__(SMF_TH) k_sm_field(const __grid_constant__ sm_
         a[3 + 2 * j] += t1.im;
       }
     }
-    const double sg = D.sid[s] < 0 ? -1.0 : 1.0, iR = 1.0 / sqrt(dot3(vR, vR)), i3 = iR * iR * iR, rdW = dot3(vR, vW) * iR;
-    a[8] += sg * w * rdW * iR * iR;
-    for (int j = 0; j < 3; ++j) a[9 + j] += sg * w * i3 * (3.0 * vR[j] * iR * rdW - vW[j]);
+    fld_geom(vR, vW, D.sid[s] < 0 ? -w : w, a + 8);
   }
   met = __syncthreads_or(met);
   if (tid == 0) again[ip] = met;
