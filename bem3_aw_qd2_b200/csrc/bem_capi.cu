@@ -408,15 +408,13 @@ static int smooth_setup(bemgpu_ctx *c, int inst, const bem_qp *qps) {
   std::vector<double> h(bem_smooth_layout(&c->sm).total);
   bem_smooth_tables(&c->sm, qps, h.data());
   // one allocation: tables, what is kept, and the workspace where it is not in A
-  const size_t tab = (h.size() + 31) / 32 * 32, keep = (bem_smooth_keep_doubles(&c->sm) + 31) / 32 * 32;
-  const size_t need = bem_smooth_ws_doubles(&c->sm, c->dom_ne[0]);
-  const bool in_A = inst == 1 && need <= 2 * (size_t)c->n * c->n;
-  CK(falloc(c, &c->sm_buf, tab + keep + (in_A ? 0 : need)), "expansion");
+  const bem_smooth_room room = bem_smooth_need(&c->sm, c->dom_ne[0], 2 * (size_t)c->n * c->n);
+  CK(falloc(c, &c->sm_buf, room.tab + room.keep + room.ws), "expansion");
   CK(cudaMemcpyAsync(c->sm_buf, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream), "expansion tables");
   c->sm.tab = c->sm_buf;
-  c->sm.keep = c->sm_buf + tab;
+  c->sm.keep = c->sm_buf + room.tab;
   c->sm.have0 = c->sm.have1 = 0;
-  c->sm.ws = in_A ? c->A : c->sm_buf + tab + keep;
+  c->sm.ws = room.ws ? c->sm_buf + room.tab + room.keep : c->A;
   return 0;
 }
 

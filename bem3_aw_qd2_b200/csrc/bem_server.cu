@@ -32,6 +32,8 @@
 #include <thread>
 #include <vector>
 #include "../../include/bemgpu.h"
+#include "bem_lattice.h"
+#include "bem_smooth.h"
 
 #define BACKFILL_MS 2000.0
 
@@ -75,7 +77,8 @@ struct owned_problem {
 // device bytes a resident problem holds: global matrix n^2 16 B, per domain
 // G, H, dpv factors 3 N_d^2 16 B (+ dG, dH 4 N_d^2 16 B for interior domains
 // when they are kept, else one 512 MiB block of recomputed rows), FP32 factors
-// in mixed precision, and element tables / scratch
+// in mixed precision, the split of the periodic domain (up to 60 MB at the highest
+// degrees), and element tables / scratch
 size_t problem_bytes(const bemgpu_problem *p, int precision, bool keep_dgh) {
   const size_t n = 2 * (size_t)p->NN;
   size_t b = n * n * 16, f32 = n * n * 8;
@@ -88,6 +91,12 @@ size_t problem_bytes(const bemgpu_problem *p, int precision, bool keep_dgh) {
   }
   if (precision) b += f32;
   if (!keep_dgh && p->MN >= 1) b += (size_t)512 << 20;
+  bem_qp q;
+  bem_qp_prepare(p->qp, &q);
+  bem_smooth S;
+  bem_smooth_plan(&S, &q, p->cr, p->npe, p->sid, p->dom_ne[0]);
+  const bem_smooth_room room = bem_smooth_need(&S, p->dom_ne[0], 2 * n * n);
+  b += (room.tab + room.keep + room.ws) * sizeof(double);
   return b + (size_t)p->Ne * 512 + (64u << 20);  // tables, workspace of the solvers
 }
 

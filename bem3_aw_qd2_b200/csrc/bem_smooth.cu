@@ -429,6 +429,12 @@ static sm_ws ws_layout(const bem_smooth *S, int ne) {
 }
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne) { return ws_layout(S, ne).total; }
 
+bem_smooth_room bem_smooth_need(const bem_smooth *S, int ne, size_t lent) {
+  if (!S->on) return {0, 0, 0};
+  const size_t tab = bem_smooth_layout(S).total, ws = bem_smooth_ws_doubles(S, ne);
+  return {(tab + 31) / 32 * 32, (bem_smooth_keep_doubles(S) + 31) / 32 * 32, S->inst == 1 && ws <= lent ? 0 : ws};
+}
+
 struct sm_qps { bem_qp q[BEM_SM_BAT]; };
 struct sm_out { double *G[BEM_SM_BAT], *H[BEM_SM_BAT]; };
 

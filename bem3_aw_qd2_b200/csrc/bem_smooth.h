@@ -47,6 +47,11 @@ double bem_smooth_plan_field(bem_smooth *F, const bem_smooth *S, const bem_qp *q
                              double limit);
 size_t bem_smooth_keep_doubles(const bem_smooth *S);
 size_t bem_smooth_ws_doubles(const bem_smooth *S, int ne);
+// what a problem of ne elements allocates for its split (0 where it is off), doubles: the
+// tables, what is kept, and the scratch of several instances or of one that is larger
+// than the lent doubles (the global matrix, which holds nothing during an assembly)
+struct bem_smooth_room { size_t tab, keep, ws; };
+bem_smooth_room bem_smooth_need(const bem_smooth *S, int ne, size_t lent);
 
 extern "C" {
 // constant tables of this translation unit (quad: bem_quad, wc: bem_wconst) and its
