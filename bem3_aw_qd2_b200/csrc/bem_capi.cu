@@ -664,13 +664,19 @@ extern "C" int bemgpu_set_ewald_scale(bemgpu_ctx *c, double scale) {
 
 static bem_dom_dev dom_view(bemgpu_ctx *c, int d);
 
-// Ewald-parameter autotuner: time the periodic regular-pair kernel on a
+// Ewald-parameter autotuner: time the periodic regular-pair kernels on a
 // sample of the pairs for the rule's scale and three neighbours (larger
 // factors meet the per-point cap and lose the tabulated terms) and keep the
-// fastest.
+// fastest.  Where the assembly takes images and expansion those kernels run for
+// the pairs on a lattice plane alone: there is nothing to time, the rule's scale stays.
 extern "C" int bemgpu_autotune(bemgpu_ctx *c, double *best_scale) {
   if (!c->bat.empty()) { snprintf(c->err, sizeof(c->err), "a batch is loaded (load a single problem first)"); return -2; }
   if (!c->loaded) { snprintf(c->err, sizeof(c->err), "no problem loaded"); return -2; }
+  if (c->sm.on) {
+    const double rule = ewald_rule_scale(c->qp);
+    if (best_scale) *best_scale = rule;
+    return bemgpu_set_ewald_scale(c, rule);
+  }
   bem_dom_dev D = dom_view(c, 0);
   if (bem_launch_classify(&D, &c->qp, 1, c->k0[0], &c->scr, c->stream)) return fail(c, "autotune", cudaGetLastError());
   double *tab = nullptr, *stab = nullptr;

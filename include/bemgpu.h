@@ -115,9 +115,11 @@ int bemgpu_set_far_rule(bemgpu_ctx *ctx, int on);
 int bemgpu_rule_pairs(bemgpu_ctx *ctx, unsigned long long counts[6]);
 
 /* Autotuner of the Ewald parameter for the loaded problem: times the periodic
- * regular-pair kernel on an eighth of the pairs for the rule's scale and three
+ * regular-pair kernels on an eighth of the pairs for the rule's scale and three
  * neighbours and sets the fastest (bemgpu_set_ewald_scale); *best_scale gets it.
- * Costs about half of one regular-pair launch. */
+ * Costs about half of one regular-pair launch.  A problem whose assembly takes lattice
+ * images and an expansion has no such launch to tune (the parameter is left to pairs
+ * on a lattice plane and the point evaluators): the rule's scale is set, nothing timed. */
 int bemgpu_autotune(bemgpu_ctx *ctx, double *best_scale);
 
 /* Batches of Bloch vectors (form 2; no counterpart in the reference, which
