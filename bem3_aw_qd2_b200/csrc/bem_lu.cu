@@ -136,15 +136,14 @@ __device__ __forceinline__ unsigned pivot_key(float a, int t) {
 // would keep the compiler from scheduling it beside the updates): a scaled by a
 // power of two to |re| + |im| in [1, 2), so that re^2 + im^2 neither over- nor
 // underflows, and 1 / (re^2 + im^2) from the hardware's approximation by one
-// third-order Newton step r (1 + e + e^2), e = 1 - d r.  Of zero it is zero (d kept off
-// zero, the least of a subnormal number's is above the bound; the scale last, whose
-// product with r alone would overflow): a column without a non-zero entry among a
-// slice's rows then leaves them as they are, and the columns after it still choose
-// among them.
+// third-order Newton step r (1 + e + e^2), e = 1 - d r.  Of zero it is zero (a summand
+// far below the least d keeps r finite; the scale comes last, whose product with r alone
+// would overflow): a column without a non-zero entry among a slice's rows then leaves
+// them as they are, and the columns after it still choose among them.
 __device__ __forceinline__ double2 pivot_rcp(double2 a) {
   const int e = (__double2hiint(cabs1(a)) >> 20) & 2047;
   const double sc = __hiloint2double(max(2046 - e, 1) << 20, 0);
-  const double x = a.x * sc, y = a.y * sc, d = fmax(fma(x, x, y * y), 0x1p-110);
+  const double x = a.x * sc, y = a.y * sc, d = fma(x, x, fma(y, y, 0x1p-200));
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
   const double q = fma(-d, r, 1.0);
@@ -154,7 +153,7 @@ __device__ __forceinline__ double2 pivot_rcp(double2 a) {
 __device__ __forceinline__ float2 pivot_rcp(float2 a) {
   const int e = (__float_as_int(cabs1(a)) >> 23) & 255;
   const float sc = __int_as_float(max(254 - e, 1) << 23);
-  const float x = a.x * sc, y = a.y * sc, d = fmaxf(fmaf(x, x, y * y), 0x1p-50f);
+  const float x = a.x * sc, y = a.y * sc, d = fmaf(x, x, fmaf(y, y, 0x1p-100f));
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   r = fmaf(r, fmaf(-d, r, 1.0f), r);
