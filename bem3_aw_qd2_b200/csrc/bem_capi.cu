@@ -1430,9 +1430,8 @@ static std::vector<int> sample_points(int n) {
 // plane waves alone do not do, and the point keeps the distance from the body's ball
 // below which the Ewald parameter is capped (bem_ewald_eta: a warp would run both forms).
 // A build takes 50 to 90 us and saves a quarter or more of the sums of the points that
-// it serves and the own table does not: 30 points of 96 flat quads, period 1, 9-point
-// rule, 1.03 -> 0.82 ms (7 strides of 128 sources; 3 are worth it), 3000 of them 11.1 ->
-// 6.6.  Within one wave of blocks the slowest point decides, so that second derivatives
+// it serves and the own table does not: 30 points of 96 flat quads, 9-point rule, 1.04 ->
+// 0.85 ms at period 1, 1.85 -> 1.31 at 1.6 (7 strides of 128 sources; 3 are worth it).  Within one wave of blocks the slowest point decides, so that second derivatives
 // (whose direct forms are code of their own) ask for every point to be served, beyond
 // it for half.
 static int field_tables(bemgpu_ctx *c, int n, const double *r, long long sources, int grad, bem_qp *q, int *spec) {

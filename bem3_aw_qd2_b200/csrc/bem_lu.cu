@@ -23,13 +23,17 @@
 //               64 x 64 complex tiles, the complex product as four real ones.
 //
 // A small factorisation's sequence is captured once as a CUDA graph and replayed,
-// a large one runs on two streams of its own (factor_blocks).  Solves: forward substitution L y = P b and back substitution
-// U x = y in one launch each, one CTA per 32-row block; blocks are written in
-// dependency order and a block folds in each block it needs as soon as a
-// progress counter in global memory has passed it (bounded waits: a wait that
-// gives up sets BEM_LU_ST_WAIT and the call reports it; nothing hangs).  The
-// launches are cooperative, so every CTA is resident and blocks are taken in
-// order: the waits cannot deadlock.
+// a large one runs on two streams of its own (factor_blocks).
+//
+// Solves: forward substitution L y = P b and back substitution U x = y in one launch
+// each, one CTA per 32-row block, its diagonal block applied as an inverse formed ahead.
+// The values are their own flags: the output is filled with all-ones words before the
+// launch, a block polls the values that it needs and takes each 8-byte component
+// (4 in FP32) once it is no longer that pattern (a 16-byte access is not one atomic), and
+// a value that comes out as the pattern, a NaN handed in, is stored as another NaN.
+// Waits are bounded: one that gives up sets BEM_LU_ST_WAIT and the call reports it;
+// nothing hangs.  The launches are cooperative, so every CTA is resident and blocks are
+// taken in order: the waits cannot deadlock.
 #include "bem_count.h"
 #include <cuda_runtime.h>
 #include <stdint.h>

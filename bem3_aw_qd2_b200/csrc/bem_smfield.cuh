@@ -4,7 +4,7 @@
 // operations a pair; here a pair is 10 to 40 images of 160 (e^{ikR} / R, its
 // gradient and its second derivatives along W), and the rest of all sources is one
 // sum of K regular waves a point.  1500 points of 216 quads on the 9-point rule: 11.0
-// ms with the tabled lattice sums of k_field, 1.75 ms like this, of which the sums
+// ms with the tabled lattice sums of k_field, 1.54 ms like this, of which the sums
 // take 1.02 (images, 40 % of the FP64 pipe's peak).  A
 // point with a source on its lattice plane is left to k_field.
 #pragma once

@@ -276,7 +276,6 @@ static void finish_plan(bem_smooth *S, const bem_qp *q) {
   S->s1 = (int)(cuts * hypot(q->d1x, q->d1y) / tp) + 2;
   S->s2 = (int)(cuts * hypot(q->d2x, q->d2y) / tp) + 2;
   // a batch's instances share the window: centred on n2 = 0, wide enough for |k_par| <= k
-  S->sc2 = 0;
   S->s2 += (int)(S->k * hypot(q->d2x, q->d2y) / tp) + 1;
   if ((double)(2 * S->r1 + 1) * (2 * S->r2 + 1) > 20000.0 || (double)(2 * S->s1 + 1) * (2 * S->s2 + 1) > 20000.0) {
     S->on = 0;
@@ -383,7 +382,7 @@ struct sm_dev {
   int lmax, Lmax, Mx, K, Kp, nt, nphi, nimg, nlm;  // nlm: pairs (l, m >= 0) up to Lmax
   double cx, cy, cz, R0, iR0, kR0, rho, k, cut;
   double eta;                       // Ewald parameter of the samples
-  int nreal, r1, r2, nspec, s1, s2, sc2;  // its windows: l1 in [-r1, r1], l2 in [-r2, r2]; n1 - nc1 in [-s1, s1], ...
+  int nreal, r1, r2, nspec, s1, s2;  // its windows: l1 in [-r1, r1], l2 in [-r2, r2]; n1 - nc1 in [-s1, s1], n2 in [-s2, s2]
   int iml[2 * BEM_SM_MAXIMG];       // the images' indices
   int lcut[8];                      // degrees of the expansion about a point at |R| <= (i + 1) 2 R0 / 8
   const double *x, *w, *ca, *cb, *dL, *el, *rec, *img;
@@ -514,7 +513,7 @@ __global__ void __launch_bounds__(SMP_TH) k_sm_sample(const __grid_constant__ sm
     const double c2 = 0.25 * q.aidet, dz = Z / (2.0 * ve);
     bool ray = false;
     for (int e = lane; e < S.nspec; e += 32) {
-      const int n1 = q.nc1 + e / (2 * S.s2 + 1) - S.s1, n2 = S.sc2 + e % (2 * S.s2 + 1) - S.s2;
+      const int n1 = q.nc1 + e / (2 * S.s2 + 1) - S.s1, n2 = e % (2 * S.s2 + 1) - S.s2;
       const double ax = bem_an(-q.kx, n1, q.g1x, n2, q.g2x), ay = bem_an(-q.ky, n1, q.g1y, n2, q.g2y);
       const double bn2 = __dadd_rn(__dadd_rn(__dmul_rn(q.k, q.k), -__dmul_rn(ax, ax)), -__dmul_rn(ay, ay));
       if (bn2 * ve * ve < -42.0) continue;
@@ -1203,7 +1202,7 @@ static sm_dev dev_view(const bem_smooth *S, int ne, int b0, bool held = false) {
   d.lmax = S->lmax; d.Lmax = S->Lmax; d.K = S->K; d.Kp = S->Kp; d.nt = S->nt; d.nphi = S->nphi; d.nimg = S->nimg;
   d.eta = S->eta;
   d.r1 = S->r1; d.r2 = S->r2; d.nreal = (2 * S->r1 + 1) * (2 * S->r2 + 1);
-  d.s1 = S->s1; d.s2 = S->s2; d.sc2 = S->sc2; d.nspec = (2 * S->s1 + 1) * (2 * S->s2 + 1);
+  d.s1 = S->s1; d.s2 = S->s2; d.nspec = (2 * S->s1 + 1) * (2 * S->s2 + 1);
   for (int i = 0; i < S->nimg; ++i) { d.iml[2 * i] = S->l1[i]; d.iml[2 * i + 1] = S->l2[i]; }
   d.nlm = (S->Lmax + 1) * (S->Lmax + 2) / 2;
   d.cx = S->ctr[0]; d.cy = S->ctr[1]; d.cz = S->ctr[2];
@@ -1281,7 +1280,15 @@ extern "C" int bem_launch_smooth(bem_smooth *S, const bem_dom_dev *D, const bem_
         d.U, 0, S->Kp, d.T, sT, 2 * S->Kp, N, 2 * S->Kp, S->Kp, d.A, sA, 2 * S->Kp, O);
     k_sm_gemm<true><<<dim3((8 * ne + GM_BN - 1) / GM_BN, (2 * N + GM_BM - 1) / GM_BM, n), GM_TH, GM_SMEM, st>>>(
         d.A, sA, S->Kp, d.V, 0, 8 * ne, 2 * N, 8 * ne, S->Kp, nullptr, 0, 0, O);
-    // lanes per pair: enough threads for several waves of the GPU's 75,000 resident ones
+    // Lanes per pair: 32 where a thread a pair leaves most of the GPU's 75,000 resident
+    // threads idle, then 4, 1 where pairs alone are many waves and a lane's share of a
+    // short rule gets small.  Measured, us with 32 / 4 / 1 lanes (square lattice, period
+    // 0.8): 24 quads (2304 pairs) 37 / 117 / 440, 80 triangles (25,600) 192 / 451 / 1123, 96
+    // quads (36,864) 213 / 192 / 371, 216 (186,624) 958 / 672 / 799, 600 (1.44e6) 7117 / 3711 /
+    // 3824, 726 (2.1e6) 8152 / 3849 / 3884, 1014 (4.1e6) 16178 / 7212 / 7038, 1536 (9.4e6) 36612
+    // / 15878 / 15099.  The lines lie where quads and triangles together lose least below
+    // (32 to 4) and where 4 and 1 are within 3 % of each other on quads; 1280 triangles
+    // (6.6e6) would take 9441 with 4 for 10902.
     const long long work = npairs * n;
     if (work >= 1500000) launch_images<1>(d, D, n, scr->flag, O, st);
     else if (work >= 60000) launch_images<4>(d, D, n, scr->flag, O, st);

@@ -17,7 +17,7 @@ struct bem_smooth {
   double ctr[3] = {0, 0, 0}, R0 = 0.0, rho = 0.0, k = 0.0;
   double cut = 0.0;             // least distance of an image left in from an element, seen from a node
   double eta = 0.0;             // Ewald parameter and windows of the samples
-  int r1 = 0, r2 = 0, s1 = 0, s2 = 0, sc2 = 0;
+  int r1 = 0, r2 = 0, s1 = 0, s2 = 0;
   int l1[BEM_SM_MAXIMG], l2[BEM_SM_MAXIMG];  // the images' lattice indices, (0, 0) first
   int np = 0;                   // the nearest lattice points, by distance (as many as a split
   double pr[BEM_SM_MAXIMG + 1]; // can look at: its images and the first shell left in)
